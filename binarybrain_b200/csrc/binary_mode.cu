@@ -218,157 +218,357 @@ k_bit_gather_forward(const uint32_t *__restrict__ x, float *__restrict__ y, cons
 
 // --------------------------------------------------------------------------------------------- backward of bit-input layers
 // With bit inputs the backward pass also factors through the pattern p of a frame:
-//   dx_j(f) = g(f) * D_j[p(f)]          D_j[p] = dy/du_j at pattern p, six values per pattern and node
+//   dx_j(f) = g(f) * D_j[p(f)]          D_j[p] = dy/du_j at pattern p; y is linear in u_j, so D_j does not depend on bit j of p
 //   dW      = K^T Hg                    Hg[p] = sum of g over the frames with pattern p; K[i][p] = prod_j k(bit_j(i), bit_j(p)),
 //                                        k = 0.5 + bias where the bits agree, 0.5 - bias where they differ (one butterfly per input)
 // and for the batch-norm form g(f) = mask[p] dy(f) gamma rstd + dmean + Y[p] dvar / F, so Hg and the two batch sums
 // (include/bb/DifferentiableLutN.h:1190-1258) follow from Hdy[p] = sum of dy per pattern and the pattern counts H[p].
-// Per frame that leaves: the pattern (bit inputs: a 32 x 32 bit transpose per row and 32 words, then four patterns at a time, one per
-// byte), 6 table reads, 6 multiplies and the 6 dx reductions.
-
-enum { kBwdPlainAll = 0, kBwdHistOnly = 1, kBwdNormDx = 2 };
+// Kernels: the sums per pattern and the pattern of every frame (k_pattern_sums); everything per node (k_bit_backward_finalize:
+// batch sums, dW, the look-up tables of the last pass); dx (k_pattern_gather).
+//
+// dx is gathered by input row, not scattered by node: reductions into L2 run at 6 TB/s on B200 whatever their width (measured, 512
+// bytes in 24 clocks per SM), so six of them per node-frame cost 0.54 ms for 8192 nodes x 16384 frames, while loads that hit L2 run
+// at 18 TB/s.  An input row therefore sums over its consumers (a list made once per launch), reading their dy and pattern
+// bytes, and is written once: no clear, no read-modify-write, 5 bytes per node-frame and consumer.
+//
+// In all of them lane l owns the frames 4l .. 4l+3 of every 128, so that dy is read and dx is written 16 bytes at a time.
 
 struct BitBwdArgs {
-    const uint32_t *x;                  // bit-packed rows, or (XF32 kernels) fp32 rows reinterpreted: an input is "set" where x > 0.5
-    uint32_t *hist;                     // XF32 only: [O][64] pattern counts (added to by the histogram pass)
-    unsigned char *pat;                 // XF32 with batch norm: [O][fs] pattern bytes, written by the histogram pass, read by the dx pass
+    const uint32_t *x;                  // bit-packed rows, or (k_pattern_sums<true>) fp32 rows reinterpreted: an input is "set" where x > 0.5
     const float *dy;
     float *dx;
     const int *idx;
-    const float *W;
-    float *hdy;                         // [O][64] per-pattern sums of dy (added to)
-    const float *mean, *rstd, *dmean, *dvar;
-    float gamma, beta, bias, rF;
-    int O, F, groups, tile_words, lut_binarize;
-    long long xs, fs;                   // word stride of x, float stride of dy / dx
+    float *hdy;                         // [O][64] sums of dy per pattern
+    uint32_t *hist;                     // [O][64] pattern counts
+    uint2 *mask;                        // [O] hard-tanh masks of the 64 patterns (batch norm only)
+    uint16_t *pat;                      // [O][ps] doubled patterns p | p << 6, bit 15: the mask passes
+    float *etab;                        // [6 O][64] look-up tables, see k_bit_backward_finalize
+    float2 *ntab;                       // [O] gamma rstd, dvar bias / F
+    const int *edge_end, *edge_count, *edges;      // consumers of every input row (8 node + input number)
+    int I, O, F, groups, tile_frames, tiles, split;
+    int vec;                            // dy and dx (and fp32 x) rows start on 16-byte boundaries
+    long long xs, fs, ps;               // word stride of x, float stride of dy / dx, stride of pat
 };
 
-// Four CTAs per SM (64 registers): the frame loop needs few registers and hides its load latency with warps; the table set-up at the
-// top, which would like ~130, runs once per tile and may spill.
-// XF32: the layer is in binary mode on fp32 frames (include/bb/DifferentiableLutN.h:779-786 maps x to 0.5 +- bias by x > 0.5), so the
-// pattern of a frame comes from six compares instead of six bits, and the histogram pass also counts the patterns.
-template <int MODE, bool XF32>
-__global__ void __launch_bounds__(kWarpsPerCta * 32, 4)
-k_bit_backward_frames(const BitBwdArgs a)
+// bits of four frames (4l .. 4l+3 of the chunk, words of the 32 frames they are in) -> four patterns, one per byte
+__device__ __forceinline__ uint32_t pattern_bytes(const uint32_t (&w)[6], int lane)
 {
-    __shared__ float4 s_tab[kWarpsPerCta][16];
-    __shared__ float s_D[kWarpsPerCta][6][64];
-    __shared__ float s_A[kWarpsPerCta][64], s_B[kWarpsPerCta][64], s_H[kWarpsPerCta][64];
-    __shared__ unsigned s_C[XF32 ? kWarpsPerCta : 1][64];
+    const int sh = 4 * (lane & 7);
+    uint32_t p4 = 0u;
+#pragma unroll
+    for (int j = 0; j < 6; ++j) p4 |= (((w[j] >> sh) & 0xfu) * (0x00204081u << j)) & (0x01010101u << j);
+    return p4;
+}
+
+// four consecutive floats of a row; frames from F on read as 0
+__device__ __forceinline__ float4 load_frames(const float *row, long long f, int F, int vec)
+{
+    if (vec && f + 3 < F) return __ldg(reinterpret_cast<const float4 *>(row + f));
+    return make_float4(f < F ? __ldg(row + f) : 0.0f, f + 1 < F ? __ldg(row + f + 1) : 0.0f, f + 2 < F ? __ldg(row + f + 2) : 0.0f,
+                       f + 3 < F ? __ldg(row + f + 3) : 0.0f);
+}
+
+// bits[i][w]: frames 32 w .. 32 w + 31 of row i, set where x > 0.5.  A warp packs 32 words (1024 frames); bound by reading x.
+__global__ void __launch_bounds__(kWarpsPerCta * 32)
+k_pack_bits(const float *__restrict__ x, uint32_t *__restrict__ bits, int I, int F, long long xs, long long ws, int runs)
+{
+    const int lane = threadIdx.x & 31;
+    const long long unit = (long long)blockIdx.x * kWarpsPerCta + (threadIdx.x >> 5);
+    const int row = (int)(unit / runs), run = (int)(unit - (long long)row * runs);
+    if (row >= I) return;
+    const float *src = x + (size_t)row * xs + run * 1024 + lane;
+    const int left = F - run * 1024 - lane;
+    uint32_t mine = 0u;
+#pragma unroll
+    for (int h = 0; h < 32; h += 16) {
+        float v[16];
+#pragma unroll
+        for (int k = 0; k < 16; ++k) v[k] = 32 * (h + k) < left ? __ldg(src + 32 * (h + k)) : 0.0f;
+#pragma unroll
+        for (int k = 0; k < 16; ++k) {
+            const uint32_t word = __ballot_sync(kFull, v[k] > 0.5f);
+            if (lane == h + k) mine = word;
+        }
+    }
+    if (run * 32 + lane < ws) bits[(size_t)row * ws + run * 32 + lane] = mine;
+}
+
+// Sums of dy per pattern, with BN the pattern counts, and the patterns as bytes.  Every lane keeps a histogram of its own in shared memory
+// -- column `lane` of [64 patterns][32 lanes], free of bank conflicts and of atomics -- and the columns are added up once per tile.
+// (Float atomics on one shared histogram per warp, compare-and-swap loops in hardware, took 0.68 ms for 8192 nodes x 16384 frames.)
+// Shared memory takes four clocks per warp and 32 frames (a 64-bit load and store per frame), about as long as reading dy takes; with
+// only 12 warps per SM (16 KiB of columns each) the loads have to be far ahead, so 512 frames of dy are in flight per warp.
+constexpr int kPsWarps = 4;
+template <bool BN> struct PatternSlot { float s; uint32_t n; };      // n: count, bit 31: the pattern's mask bit
+template <> struct PatternSlot<false> { float s; };
+
+// Adds four frames (patterns one per byte, frames from `live` on do not count) to a lane's column; returns their doubled patterns with the
+// mask bits, which come with the slots.
+template <bool BN>
+__device__ __forceinline__ uint2 pattern_columns_add(PatternSlot<BN> *mine, uint32_t p4, const float4 &g, int live)
+{
+    const float gv[4] = {g.x, g.y, g.z, g.w};
+    uint32_t q[2] = {__byte_perm(p4, 0u, 0x4140) * 65u, __byte_perm(p4, 0u, 0x4342) * 65u};
+#pragma unroll
+    for (int i = 0; i < 4; ++i) {
+        PatternSlot<BN> *slot = mine + 32 * __byte_perm(p4, 0u, 0x4440 + i);
+        PatternSlot<BN> v = *slot;
+        v.s += gv[i];
+        if constexpr (BN) {
+            q[i >> 1] |= i & 1 ? v.n & 0x80000000u : (v.n >> 16) & 0x8000u;
+            v.n += i < live ? 1u : 0u;
+        }
+        *slot = v;
+    }
+    return make_uint2(q[0], q[1]);
+}
+
+// adds the 32 columns of every pattern: lane l returns patterns l and l + 32
+template <bool BN>
+__device__ __forceinline__ void pattern_columns_reduce(const PatternSlot<BN> *slots, int lane, float (&s)[2], uint32_t (&n)[2])
+{
+#pragma unroll
+    for (int h = 0; h < 2; ++h) {
+        s[h] = 0.0f;
+        n[h] = 0u;
+#pragma unroll 8
+        for (int k = 0; k < 32; ++k) {
+            const PatternSlot<BN> v = slots[(lane + 32 * h) * 32 + ((k + lane) & 31)];      // rotated: 32 different banks
+            s[h] += v.s;
+            if constexpr (BN) n[h] += v.n & 0x7fffffffu;
+        }
+    }
+}
+
+template <bool XF32, bool BN>
+__global__ void __launch_bounds__(kPsWarps * 32)
+k_pattern_sums(const BitBwdArgs a)
+{
+    extern __shared__ __align__(16) unsigned char smem_raw[];
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
     const int tile = blockIdx.x / a.groups;
-    const int node = (blockIdx.x % a.groups) * kWarpsPerCta + warp;
+    const int node = (blockIdx.x % a.groups) * kPsWarps + warp;
     if (node >= a.O) return;
-    // the node's per-pattern tables: this lane works out patterns `lane` and `lane + 32`
-    stage_table_halves(s_tab[warp], a.W, node, lane, a.lut_binarize);
+    PatternSlot<BN> *slots = reinterpret_cast<PatternSlot<BN> *>(smem_raw) + warp * 64 * 32, *mine = slots + lane;
+    if constexpr (BN) {
+        const uint2 mask = a.mask[node];
+#pragma unroll 8
+        for (int p = 0; p < 64; ++p) mine[p * 32] = PatternSlot<true>{0.0f, ((p < 32 ? mask.x : mask.y) << (31 - (p & 31))) & 0x80000000u};
+    } else {
+#pragma unroll 8
+        for (int p = 0; p < 64; ++p) mine[p * 32] = PatternSlot<false>{0.0f};
+    }
+    const uint32_t *rows[6];
 #pragma unroll
-    for (int half = 0; half < 2; ++half) {
-        const int p = lane + 32 * half;
-        float u[6];
+    for (int j = 0; j < 6; ++j) rows[j] = a.x + (size_t)__ldg(a.idx + (size_t)node * 6 + j) * a.xs;
+    const float *dyrow = a.dy + (size_t)node * a.fs;
+    uint16_t *prow = a.pat + (size_t)node * a.ps;
+    const int f_begin = tile * a.tile_frames, f_end = min(a.F, f_begin + a.tile_frames);
+
+    int f = f_begin + 4 * lane;
+    if constexpr (!XF32) {
+        // 512 frames per step while whole steps are left; the loads of the next step are issued before this one is used, into the
+        // other of two sets of registers
+        constexpr int NC = 4, kStep = 128 * NC;
+        struct Set { uint32_t w[NC][6]; float4 dy[NC]; };
+        const int steps = a.vec ? (f_end - f_begin) / kStep : 0;
+        auto fetch = [&](Set &b, int k) {
+            if (k < steps) {
 #pragma unroll
-        for (int j = 0; j < 6; ++j) u[j] = ((p >> j) & 1) ? a.bias : -a.bias;
-        KeptHalves K;
-        const float v = lut6_forward_keep_halves(s_tab[warp], u, K);
-        if (MODE != kBwdHistOnly) {
-            f32x2 unused[32];
+                for (int c = 0; c < NC; ++c) {
 #pragma unroll
-            for (int i = 0; i < 32; ++i) unused[i] = 0ull;
-            float d[6];
-            lut6_reverse_halves(s_tab[warp], u, K, 1.0f, unused, d);
+                    for (int j = 0; j < 6; ++j) b.w[c][j] = __ldg(rows[j] + ((f + k * kStep) >> 5) + 4 * c);
+                    b.dy[c] = __ldg(reinterpret_cast<const float4 *>(dyrow + f + k * kStep + 128 * c));
+                }
+            }
+        };
+        auto use = [&](const Set &b, int k) {
+            if (k < steps) {
 #pragma unroll
-            for (int j = 0; j < 6; ++j) s_D[warp][j][p] = d[j];
+                for (int c = 0; c < NC; ++c)
+                    *reinterpret_cast<uint2 *>(prow + f + k * kStep + 128 * c) = pattern_columns_add<BN>(mine, pattern_bytes(b.w[c], lane), b.dy[c], 4);
+            }
+        };
+        Set s0, s1;
+        fetch(s0, 0);
+        for (int k = 0; k < steps; k += 2) {
+            fetch(s1, k + 1);
+            use(s0, k);
+            fetch(s0, k + 2);
+            use(s1, k + 1);
         }
-        if (MODE == kBwdNormDx) {
-            const float mean = a.mean[node], rstd = a.rstd[node];
-            const float tanh_x = ((v - mean) * rstd) * a.gamma + a.beta;
-            s_A[warp][p] = (tanh_x <= 0.0f || tanh_x >= 1.0f) ? 0.0f : 1.0f;              // hard-tanh mask of the pattern
-            s_B[warp][p] = a.dmean[node] + (v * a.dvar[node] * a.rF);
+        f += steps * kStep;
+    }
+    for (; f < f_end; f += 128) {                          // what is left, unaligned rows, and fp32 rows
+        uint32_t p4;
+        if constexpr (XF32) {
+            p4 = 0u;
+#pragma unroll
+            for (int j = 0; j < 6; ++j) {
+                const float4 v = load_frames(reinterpret_cast<const float *>(rows[j]), f, a.F, a.vec);
+                p4 |= ((v.x > 0.5f ? 1u : 0u) | (v.y > 0.5f ? 0x100u : 0u) | (v.z > 0.5f ? 0x10000u : 0u) | (v.w > 0.5f ? 0x1000000u : 0u)) << j;
+            }
+        } else {
+            uint32_t w[6];
+#pragma unroll
+            for (int j = 0; j < 6; ++j) w[j] = __ldg(rows[j] + (f >> 5));
+            p4 = pattern_bytes(w, lane);
         }
-        if (MODE != kBwdNormDx) s_H[warp][p] = 0.0f;
-        if (XF32 && MODE == kBwdHistOnly) s_C[warp][p] = 0u;
+        *reinterpret_cast<uint2 *>(prow + f) = pattern_columns_add<BN>(mine, p4, load_frames(dyrow, f, a.F, a.vec), a.F - f);      // rows of pat are padded
     }
     __syncwarp();
-    const float grstd_gamma = a.gamma, rstd_n = (MODE == kBwdNormDx) ? a.rstd[node] : 0.0f;
+    float s[2];
+    uint32_t n[2];
+    pattern_columns_reduce<BN>(slots, lane, s, n);
+#pragma unroll
+    for (int h = 0; h < 2; ++h) {
+        const size_t at = (size_t)node * 64 + 32 * h + lane;
+        if (a.tiles == 1) {
+            a.hdy[at] = s[h];
+            if (BN) a.hist[at] = n[h];
+        } else {                                              // several tiles: the launcher has cleared the sums
+            atomicAdd(a.hdy + at, s[h]);
+            if (BN) atomicAdd(a.hist + at, n[h]);
+        }
+    }
+}
 
-    const uint32_t *rows[6];
-    long long off[6];
+// ---- the consumers of every input row, as lists of 8 node + input number
+__global__ void k_edge_count(const int *__restrict__ idx, int *count, int edges)
+{
+    const int e = blockIdx.x * blockDim.x + threadIdx.x;
+    if (e < edges) atomicAdd(count + idx[e], 1);
+}
+
+// room for every row's list, in no particular order: `total` is a bump pointer, advanced once per warp
+__global__ void k_edge_room(const int *__restrict__ count, int *cursor, int *total, int I)
+{
+    const int i = blockIdx.x * blockDim.x + threadIdx.x, lane = threadIdx.x & 31;
+    const int n = i < I ? count[i] : 0;
+    int at = n;
 #pragma unroll
-    for (int j = 0; j < 6; ++j) {
-        const int r = __ldg(a.idx + (size_t)node * 6 + j);
-        rows[j] = a.x + (size_t)r * a.xs;
-        off[j] = (long long)r * a.fs;
+    for (int d = 1; d < 32; d <<= 1) {
+        const int t = __shfl_up_sync(kFull, at, d);
+        if (lane >= d) at += t;
     }
-    const int words = (a.F + 31) >> 5;
-    const int w_end = min(words, (tile + 1) * a.tile_words);
-    const float *dyrow = a.dy + (size_t)node * a.fs;
-    const BitTranspose transpose(lane);
-    for (int w0 = tile * a.tile_words; w0 < w_end; w0 += 32) {
-        uint32_t xw[6];                       // bit inputs: after the transpose, bit k of xw[j] is frame `lane` of word w0 + k
-        if (!XF32) {
+    int base = 0;
+    if (lane == 31) base = atomicAdd(total, at);
+    base = __shfl_sync(kFull, base, 31);
+    if (i < I) cursor[i] = base + at - n;
+}
+
+// afterwards cursor[i] is the end of row i's list
+__global__ void k_edge_fill(const int *__restrict__ idx, int *cursor, int *list, int edges)
+{
+    const int e = blockIdx.x * blockDim.x + threadIdx.x;
+    if (e < edges) list[atomicAdd(cursor + idx[e], 1)] = e + 2 * (e / 6);
+}
+
+template <unsigned SEL>
+__device__ __forceinline__ uint32_t prmt(uint32_t v)
+{
+    uint32_t r;
+    asm("prmt.b32 %0, %1, 0, %2;" : "=r"(r) : "r"(v), "n"(SEL));
+    return r;
+}
+
+// dx_i(f) = sum over the consumers (node o, input j) of row i of g_o(f) D_j[p_o(f)], frames from F on 0.  A CTA is one row and NC
+// chunks of 128 frames; `split` warps share the consumers (rows with many of them, or few rows).  One warp per CTA otherwise, because
+// the number of consumers varies from row to row and a CTA of several rows waits for the longest.
+// The tables of a consumer live in registers, one entry per lane, and a look-up is a shuffle whose source lane is a field of the doubled
+// pattern: bits j+1 .. j+5 are the other five inputs, bit j+6 is input j.  With batch norm g is put together here, ten
+// instructions per consumer and 32 frames in all, which is what bounds the kernel; writing g out once and reading it back would
+// leave three, but costs 10 bytes per node-frame of HBM traffic.
+template <bool BN, int NC, bool WHOLE>
+__device__ __forceinline__ void pattern_gather(const BitBwdArgs &a, int row, int part, int f0, int lane, float (&acc)[NC][4])
+{
+    const int n = __ldg(a.edge_count + row);
+    const int *list = a.edges + (__ldg(a.edge_end + row) - n);
+    int e_n = part < n ? __ldg(list + part) : 0;
+    for (int k = part; k < n; k += a.split) {
+        const int node = e_n >> 3, j = e_n & 7;
+        if (k + a.split < n) e_n = __ldg(list + k + a.split);
+        const float *t = a.etab + (size_t)(6 * node + j) * 64 + lane;
+        const float D = __ldg(t);
+        const float base = BN ? __ldg(t + 32) : 0.0f;
+        const float2 gs = BN ? __ldg(a.ntab + node) : make_float2(1.0f, 0.0f);
+        const uint32_t minus_slope = __float_as_uint(-gs.y);
+        const float *dyrow = a.dy + (size_t)node * a.fs;
+        const uint16_t *prow = a.pat + (size_t)node * a.ps;
+        float4 dyq[NC];
+        uint2 q2[NC];
 #pragma unroll
-            for (int j = 0; j < 6; ++j) xw[j] = transpose((w0 + lane < w_end) ? __ldg(rows[j] + w0 + lane) : 0u);
-        }
-        uint32_t p4 = 0u;                     // bit inputs: the patterns of four consecutive words, one per byte
-        const int kn = min(32, w_end - w0);
-        // dy of the next word is fetched while this one is processed
-        long long f = (long long)w0 * 32 + lane;
-        float dy_next = f < a.F ? __ldg(dyrow + f) : 0.0f;
-        // fp32 frames: this step's inputs were fetched during the previous step.  With batch norm the histogram pass leaves one pattern
-        // byte per frame behind and the dx pass reads that instead of gathering the six rows a second time.
-        constexpr bool kFromBytes = XF32 && MODE == kBwdNormDx;
-        float x_next[(XF32 && !kFromBytes) ? 6 : 1];
-        unsigned char p_next = 0;
-        const unsigned char *prow = XF32 && a.pat != nullptr ? a.pat + (size_t)node * a.fs : nullptr;
-        if (kFromBytes) {
-            p_next = f < a.F ? prow[f] : (unsigned char)0;
-        } else if (XF32) {
-#pragma unroll
-            for (int j = 0; j < 6; ++j) x_next[j] = f < a.F ? __ldg(reinterpret_cast<const float *>(a.x) + f + off[j]) : 0.0f;
-        }
-        for (int k = 0; k < kn; ++k, f += 32) {
-            uint32_t p = 0;
-            if (kFromBytes) {
-                p = p_next;
-                if (k + 1 < kn && f + 32 < a.F) p_next = prow[f + 32];
-            } else if (XF32) {
-#pragma unroll
-                for (int j = 5; j >= 0; --j) p = (p << 1) | (x_next[j] > 0.5f ? 1u : 0u);
-                if (k + 1 < kn && f + 32 < a.F) {
-                    const float *xf = reinterpret_cast<const float *>(a.x) + f + 32;
-#pragma unroll
-                    for (int j = 0; j < 6; ++j) x_next[j] = __ldg(xf + off[j]);
-                }
-                if (MODE == kBwdHistOnly && f < a.F) const_cast<unsigned char *>(prow)[f] = (unsigned char)p;
+        for (int c = 0; c < NC; ++c) {
+            const int f = f0 + 128 * c;
+            if (WHOLE) {
+                dyq[c] = __ldg(reinterpret_cast<const float4 *>(dyrow + f));
+                q2[c] = __ldg(reinterpret_cast<const uint2 *>(prow + f));
             } else {
-                if ((k & 3) == 0) {
-                    p4 = 0u;
-#pragma unroll
-                    for (int j = 0; j < 6; ++j) p4 |= ((((xw[j] >> k) & 0xfu) * 0x00204081u) & 0x01010101u) << j;
-                }
-                p = (p4 >> (8 * (k & 3))) & 63u;
+                dyq[c] = load_frames(dyrow, f, a.F, a.vec);
+                q2[c] = f < a.F ? __ldg(reinterpret_cast<const uint2 *>(prow + f)) : make_uint2(0u, 0u);
             }
-            const float dyv = dy_next;
-            if (k + 1 < kn && f + 32 < a.F) dy_next = __ldg(dyrow + f + 32);
-            if (f < a.F) {
-                if (MODE != kBwdNormDx) atomicAdd(&s_H[warp][p], dyv);
-                if (XF32 && MODE == kBwdHistOnly) atomicAdd(&s_C[warp][p], 1u);
-                if (MODE != kBwdHistOnly) {
-                    float g = dyv;
-                    if (MODE == kBwdNormDx) g = ((dyv * s_A[warp][p]) * grstd_gamma) * rstd_n + s_B[warp][p];
-                    float *dxf = a.dx + f;
+        }
 #pragma unroll
-                    for (int j = 0; j < 6; ++j) atomicAdd(dxf + off[j], g * s_D[warp][j][p]);
+        for (int c = 0; c < NC; ++c) {
+            const float dyv[4] = {dyq[c].x, dyq[c].y, dyq[c].z, dyq[c].w};
+#pragma unroll
+            for (int i = 0; i < 4; ++i) {
+                const uint32_t q = i < 2 ? q2[c].x : q2[c].y;
+                const uint32_t r = q >> (j + 1 + 16 * (i & 1));
+                const float d = __shfl_sync(kFull, D, r);
+                float g = dyv[i];
+                if (BN) {
+                    const float slope = __uint_as_float(((r << 26) & 0x80000000u) ^ minus_slope);      // +slope where input j is set
+                    const uint32_t pass = i & 1 ? prmt<0xbbbb>(q) : prmt<0x9999>(q);                   // bit 15 of the frame's half, replicated
+                    g = fmaf(__uint_as_float(__float_as_uint(g) & pass), gs.x, fmaf(slope, d, __shfl_sync(kFull, base, r)));
                 }
+                acc[c][i] = fmaf(g, d, acc[c][i]);
             }
         }
     }
-    if (MODE != kBwdNormDx) {
-        __syncwarp();
-        atomicAdd(a.hdy + (size_t)node * 64 + lane, s_H[warp][lane]);
-        atomicAdd(a.hdy + (size_t)node * 64 + 32 + lane, s_H[warp][lane + 32]);
-        if (XF32 && MODE == kBwdHistOnly) {
-            atomicAdd(a.hist + (size_t)node * 64 + lane, s_C[warp][lane]);
-            atomicAdd(a.hist + (size_t)node * 64 + 32 + lane, s_C[warp][lane + 32]);
+}
+
+template <bool BN, int NC>
+__global__ void __launch_bounds__(kWarpsPerCta * 32, 4)
+k_pattern_gather(const BitBwdArgs a)
+{
+    extern __shared__ __align__(16) unsigned char smem_raw[];           // split > 1: float4 [split][NC][32]
+    float4 *s_part = reinterpret_cast<float4 *>(smem_raw);
+    const int part = threadIdx.x >> 5, lane = threadIdx.x & 31;
+    const int tile = blockIdx.x / a.I, row = blockIdx.x - tile * a.I;
+    const int f_begin = tile * (128 * NC), f0 = f_begin + 4 * lane;
+    float acc[NC][4];
+#pragma unroll
+    for (int c = 0; c < NC; ++c)
+#pragma unroll
+        for (int i = 0; i < 4; ++i) acc[c][i] = 0.0f;
+    if (a.vec && f_begin + 128 * NC <= a.F) pattern_gather<BN, NC, true>(a, row, part, f0, lane, acc);
+    else if (f_begin < a.F)                 pattern_gather<BN, NC, false>(a, row, part, f0, lane, acc);
+    if (a.split > 1) {
+#pragma unroll
+        for (int c = 0; c < NC; ++c) s_part[(part * NC + c) * 32 + lane] = make_float4(acc[c][0], acc[c][1], acc[c][2], acc[c][3]);
+        __syncthreads();
+        if (part != 0) return;
+        for (int k = 1; k < a.split; ++k)
+#pragma unroll
+            for (int c = 0; c < NC; ++c) {
+                const float4 v = s_part[(k * NC + c) * 32 + lane];
+                acc[c][0] += v.x; acc[c][1] += v.y; acc[c][2] += v.z; acc[c][3] += v.w;
+            }
+    }
+    float *out = a.dx + (size_t)row * a.fs;
+#pragma unroll
+    for (int c = 0; c < NC; ++c) {
+        const int f = f0 + 128 * c;
+#pragma unroll
+        for (int i = 0; i < 4; ++i)
+            if (f + i >= a.F) acc[c][i] = 0.0f;
+        if (a.vec && f + 3 < a.fs) {
+            *reinterpret_cast<float4 *>(out + f) = make_float4(acc[c][0], acc[c][1], acc[c][2], acc[c][3]);
+        } else {
+#pragma unroll
+            for (int i = 0; i < 4; ++i)
+                if (f + i < a.fs) out[f + i] = acc[c][i];
         }
     }
 }
@@ -388,33 +588,112 @@ __device__ __forceinline__ float2 pattern_sums_to_table_grads(float2 v, int lane
     return v;
 }
 
-// One warp per node.  BN = false: dW += K^T Hdy.  BN = true: the batch sums, dmean / dvar, then dW += K^T Hg with
-// Hg[p] = mask[p] gamma rstd Hdy[p] + (dmean + Y[p] dvar / F) H[p].
+// LUT value and the six input derivatives at patterns `lane` and `lane + 32` of a node whose table is staged in `tab2`.
+__device__ __forceinline__ void eval_pattern_pair(const float4 *tab2, int lane, float bias, float (&y)[2], float (&d)[2][6])
+{
+#pragma unroll
+    for (int h = 0; h < 2; ++h) {
+        float u[6];
+#pragma unroll
+        for (int j = 0; j < 5; ++j) u[j] = ((lane >> j) & 1) ? bias : -bias;
+        u[5] = h ? bias : -bias;
+        KeptHalves K;
+        f32x2 unused[32];
+#pragma unroll
+        for (int i = 0; i < 32; ++i) unused[i] = 0ull;
+        y[h] = lut6_forward_keep_halves(tab2, u, K);
+        lut6_reverse_halves(tab2, u, K, 1.0f, unused, d[h]);
+    }
+}
+
+// The look-up tables of a node's six edges, 64 floats each: D_j for the 32 values of the other five bits -- entry m belongs to the
+// patterns whose bits j+1 .. j+5 (mod 6) are m, a field of the doubled pattern p | p << 6 -- and, with batch norm, the part of
+// dmean + Y[p] dvar / F that does not depend on bit j (the rest is +-D_j times dvar bias / F).
+template <bool BN>
+__device__ __forceinline__ void store_edge_tables(float *etab, int lane, const float (&y)[2], const float (&d)[2][6], float dmean, float dvar_rF)
+{
+#pragma unroll
+    for (int j = 0; j < 6; ++j) {
+#pragma unroll
+        for (int h = 0; h < 2; ++h) {
+            const unsigned p = lane + 32 * h, q = p | (p << 6);
+            const float other = j == 5 ? y[1 - h] : __shfl_xor_sync(kFull, y[h], 1 << (j & 31));
+            if (!((p >> j) & 1u)) {                                                          // D_j is the same with bit j set
+                float *t = etab + 64 * j + ((q >> (j + 1)) & 31u);
+                t[0] = d[h][j];
+                if (BN) t[32] = dmean + (0.5f * (y[h] + other)) * dvar_rF;
+            }
+        }
+    }
+}
+
+__global__ void __launch_bounds__(kWarpsPerCta * 32)
+k_pattern_derivatives(const float *__restrict__ W, float *__restrict__ etab, float bias, int O, int lut_binarize)
+{
+    __shared__ float4 s_tab[kWarpsPerCta][16];
+    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+    const int node = blockIdx.x * kWarpsPerCta + warp;
+    if (node >= O) return;
+    stage_table_halves(s_tab[warp], W, node, lane, lut_binarize);
+    float y[2], d[2][6];
+    eval_pattern_pair(s_tab[warp], lane, bias, y, d);
+    store_edge_tables<false>(etab + (size_t)node * 6 * 64, lane, y, d, 0.0f, 0.0f);
+}
+
+// Hard-tanh mask of every pattern of every node: the gradient passes where 0 < affine(Y[p]) < 1 (include/bb/DifferentiableLutN.h:1204-1206).
+__global__ void __launch_bounds__(kWarpsPerCta * 32)
+k_pattern_masks(const float *__restrict__ W, uint2 *__restrict__ mask, const float *__restrict__ mean_buf, const float *__restrict__ rstd_buf, float gamma,
+                float beta, float bias, int O, int lut_binarize)
+{
+    __shared__ float4 s_tab[kWarpsPerCta][16];
+    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+    const int node = blockIdx.x * kWarpsPerCta + warp;
+    if (node >= O) return;
+    stage_table_halves(s_tab[warp], W, node, lane, lut_binarize);
+    const float mean = mean_buf[node], rstd = rstd_buf[node];
+    unsigned m[2];
+#pragma unroll
+    for (int h = 0; h < 2; ++h) {
+        float u[6];
+#pragma unroll
+        for (int j = 0; j < 5; ++j) u[j] = ((lane >> j) & 1) ? bias : -bias;
+        u[5] = h ? bias : -bias;
+        const float t = ((lut6_forward_halves(s_tab[warp], u) - mean) * rstd) * gamma + beta;
+        m[h] = __ballot_sync(kFull, !(t <= 0.0f || t >= 1.0f));
+    }
+    if (lane == 0) mask[node] = make_uint2(m[0], m[1]);
+}
+
+// One warp per node.  BN = false: dW += K^T Hdy.  BN = true: the batch sums, dmean / dvar, dW += K^T Hg with
+// Hg[p] = mask[p] gamma rstd Hdy[p] + (dmean + Y[p] dvar / F) H[p], and the look-up tables of k_pattern_gather.
 // `sums_out` (frame-sharded callers): the node's local (dstd, dmeanx) go out as fp64 and nothing else is done.
 // `sums_in`: the sums over ALL ranks' frames come in instead of being formed from this rank's Hdy; rF = 1 / total frames.
 template <bool BN>
 __global__ void __launch_bounds__(kWarpsPerCta * 32)
-k_bit_backward_finalize(const float *__restrict__ hdy, const uint32_t *__restrict__ hist, const float *__restrict__ Y, float *dW,
-                        const float *__restrict__ mean_buf, const float *__restrict__ rstd_buf, float *dmean_out, float *dvar_out, float gamma,
-                        float beta, float bias, int O, float rF, double *sums_out, const double *__restrict__ sums_in)
+k_bit_backward_finalize(const float *__restrict__ hdy, const uint32_t *__restrict__ hist, const uint2 *__restrict__ mask, const float *__restrict__ W,
+                        float *__restrict__ etab, float2 *__restrict__ ntab, float *dW, const float *__restrict__ mean_buf, const float *__restrict__ rstd_buf, float *dmean_out, float *dvar_out, float gamma,
+                        float beta, float bias, int O, float rF, int lut_binarize, double *sums_out, const double *__restrict__ sums_in)
 {
+    __shared__ float4 s_tab[BN ? kWarpsPerCta : 1][16];
+    __shared__ float s_hg[kWarpsPerCta][64];
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
     const int node = blockIdx.x * kWarpsPerCta + warp;
     if (node >= O) return;
-    float2 hg = reinterpret_cast<const float2 *>(hdy + (size_t)node * 64)[lane];             // patterns 2l, 2l + 1
+    float hg[2] = {hdy[(size_t)node * 64 + lane], hdy[(size_t)node * 64 + 32 + lane]};                // patterns lane, lane + 32
     if (BN) {
-        const float2 y = reinterpret_cast<const float2 *>(Y + (size_t)node * 64)[lane];
-        const uint2 h = reinterpret_cast<const uint2 *>(hist + (size_t)node * 64)[lane];
+        stage_table_halves(s_tab[warp], W, node, lane, lut_binarize);
+        float y[2], d[2][6];
+        eval_pattern_pair(s_tab[warp], lane, bias, y, d);
         const float mean = mean_buf[node], rstd = rstd_buf[node], rstd2 = rstd * rstd;
-        const float t0 = ((y.x - mean) * rstd) * gamma + beta, t1 = ((y.y - mean) * rstd) * gamma + beta;
-        const float m0 = (t0 <= 0.0f || t0 >= 1.0f) ? 0.0f : 1.0f, m1 = (t1 <= 0.0f || t1 >= 1.0f) ? 0.0f : 1.0f;
-        const float dxn0 = gamma * (m0 * hg.x), dxn1 = gamma * (m1 * hg.y);                   // sum over the pattern's frames of gamma * masked dy
+        const uint2 mw = mask[node];
+        const bool m0 = (mw.x >> lane) & 1u, m1 = (mw.y >> lane) & 1u;
+        const float dxn0 = m0 ? gamma * hg[0] : 0.0f, dxn1 = m1 ? gamma * hg[1] : 0.0f;       // sum over the pattern's frames of gamma * masked dy
         double dstd, dmeanx;
         if (sums_in != nullptr) {
             dstd = sums_in[2 * (size_t)node];
             dmeanx = sums_in[2 * (size_t)node + 1];
         } else {
-            dstd = -((double)(dxn0 * (y.x - mean) * rstd2) + (double)(dxn1 * (y.y - mean) * rstd2));
+            dstd = -((double)(dxn0 * (y[0] - mean) * rstd2) + (double)(dxn1 * (y[1] - mean) * rstd2));
             dmeanx = -((double)(dxn0 * rstd) + (double)(dxn1 * rstd));
             dstd = warp_sum(dstd);
             dmeanx = warp_sum(dmeanx);
@@ -426,10 +705,15 @@ k_bit_backward_finalize(const float *__restrict__ hdy, const uint32_t *__restric
         const float dvar = (float)dstd * rstd;
         const float dmean = ((float)dmeanx - (mean * dvar)) * rF;
         if (lane == 0) { dvar_out[node] = dvar; dmean_out[node] = dmean; }
-        hg.x = (dxn0 * rstd) + (dmean + (y.x * dvar * rF)) * (float)h.x;
-        hg.y = (dxn1 * rstd) + (dmean + (y.y * dvar * rF)) * (float)h.y;
+        hg[0] = (dxn0 * rstd) + (dmean + (y[0] * dvar * rF)) * (float)hist[(size_t)node * 64 + lane];
+        hg[1] = (dxn1 * rstd) + (dmean + (y[1] * dvar * rF)) * (float)hist[(size_t)node * 64 + 32 + lane];
+        store_edge_tables<true>(etab + (size_t)node * 6 * 64, lane, y, d, dmean, dvar * rF);
+        if (lane == 0) ntab[node] = make_float2(gamma * rstd, bias * dvar * rF);
     }
-    const float2 gw = pattern_sums_to_table_grads(hg, lane, bias);
+    s_hg[warp][lane] = hg[0];
+    s_hg[warp][lane + 32] = hg[1];
+    __syncwarp();
+    const float2 gw = pattern_sums_to_table_grads(reinterpret_cast<const float2 *>(s_hg[warp])[lane], lane, bias);
     float *dst = dW + (size_t)node * 64 + 2 * lane;
     dst[0] += gw.x;
     dst[1] += gw.y;
@@ -564,7 +848,7 @@ struct Scratch {
 // bytes), so that the apply half that follows it on the same stream need not repeat that pass.  Any other use of the scratch
 // forgets it; the apply half checks every field and redoes the pass when something differs.
 struct PassOneRecord {
-    const void *x = nullptr, *dy = nullptr, *W = nullptr;
+    const void *x = nullptr, *dy = nullptr, *W = nullptr, *mean = nullptr, *rstd = nullptr;
     int O = 0, F = 0;
     long long fs = 0;
 };
@@ -727,157 +1011,187 @@ int f32_binary_forward_by_table(int mode, const float *x, float *y, const int *i
     return launch_status();
 }
 
-// Backward of the bit-input layers (StochasticLut6: bn = false; DifferentiableLut6: bn = true).  dx must be zero on entry.
-int bit_backward_by_table(bool bn, bool x_is_fp32, const void *x, const float *dy, float *dx, const int *idx, const float *W, float *dW,
-                          const float *mean, const float *rstd, float *dmean_out, float *dvar_out, float gamma, float beta, float bias, int O, int F,
-                          long long xs, long long fs, int lut_binarize, cudaStream_t st)
+// ---------------------------------------------------------------------------------------------- backward launchers
+namespace {
+
+// Scratch and arguments shared by all backward calls.  The block in slot 1 has the same size whatever the call (sums, counts, masks,
+// look-up tables, pattern bytes), so that the apply half of a frame-sharded backward finds what its statistics half left there.
+bool backward_setup(BitBwdArgs &a, const void *x, const float *dy, const int *idx, int O, int F, long long xs, long long fs, cudaStream_t st)
 {
-    if (x_is_fp32 && xs != fs) return BBCU_ERR_NO_MEMORY;          // fp32 x shares the stride of dy / dx in every caller; otherwise decline
-    if (O == 0 || F == 0) return BBCU_OK;
-    const size_t pat_bytes = (x_is_fp32 && bn) ? (size_t)O * (size_t)fs : 0;      // pattern bytes handed from the histogram pass to the dx pass
-    if (pat_bytes > ((size_t)1 << 30)) return BBCU_ERR_NO_MEMORY;
+    const long long ps = ((long long)F + 127) / 128 * 128;
+    const size_t tables = (size_t)O * (6 * 64 * sizeof(float) + sizeof(float2) + sizeof(uint2));
+    if ((size_t)O * (size_t)ps > ((size_t)1 << 32)) return false;        // 8 GiB of patterns at most
     Scratch s;
-    if (!carve(s, O, st, pat_bytes)) return BBCU_ERR_NO_MEMORY;
-    float *hdy = reinterpret_cast<float *>(s.hist) + (size_t)O * 64;       // the block between the pattern counts and the truth tables
-    BitBwdArgs a = {};
-    a.x = static_cast<const uint32_t *>(x); a.dy = dy; a.dx = dx; a.idx = idx; a.W = W; a.hdy = hdy; a.hist = s.hist; a.pat = pat_bytes ? s.pat : nullptr;
-    a.mean = mean; a.rstd = rstd; a.dmean = dmean_out; a.dvar = dvar_out;
-    a.gamma = gamma; a.beta = beta; a.bias = bias; a.rF = 1.0f / (float)F;
-    a.O = O; a.F = F; a.xs = xs; a.fs = fs; a.lut_binarize = lut_binarize;
-    a.groups = (O + kWarpsPerCta - 1) / kWarpsPerCta;
-    const int words = (F + 31) / 32;
-    // tiles of 4096 frames unless that leaves the GPU short of CTAs (each warp pays ~1000 instructions of table set-up per tile)
-    a.tile_words = 128;
-    while (a.tile_words > 32 && (long long)a.groups * ((words + a.tile_words - 1) / a.tile_words) < 2LL * device_info().sm_count) a.tile_words /= 2;
-    const long long blocks = (long long)a.groups * ((words + a.tile_words - 1) / a.tile_words);
+    if (!carve(s, O, st, ((tables + 255) & ~(size_t)255) + (size_t)O * (size_t)ps * sizeof(uint16_t))) return false;
+    a = BitBwdArgs{};
+    a.x = static_cast<const uint32_t *>(x); a.dy = dy; a.idx = idx;
+    a.hist = s.hist;
+    a.hdy = reinterpret_cast<float *>(s.hist) + (size_t)O * 64;          // the block between the pattern counts and the truth tables
+    a.etab = reinterpret_cast<float *>(s.pat);
+    a.ntab = reinterpret_cast<float2 *>(a.etab + (size_t)O * 6 * 64);
+    a.mask = reinterpret_cast<uint2 *>(a.ntab + O);
+    a.pat = reinterpret_cast<uint16_t *>(s.pat + ((tables + 255) & ~(size_t)255));
+    a.O = O; a.F = F; a.xs = xs; a.fs = fs; a.ps = ps;
+    a.vec = (reinterpret_cast<uintptr_t>(dy) & 15) == 0 && fs % 4 == 0;
+    return true;
+}
+
+// Slot 3 of the stream's scratch: consumer lists, and the bits of the I fp32 rows when `pack`.
+bool input_side(BitBwdArgs &a, int I, bool pack, cudaStream_t st)
+{
+    if (I == 0) return false;
+    a.I = I;
+    const int edges = 6 * a.O;
+    const long long ws = (a.F + 31) / 32;
+    const size_t list_bytes = ((2 * (size_t)I + 1 + (size_t)edges) * sizeof(int) + 255) & ~(size_t)255;
+    const size_t bit_bytes = pack ? (size_t)I * (size_t)ws * 4 : 0;
+    if (bit_bytes > ((size_t)1 << 30)) return false;
+    int *count = static_cast<int *>(stream_scratch(st, list_bytes + bit_bytes, 3));
+    if (count == nullptr) return false;
+    int *total = count + I, *cursor = total + 1, *list = cursor + I;
+    a.edge_count = count; a.edge_end = cursor; a.edges = list;
+    cudaMemsetAsync(count, 0, ((size_t)I + 1) * sizeof(int), st);
+    k_edge_count<<<(edges + 255) / 256, 256, 0, st>>>(a.idx, count, edges);
+    k_edge_room<<<(I + 255) / 256, 256, 0, st>>>(count, cursor, total, I);
+    k_edge_fill<<<(edges + 255) / 256, 256, 0, st>>>(a.idx, cursor, list, edges);
+    if (pack) {
+        uint32_t *bits = reinterpret_cast<uint32_t *>(reinterpret_cast<unsigned char *>(count) + list_bytes);
+        const int runs = (int)((ws + 31) / 32);
+        const long long blocks = ((long long)I * runs + kWarpsPerCta - 1) / kWarpsPerCta;
+        if (blocks >= (1LL << 31)) return false;
+        k_pack_bits<<<(unsigned)blocks, kWarpsPerCta * 32, 0, st>>>(reinterpret_cast<const float *>(a.x), bits, I, a.F, a.xs, ws, runs);
+        a.x = bits;
+        a.xs = ws;
+    }
+    return true;
+}
+
+// Pattern sums (and counts) and pattern bytes.  Tiles as wide as still give every SM two rounds of warps: the columns of a tile cost
+// about as much to clear and add up as 500 frames.
+template <bool XF32>
+int launch_pattern_sums(BitBwdArgs a, bool bn, cudaStream_t st)
+{
+    a.groups = (a.O + kPsWarps - 1) / kPsWarps;
+    if (XF32) a.vec = a.vec && (reinterpret_cast<uintptr_t>(a.x) & 15) == 0 && a.xs % 4 == 0;
+    long long tile = ((long long)a.F + 127) / 128 * 128;
+    while (tile > 1024 && (long long)a.O * ((a.F + tile - 1) / tile) < 24LL * device_info().sm_count) tile = (tile / 2 + 127) / 128 * 128;
+    a.tile_frames = (int)tile;
+    a.tiles = (int)((a.F + tile - 1) / tile);
+    const long long blocks = (long long)a.groups * a.tiles;
     BB200_REQUIRE(blocks < (1LL << 31), BBCU_ERR_TOO_LARGE);
-    BB200_CUDA(cudaMemsetAsync(hdy, 0, (size_t)O * 256, st));
-    const unsigned nb = (unsigned)blocks, threads = kWarpsPerCta * 32;
-    if (!bn) {
-        if (x_is_fp32) k_bit_backward_frames<kBwdPlainAll, true><<<nb, threads, 0, st>>>(a);
-        else           k_bit_backward_frames<kBwdPlainAll, false><<<nb, threads, 0, st>>>(a);
-        BB200_CUDA(cudaPeekAtLastError());
-        k_bit_backward_finalize<false><<<a.groups, threads, 0, st>>>(hdy, nullptr, nullptr, dW, nullptr, nullptr, nullptr, nullptr, 0.0f, 0.0f, bias, O, 0.0f, nullptr, nullptr);
-        return launch_status();
+    if (a.tiles > 1) {
+        BB200_CUDA(cudaMemsetAsync(a.hdy, 0, (size_t)a.O * 256, st));
+        if (bn) BB200_CUDA(cudaMemsetAsync(a.hist, 0, (size_t)a.O * 256, st));
     }
-    k_pattern_values<kTableNone><<<a.groups, threads, 0, st>>>(W, s.Y, nullptr, nullptr, nullptr, 0.0f, 0.0f, bias, O, lut_binarize);
-    BB200_CUDA(cudaPeekAtLastError());
-    BB200_CUDA(cudaMemsetAsync(s.hist, 0, (size_t)O * 256, st));
-    if (!x_is_fp32) {                                   // fp32 frames: the histogram pass below counts the patterns itself
-        int tw = 4096;
-        while (tw > 32 && (long long)a.groups * ((words + tw - 1) / tw) < 2LL * device_info().sm_count) tw /= 2;
-        const long long hb = (long long)a.groups * ((words + tw - 1) / tw);
-        k_pattern_histogram<<<(unsigned)hb, threads, 0, st>>>(a.x, idx, s.hist, O, F, xs, a.groups, tw);
-        BB200_CUDA(cudaPeekAtLastError());
-    }
-    if (x_is_fp32) k_bit_backward_frames<kBwdHistOnly, true><<<nb, threads, 0, st>>>(a);
-    else           k_bit_backward_frames<kBwdHistOnly, false><<<nb, threads, 0, st>>>(a);
-    BB200_CUDA(cudaPeekAtLastError());
-    k_bit_backward_finalize<true><<<a.groups, threads, 0, st>>>(hdy, s.hist, s.Y, dW, mean, rstd, dmean_out, dvar_out, gamma, beta, bias, O, 1.0f / (float)F, nullptr, nullptr);
-    BB200_CUDA(cudaPeekAtLastError());
-    if (x_is_fp32) k_bit_backward_frames<kBwdNormDx, true><<<nb, threads, 0, st>>>(a);
-    else           k_bit_backward_frames<kBwdNormDx, false><<<nb, threads, 0, st>>>(a);
+    const int smem = kPsWarps * 64 * 32 * (int)(bn ? sizeof(PatternSlot<true>) : sizeof(PatternSlot<false>));
+    auto kern = bn ? k_pattern_sums<XF32, true> : k_pattern_sums<XF32, false>;
+    BB200_CUDA(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, smem));
+    kern<<<(unsigned)blocks, kPsWarps * 32, smem, st>>>(a);
     return launch_status();
 }
 
-
-// ---- the two halves of the batch-norm backward for frame-sharded callers (binary mode; bit rows or fp32 rows)
-namespace {
-
-// pass 1: pattern values, pattern counts and per-pattern dy sums (and, for fp32 rows, the pattern bytes) of this rank's frames
-int backward_pass_one(bool x_is_fp32, BitBwdArgs &a, Scratch &s, float *&hdy, const void *x, const float *dy, const int *idx, const float *W,
-                      float bias, int O, int F, long long xs, long long fs, int lut_binarize, cudaStream_t st, bool reuse)
+// dx.  The tile is 512 frames (the tables of a consumer are loaded once per tile) unless the dy and pattern rows of such a tile, 6
+// bytes per node and frame, exceed two thirds of L2, or the GPU would run short of warps.
+int launch_pattern_gather(BitBwdArgs a, bool bn, cudaStream_t st)
 {
-    const size_t pat_bytes = x_is_fp32 ? (size_t)O * (size_t)fs : 0;
-    if (pat_bytes > ((size_t)1 << 30)) return BBCU_ERR_NO_MEMORY;
-    bool have = false;
-    if (reuse) {
-        std::lock_guard<std::mutex> g(g_record_mu);
-        auto it = g_records.find(record_key(st));
-        have = it != g_records.end() && it->second.x == x && it->second.dy == dy && it->second.W == W && it->second.O == O && it->second.F == F &&
-               it->second.fs == fs;
-    }
-    if (!carve(s, O, st, pat_bytes)) return BBCU_ERR_NO_MEMORY;           // same size as before: the same block (and it forgets the record)
-    hdy = reinterpret_cast<float *>(s.hist) + (size_t)O * 64;
-    a = BitBwdArgs{};
-    a.x = static_cast<const uint32_t *>(x); a.dy = dy; a.idx = idx; a.W = W; a.hdy = hdy; a.hist = s.hist; a.pat = pat_bytes ? s.pat : nullptr;
-    a.bias = bias; a.O = O; a.F = F; a.xs = xs; a.fs = fs; a.lut_binarize = lut_binarize;
-    a.groups = (O + kWarpsPerCta - 1) / kWarpsPerCta;
-    const int words = (F + 31) / 32;
-    a.tile_words = 128;
-    while (a.tile_words > 32 && (long long)a.groups * ((words + a.tile_words - 1) / a.tile_words) < 2LL * device_info().sm_count) a.tile_words /= 2;
-    const long long blocks = (long long)a.groups * ((words + a.tile_words - 1) / a.tile_words);
+    a.vec = a.vec && (reinterpret_cast<uintptr_t>(a.dx) & 15) == 0;
+    const DeviceInfo &di = device_info();
+    const long long fan = (6LL * a.O + a.I - 1) / a.I;                                // consumers per row, on average
+    int nc = 4;
+    while (nc > 1 && (6LL * a.O * 128 * nc > (long long)(di.l2_bytes / 3 * 2) || (long long)a.I * ((a.fs + 128 * nc - 1) / (128 * nc)) < 16LL * di.sm_count)) nc /= 2;
+    const long long blocks = (long long)a.I * ((a.fs + 128 * nc - 1) / (128 * nc));
     BB200_REQUIRE(blocks < (1LL << 31), BBCU_ERR_TOO_LARGE);
-    if (!have) {
-        const unsigned threads = kWarpsPerCta * 32;
-        BB200_CUDA(cudaMemsetAsync(hdy, 0, (size_t)O * 256, st));
-        k_pattern_values<kTableNone><<<a.groups, threads, 0, st>>>(W, s.Y, nullptr, nullptr, nullptr, 0.0f, 0.0f, bias, O, lut_binarize);
-        BB200_CUDA(cudaPeekAtLastError());
-        BB200_CUDA(cudaMemsetAsync(s.hist, 0, (size_t)O * 256, st));
-        if (!x_is_fp32) {
-            int tw = 4096;
-            while (tw > 32 && (long long)a.groups * ((words + tw - 1) / tw) < 2LL * device_info().sm_count) tw /= 2;
-            const long long hb = (long long)a.groups * ((words + tw - 1) / tw);
-            k_pattern_histogram<<<(unsigned)hb, threads, 0, st>>>(a.x, idx, s.hist, O, F, xs, a.groups, tw);
-            BB200_CUDA(cudaPeekAtLastError());
-        }
-        if (x_is_fp32) k_bit_backward_frames<kBwdHistOnly, true><<<(unsigned)blocks, threads, 0, st>>>(a);
-        else           k_bit_backward_frames<kBwdHistOnly, false><<<(unsigned)blocks, threads, 0, st>>>(a);
-        BB200_CUDA(cudaPeekAtLastError());
-    }
-    return BBCU_OK;
+    a.split = 1;
+    while (a.split < kWarpsPerCta && (fan >= 32LL * a.split || (fan >= 4LL * a.split && blocks * a.split < 8LL * di.sm_count))) a.split *= 2;
+    const int smem = a.split > 1 ? a.split * nc * 32 * (int)sizeof(float4) : 0;
+    auto kern = bn ? (nc == 4 ? k_pattern_gather<true, 4> : nc == 2 ? k_pattern_gather<true, 2> : k_pattern_gather<true, 1>)
+                   : (nc == 4 ? k_pattern_gather<false, 4> : nc == 2 ? k_pattern_gather<false, 2> : k_pattern_gather<false, 1>);
+    kern<<<(unsigned)blocks, a.split * 32, smem, st>>>(a);
+    return launch_status();
 }
 
 }   // namespace
 
-// Statistics half: this rank's (dstd, dmeanx) per node into `sums` ([O][2] fp64), to be added over the ranks by the caller.
-int bit_backward_stats_by_table(bool x_is_fp32, const void *x, const float *dy, const int *idx, const float *W, const float *mean, const float *rstd,
-                                double *sums, float gamma, float beta, float bias, int O, int F, long long xs, long long fs, int lut_binarize,
-                                cudaStream_t st)
+// Backward of the bit-input layers (StochasticLut6: bn = false; DifferentiableLut6: bn = true); writes all of dx's I rows.
+int bit_backward_by_table(bool bn, bool x_is_fp32, const void *x, const float *dy, float *dx, const int *idx, const float *W, float *dW,
+                          const float *mean, const float *rstd, float *dmean_out, float *dvar_out, float gamma, float beta, float bias, int I, int O,
+                          int F, long long xs, long long fs, int lut_binarize, cudaStream_t st)
 {
-    if (x_is_fp32 && xs != fs) return BBCU_ERR_NO_MEMORY;
+    if (x_is_fp32 && xs != fs) return BBCU_ERR_NO_MEMORY;          // fp32 x shares the stride of dy / dx in every caller; otherwise decline
+    BitBwdArgs a;
+    if (!backward_setup(a, x, dy, idx, O, F, xs, fs, st) || !input_side(a, I, x_is_fp32, st)) return BBCU_ERR_NO_MEMORY;
+    BB200_CUDA(cudaPeekAtLastError());
+    a.dx = dx;
+    const unsigned blocks = (unsigned)((O + kWarpsPerCta - 1) / kWarpsPerCta), threads = kWarpsPerCta * 32;
+    if (bn) k_pattern_masks<<<blocks, threads, 0, st>>>(W, a.mask, mean, rstd, gamma, beta, bias, O, lut_binarize);
+    else    k_pattern_derivatives<<<blocks, threads, 0, st>>>(W, a.etab, bias, O, lut_binarize);
+    BB200_CUDA(cudaPeekAtLastError());
+    const int rc = launch_pattern_sums<false>(a, bn, st);
+    if (rc) return rc;
+    if (bn) k_bit_backward_finalize<true><<<blocks, threads, 0, st>>>(a.hdy, a.hist, a.mask, W, a.etab, a.ntab, dW, mean, rstd, dmean_out, dvar_out, gamma, beta,
+                                                                     bias, O, 1.0f / (float)F, lut_binarize, nullptr, nullptr);
+    else    k_bit_backward_finalize<false><<<blocks, threads, 0, st>>>(a.hdy, nullptr, nullptr, nullptr, nullptr, nullptr, dW, nullptr, nullptr, nullptr, nullptr,
+                                                                      0.0f, 0.0f, bias, O, 0.0f, lut_binarize, nullptr, nullptr);
+    BB200_CUDA(cudaPeekAtLastError());
+    return launch_pattern_gather(a, bn, st);
+}
+
+// ---- the two halves of the batch-norm backward for frame-sharded callers (binary mode on fp32 rows)
+// Statistics half: this rank's (dstd, dmeanx) per node into `sums` ([O][2] fp64), to be added over the ranks by the caller.  (The number of
+// input rows is not known here, so the patterns come straight from the fp32 rows.)
+int bit_backward_stats_by_table(const float *x, const float *dy, const int *idx, const float *W, const float *mean, const float *rstd, double *sums,
+                                float gamma, float beta, float bias, int O, int F, long long fs, int lut_binarize, cudaStream_t st)
+{
     if (O == 0) return BBCU_OK;
     if (F == 0) { BB200_CUDA(cudaMemsetAsync(sums, 0, sizeof(double) * 2 * (size_t)O, st)); return BBCU_OK; }
     BitBwdArgs a;
-    Scratch s;
-    float *hdy = nullptr;
-    int rc = backward_pass_one(x_is_fp32, a, s, hdy, x, dy, idx, W, bias, O, F, xs, fs, lut_binarize, st, false);
+    if (!backward_setup(a, x, dy, idx, O, F, fs, fs, st)) return BBCU_ERR_NO_MEMORY;
+    const unsigned blocks = (unsigned)((O + kWarpsPerCta - 1) / kWarpsPerCta), threads = kWarpsPerCta * 32;
+    k_pattern_masks<<<blocks, threads, 0, st>>>(W, a.mask, mean, rstd, gamma, beta, bias, O, lut_binarize);
+    BB200_CUDA(cudaPeekAtLastError());
+    int rc = launch_pattern_sums<true>(a, true, st);
     if (rc) return rc;
-    k_bit_backward_finalize<true><<<a.groups, kWarpsPerCta * 32, 0, st>>>(hdy, s.hist, s.Y, nullptr, mean, rstd, nullptr, nullptr, gamma, beta, bias, O,
-                                                                          0.0f, sums, nullptr);
+    k_bit_backward_finalize<true><<<blocks, threads, 0, st>>>(a.hdy, a.hist, a.mask, W, nullptr, nullptr, nullptr, mean, rstd, nullptr, nullptr, gamma, beta, bias,
+                                                             O, 0.0f, lut_binarize, sums, nullptr);
     rc = launch_status();
     if (rc == BBCU_OK) {
         PassOneRecord r;
-        r.x = x; r.dy = dy; r.W = W; r.O = O; r.F = F; r.fs = fs;
+        r.x = x; r.dy = dy; r.W = W; r.mean = mean; r.rstd = rstd; r.O = O; r.F = F; r.fs = fs;
         std::lock_guard<std::mutex> g(g_record_mu);
         g_records[record_key(st)] = r;
     }
     return rc;
 }
 
-// Apply half: `sums` hold (dstd, dmeanx) over the frames of ALL ranks, total_frames is their number.  dx must be zero on entry;
+// Apply half: `sums` hold (dstd, dmeanx) over the frames of ALL ranks, total_frames is their number; writes all of dx's I rows,
 // dW receives this rank's share.
-int bit_backward_apply_by_table(bool x_is_fp32, const void *x, const float *dy, float *dx, const int *idx, const float *W, float *dW, const float *mean,
-                                const float *rstd, const double *sums, float *dmean_out, float *dvar_out, float gamma, float beta, float bias, int O,
-                                int F, long long xs, long long fs, long long total_frames, int lut_binarize, cudaStream_t st)
+int bit_backward_apply_by_table(const float *x, const float *dy, float *dx, const int *idx, const float *W, float *dW, const float *mean,
+                                const float *rstd, const double *sums, float *dmean_out, float *dvar_out, float gamma, float beta, float bias, int I,
+                                int O, int F, long long fs, long long total_frames, int lut_binarize, cudaStream_t st)
 {
-    if (x_is_fp32 && xs != fs) return BBCU_ERR_NO_MEMORY;
-    if (O == 0 || F == 0) return BBCU_OK;
+    bool have = false;
+    {
+        std::lock_guard<std::mutex> g(g_record_mu);
+        auto it = g_records.find(record_key(st));
+        have = it != g_records.end() && it->second.x == x && it->second.dy == dy && it->second.W == W && it->second.mean == mean && it->second.rstd == rstd &&
+               it->second.O == O && it->second.F == F && it->second.fs == fs;
+    }
     BitBwdArgs a;
-    Scratch s;
-    float *hdy = nullptr;
-    int rc = backward_pass_one(x_is_fp32, a, s, hdy, x, dy, idx, W, bias, O, F, xs, fs, lut_binarize, st, true);
-    if (rc) return rc;
-    const float rF = 1.0f / (float)total_frames;
-    const unsigned threads = kWarpsPerCta * 32;
-    k_bit_backward_finalize<true><<<a.groups, threads, 0, st>>>(hdy, s.hist, s.Y, dW, mean, rstd, dmean_out, dvar_out, gamma, beta, bias, O, rF, nullptr,
-                                                                sums);
+    if (!backward_setup(a, x, dy, idx, O, F, fs, fs, st)) return BBCU_ERR_NO_MEMORY;      // the same block as before (and it forgets the record)
+    if (!input_side(a, I, !have, st)) return BBCU_ERR_NO_MEMORY;
     BB200_CUDA(cudaPeekAtLastError());
-    a.dx = dx; a.mean = mean; a.rstd = rstd; a.dmean = dmean_out; a.dvar = dvar_out; a.gamma = gamma; a.beta = beta; a.rF = rF;
-    const long long blocks = (long long)a.groups * (((F + 31) / 32 + a.tile_words - 1) / a.tile_words);
-    if (x_is_fp32) k_bit_backward_frames<kBwdNormDx, true><<<(unsigned)blocks, threads, 0, st>>>(a);
-    else           k_bit_backward_frames<kBwdNormDx, false><<<(unsigned)blocks, threads, 0, st>>>(a);
-    return launch_status();
+    const unsigned blocks = (unsigned)((O + kWarpsPerCta - 1) / kWarpsPerCta), threads = kWarpsPerCta * 32;
+    if (!have) {
+        k_pattern_masks<<<blocks, threads, 0, st>>>(W, a.mask, mean, rstd, gamma, beta, bias, O, lut_binarize);
+        BB200_CUDA(cudaPeekAtLastError());
+        const int rc = launch_pattern_sums<false>(a, true, st);
+        if (rc) return rc;
+    }
+    a.dx = dx;
+    k_bit_backward_finalize<true><<<blocks, threads, 0, st>>>(a.hdy, a.hist, a.mask, W, a.etab, a.ntab, dW, mean, rstd, dmean_out, dvar_out, gamma, beta, bias,
+                                                             O, 1.0f / (float)total_frames, lut_binarize, nullptr, sums);
+    BB200_CUDA(cudaPeekAtLastError());
+    return launch_pattern_gather(a, true, st);
 }
 
 }   // namespace bb200

@@ -31,8 +31,9 @@ const DeviceInfo &device_info();
 // later calls on the same stream and is released by bbcu_LocalHeap_GarbageCollect().  Stream order
 // makes back-to-back calls on one stream safe; different streams get different blocks.  A stream has
 // kScratchSlots independent blocks, for callers whose scratch is alive at the same time (slot 0: batch-norm
-// sums, slot 1: per-node coefficient / pattern tables of the LUT operators, slot 2: the piece table of the bit Im2Col).
-constexpr int kScratchSlots = 3;
+// sums, slot 1: per-node coefficient / pattern tables of the LUT operators, slot 2: the piece table of the bit Im2Col,
+// slot 3: fp32 rows packed to bits).
+constexpr int kScratchSlots = 4;
 void *stream_scratch(cudaStream_t stream, size_t bytes, int slot = 0);
 
 // Pass 1 of the DifferentiableLut6 training forward (raw LUT values into y, fp64 sums per node); with may_allocate = false
@@ -58,17 +59,16 @@ int bit_fp32_forward_by_table(const int *x, float *y, const int *idx, const floa
                               int lut_binarize, cudaStream_t st);
 
 int bit_backward_by_table(bool bn, bool x_is_fp32, const void *x, const float *dy, float *dx, const int *idx, const float *W, float *dW,
-                          const float *mean, const float *rstd, float *dmean_out, float *dvar_out, float gamma, float beta, float bias, int O, int F,
-                          long long xs, long long fs, int lut_binarize, cudaStream_t st);
+                          const float *mean, const float *rstd, float *dmean_out, float *dvar_out, float gamma, float beta, float bias, int I, int O,
+                          int F, long long xs, long long fs, int lut_binarize, cudaStream_t st);
 
-// The batch-norm backward of a binary-mode layer in two halves for frame-sharded callers (the caller adds `sums` over the ranks in
-// between); both decline with BBCU_ERR_NO_MEMORY like the calls above.
-int bit_backward_stats_by_table(bool x_is_fp32, const void *x, const float *dy, const int *idx, const float *W, const float *mean, const float *rstd,
-                                double *sums, float gamma, float beta, float bias, int O, int F, long long xs, long long fs, int lut_binarize,
-                                cudaStream_t st);
-int bit_backward_apply_by_table(bool x_is_fp32, const void *x, const float *dy, float *dx, const int *idx, const float *W, float *dW, const float *mean,
-                                const float *rstd, const double *sums, float *dmean_out, float *dvar_out, float gamma, float beta, float bias, int O,
-                                int F, long long xs, long long fs, long long total_frames, int lut_binarize, cudaStream_t st);
+// The batch-norm backward of a binary-mode layer on fp32 frames in two halves for frame-sharded callers (the caller adds `sums` over the
+// ranks in between); both decline with BBCU_ERR_NO_MEMORY like the calls above.
+int bit_backward_stats_by_table(const float *x, const float *dy, const int *idx, const float *W, const float *mean, const float *rstd, double *sums,
+                                float gamma, float beta, float bias, int O, int F, long long fs, int lut_binarize, cudaStream_t st);
+int bit_backward_apply_by_table(const float *x, const float *dy, float *dx, const int *idx, const float *W, float *dW, const float *mean,
+                                const float *rstd, const double *sums, float *dmean_out, float *dvar_out, float gamma, float beta, float bias, int I,
+                                int O, int F, long long fs, long long total_frames, int lut_binarize, cudaStream_t st);
 
 int f32_binary_forward_by_table(int mode, const float *x, float *y, const int *idx, const float *W, float *mean, float *rstd, float *rmean,
                                 float *rvar, float gamma, float beta, float momentum, float bias, int O, int F, long long fs, int lut_binarize,

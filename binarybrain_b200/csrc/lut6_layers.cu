@@ -1194,25 +1194,25 @@ template <bool XBIT>
 static int backward_common(BwdArgs a, bool bn, long long total_frames, float *dmean_out, float *dvar_out, const double *ext_sums,
                            int I, cudaStream_t st, void *tmp = nullptr, size_t tmp_bytes = 0)
 {
+    if ((XBIT || a.binary) && ext_sums == nullptr && a.dys == a.dxs && total_frames == a.F && a.O > 0 && a.F > 0) {
+        // two-valued inputs (bit frames, or fp32 frames in binary mode): everything factors through the 6-bit input pattern of a
+        // frame (binary_mode.cu)
+        const int rc = bit_backward_by_table(bn, !XBIT, a.x, a.dy, a.dx, a.idx, a.W, a.dW, a.mean, a.rstd, dmean_out, dvar_out, a.gamma, a.beta,
+                                             a.bias, I, a.O, a.F, a.xs, a.dxs, a.lut_binarize, st);
+        if (rc != BBCU_ERR_NO_MEMORY) return rc;
+    }
+    if (!XBIT && a.binary && bn && ext_sums != nullptr && a.dys == a.dxs && a.xs == a.dxs && a.O > 0 && a.F > 0) {
+        // frame-sharded caller: the apply half of the same route, with the batch sums of all ranks
+        const int rc = bit_backward_apply_by_table(static_cast<const float *>(a.x), a.dy, a.dx, a.idx, a.W, a.dW, a.mean, a.rstd, ext_sums, dmean_out,
+                                                   dvar_out, a.gamma, a.beta, a.bias, I, a.O, a.F, a.dxs, total_frames, a.lut_binarize, st);
+        if (rc != BBCU_ERR_NO_MEMORY) return rc;
+    }
     // dx starts from zero (the reference's CPU path: dx_buf.FillZero(), DifferentiableLutN.h:1159)
     if (I > 0 && a.dxs > 0) {
         const int rc = zero_async(a.dx, sizeof(float) * (size_t)I * a.dxs, st);
         if (rc) return rc;
     }
     if (a.O == 0 || a.F == 0) return BBCU_OK;
-    if ((XBIT || a.binary) && ext_sums == nullptr && a.dys == a.dxs && total_frames == a.F) {
-        // two-valued inputs (bit frames, or fp32 frames in binary mode): everything factors through the 6-bit input pattern of a
-        // frame (binary_mode.cu)
-        const int rc = bit_backward_by_table(bn, !XBIT, a.x, a.dy, a.dx, a.idx, a.W, a.dW, a.mean, a.rstd, dmean_out, dvar_out, a.gamma, a.beta,
-                                             a.bias, a.O, a.F, a.xs, a.dxs, a.lut_binarize, st);
-        if (rc != BBCU_ERR_NO_MEMORY) return rc;
-    }
-    if ((XBIT || a.binary) && bn && ext_sums != nullptr && a.dys == a.dxs) {
-        // frame-sharded caller: the apply half of the same route, with the batch sums of all ranks
-        const int rc = bit_backward_apply_by_table(!XBIT, a.x, a.dy, a.dx, a.idx, a.W, a.dW, a.mean, a.rstd, ext_sums, dmean_out, dvar_out, a.gamma,
-                                                   a.beta, a.bias, a.O, a.F, a.xs, a.dxs, total_frames, a.lut_binarize, st);
-        if (rc != BBCU_ERR_NO_MEMORY) return rc;
-    }
     a.groups = (a.O + kWarpsPerCta - 1) / kWarpsPerCta;
     const long long rows = (long long)(I < 6LL * a.O ? I : 6LL * a.O);
     // Wide tiles: a warp reduces its 64 dW accumulators across lanes once per (node, tile), about 250 instructions, so the
@@ -1570,8 +1570,8 @@ extern "C" int bbcu_fp32_DifferentiableLut6_BackwardStats(const float *x, const 
     BB200_REQUIRE(frame_stride >= frame_size, BBCU_ERR_BAD_STRIDE);
     cudaStream_t st = as_stream(stream);
     if (binary_mode) {        // two-valued inputs: the sums follow from the per-pattern dy sums (binary_mode.cu)
-        rc = bit_backward_stats_by_table(true, x, dy, idx, W, mean, rstd, dev_sums, gamma, beta, unbinarize_bias, node_size, frame_size, frame_stride,
-                                         frame_stride, lut_binarize, st);
+        rc = bit_backward_stats_by_table(x, dy, idx, W, mean, rstd, dev_sums, gamma, beta, unbinarize_bias, node_size, frame_size, frame_stride,
+                                         lut_binarize, st);
         if (rc != BBCU_ERR_NO_MEMORY) return rc;
     }
     BB200_CUDA(cudaMemsetAsync(dev_sums, 0, sizeof(double) * 2 * (size_t)node_size, st));
