@@ -20,6 +20,7 @@
 #include <mutex>
 
 #include "common.cuh"
+#include "async_copy.cuh"
 #include "bit_transpose.cuh"
 #include "lut6_core.cuh"
 
@@ -28,6 +29,8 @@ namespace bb200 {
 namespace {
 
 enum { kTableRaw = 0, kTableNorm = 1, kTableNone = 2 };
+
+constexpr long long kSmallLayer = 1LL << 21;         // node-frames, see small_layer()
 
 // One warp per node: lane l evaluates patterns l and l + 32 as one packed pair (they differ in input 5 only).
 // MODE kTableRaw : B[p] = Y[p] > 0.5                                   (StochasticLut6, bit -> bit)
@@ -837,6 +840,269 @@ k_counts_to_sums(const float *__restrict__ Y, const uint32_t *__restrict__ hist,
     if (lane == 0) { sums[2 * (size_t)node] = s1; sums[2 * (size_t)node + 1] = s2; }
 }
 
+// --------------------------------------------------------------------------------------------- small layers: one launch per direction
+// Where a layer has up to a million or two node-frames, the kernels above take a few microseconds each and the launches between them take as
+// long again.  Here one CTA is one node with all of its frames (1 to 8 warps): tables, counts, statistics and output without
+// leaving the SM.  The rows are read twice (the second time from L1 or L2), counts and sums go through shared-memory atomics, and the
+// backward scatters dx with reductions in L2 (36 clocks per SM, warp and 32 frames; dx must be zero on entry) -- which is why larger layers
+// do not come here: see small_layer().
+
+struct SmallBinArgs {
+    const void *x;                      // fp32 rows, or bit rows
+    void *y;                            // forward: fp32 rows (0 / 1), or bit rows
+    const float *dy;
+    float *dx;
+    const int *idx;
+    const float *W;
+    float *dW;
+    const float *mean_in, *rstd_in;     // backward
+    float *mean, *rstd, *running_mean, *running_var, *dmean, *dvar;
+    float gamma, beta, momentum, bias;
+    int F, lut_binarize, vec;           // vec: fp32 rows start on 16-byte boundaries
+    long long xs, ys, fs;               // strides of x, y and dy / dx
+};
+
+// the patterns of frames f .. f+3 (one per byte) of a node with input rows `rows`
+template <bool XBIT>
+__device__ __forceinline__ uint32_t small_patterns(const SmallBinArgs &a, const size_t (&rows)[6], int f, int lane)
+{
+    if (XBIT) {
+        uint32_t w[6];
+#pragma unroll
+        for (int j = 0; j < 6; ++j) w[j] = f < a.F ? __ldg(static_cast<const uint32_t *>(a.x) + rows[j] + (f >> 5)) : 0u;
+        return pattern_bytes(w, lane);
+    }
+    uint32_t p4 = 0u;
+#pragma unroll
+    for (int j = 0; j < 6; ++j) {
+        const float4 v = load_frames(static_cast<const float *>(a.x) + rows[j], f, a.F, a.vec);
+        p4 |= ((v.x > 0.5f ? 1u : 0u) | (v.y > 0.5f ? 0x100u : 0u) | (v.z > 0.5f ? 0x10000u : 0u) | (v.w > 0.5f ? 0x1000000u : 0u)) << j;
+    }
+    return p4;
+}
+
+// Training forward of a batch-normalised layer on two-valued inputs: the arithmetic of k_pattern_values and k_dl6_bit_train_finalize.
+template <bool XBIT>
+__global__ void __launch_bounds__(kWarpsPerCta * 32)
+k_small_binary_forward(const SmallBinArgs a)
+{
+    __shared__ float4 s_tab[32];
+    __shared__ unsigned s_cnt[64];
+    __shared__ unsigned s_table[2];
+    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, node = blockIdx.x;
+    size_t rows[6];
+#pragma unroll
+    for (int j = 0; j < 6; ++j) rows[j] = (size_t)__ldg(a.idx + (size_t)node * 6 + j) * a.xs;
+    float y0 = 0.0f, y1 = 0.0f;
+    if (warp == 0) {
+        s_cnt[lane] = 0u;
+        s_cnt[lane + 32] = 0u;
+        stage_table_x2(s_tab, a.W, node, lane, a.lut_binarize);
+        f32x2 up[6][1], yp[1];
+#pragma unroll
+        for (int j = 0; j < 5; ++j) {
+            const float u = ((lane >> j) & 1) ? a.bias : -a.bias;
+            up[j][0] = pack2(u, u);
+        }
+        up[5][0] = pack2(-a.bias, a.bias);
+        lut6_forward_x2<1>(s_tab, up, yp);
+        unpack2(yp[0], y0, y1);                                              // patterns lane, lane + 32
+    }
+    __syncthreads();
+    const int step = 4 * (int)blockDim.x;
+    for (int f = 4 * (int)threadIdx.x; f < a.F; f += step) {
+        const uint32_t p4 = small_patterns<XBIT>(a, rows, f, lane);
+#pragma unroll
+        for (int i = 0; i < 4; ++i)
+            if (f + i < a.F) atomicAdd(&s_cnt[(p4 >> (8 * i)) & 63u], 1u);
+    }
+    __syncthreads();
+    if (warp == 0) {
+        const double h0 = (double)s_cnt[lane], h1 = (double)s_cnt[lane + 32];
+        const double s1 = warp_sum(h0 * (double)y0 + h1 * (double)y1);
+        const double s2 = warp_sum(h0 * ((double)y0 * (double)y0) + h1 * ((double)y1 * (double)y1));
+        const float rF   = 1.0f / (float)a.F;
+        const float mean = (float)s1 * rF;
+        const float var  = fmaxf(1.0e-5f, fmaf((float)s2, rF, -(mean * mean)));
+        const float rstd = 1.0f / sqrtf(var);
+        float lo = (y0 - mean) * rstd, hi = (y1 - mean) * rstd;
+        lo = lo * a.gamma + a.beta;
+        hi = hi * a.gamma + a.beta;
+        const unsigned w_lo = __ballot_sync(kFull, lo > 0.5f), w_hi = __ballot_sync(kFull, hi > 0.5f);
+        if (lane == 0) {
+            s_table[0] = w_lo;
+            s_table[1] = w_hi;
+            a.running_mean[node] = a.running_mean[node] * a.momentum + mean * (1.0f - a.momentum);
+            a.running_var[node]  = a.running_var[node]  * a.momentum + var  * (1.0f - a.momentum);
+            a.mean[node] = mean;
+            a.rstd[node] = rstd;
+        }
+    }
+    __syncthreads();
+    const uint32_t lo = s_table[0], hi = s_table[1];
+    for (int base = 4 * 32 * warp; base < a.F; base += step) {               // warp-uniform: bit outputs shuffle
+        const int f = base + 4 * lane;
+        const uint32_t p4 = small_patterns<XBIT>(a, rows, f, lane);
+        uint32_t bits = 0u;
+#pragma unroll
+        for (int i = 0; i < 4; ++i) {
+            const uint32_t p = p4 >> (8 * i);
+            bits |= f + i < a.F ? (((p & 32u ? hi : lo) >> (p & 31u)) & 1u) << i : 0u;
+        }
+        if (XBIT) {
+            bits <<= 4 * (lane & 7);
+#pragma unroll
+            for (int m = 1; m < 8; m <<= 1) bits |= __shfl_xor_sync(kFull, bits, m);
+            if ((lane & 7) == 0 && f < a.F) static_cast<uint32_t *>(a.y)[(size_t)node * a.ys + (f >> 5)] = bits;
+        } else {
+            float *out = static_cast<float *>(a.y) + (size_t)node * a.ys + f;
+            const float4 o = make_float4(bits & 1u ? 1.0f : 0.0f, bits & 2u ? 1.0f : 0.0f, bits & 4u ? 1.0f : 0.0f, bits & 8u ? 1.0f : 0.0f);
+            if (a.vec && f + 3 < a.F) {
+                *reinterpret_cast<float4 *>(out) = o;
+            } else {
+                if (f < a.F) out[0] = o.x;
+                if (f + 1 < a.F) out[1] = o.y;
+                if (f + 2 < a.F) out[2] = o.z;
+                if (f + 3 < a.F) out[3] = o.w;
+            }
+        }
+    }
+}
+
+// Backward (BN: batch-normalised layer): the arithmetic of k_bit_backward_finalize and k_pattern_gather.
+template <bool XBIT, bool BN>
+__global__ void __launch_bounds__(kWarpsPerCta * 32)
+k_small_binary_backward(const SmallBinArgs a)
+{
+    __shared__ float4 s_tab[16];
+    __shared__ float s_hdy[64], s_hg[64];
+    __shared__ unsigned s_cnt[64];
+    __shared__ float s_edge[6 * 64];
+    __shared__ float s_node[2];
+    __shared__ unsigned s_mask[2];
+    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, node = blockIdx.x;
+    size_t rows[6], out[6];
+#pragma unroll
+    for (int j = 0; j < 6; ++j) {
+        const size_t r = (size_t)__ldg(a.idx + (size_t)node * 6 + j);
+        rows[j] = r * a.xs;
+        out[j] = r * a.fs;
+    }
+    float y[2], d[2][6], mean = 0.0f, rstd = 0.0f;
+    bool m[2] = {false, false};
+    if (warp == 0) {
+        s_hdy[lane] = 0.0f;
+        s_hdy[lane + 32] = 0.0f;
+        s_cnt[lane] = 0u;
+        s_cnt[lane + 32] = 0u;
+        stage_table_halves(s_tab, a.W, node, lane, a.lut_binarize);
+        eval_pattern_pair(s_tab, lane, a.bias, y, d);
+        if (BN) {
+            mean = a.mean_in[node];
+            rstd = a.rstd_in[node];
+#pragma unroll
+            for (int h = 0; h < 2; ++h) {
+                const float t = ((y[h] - mean) * rstd) * a.gamma + a.beta;
+                m[h] = !(t <= 0.0f || t >= 1.0f);
+                const unsigned w = __ballot_sync(kFull, m[h]);
+                if (lane == 0) s_mask[h] = w;
+            }
+        } else {
+            store_edge_tables<false>(s_edge, lane, y, d, 0.0f, 0.0f);
+        }
+    }
+    __syncthreads();
+    const float *dyrow = a.dy + (size_t)node * a.fs;
+    const int step = 4 * (int)blockDim.x;
+    for (int f = 4 * (int)threadIdx.x; f < a.F; f += step) {
+        const uint32_t p4 = small_patterns<XBIT>(a, rows, f, lane);
+        const float4 g = load_frames(dyrow, f, a.F, a.vec);
+        const float gv[4] = {g.x, g.y, g.z, g.w};
+#pragma unroll
+        for (int i = 0; i < 4; ++i)
+            if (f + i < a.F) {
+                const uint32_t p = (p4 >> (8 * i)) & 63u;
+                atomicAdd(&s_hdy[p], gv[i]);
+                if (BN) atomicAdd(&s_cnt[p], 1u);
+            }
+    }
+    __syncthreads();
+    if (warp == 0) {
+        float hg[2] = {s_hdy[lane], s_hdy[lane + 32]};
+        if (BN) {
+            const float rF = 1.0f / (float)a.F, rstd2 = rstd * rstd;
+            const float dxn0 = m[0] ? a.gamma * hg[0] : 0.0f, dxn1 = m[1] ? a.gamma * hg[1] : 0.0f;
+            const double dstd = warp_sum(-((double)(dxn0 * (y[0] - mean) * rstd2) + (double)(dxn1 * (y[1] - mean) * rstd2)));
+            const double dmeanx = warp_sum(-((double)(dxn0 * rstd) + (double)(dxn1 * rstd)));
+            const float dvar = (float)dstd * rstd;
+            const float dmean = ((float)dmeanx - (mean * dvar)) * rF;
+            hg[0] = (dxn0 * rstd) + (dmean + (y[0] * dvar * rF)) * (float)s_cnt[lane];
+            hg[1] = (dxn1 * rstd) + (dmean + (y[1] * dvar * rF)) * (float)s_cnt[lane + 32];
+            store_edge_tables<true>(s_edge, lane, y, d, dmean, dvar * rF);
+            if (lane == 0) {
+                a.dvar[node] = dvar;
+                a.dmean[node] = dmean;
+                s_node[0] = a.gamma * rstd;
+                s_node[1] = a.bias * dvar * rF;
+            }
+        }
+        s_hg[lane] = hg[0];
+        s_hg[lane + 32] = hg[1];
+        __syncwarp();
+        const float2 gw = pattern_sums_to_table_grads(reinterpret_cast<const float2 *>(s_hg)[lane], lane, a.bias);
+        float *dst = a.dW + (size_t)node * 64 + 2 * lane;
+        dst[0] += gw.x;
+        dst[1] += gw.y;
+    }
+    __syncthreads();
+    float D[6], base[6];
+#pragma unroll
+    for (int j = 0; j < 6; ++j) {
+        D[j] = s_edge[64 * j + lane];
+        base[j] = BN && j == 5 ? s_edge[64 * j + 32 + lane] : 0.0f;          // input 5 is split off here, so one base table serves all six
+    }
+    const float gain = BN ? s_node[0] : 1.0f, slope = BN ? s_node[1] : 0.0f;
+    const uint32_t mask_lo = BN ? s_mask[0] : 0u, mask_hi = BN ? s_mask[1] : 0u;
+    for (int f_warp = 4 * 32 * warp; f_warp < a.F; f_warp += step) {
+        const int f = f_warp + 4 * lane;
+        const uint32_t p4 = small_patterns<XBIT>(a, rows, f, lane);
+        const float4 gq = load_frames(dyrow, f, a.F, a.vec);
+        float g[4] = {gq.x, gq.y, gq.z, gq.w};
+        const uint32_t q2[2] = {__byte_perm(p4, 0u, 0x4140) * 65u, __byte_perm(p4, 0u, 0x4342) * 65u};
+        if (BN) {
+#pragma unroll
+            for (int i = 0; i < 4; ++i) {
+                const uint32_t q = q2[i >> 1] >> (16 * (i & 1));
+                const bool upper = (q & 32u) != 0u;
+                const float add = fmaf(upper ? slope : -slope, __shfl_sync(kFull, D[5], q), __shfl_sync(kFull, base[5], q));
+                const bool pass = ((upper ? mask_hi : mask_lo) >> (q & 31u)) & 1u;
+                g[i] = f + i < a.F ? fmaf(pass ? g[i] : 0.0f, gain, add) : 0.0f;
+            }
+        }
+#pragma unroll
+        for (int j = 0; j < 6; ++j) {
+            float v[4];
+#pragma unroll
+            for (int i = 0; i < 4; ++i) v[i] = g[i] * __shfl_sync(kFull, D[j], q2[i >> 1] >> (16 * (i & 1) + j + 1));
+            float *dst = a.dx + out[j] + f;
+            if (a.vec) {
+                if (f < a.F) red_add_v4(dst, v[0], v[1], v[2], v[3]);        // rows are padded to whole quads; frames from F on add 0
+            } else {
+#pragma unroll
+                for (int i = 0; i < 4; ++i)
+                    if (f + i < a.F) atomicAdd(dst + i, v[i]);
+            }
+        }
+    }
+}
+
+// Where the one-launch kernels pay.  Measured on B200, forward + backward of a layer on fp32 frames against the general kernels: 360
+// nodes x 100 frames 17 / 55 us, 1024 x 1024 41 / 66, 2048 x 1000 (2^21 node-frames) 70 / 86, 8192 x 256 71 / 120, but 4096 x 1000
+// 129 / 115; and however few the nodes, a CTA works through its frames alone: 64 x 16384 125 / 64.
+bool small_layer(int O, int F) { return (long long)O * F <= kSmallLayer && F <= 4096; }
+
+unsigned small_threads(int F) { return 32u * (unsigned)(F > 128 * kWarpsPerCta ? kWarpsPerCta : (F + 127) / 128); }
+
 struct Scratch {
     float    *Y;        // [O][64]
     uint32_t *hist;     // [O][64]
@@ -912,6 +1178,13 @@ int dl6_bit_forward_training_by_table(const int *x, int *y, const int *idx, cons
                                       cudaStream_t st)
 {
     if (O == 0 || F == 0) return BBCU_OK;
+    if (small_layer(O, F)) {
+        SmallBinArgs a = {};
+        a.x = x; a.y = y; a.idx = idx; a.W = W; a.mean = mean; a.rstd = rstd; a.running_mean = rmean; a.running_var = rvar;
+        a.gamma = gamma; a.beta = beta; a.momentum = momentum; a.bias = bias; a.F = F; a.lut_binarize = lut_binarize; a.xs = stride; a.ys = stride;
+        k_small_binary_forward<true><<<O, small_threads(F), 0, st>>>(a);
+        return launch_status();
+    }
     Scratch s;
     if (!carve(s, O, st)) return BBCU_ERR_NO_MEMORY;
     const int groups = (O + kWarpsPerCta - 1) / kWarpsPerCta;
@@ -961,7 +1234,15 @@ int f32_binary_forward_by_table(int mode, const float *x, float *y, const int *i
                                 cudaStream_t st)
 {
     if (O == 0 || F == 0) return BBCU_OK;
-    if (((reinterpret_cast<uintptr_t>(x) | reinterpret_cast<uintptr_t>(y)) & 15) != 0 || (fs % 4) != 0) return BBCU_ERR_NO_MEMORY;
+    const bool aligned = ((reinterpret_cast<uintptr_t>(x) | reinterpret_cast<uintptr_t>(y)) & 15) == 0 && fs % 4 == 0;
+    if (mode == 2 && small_layer(O, F)) {
+        SmallBinArgs a = {};
+        a.x = x; a.y = y; a.idx = idx; a.W = W; a.mean = mean; a.rstd = rstd; a.running_mean = rmean; a.running_var = rvar;
+        a.gamma = gamma; a.beta = beta; a.momentum = momentum; a.bias = bias; a.F = F; a.lut_binarize = lut_binarize; a.xs = fs; a.ys = fs; a.vec = aligned;
+        k_small_binary_forward<false><<<O, small_threads(F), 0, st>>>(a);
+        return launch_status();
+    }
+    if (!aligned) return BBCU_ERR_NO_MEMORY;
     const size_t pat_bytes = mode == 2 ? (size_t)O * (size_t)fs : 0;
     if (pat_bytes > ((size_t)1 << 30)) return BBCU_ERR_NO_MEMORY;
     Scratch s;
@@ -1118,6 +1399,17 @@ int bit_backward_by_table(bool bn, bool x_is_fp32, const void *x, const float *d
                           int F, long long xs, long long fs, int lut_binarize, cudaStream_t st)
 {
     if (x_is_fp32 && xs != fs) return BBCU_ERR_NO_MEMORY;          // fp32 x shares the stride of dy / dx in every caller; otherwise decline
+    if (small_layer(O, F)) {
+        SmallBinArgs a = {};
+        a.x = x; a.dy = dy; a.dx = dx; a.idx = idx; a.W = W; a.dW = dW; a.mean_in = mean; a.rstd_in = rstd; a.dmean = dmean_out; a.dvar = dvar_out;
+        a.gamma = gamma; a.beta = beta; a.bias = bias; a.F = F; a.lut_binarize = lut_binarize; a.xs = xs; a.fs = fs;
+        a.vec = ((reinterpret_cast<uintptr_t>(dy) | reinterpret_cast<uintptr_t>(dx) | (x_is_fp32 ? reinterpret_cast<uintptr_t>(x) : 0)) & 15) == 0 && fs % 4 == 0;
+        BB200_CUDA(cudaMemsetAsync(dx, 0, sizeof(float) * (size_t)I * (size_t)fs, st));
+        auto kern = x_is_fp32 ? (bn ? k_small_binary_backward<false, true> : k_small_binary_backward<false, false>)
+                              : (bn ? k_small_binary_backward<true, true> : k_small_binary_backward<true, false>);
+        kern<<<O, small_threads(F), 0, st>>>(a);
+        return launch_status();
+    }
     BitBwdArgs a;
     if (!backward_setup(a, x, dy, idx, O, F, xs, fs, st) || !input_side(a, I, x_is_fp32, st)) return BBCU_ERR_NO_MEMORY;
     BB200_CUDA(cudaPeekAtLastError());

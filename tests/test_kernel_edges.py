@@ -3,7 +3,8 @@ the CPU oracle."""
 import numpy as np
 import pytest
 
-from oracle import port
+import test_gpu_parity as parity
+from oracle import port, pack_bits, unpack_bits
 
 pytestmark = pytest.mark.gpu
 
@@ -52,3 +53,37 @@ def test_binary_lut6_host_chunks(ops, n_in, n_out, words, spare):
     live = np.full(words, 0xffffffff, np.uint32)
     live[-1] >>= spare
     assert ((y.numpy().view(np.uint32)[:, :words] ^ want[:, :words]) & live == 0).all()
+
+
+# two-valued inputs.  One launch per direction (up to 2^21 node-frames and 4096 frames): one warp, whole warps, a ragged last one, eight
+# warps and several rounds of them.  General kernels: many consumers per input row (shared between warps) and rows without any, rows
+# that are not 16-byte aligned, tiles of 512 frames with every kind of remainder, several tiles per node.
+@pytest.mark.parametrize("I,O,F,stride", [(6, 1, 1, None), (9, 5, 3, 4), (40, 64, 127, None), (33, 70, 128, None), (50, 31, 129, 131), (30, 40, 1153, None),
+                                          (48, 33, 4096, None),
+                                          (40, 64, 4100, None), (7, 48, 5000, None), (3000, 400, 5377, 5380), (20, 30, 4609, 4611), (500, 1100, 2113, None)])
+def test_two_valued_layers_edges(ops, I, O, F, stride):
+    import torch
+    from gpu_util import dev, dev_bits, dev_fp32, err, host_bits, host_fp32, wiring
+    rng = np.random.default_rng(I + O + F)
+    idx = wiring(rng, I, O)
+    W = np.clip(rng.normal(0.5, 0.25, (O, 64)), 0, 1).astype(np.float32)
+    x, dy = rng.random((I, F), dtype=np.float32), rng.standard_normal((O, F), dtype=np.float32)
+    rm, rv = rng.random(O, dtype=np.float32), rng.random(O, dtype=np.float32) + 0.5
+    parity._dl6_fp32_check(ops, x, idx, W, dy, rm, rv, dict(binary=1, lut_binarize=0), stride)
+    xb = pack_bits(x > 0.5)
+    for src, bits in ((dev_fp32(x, stride), False), (dev_bits(xb, F), True)):
+        dW = torch.zeros((O, 64), device="cuda")
+        dx = ops.stochastic_lut6_backward(src, dev_fp32(dy, stride), dev(idx), dev(W), dW, I, F, binary=True)
+        dx_w, dW_w = port.sl6_backward(x, dy, idx, W, I, binary=1)
+        assert err(host_fp32(dx, F), dx_w) <= parity.TOL and err(dW.cpu().numpy(), dW_w) <= parity.TOL
+        assert not dx[:, F:].any()                                                    # the padding of dx stays clear
+    p = port.dl6_forward_train(xb, idx, W, rm, rv, frames=F)
+    amp = max(1.0, 0.3 * float(p["rstd"].max()))
+    y, mean, rstd = ops.differentiable_lut6_forward_training(dev_bits(xb, F), dev(idx), dev(W), dev(rm.copy()), dev(rv.copy()), F)
+    bad = unpack_bits(host_bits(y, F), F) != unpack_bits(p["y_bits"], F)
+    assert (np.abs(p["y_pre"][bad] - 0.5) < 1e-4 * amp).all() and err(mean.cpu().numpy(), p["mean"]) <= parity.TOL
+    dy = np.where(parity._edges(p["y_pre"], amp), np.float32(0), dy).astype(np.float32)
+    dx_w, dW_w = port.dl6_backward(xb, dy, idx, W, p["mean"], p["rstd"], I)
+    dW = torch.zeros((O, 64), device="cuda")
+    dx = ops.differentiable_lut6_backward(dev_bits(xb, F), dev_fp32(dy, stride), dev(idx), dev(W), dW, dev(p["mean"]), dev(p["rstd"]), I, F)
+    assert err(host_fp32(dx, F), dx_w) <= parity.BN_GRAD_FACTOR * parity.TOL * amp and err(dW.cpu().numpy(), dW_w) <= parity.BN_GRAD_FACTOR * parity.TOL * amp
