@@ -56,6 +56,8 @@ SIGNATURES = {
     "bbcu_fp32_Vector_clamp": (_i, [_vp, _vp, _f, _f, _i, _vp]),
     "bbcu_fp32_Vector_set": (_i, [_vp, _f, _i, _vp]),
     "bbcu_fp32_OptimizerAdam": (_i, [_i] + [_vp] * 5 + [_f] * 3 + [_vp]),
+    "bbcu_fp32_OptimizerAdamUpdate": (_i, [_i] + [_vp] * 5 + [_f] * 3 + [_vp]),
+    "bbcu_fp32_LossSoftmaxCrossEntropyMean": (_i, [_vp] * 4 + [_i] * 4 + [_vp]),
     "bbcu_fp32_LossSoftmaxCrossEntropy": (_i, [_vp] * 4 + [_f] + [_i] * 4 + [_vp]),
     "bbcu_fp32_LossMeanSquaredError": (_i, [_vp] * 4 + [_i] * 4 + [_f, C.c_double, _vp]),
     "bbcu_fp32_Reduce_Forward": (_i, [_vp] * 2 + [_i] * 5 + [_vp]),
@@ -80,6 +82,7 @@ SIGNATURES = {
     "bbcu_fp32_DifferentiableLut6_ForwardTraining_NoAlloc": (_i, [_vp] * 8 + [_f] * 4 + [_i] * 5 + [_vp]),
     "bbcu_fp32_DifferentiableLut6_ForwardTraining_NoAlloc_MaxNodes": (_i, []),
     "bbcu_fp32_DifferentiableLut6_BackwardStatsFromOutput": (_i, [_vp] * 4 + [_f] * 2 + [_i] * 4 + [_vp]),
+    "bbcu_fp32_DifferentiableLut6_BackwardFromOutput": (_i, [_vp] * 11 + [_f] * 2 + [_i] * 5 + [_vp]),
     "bbcu_fp32_DifferentiableLut6_BackwardApply": (_i, [_vp] * 11 + [_f] * 3 + [_i] * 4 + [_ll, _i, _i, _vp]),
 }
 

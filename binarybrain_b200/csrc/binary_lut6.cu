@@ -512,14 +512,7 @@ extern "C" int bbcu_bit_BinaryLut6_Forward(const int *x, int *y, const int *idx,
     BB200_REQUIRE(blocks < (1LL << 31), BBCU_ERR_TOO_LARGE);
     if (vec) {
         // persistent pipeline: two CTAs per SM, each walking (tile, node group) items
-        static bool attr_done[64] = {};              // the opt-in to > 48 KB of dynamic shared memory is per device
-        const int dev_id = bbcu_GetDevice();
-        bool attr_ok = dev_id >= 0 && dev_id < 64 && attr_done[dev_id];
-        if (!attr_ok && dev_id >= 0 && dev_id < 64) {
-            attr_ok = cudaFuncSetAttribute(k_binary_lut6_pipe, cudaFuncAttributeMaxDynamicSharedMemorySize, kPipeSmem) == cudaSuccess;
-            attr_done[dev_id] = attr_ok;
-            if (!attr_ok) cudaGetLastError();
-        }
+        const bool attr_ok = allow_big_smem(k_binary_lut6_pipe, kPipeSmem);
         int *fault = fault_word();
         if (attr_ok && fault != nullptr) {
             const long long n_items = (long long)((a.nwords + kPipeWords - 1) / kPipeWords) * a.groups;
@@ -555,7 +548,7 @@ extern "C" int bbcu_bit_BinaryLut6_Forward_Lop3Immediate(const int *x, int *y, c
     a.nwords = ((frame_size + 31) / 32 + 3) & ~3;
     a.groups = (node_size + kBlWarps - 1) / kBlWarps;
     a.Tw = kImmWords;
-    BB200_CUDA(cudaFuncSetAttribute(k_binary_lut6_imm, cudaFuncAttributeMaxDynamicSharedMemorySize, kImmSmem));
+    BB200_REQUIRE(allow_big_smem(k_binary_lut6_imm, kImmSmem), BBCU_ERR_TOO_LARGE);
     const int n_tiles = (a.nwords + kImmWords - 1) / kImmWords;
     const long long n_items = (long long)n_tiles * a.groups;
     BB200_REQUIRE(n_items < (1LL << 31) - 4096, BBCU_ERR_TOO_LARGE);

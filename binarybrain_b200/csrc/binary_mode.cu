@@ -1366,7 +1366,7 @@ int launch_pattern_sums(BitBwdArgs a, bool bn, cudaStream_t st)
     }
     const int smem = kPsWarps * 64 * 32 * (int)(bn ? sizeof(PatternSlot<true>) : sizeof(PatternSlot<false>));
     auto kern = bn ? k_pattern_sums<XF32, true> : k_pattern_sums<XF32, false>;
-    BB200_CUDA(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, smem));
+    BB200_REQUIRE(allow_big_smem(kern, smem), BBCU_ERR_NO_MEMORY);
     kern<<<(unsigned)blocks, kPsWarps * 32, smem, st>>>(a);
     return launch_status();
 }

@@ -74,8 +74,29 @@ int f32_binary_forward_by_table(int mode, const float *x, float *y, const int *i
                                 float *rvar, float gamma, float beta, float momentum, float bias, int O, int F, long long fs, int lut_binarize,
                                 cudaStream_t st);
 
+// Small layers in probability mode, one launch per direction (lut6_small.cu).  All rows share the frame stride fs; vec: x, y, dy and dx rows
+// start on 16-byte boundaries.  small_forward(): mode 0 y = clip(LUT), 1 training with batch norm, 2 inference (mean_in, and the running
+// variance in rstd_in); small_backward() clears dx and adds to dW.
+struct SmallLayerArgs {
+    const float *x, *dy, *W, *mean_in, *rstd_in;
+    const int *idx;
+    float *y, *dx, *dW, *mean, *rstd, *running_mean, *running_var, *dmean, *dvar;
+    float gamma, beta, momentum;
+    int F, lut_binarize, vec;
+    long long fs;
+};
+constexpr long long kSmallProbability = 1LL << 21;       // node-frames, see small_probability_layer()
+bool small_probability_layer(int O, int F);
+int small_forward(int mode, const SmallLayerArgs &a, int O, cudaStream_t st);
+int small_backward(bool bn, const SmallLayerArgs &a, int I, int O, cudaStream_t st);
+
 // Per-device int in the library's device image (zero until a kernel records a fault); nothing is allocated for it.
 int *fault_word();
+
+// Opt-in to more than 48 KB of dynamic shared memory, once per kernel and device (the attribute stays set, the call costs about as much
+// as a small launch).  False when it is refused.
+bool allow_big_smem_once(const void *kernel, int bytes);
+template <typename K> inline bool allow_big_smem(K *kernel, int bytes) { return allow_big_smem_once(reinterpret_cast<const void *>(kernel), bytes); }
 
 inline cudaStream_t as_stream(bbcu_stream_t s) { return reinterpret_cast<cudaStream_t>(s); }
 

@@ -10,12 +10,27 @@
 
 namespace bb200 {
 
-// one thread per (frame, pixel): softmax over the ch_size channel rows node = ch * pix_size + pix
-__global__ void k_softmax_cross_entropy(const float *__restrict__ y, const float *__restrict__ t, float *dy, double *loss_buf, float t_sum,
-                                        int pix_size, int ch_size, int F, long long stride)
+// The mean loss over frames in one go: work[0] = sum of all targets, work[1] = sum of the per-frame losses, *loss = -work[1] / work[0].
+// Up to kOneCta target values a single CTA does everything in one launch (ten classes x 512 frames: a read of the target sum by the
+// host, three reductions and a kernel took 58 us of host time); above, the sums go through `work`, which the caller clears.
+constexpr int kOneCta = 1 << 15;
+
+__device__ __forceinline__ double cta_sum(double v, double *red)
 {
-    const int f = blockIdx.x * blockDim.x + threadIdx.x;
-    if (f >= F) return;
+#pragma unroll
+    for (int m = 16; m > 0; m >>= 1) v += __shfl_xor_sync(0xffffffffu, v, m);
+    __syncthreads();
+    if ((threadIdx.x & 31) == 0) red[threadIdx.x >> 5] = v;
+    __syncthreads();
+    v = 0.0;
+    for (unsigned w = 0; w < blockDim.x >> 5; ++w) v += red[w];
+    return v;
+}
+
+// one frame: softmax over the channel rows of every pixel, dy, and the frame's loss
+__device__ __forceinline__ double softmax_frame(const float *__restrict__ y, const float *__restrict__ t, float *dy, float t_sum, int pix_size, int ch_size,
+                                                int f, long long stride)
+{
     const float eps = 1.0e-7f;
     double loss = 0.0;
     for (int pix = 0; pix < pix_size; ++pix) {
@@ -36,8 +51,54 @@ __global__ void k_softmax_cross_entropy(const float *__restrict__ y, const float
             dy[o] = (t_max * softmax - tv) / t_sum;
         }
     }
-    loss_buf[f] = loss;
+    return loss;
 }
+
+__global__ void k_softmax_cross_entropy(const float *__restrict__ y, const float *__restrict__ t, float *dy, double *loss_buf, float t_sum,
+                                        int pix_size, int ch_size, int F, long long stride)
+{
+    const int f = blockIdx.x * blockDim.x + threadIdx.x;
+    if (f < F) loss_buf[f] = softmax_frame(y, t, dy, t_sum, pix_size, ch_size, f, stride);
+}
+
+__global__ void __launch_bounds__(1024)
+k_softmax_cross_entropy_one(const float *__restrict__ y, const float *__restrict__ t, float *dy, double *loss, int pix_size, int ch_size, int F,
+                            long long stride)
+{
+    __shared__ double red[32];
+    double s = 0.0;
+    for (int row = threadIdx.x / 128; row < pix_size * ch_size; row += blockDim.x / 128)
+        for (int f = threadIdx.x % 128; f < F; f += 128) s += (double)t[(size_t)row * stride + f];
+    const double t_total = cta_sum(s, red);
+    double l = 0.0;
+    for (int f = threadIdx.x; f < F; f += blockDim.x) l += softmax_frame(y, t, dy, (float)t_total, pix_size, ch_size, f, stride);
+    l = cta_sum(l, red);
+    if (threadIdx.x == 0) *loss = -l / t_total;
+}
+
+__global__ void __launch_bounds__(256)
+k_target_sum(const float *__restrict__ t, double *work, int rows, int F, long long stride)
+{
+    __shared__ double red[8];
+    double s = 0.0;
+    for (int row = blockIdx.y; row < rows; row += gridDim.y)
+        for (int f = blockIdx.x * blockDim.x + threadIdx.x; f < F; f += gridDim.x * blockDim.x) s += (double)t[(size_t)row * stride + f];
+    s = cta_sum(s, red);
+    if (threadIdx.x == 0) atomicAdd(work, s);
+}
+
+__global__ void __launch_bounds__(128)
+k_softmax_cross_entropy_sums(const float *__restrict__ y, const float *__restrict__ t, float *dy, double *work, int pix_size, int ch_size, int F,
+                             long long stride)
+{
+    __shared__ double red[4];
+    const int f = blockIdx.x * blockDim.x + threadIdx.x;
+    double l = f < F ? softmax_frame(y, t, dy, (float)work[0], pix_size, ch_size, f, stride) : 0.0;
+    l = cta_sum(l, red);
+    if (threadIdx.x == 0) atomicAdd(work + 1, l);
+}
+
+__global__ void k_mean_loss(const double *__restrict__ work, double *loss) { *loss = -work[1] / work[0]; }
 
 // dy = grad_reduction * (y - t);  loss_buf[block % loss_buf_size] += sum (y - t)^2 * loss_reduction  (NaN terms skipped)
 __global__ void __launch_bounds__(256)
@@ -99,6 +160,31 @@ extern "C" int bbcu_fp32_LossSoftmaxCrossEntropy(const float *y, const float *t,
     if (frame_size == 0) return BBCU_OK;
     k_softmax_cross_entropy<<<(frame_size + 127) / 128, 128, 0, as_stream(stream)>>>(y, t, dy, loss_buf, t_sum, pix_size, ch_size, frame_size,
                                                                                    frame_stride);
+    return launch_status();
+}
+
+extern "C" int bbcu_fp32_LossSoftmaxCrossEntropyMean(const float *y, const float *t, float *dy, double *loss, int pix_size, int ch_size, int frame_size,
+                                                     int frame_stride, bbcu_stream_t stream)
+{
+    BB200_REQUIRE_PTR(y); BB200_REQUIRE_PTR(t); BB200_REQUIRE_PTR(dy); BB200_REQUIRE_PTR(loss);
+    BB200_REQUIRE(pix_size > 0 && ch_size > 0 && frame_size >= 0, BBCU_ERR_BAD_SIZE);
+    BB200_REQUIRE(frame_stride >= frame_size, BBCU_ERR_BAD_STRIDE);
+    cudaStream_t st = as_stream(stream);
+    const long long rows = (long long)pix_size * ch_size;
+    if (rows * frame_size <= kOneCta) {
+        k_softmax_cross_entropy_one<<<1, 1024, 0, st>>>(y, t, dy, loss, pix_size, ch_size, frame_size, frame_stride);
+        return launch_status();
+    }
+    double *work = static_cast<double *>(stream_scratch(st, 2 * sizeof(double)));
+    BB200_REQUIRE(work != nullptr, BBCU_ERR_NO_MEMORY);
+    BB200_REQUIRE(rows < (1LL << 31), BBCU_ERR_TOO_LARGE);
+    BB200_CUDA(cudaMemsetAsync(work, 0, 2 * sizeof(double), st));
+    const unsigned bx = (unsigned)((frame_size + 2047) / 2048);
+    k_target_sum<<<dim3(bx, (unsigned)(rows < 64 ? rows : 64)), 256, 0, st>>>(t, work, (int)rows, frame_size, frame_stride);
+    BB200_CUDA(cudaPeekAtLastError());
+    k_softmax_cross_entropy_sums<<<(frame_size + 127) / 128, 128, 0, st>>>(y, t, dy, work, pix_size, ch_size, frame_size, frame_stride);
+    BB200_CUDA(cudaPeekAtLastError());
+    k_mean_loss<<<1, 1, 0, st>>>(work, loss);
     return launch_status();
 }
 

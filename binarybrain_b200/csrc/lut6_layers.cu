@@ -1025,14 +1025,6 @@ static int check_common(const void *x, const void *y, const int *idx, const floa
     return BBCU_OK;
 }
 
-// opt-in to more than 48 KB of dynamic shared memory (per kernel and device; the call is a host-side attribute write)
-template <typename K>
-static bool allow_big_smem(K kernel, int bytes)
-{
-    if (cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, bytes) != cudaSuccess) { cudaGetLastError(); return false; }
-    return true;
-}
-
 template <bool XBIT, int PHASE, bool YBIT>
 static int launch_forward(FwdArgs a, int max_tile, cudaStream_t st)
 {
@@ -1190,6 +1182,16 @@ static int zero_async(void *ptr, size_t bytes, cudaStream_t st)
     return BBCU_OK;
 }
 
+static SmallLayerArgs small_args(const float *x, const int *idx, const float *W, int F, long long fs, int lut_binarize, const void *p, const void *q,
+                                 const void *r)
+{
+    SmallLayerArgs a = {};
+    a.x = x; a.idx = idx; a.W = W; a.F = F; a.fs = fs; a.lut_binarize = lut_binarize;
+    a.vec = fs % 4 == 0 && ((reinterpret_cast<uintptr_t>(x) | reinterpret_cast<uintptr_t>(p) | reinterpret_cast<uintptr_t>(q) |
+                             reinterpret_cast<uintptr_t>(r)) & 15) == 0;
+    return a;
+}
+
 template <bool XBIT>
 static int backward_common(BwdArgs a, bool bn, long long total_frames, float *dmean_out, float *dvar_out, const double *ext_sums,
                            int I, cudaStream_t st, void *tmp = nullptr, size_t tmp_bytes = 0)
@@ -1206,6 +1208,12 @@ static int backward_common(BwdArgs a, bool bn, long long total_frames, float *dm
         const int rc = bit_backward_apply_by_table(static_cast<const float *>(a.x), a.dy, a.dx, a.idx, a.W, a.dW, a.mean, a.rstd, ext_sums, dmean_out,
                                                    dvar_out, a.gamma, a.beta, a.bias, I, a.O, a.F, a.dxs, total_frames, a.lut_binarize, st);
         if (rc != BBCU_ERR_NO_MEMORY) return rc;
+    }
+    if (!XBIT && !a.binary && ext_sums == nullptr && a.xs == a.dxs && a.dys == a.dxs && total_frames == a.F && small_probability_layer(a.O, a.F)) {
+        SmallLayerArgs s = small_args(static_cast<const float *>(a.x), a.idx, a.W, a.F, a.dxs, a.lut_binarize, a.dy, a.dx, nullptr);
+        s.dy = a.dy; s.dx = a.dx; s.dW = a.dW; s.mean_in = a.mean; s.rstd_in = a.rstd; s.dmean = dmean_out; s.dvar = dvar_out;
+        s.gamma = a.gamma; s.beta = a.beta;
+        return small_backward(bn, s, I, a.O, st);
     }
     // dx starts from zero (the reference's CPU path: dx_buf.FillZero(), DifferentiableLutN.h:1159)
     if (I > 0 && a.dxs > 0) {
@@ -1280,6 +1288,11 @@ extern "C" int bbcu_fp32_StochasticLut6_Forward(const float *x, float *y, const 
         rc = f32_binary_forward_by_table(0, x, y, idx, W, nullptr, nullptr, nullptr, nullptr, 0.0f, 0.0f, 0.0f, unbinarize_bias, node_size, frame_size,
                                          frame_stride, lut_binarize, as_stream(stream));
         if (rc != BBCU_ERR_NO_MEMORY) return rc;
+    }
+    if (!input_binary && small_probability_layer(node_size, frame_size)) {
+        SmallLayerArgs a = small_args(x, idx, W, frame_size, frame_stride, lut_binarize, y, nullptr, nullptr);
+        a.y = y;
+        return small_forward(0, a, node_size, as_stream(stream));
     }
     return forward_plain<false>(x, y, nullptr, idx, W, node_size, frame_size, frame_stride, frame_stride, input_binary, lut_binarize,
                                 unbinarize_bias, as_stream(stream));
@@ -1427,6 +1440,13 @@ extern "C" int bbcu_fp32_DifferentiableLut6_ForwardTraining(const float *x, floa
         rcb = f32_binary_forward_by_table(2, x, y, idx, W, mean, rstd, rmean, rvar, gamma, beta, momentum, unbinarize_bias, node_size, frame_size,
                                           frame_stride, lut_binarize, st);
         if (rcb != BBCU_ERR_NO_MEMORY) return rcb;
+    } else if (small_probability_layer(node_size, frame_size)) {
+        const int rcs = check_common(x, y, idx, W, node_size, frame_size, frame_stride);
+        if (rcs) return rcs;
+        BB200_REQUIRE(frame_stride >= frame_size, BBCU_ERR_BAD_STRIDE);
+        SmallLayerArgs a = small_args(x, idx, W, frame_size, frame_stride, lut_binarize, y, nullptr, nullptr);
+        a.y = y; a.mean = mean; a.rstd = rstd; a.running_mean = rmean; a.running_var = rvar; a.gamma = gamma; a.beta = beta; a.momentum = momentum;
+        return small_forward(1, a, node_size, st);
     }
     double *sums = static_cast<double *>(stream_scratch(st, sizeof(double) * 2 * (size_t)(node_size > 0 ? node_size : 0)));
     BB200_REQUIRE(sums != nullptr, BBCU_ERR_NO_MEMORY);
@@ -1482,6 +1502,10 @@ extern "C" int bbcu_fp32_DifferentiableLut6_ForwardInference(const float *x, flo
         rc = f32_binary_forward_by_table(1, x, y, idx, W, nullptr, nullptr, const_cast<float *>(rmean), const_cast<float *>(rvar), gamma, beta, 0.0f,
                                          unbinarize_bias, node_size, frame_size, frame_stride, lut_binarize, as_stream(stream));
         if (rc != BBCU_ERR_NO_MEMORY) return rc;
+    } else if (small_probability_layer(node_size, frame_size)) {
+        SmallLayerArgs sa = small_args(x, idx, W, frame_size, frame_stride, lut_binarize, y, nullptr, nullptr);
+        sa.y = y; sa.mean_in = rmean; sa.rstd_in = rvar; sa.gamma = gamma; sa.beta = beta;
+        return small_forward(2, sa, node_size, as_stream(stream));
     }
     FwdArgs a = {};
     a.x = x; a.y = y; a.idx = idx; a.W = W; a.mean = rmean; a.rstd = rvar; a.stat_is_var = 1; a.bias = unbinarize_bias;
@@ -1620,4 +1644,24 @@ extern "C" int bbcu_fp32_DifferentiableLut6_BackwardApply(const float *x, const 
                                frame_stride, frame_stride, lut_binarize, binary_mode);
     if (rc) return rc;
     return backward_common<false>(a, true, total_frame_size, dmean_tmp, dvar_tmp, dev_sums, input_node_size, as_stream(stream));
+}
+
+extern "C" int bbcu_fp32_DifferentiableLut6_BackwardFromOutput(const float *x, const float *y, const float *dy, float *dx, const int *idx, const float *W,
+                                                               float *dW, const float *mean, const float *rstd, float *dmean_tmp, float *dvar_tmp,
+                                                               float gamma, float beta, int input_node_size, int output_node_size, int frame_size,
+                                                               int frame_stride, int lut_binarize, bbcu_stream_t stream)
+{
+    BB200_REQUIRE_PTR(y); BB200_REQUIRE_PTR(dmean_tmp); BB200_REQUIRE_PTR(dvar_tmp);
+    BwdArgs a;
+    int rc = dl6_backward_args(a, x, dy, dx, idx, W, dW, mean, rstd, gamma, beta, 0.0f, input_node_size, output_node_size, frame_size, frame_stride,
+                               frame_stride, lut_binarize, 0);
+    if (rc) return rc;
+    cudaStream_t st = as_stream(stream);
+    if (small_probability_layer(output_node_size, frame_size))        // one launch, which evaluates the LUT anyway
+        return backward_common<false>(a, true, frame_size, dmean_tmp, dvar_tmp, nullptr, input_node_size, st);
+    double *sums = static_cast<double *>(stream_scratch(st, sizeof(double) * 2 * (size_t)output_node_size));
+    BB200_REQUIRE(sums != nullptr, BBCU_ERR_NO_MEMORY);
+    rc = bbcu_fp32_DifferentiableLut6_BackwardStatsFromOutput(y, dy, rstd, sums, gamma, beta, output_node_size, frame_size, frame_stride, 0, stream);
+    if (rc) return rc;
+    return backward_common<false>(a, true, frame_size > 0 ? frame_size : 1, dmean_tmp, dvar_tmp, sums, input_node_size, st);
 }

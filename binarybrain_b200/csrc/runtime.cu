@@ -11,6 +11,7 @@
 //     the high-water mark, i.e. on nearly every step of a network with layers of different sizes);
 //   - block sizes are rounded up to 512 bytes so that every row a caller carves out of a block
 //     keeps the 256-byte alignment cudaMalloc gives.
+#include <atomic>
 #include <map>
 #include <mutex>
 #include <unordered_map>
@@ -73,6 +74,24 @@ const DeviceInfo &device_info()
         it = infos.emplace(dev, di).first;
     }
     return it->second;
+}
+
+bool allow_big_smem_once(const void *kernel, int bytes)
+{
+    static std::mutex mu;
+    static std::map<std::pair<int, const void *>, int> done;             // (device, kernel) -> bytes granted
+    int dev = 0;
+    cudaGetDevice(&dev);
+    const std::pair<int, const void *> key(dev, kernel);
+    {
+        std::lock_guard<std::mutex> g(mu);
+        auto it = done.find(key);
+        if (it != done.end() && it->second >= bytes) return true;
+    }
+    if (cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, bytes) != cudaSuccess) { cudaGetLastError(); return false; }
+    std::lock_guard<std::mutex> g(mu);
+    done[key] = bytes;
+    return true;
 }
 
 int frame_tile(long long rows_touched, int bits_per_row_frame, int node_groups, int frame_size, int max_tile)
@@ -206,8 +225,11 @@ extern "C" int bbcu_b200_selftest_wait_expiry(bbcu_stream_t stream)
 // ---------------------------------------------------------------------------------------------- manager
 extern "C" int bbcu_GetDeviceCount(void)
 {
-    int n = 0;
+    static std::atomic<int> count{0};              // asked for on every access to a host class's buffer; does not change once there are devices
+    int n = count.load(std::memory_order_relaxed);
+    if (n > 0) return n;
     if (cudaGetDeviceCount(&n) != cudaSuccess) { cudaGetLastError(); return 0; }
+    count.store(n, std::memory_order_relaxed);
     return n;
 }
 

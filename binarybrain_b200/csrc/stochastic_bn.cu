@@ -187,21 +187,39 @@ __global__ void k_set(float *dst, float a, int n)
     for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x) dst[i] = a;
 }
 
-// One grid row per tensor of the table (the reference: one block per tensor, cuda/OptimizerAdam.cu:12-48).
-__global__ void k_adam(const int *__restrict__ size_table, float *const *params, float *const *grads, float *const *m_tab, float *const *v_tab,
-                       float lr_t, float beta1, float beta2)
+// One grid row per tensor of the table (the reference: one block per tensor, cuda/OptimizerAdam.cu:12-48).  CLEAR: the gradient is
+// cleared on the way (Optimizer::Update = Step + ZeroGrad, include/bb/Optimizer.h:29-33), which saves its own launch per tensor.
+template <bool CLEAR>
+__global__ void __launch_bounds__(256)
+k_adam(const int *__restrict__ size_table, float *const *params, float *const *grads, float *const *m_tab, float *const *v_tab, float lr_t,
+       float beta1, float beta2)
 {
     const int t = blockIdx.y;
     const int n = size_table[t];
-    float *p = params[t], *m = m_tab[t], *v = v_tab[t];
-    const float *g = grads[t];
-    for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x) {
-        float gi = g[i], mi = m[i], vi = v[i];
+    float *p = params[t], *m = m_tab[t], *v = v_tab[t], *g = grads[t];
+    auto one = [&](float &pi, float gi, float &mi, float &vi) {
         mi += (1.0f - beta1) * (gi - mi);
         vi += (1.0f - beta2) * (gi * gi - vi);
-        p[i] -= lr_t * mi / (sqrtf(vi) + 1.0e-7f);
+        pi -= lr_t * mi / (sqrtf(vi) + 1.0e-7f);
+    };
+    const bool vec = ((reinterpret_cast<uintptr_t>(p) | reinterpret_cast<uintptr_t>(m) | reinterpret_cast<uintptr_t>(v) | reinterpret_cast<uintptr_t>(g)) & 15) == 0;
+    const int quads = vec ? n / 4 : 0, threads = gridDim.x * blockDim.x, id = blockIdx.x * blockDim.x + threadIdx.x;
+    for (int i = id; i < quads; i += threads) {
+        float4 pq = reinterpret_cast<float4 *>(p)[i], mq = reinterpret_cast<float4 *>(m)[i], vq = reinterpret_cast<float4 *>(v)[i];
+        const float4 gq = reinterpret_cast<float4 *>(g)[i];
+        one(pq.x, gq.x, mq.x, vq.x); one(pq.y, gq.y, mq.y, vq.y); one(pq.z, gq.z, mq.z, vq.z); one(pq.w, gq.w, mq.w, vq.w);
+        reinterpret_cast<float4 *>(p)[i] = pq;
+        reinterpret_cast<float4 *>(m)[i] = mq;
+        reinterpret_cast<float4 *>(v)[i] = vq;
+        if (CLEAR) reinterpret_cast<float4 *>(g)[i] = make_float4(0.0f, 0.0f, 0.0f, 0.0f);
+    }
+    for (int i = 4 * quads + id; i < n; i += threads) {
+        float pi = p[i], mi = m[i], vi = v[i];
+        one(pi, g[i], mi, vi);
+        p[i] = pi;
         m[i] = mi;
         v[i] = vi;
+        if (CLEAR) g[i] = 0.0f;
     }
 }
 
@@ -307,12 +325,25 @@ extern "C" int bbcu_fp32_Vector_set(float *dst, float a, int size, bbcu_stream_t
     return launch_status();
 }
 
-extern "C" int bbcu_fp32_OptimizerAdam(int size, const int *size_table, float *const *params, float *const *grads, float *const *m_tab,
-                                       float *const *v_tab, float lr_t, float beta1, float beta2, bbcu_stream_t stream)
+static int adam(bool clear, int size, const int *size_table, float *const *params, float *const *grads, float *const *m_tab, float *const *v_tab,
+                float lr_t, float beta1, float beta2, bbcu_stream_t stream)
 {
     BB200_REQUIRE_PTR(size_table); BB200_REQUIRE_PTR(params); BB200_REQUIRE_PTR(grads); BB200_REQUIRE_PTR(m_tab); BB200_REQUIRE_PTR(v_tab);
     BB200_REQUIRE(size >= 0 && size <= 65535, BBCU_ERR_BAD_SIZE);
     if (size == 0) return BBCU_OK;
-    k_adam<<<dim3(296, size), 256, 0, as_stream(stream)>>>(size_table, params, grads, m_tab, v_tab, lr_t, beta1, beta2);
+    auto kern = clear ? k_adam<true> : k_adam<false>;
+    kern<<<dim3(296, size), 256, 0, as_stream(stream)>>>(size_table, params, grads, m_tab, v_tab, lr_t, beta1, beta2);
     return launch_status();
+}
+
+extern "C" int bbcu_fp32_OptimizerAdam(int size, const int *size_table, float *const *params, float *const *grads, float *const *m_tab,
+                                       float *const *v_tab, float lr_t, float beta1, float beta2, bbcu_stream_t stream)
+{
+    return adam(false, size, size_table, params, grads, m_tab, v_tab, lr_t, beta1, beta2, stream);
+}
+
+extern "C" int bbcu_fp32_OptimizerAdamUpdate(int size, const int *size_table, float *const *params, float *const *grads, float *const *m_tab,
+                                             float *const *v_tab, float lr_t, float beta1, float beta2, bbcu_stream_t stream)
+{
+    return adam(true, size, size_table, params, grads, m_tab, v_tab, lr_t, beta1, beta2, stream);
 }

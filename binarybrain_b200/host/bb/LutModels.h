@@ -559,9 +559,15 @@ public:
         FrameBuffer y_saved;
         if (!m_y_stack.empty()) { y_saved = m_y_stack.back(); m_y_stack.pop_back(); }
         const bool from_output = !this->m_binary_mode && !y_saved.Empty() && y_saved.GetFrameSize() == dy_buf.GetFrameSize();
-        if (m_batch_norm && !kBit && (m_total_frames > 0 || from_output)) {
-            // the two halves of the backward: per-rank sums, their exchange when this object holds a frame shard, then the gradients
-            const long long total = m_total_frames > 0 ? (long long)m_total_frames : (long long)F;
+        if (m_batch_norm && !kBit && m_total_frames == 0 && from_output) {
+            // probability mode: the batch sums come from the saved output (8 bytes per node-frame) instead of a second LUT evaluation
+            Tensor dmean(indices_t{O}), dvar(indices_t{O});
+            BBCU_CHECK(bbcu_fp32_DifferentiableLut6_BackwardFromOutput(
+                    (float const *)x_buf.LockDeviceMemoryConst(), (float const *)y_saved.LockDeviceMemoryConst(), (float const *)dy_buf.LockDeviceMemoryConst(),
+                    (float *)dx_buf.LockDeviceMemory(true), idx, this->m_W->DevConst(), this->m_dW->Dev(), m_mean.DevConst(), m_rstd.DevConst(),
+                    dmean.Dev(true), dvar.Dev(true), m_gamma, m_beta, I, O, F, fs, this->m_lut_binarize, st));
+        } else if (m_batch_norm && !kBit && m_total_frames > 0) {
+            // this object holds a frame shard: the two halves of the backward with the exchange of the per-rank sums in between
             Tensor dmean(indices_t{O}), dvar(indices_t{O});
             m_sums.Resize({(index_t)O, 2});
             float const *xp = (float const *)x_buf.LockDeviceMemoryConst(), *dyp = (float const *)dy_buf.LockDeviceMemoryConst();
@@ -575,12 +581,12 @@ public:
                                                                       this->m_lut_binarize, this->m_binary_mode, st));
             }
             y_saved = FrameBuffer();
-            if (m_total_frames > 0) m_allreduce_sums(m_sums.Dev(), (std::size_t)O * 2, st);
+            m_allreduce_sums(m_sums.Dev(), (std::size_t)O * 2, st);
             BBCU_CHECK(bbcu_fp32_DifferentiableLut6_BackwardApply(xp, dyp, (float *)dx_buf.LockDeviceMemory(true), idx, this->m_W->DevConst(),
                                                                   this->m_dW->Dev(), m_mean.DevConst(), m_rstd.DevConst(), m_sums.DevConst(),
                                                                   dmean.Dev(true), dvar.Dev(true), m_gamma, m_beta, this->m_unbinarize_bias, I, O, F, fs,
-                                                                  total, this->m_lut_binarize, this->m_binary_mode, st));
-            if (m_total_frames > 0 && m_allreduce_grads) m_allreduce_grads(this->m_dW->Dev(), (std::size_t)this->m_dW->GetSize(), st);
+                                                                  (long long)m_total_frames, this->m_lut_binarize, this->m_binary_mode, st));
+            if (m_allreduce_grads) m_allreduce_grads(this->m_dW->Dev(), (std::size_t)this->m_dW->GetSize(), st);
         } else if (m_batch_norm) {
             Tensor dmean(indices_t{O}), dvar(indices_t{O});
             if (kBit) BBCU_CHECK(bbcu_bit_fp32_DifferentiableLut6_Backward(
@@ -977,7 +983,8 @@ class OptimizerAdam
 {
     std::vector<std::shared_ptr<Tensor>> m_params, m_grads, m_m, m_v;
     Tensor_<std::int32_t> m_sizes;
-    Tensor_<std::int64_t> m_ptab[4];
+    Tensor_<std::int64_t> m_tables;             // addresses of the parameters, gradients and both moments, one row each
+    std::vector<std::int64_t> m_addresses;      // what m_tables holds
     float m_lr, m_beta1, m_beta2, m_b1, m_b2;
 
 public:
@@ -999,31 +1006,40 @@ public:
         m_m.push_back(m); m_v.push_back(v);
     }
 
-    void Step()
-    {
-        if (m_params.empty()) return;
-        int n = (int)m_params.size();
-        m_sizes.Resize(n);
-        for (auto &t : m_ptab) t.Resize(n);
-        auto sz = m_sizes.Host(true);
-        std::int64_t *p[4] = {m_ptab[0].Host(true), m_ptab[1].Host(true), m_ptab[2].Host(true), m_ptab[3].Host(true)};
-        for (int i = 0; i < n; ++i) {
-            sz[i] = (std::int32_t)m_params[i]->GetSize();
-            p[0][i] = (std::int64_t)m_params[i]->Dev(); p[1][i] = (std::int64_t)m_grads[i]->Dev();
-            p[2][i] = (std::int64_t)m_m[i]->Dev();      p[3][i] = (std::int64_t)m_v[i]->Dev();
-        }
-        float lr_t = m_lr * std::sqrt(1.0f - m_b2) / (1.0f - m_b1);
-        BBCU_CHECK(bbcu_fp32_OptimizerAdam(n, m_sizes.DevConst(), (float *const *)m_ptab[0].DevConst(), (float *const *)m_ptab[1].DevConst(),
-                                           (float *const *)m_ptab[2].DevConst(), (float *const *)m_ptab[3].DevConst(), lr_t, m_beta1, m_beta2,
-                                           Manager::Stream()));
-        m_b1 *= m_beta1;
-        m_b2 *= m_beta2;
-    }
+    void Step() { Apply(false); }
     void ZeroGrad()
     {
         for (auto &g : m_grads) BBCU_CHECK(bbcu_fp32_Vector_set(g->Dev(true), 0.0f, (int)g->GetSize(), Manager::Stream()));
     }
-    void Update() { Step(); ZeroGrad(); }      // include/bb/Optimizer.h:29-33
+    void Update() { Apply(true); }             // Step + ZeroGrad (include/bb/Optimizer.h:29-33), one pass over the tables
+
+private:
+    void Apply(bool clear_grads)
+    {
+        if (m_params.empty()) return;
+        // the tables go up when they are new or an address has changed (a tensor was resized), not on every step
+        const std::size_t n = m_params.size();
+        std::vector<std::int64_t> now(4 * n);
+        for (std::size_t i = 0; i < n; ++i) {
+            now[i] = (std::int64_t)m_params[i]->Dev();    now[n + i] = (std::int64_t)m_grads[i]->Dev();
+            now[2 * n + i] = (std::int64_t)m_m[i]->Dev(); now[3 * n + i] = (std::int64_t)m_v[i]->Dev();
+        }
+        if (now != m_addresses) {
+            std::vector<std::int32_t> sizes(n);
+            for (std::size_t i = 0; i < n; ++i) sizes[i] = (std::int32_t)m_params[i]->GetSize();
+            m_sizes.Resize((index_t)n);
+            m_sizes.FromVector(sizes);
+            m_tables.Resize((index_t)(4 * n));
+            m_tables.FromVector(now);
+            m_addresses = now;
+        }
+        auto table = [&](std::size_t k) { return (float *const *)(m_tables.DevConst() + k * n); };
+        const float lr_t = m_lr * std::sqrt(1.0f - m_b2) / (1.0f - m_b1);
+        BBCU_CHECK((clear_grads ? bbcu_fp32_OptimizerAdamUpdate : bbcu_fp32_OptimizerAdam)((int)n, m_sizes.DevConst(), table(0), table(1), table(2), table(3), lr_t,
+                                                                                          m_beta1, m_beta2, Manager::Stream()));
+        m_b1 *= m_beta1;
+        m_b2 *= m_beta2;
+    }
 };
 
 }   // namespace bb

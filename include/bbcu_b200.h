@@ -23,18 +23,19 @@
  *     exit(1), include/bbcu/bbcu_util.h:17-36);
  *   - scratch: the fp32 backward operators use the caller's dev_dx_tmp when it is given, 16-byte aligned and at least 512 bytes
  *     per output node.  Otherwise, and for the operators whose reference signature carries no scratch, the LUT operators keep
- *     per-stream work areas in the device heap below: per-node sums, coefficient and pattern tables (at most ~1 KiB per output
- *     node) and, for DifferentiableLut6 in binary mode on fp32 frames, one pattern byte per node-frame (node_size *
- *     frame_stride bytes; above 1 GiB the operator runs its scratch-free kernels instead).  The first call on a stream
- *     allocates them, later calls reuse them, and bbcu_LocalHeap_GarbageCollect releases them.
+ *     per-stream work areas in the device heap below: per-node sums, coefficient and pattern tables (at most ~3 KiB per output
+ *     node), the lists of the consumers of every input row (32 bytes per node) and, for two-valued inputs, the patterns of the frames (backward:
+ *     2 bytes per node-frame; forward of DifferentiableLut6 in binary mode on fp32 frames: 1) and fp32 rows packed to bits; when
+ *     these would exceed 8 GiB (forward: 1 GiB) the operator runs its scratch-free kernels instead.  The first call on a
+ *     stream allocates them, later calls reuse them, and bbcu_LocalHeap_GarbageCollect releases them.
  *     ..._ForwardTraining_NoAlloc is the variant that never allocates.
  *
  * Results follow the reference's CPU branches (the header-only path in include/bb), which is what
  * parity is measured against; where the reference's old CUDA kernels differ from its CPU code the
  * CPU code wins.  dev_reverse_index of the backward operators is accepted for signature compatibility and
  * not read: the input gradients of a node are added to dx with 128-bit floating-point reductions
- * (red.global.add.v4.f32) that L2 resolves, instead of going through a [nodes*6][frames] temporary and a
- * gather by reverse index; dev_dx_tmp serves as plain scratch (see above).
+ * (red.global.add.v4.f32) that L2 resolves, or (two-valued inputs) gathered through a list the call makes itself, instead of going through
+ * a [nodes*6][frames] temporary and a gather by reverse index; dev_dx_tmp serves as plain scratch (see above).
  */
 #ifndef BBCU_B200_H
 #define BBCU_B200_H
@@ -215,11 +216,18 @@ int bbcu_fp32_Vector_set(float *dev_dst, float a, int size, bbcu_stream_t stream
 int bbcu_fp32_OptimizerAdam(int size, const int *dev_size_table, float *const *dev_params_buf_table, float *const *dev_grads_buf_table,
                             float *const *dev_m_buf_table, float *const *dev_v_buf_table, float lr_t, float beta1, float beta2,
                             bbcu_stream_t stream);
+/* Additive: the same step, and the gradients are cleared (bb::Optimizer::Update = Step + ZeroGrad, include/bb/Optimizer.h:29-33). */
+int bbcu_fp32_OptimizerAdamUpdate(int size, const int *dev_size_table, float *const *dev_params_buf_table, float *const *dev_grads_buf_table,
+                                  float *const *dev_m_buf_table, float *const *dev_v_buf_table, float lr_t, float beta1, float beta2,
+                                  bbcu_stream_t stream);
 
 /* bbcu_LossSoftmaxCrossEntropy<float>, include/bbcu/bbcu.h:1507-1519: per frame and pixel a softmax over the ch_size channel rows
  * (node = ch * pix_size + pix); dy = (t_weight * softmax - t) / t_sum; dev_loss_buf[frame] = sum log(softmax + 1e-7) * t_weight. */
 int bbcu_fp32_LossSoftmaxCrossEntropy(const float *dev_y_buf, const float *dev_t_buf, float *dev_dy_buf, double *dev_loss_buf, float t_sum,
                                       int pix_size, int ch_size, int frame_size, int frame_stride, bbcu_stream_t stream);
+/* Additive: the same with t_sum, the sum of all targets, formed on the device, and the mean loss -sum(loss) / t_sum in *dev_loss. */
+int bbcu_fp32_LossSoftmaxCrossEntropyMean(const float *dev_y_buf, const float *dev_t_buf, float *dev_dy_buf, double *dev_loss, int pix_size,
+                                          int ch_size, int frame_size, int frame_stride, bbcu_stream_t stream);
 /* bbcu_fp32_LossMeanSquaredError, include/bbcu/bbcu.h:1487-1500: dy = grad_reduction * (y - t); the squared errors times loss_reduction
  * are ADDED into dev_loss_buf[0 .. loss_buf_size) (the caller sums the buffer). */
 int bbcu_fp32_LossMeanSquaredError(const float *dev_y_buf, const float *dev_t_buf, float *dev_dy_buf, double *dev_loss_buf, int loss_buf_size,
@@ -325,6 +333,14 @@ int bbcu_fp32_DifferentiableLut6_BackwardApply(const float *dev_x_buf, const flo
                                                float gamma, float beta, float unbinarize_bias, int input_node_size, int output_node_size,
                                                int frame_size, int frame_stride, long long total_frame_size,
                                                int lut_binarize, int binary_mode, bbcu_stream_t stream);
+
+/* Additive: the whole backward of a batch-normalised layer in probability mode for a caller that kept the training output y (statistics
+ * from y as above, then the gradients); equal to bbcu_fp32_DifferentiableLut6_Backward, which evaluates the LUT a second time instead. */
+int bbcu_fp32_DifferentiableLut6_BackwardFromOutput(const float *dev_x_buf, const float *dev_y_buf, const float *dev_dy_buf, float *dev_dx_buf,
+                                                    const int *dev_input_index, const float *dev_W, float *dev_dW, const float *dev_mean_buf,
+                                                    const float *dev_rstd_buf, float *dev_dmean_tmp, float *dev_dvar_tmp, float gamma, float beta,
+                                                    int input_node_size, int output_node_size, int frame_size, int frame_stride, int lut_binarize,
+                                                    bbcu_stream_t stream);
 
 /* ------------------------------------------------------------------ Additive: a training forward that allocates nothing.
  * No counterpart in the reference.  Same arguments and results as bbcu_fp32_DifferentiableLut6_ForwardTraining, for callers that

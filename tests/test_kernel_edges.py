@@ -87,3 +87,39 @@ def test_two_valued_layers_edges(ops, I, O, F, stride):
     dW = torch.zeros((O, 64), device="cuda")
     dx = ops.differentiable_lut6_backward(dev_bits(xb, F), dev_fp32(dy, stride), dev(idx), dev(W), dW, dev(p["mean"]), dev(p["rstd"]), I, F)
     assert err(host_fp32(dx, F), dx_w) <= parity.BN_GRAD_FACTOR * parity.TOL * amp and err(dW.cpu().numpy(), dW_w) <= parity.BN_GRAD_FACTOR * parity.TOL * amp
+
+
+# probability mode, one launch per direction: one warp, ragged and whole warps, eight warps and several rounds, unaligned rows, the largest
+@pytest.mark.parametrize("I,O,F,stride", [(6, 1, 1, None), (9, 5, 3, 4), (33, 70, 128, None), (50, 31, 129, 131), (30, 40, 1025, None), (12, 8, 4096, 4099),
+                                          (700, 512, 4096, None)])
+def test_small_probability_layers_edges(ops, I, O, F, stride):
+    from gpu_util import wiring
+    rng = np.random.default_rng(I + O + F)
+    idx = wiring(rng, I, O)
+    W = np.clip(rng.normal(0.5, 0.25, (O, 64)), 0, 1).astype(np.float32)
+    x = (rng.random((I, F), dtype=np.float32) * 1.2 - 0.1).astype(np.float32)
+    dy, dW0 = rng.standard_normal((O, F), dtype=np.float32), rng.random((O, 64), dtype=np.float32)
+    y = port.sl6_forward(x, idx, W)
+    dx, dW = port.sl6_backward(x, dy, idx, W, I, dW=dW0)
+    parity._sl6_check(ops, x, idx, W, dy, dW0, {}, dict(y=y, dx=dx, dW=dW), stride)
+    parity._dl6_fp32_check(ops, x, idx, W, dy, rng.random(O, dtype=np.float32), rng.random(O, dtype=np.float32) + 0.5, dict(binary=0, lut_binarize=0), stride)
+
+
+# one CTA (up to 2^15 target values) and the general form; Adam with the gradients cleared on the way, whole quads and a remainder
+@pytest.mark.parametrize("classes,frames", [(1, 1), (10, 129), (10, 3276), (10, 3277), (3, 20000)])
+def test_mean_loss_and_adam_update(ops, classes, frames):
+    import torch
+    from gpu_util import dev, dev_fp32, host_fp32
+    rng = np.random.default_rng(frames)
+    y = rng.random((classes, frames), dtype=np.float32)
+    t = np.zeros_like(y)
+    t[rng.integers(0, classes, frames), np.arange(frames)] = 1.0
+    dy, loss = ops.softmax_cross_entropy(dev_fp32(y), dev_fp32(t), frames)
+    dy_w, loss_w = port.softmax_cross_entropy(y, t)
+    assert np.abs(host_fp32(dy, frames) - dy_w).max() <= 1e-6 and abs(float(loss.item()) - loss_w) <= 1e-5
+    for n in (frames, frames + 1):
+        W, dW = rng.random(n, dtype=np.float32), rng.standard_normal(n).astype(np.float32)
+        Wd, dWd = dev(W.copy()), dev(dW.copy())
+        ops.Adam([Wd], [dWd]).update()
+        port.adam_update(W, dW, np.zeros_like(W), np.zeros_like(W), np.ones(2, np.float32))
+        assert np.abs(Wd.cpu().numpy() - W).max() <= 1e-6 and not dWd.any()
