@@ -1,6 +1,6 @@
 """Builds the sm_100a shared libraries of this package in-tree (binarybrain_b200/lib/).
 
-    python -m binarybrain_b200.build            # C-ABI kernel library (+ the pybind11 host module)
+    python -m binarybrain_b200.build            # C-ABI kernel library, pybind11 host module, native operator module
 """
 import os
 import subprocess
@@ -63,9 +63,27 @@ def build_host_module(force=False):
     return out
 
 
+def build_native_module(force=False):
+    """The CPython module `binarybrain_b200._native` (the operators on torch tensors, for ops.py)."""
+    import torch
+    from torch.utils.cpp_extension import include_paths
+
+    src = os.path.join(HERE, "host", "native_main.cpp")
+    out = os.path.join(HERE, "_native" + sysconfig.get_config_var("EXT_SUFFIX"))
+    if force or _newer(out, [src, os.path.join(HERE, "..", "include", "bbcu_b200.h")]):
+        cxx = "/usr/bin/g++" if os.path.exists("/usr/bin/g++") else "g++"
+        torch_lib = os.path.join(os.path.dirname(torch.__file__), "lib")
+        cmd = [cxx, "-O2", "-std=c++17", "-shared", "-fPIC", "-fvisibility=hidden", f"-D_GLIBCXX_USE_CXX11_ABI={int(torch._C._GLIBCXX_USE_CXX11_ABI)}",
+               src, "-o", out, "-I" + sysconfig.get_paths()["include"], "-I" + os.path.join(HERE, "..", "include"), "-I/usr/local/cuda/include",
+               *["-I" + d for d in include_paths()], "-L" + torch_lib, "-ltorch_python", "-ltorch_cpu", "-lc10_cuda", "-lc10", "-ldl"]
+        subprocess.check_call(cmd)
+    return out
+
+
 def build_all(force=False):
     lib = build_library(force)
     mod = build_host_module(force)
+    build_native_module(force)
     return lib, mod
 
 

@@ -66,12 +66,15 @@ class ShardedDifferentiableLut6:
         """x: this rank's [n_in, stride] shard with `frames` valid frames; total_frames: frames of the whole step."""
         if y is None:
             y = torch.empty((self.n_out, x.shape[1]), dtype=torch.float32, device=x.device)
-        self._fused = self.world == 1 and self.binary and hasattr(self.ops, "differentiable_lut6_forward_training")
+        # One rank needs no exchange point: the unsplit operators, which take the per-pattern table route in binary mode and run a small
+        # layer in one launch.  (A large layer in probability mode keeps the split operators, whose backward reads the saved output.)
+        self._fused = (hasattr(self.ops, "differentiable_lut6_forward_training") and self.world == 1 and
+                       (self.binary or (frames == total_frames and frames <= self.ops.SMALL_FRAMES and
+                                        frames * self.n_out <= self.ops.SMALL_NODE_FRAMES)))
         if self._fused:
-            # one rank, binary mode: the unsplit operators, which take the per-pattern table route (no exchange point is needed)
             _, mean, rstd = self.ops.differentiable_lut6_forward_training(x, self.idx, self.W, self.running_mean, self.running_var, frames, y=y,
                                                                          gamma=self.gamma, beta=self.beta, momentum=self.momentum,
-                                                                         lut_binarize=self.lut_binarize, binary=True)
+                                                                         lut_binarize=self.lut_binarize, binary=self.binary)
             self.mean, self.rstd = mean, rstd
             self._x, self._frames, self._total, self._y = x, frames, total_frames, None
             return y
