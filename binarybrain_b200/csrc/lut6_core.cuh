@@ -244,14 +244,17 @@ __device__ __forceinline__ float lut6_forward_halves(const float4 *tab2, const f
     return fmaf(u[5], b, a);
 }
 
-// Reverse pass for one frame; acc2[i] collects (dC[i], dC[i + 32]).
+// Reverse pass for one frame; acc2[i] collects (dC[i], dC[i + 32]).  The gradient is carried down to the eight packed values
+// G[b] = g * (monomial b of u2, u3, u4); the coefficient gradients are the products of those with 1, u0, u1 and u0 u1, and the
+// derivatives of u0 and u1 come from c01 + u1 c11 and the kept c10 + u0 c11.  Going down one level less saves seven packed products
+// per frame against carrying the gradient through u1 as well.
 __device__ __forceinline__ void lut6_reverse_halves(const float4 *tab2, const float (&u)[6], const KeptHalves &D, float g,
                                                     f32x2 (&acc2)[32], float (&dx)[6])
 {
     f32x2 U[5];
 #pragma unroll
     for (int j = 0; j < 5; ++j) U[j] = pack2(u[j], u[j]);
-    f32x2 gt[16], s[5];
+    f32x2 gt[8], s[5];
     dx[5] = g * D.d6;
     gt[0] = pack2(g, g * u[5]);
 
@@ -277,22 +280,20 @@ __device__ __forceinline__ void lut6_reverse_halves(const float4 *tab2, const fl
         for (int k = 2; k < 8; k += 2) { a = fma2(gt[k], D.d2[k], a); b = fma2(gt[k + 1], D.d2[k + 1], b); }
         s[1] = add2(a, b);
     }
-#pragma unroll
-    for (int k = 7; k >= 0; --k) { gt[2 * k + 1] = mul2(gt[k], U[1]); gt[2 * k] = gt[k]; }
-
     {
+        const f32x2 U01 = mul2(U[0], U[1]);
         f32x2 a = 0ull, b = 0ull;
 #pragma unroll
-        for (int k = 0; k < 16; k += 2) {
-            a = fma2(gt[k], reinterpret_cast<const ulonglong2 *>(tab2 + k)->y, a);
-            b = fma2(gt[k + 1], reinterpret_cast<const ulonglong2 *>(tab2 + k + 1)->y, b);
+        for (int k = 0; k < 8; ++k) {
+            const f32x2 e = fma2(U[1], reinterpret_cast<const ulonglong2 *>(tab2 + 2 * k + 1)->y, reinterpret_cast<const ulonglong2 *>(tab2 + 2 * k)->y);
+            if (k & 1) b = k == 1 ? mul2(gt[k], e) : fma2(gt[k], e, b);
+            else       a = k == 0 ? mul2(gt[k], e) : fma2(gt[k], e, a);
+            acc2[4 * k]     = add2(acc2[4 * k], gt[k]);
+            acc2[4 * k + 1] = fma2(gt[k], U[0], acc2[4 * k + 1]);
+            acc2[4 * k + 2] = fma2(gt[k], U[1], acc2[4 * k + 2]);
+            acc2[4 * k + 3] = fma2(gt[k], U01, acc2[4 * k + 3]);
         }
         s[0] = add2(a, b);
-#pragma unroll
-        for (int k = 0; k < 16; ++k) {
-            acc2[2 * k]     = add2(acc2[2 * k], gt[k]);
-            acc2[2 * k + 1] = fma2(gt[k], U[0], acc2[2 * k + 1]);
-        }
     }
 #pragma unroll
     for (int j = 0; j < 5; ++j) {

@@ -752,9 +752,9 @@ k_lut6_backward(const BwdArgs a)
 // Work item = (frame tile of a.T frames, group of 8 nodes), walked in tile-major order by one CTA per SM; each warp owns one node
 // of the group.  What the kernel is bound by: an SM sub-partition issues one instruction per clock and a packed f32x2
 // instruction takes two issue slots (measured: 32 packed FMAs take 65 clocks per warp, and scalar FMAs, logic ops or anything
-// else issued beside them add their own clocks in full), so the time is the weighted instruction count -- 113 packed (226
-// slots) + about 105 others per frame -- over the issue rate.  Everything here is about the "others":
-//   * the per-node table arrives ready to use (k_table_halves has converted every table once per launch);
+// else issued beside them add their own clocks in full), so the time is the weighted instruction count -- 106 packed (212
+// slots) + about 100 others per frame -- over the issue rate.  Everything here is about the "others":
+//   * the per-node table arrives ready to use (k_backward_prepare has converted every table once per launch);
 //   * global -> shared: a warp streams its item in 128-frame chunks through a three-stage ring; every lane copies 16 bytes (four
 //     consecutive frames) of each of the six input rows and of dy with cp.async, two chunks ahead of the arithmetic, so the
 //     prefetch holds no registers and the loop has no global address arithmetic per frame;
@@ -920,7 +920,7 @@ k_lut6_backward_pipe(const BwdArgs a, const float4 *__restrict__ coef, float *__
         const int node_raw = cc.group * kWarpsPerCta + warp;
         const bool live_node = node_raw < a.O;
         const int node = min(node_raw, a.O - 1);
-        const float mean = mean_n, rstd = rstd_n, dmean = dmean_n, dvar = dvar_n;
+        const float mean = mean_n, rstd = rstd_n, dmean = dmean_n, grstd = a.gamma * rstd_n, dvar_rF = dvar_n * a.rF;
         {
             BvCursor t = cc;
             next_item(t);
@@ -964,8 +964,7 @@ k_lut6_backward_pipe(const BwdArgs a, const float4 *__restrict__ coef, float *__
                     if (BN) {
                         const float tanh_x = ((v - mean) * rstd) * a.gamma + a.beta;
                         if (tanh_x <= 0.0f || tanh_x >= 1.0f) g = 0.0f;
-                        const float dxc = (g * a.gamma) * rstd;
-                        g = dxc + dmean + (v * dvar * a.rF);
+                        g = fmaf(v, dvar_rF, fmaf(g, grstd, dmean));
                     }
                     if (f0 + 64 * h + 2 * lane + e >= a.F || !live_node) g = 0.0f;
                     float dxv[6];
@@ -1114,17 +1113,28 @@ static int forward_plain(const void *x, float *y, uint32_t *ybits, const int *id
 // Frames per tile of the persistent backward.  A wide tile amortises the per-item flush of the 64 gradient sums; a narrow one keeps
 // the tile's x and dx rows (8 bytes per row and frame) in L2.  The kernel is issue-bound, so the wide tile wins until the rows
 // exceed L2 several times over -- measured on B200: 8192 rows 1.60 / 1.54 / 1.52 ms at 512 / 1024 / 2048 frames, 65536 rows
-// 3.57 / 3.42 / 3.46 ms -- hence four times L2, between 512 and 2048 frames.
+// 3.07 / 2.97 / 2.97 ms (2.94 at 1408) -- hence at most six times L2, between 512 and 2048 frames.  Below that limit the tile is the one whose busiest
+// CTA has the least to do, an item costing its frames plus about 40 frames' worth of flush: the items go to the CTAs in rounds, and a
+// last round that is nearly empty costs as much as a full one (3000 nodes x 5001 frames: 11 % over the mean with 2048-frame tiles).
 static int backward_pipe_tile(long long rows, int groups, int F)
 {
-    const DeviceInfo &di = device_info();
-    long long t = (long long)(4 * di.l2_bytes) / (8 * (rows > 0 ? rows : 1));
-    t = (t / kFramesPerIter) * kFramesPerIter;
-    if (t > 2048) t = 2048;
-    if (t < 512) t = 512;
-    // small layers: narrow the tile until every SM has a couple of items
-    while (t > kFramesPerIter && (long long)groups * ((F + t - 1) / t) < 2LL * di.sm_count) t -= kFramesPerIter;
-    return (int)t;
+    const long long ctas = device_info().sm_count;
+    long long cap = (long long)(6 * device_info().l2_bytes) / (8 * (rows > 0 ? rows : 1)) / kFramesPerIter * kFramesPerIter;
+    cap = cap > 2048 ? 2048 : cap < 512 ? 512 : cap;
+    constexpr long long kFlush = 40;
+    long long best = kFramesPerIter, best_cost = -1;
+    for (long long T = kFramesPerIter; T <= cap; T += kFramesPerIter) {
+        const long long tiles = (F + T - 1) / T, whole = (long long)groups * (tiles - 1), all = (long long)groups * tiles;
+        const long long last = ((F - (tiles - 1) * T + kFramesPerIter - 1) / kFramesPerIter) * kFramesPerIter;
+        long long cost = 0;
+        for (long long c : {0LL, whole % ctas, all % ctas}) {         // the load changes at these CTAs only
+            const long long n = all > c ? (all - c + ctas - 1) / ctas : 0, n_whole = whole > c ? (whole - c + ctas - 1) / ctas : 0;
+            const long long load = n_whole * (T + kFlush) + (n - n_whole) * (last + kFlush);
+            if (load > cost) cost = load;
+        }
+        if (best_cost < 0 || cost <= best_cost) { best = T; best_cost = cost; }
+    }
+    return (int)best;
 }
 
 // The persistent backward (k_lut6_backward_pipe); BBCU_ERR_NO_MEMORY when its scratch (512 bytes per node) cannot be had.
