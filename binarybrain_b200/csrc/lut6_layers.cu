@@ -34,7 +34,7 @@ struct FwdArgs {
     const float *W;
     const float *mean;      // PH_NORM
     const float *rstd;      // PH_NORM: rstd, or the running variance when stat_is_var
-    double     *sums;       // PH_STATS: [O][2]
+    double     *sums;       // PH_STATS, PH_BWD: [O][2], cleared by the launcher
     float gamma, beta, bias;
     int O, F, T;
     long long xs, ys;       // row strides in elements (floats / words)
@@ -286,9 +286,10 @@ __device__ __forceinline__ void fp_issue(const FwdArgs &a, FpPos pos, bool exist
     cp_async_commit();
 }
 
-// Every node's table as 32 x (c0, c0, c1, c1): the polynomial coefficients, each duplicated for the two halves of a packed operand.
+// Every node's table as 32 x (c0, c0, c1, c1): the polynomial coefficients, each duplicated for the two halves of a packed operand.  On the
+// way it clears the node's batch sums, when there are any.
 __global__ void __launch_bounds__(kWarpsPerCta * 32)
-k_table_coeffs(const float *__restrict__ W, float4 *__restrict__ coef, int O, int lut_binarize)
+k_table_coeffs(const float *__restrict__ W, float4 *__restrict__ coef, double *__restrict__ sums, int O, int lut_binarize)
 {
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
     const int node = blockIdx.x * kWarpsPerCta + warp;
@@ -297,6 +298,7 @@ k_table_coeffs(const float *__restrict__ W, float4 *__restrict__ coef, int O, in
     if (lut_binarize) { v.x = v.x > 0.5f ? 1.0f : 0.0f; v.y = v.y > 0.5f ? 1.0f : 0.0f; }
     v = table_to_coeffs(v, lane);
     coef[(size_t)node * 32 + lane] = make_float4(v.x, v.x, v.y, v.y);
+    if (sums != nullptr && lane < 2) sums[2 * (size_t)node + lane] = 0.0;
 }
 
 template <int PHASE, bool BINARY>            // BINARY: the layer's binary mode, compiled in so that input conditioning is one instruction
@@ -461,32 +463,49 @@ k_lut6_forward_pipe(const FwdArgs a, int n_tiles)
     cp_async_wait<0>();
 }
 
-// mean / var / rstd and the running statistics from the fp64 sums (DifferentiableLutN.h:804-812).
+// mean and rstd of a node from its fp64 sums (DifferentiableLutN.h:804-812)
+struct BnStatistics {
+    float mean, var, rstd;
+};
+
+__device__ __forceinline__ BnStatistics bn_statistics(const double *__restrict__ sums, int n, long long total_frames)
+{
+    const float rF = 1.0f / (float)total_frames;
+    const float s1 = (float)sums[2 * (size_t)n];
+    const float s2 = (float)sums[2 * (size_t)n + 1];
+    BnStatistics s;
+    s.mean = s1 * rF;
+    // one fused multiply-subtract, which is what the reference's build flags make of (s2*rF) - (mean*mean)
+    s.var  = fmaxf(1.0e-5f, fmaf(s2, rF, -(s.mean * s.mean)));
+    s.rstd = 1.0f / sqrtf(s.var);
+    return s;
+}
+
+__device__ __forceinline__ void bn_record(const BnStatistics &s, int n, float *mean_out, float *rstd_out, float *running_mean, float *running_var, float momentum)
+{
+    running_mean[n] = running_mean[n] * momentum + s.mean * (1.0f - momentum);
+    running_var[n]  = running_var[n]  * momentum + s.var  * (1.0f - momentum);
+    mean_out[n] = s.mean;
+    rstd_out[n] = s.rstd;
+}
+
 __global__ void k_bn_finalize(const double *__restrict__ sums, float *mean_out, float *rstd_out, float *running_mean, float *running_var,
                               float momentum, int O, long long total_frames)
 {
     int n = blockIdx.x * blockDim.x + threadIdx.x;
-    if (n >= O) return;
-    const float rF   = 1.0f / (float)total_frames;
-    const float s1   = (float)sums[2 * (size_t)n];
-    const float s2   = (float)sums[2 * (size_t)n + 1];
-    const float mean = s1 * rF;
-    // one fused multiply-subtract, which is what the reference's build flags make of (s2*rF) - (mean*mean)
-    const float var  = fmaxf(1.0e-5f, fmaf(s2, rF, -(mean * mean)));
-    const float rstd = 1.0f / sqrtf(var);
-    running_mean[n] = running_mean[n] * momentum + mean * (1.0f - momentum);
-    running_var[n]  = running_var[n]  * momentum + var  * (1.0f - momentum);
-    mean_out[n] = mean;
-    rstd_out[n] = rstd;
+    if (n < O) bn_record(bn_statistics(sums, n, total_frames), n, mean_out, rstd_out, running_mean, running_var, momentum);
 }
 
-// In-place normalise of the raw LUT values stored by PH_STATS: one CTA per (node, 4096-frame chunk).
+// In-place normalise of the raw LUT values stored by PH_STATS: one CTA per (node, 4096-frame chunk).  Every CTA takes the statistics from
+// the sums itself and the first one of a node records them, which spares a launch of its own.
 __global__ void __launch_bounds__(256)
-k_bn_normalize_inplace(float *y, const float *__restrict__ mean_buf, const float *__restrict__ rstd_buf, float gamma, float beta,
-                       int F, long long ys, int binary, int chunks)
+k_bn_normalize_inplace(float *y, const double *__restrict__ sums, float *mean_out, float *rstd_out, float *running_mean, float *running_var, float gamma,
+                       float beta, float momentum, long long total_frames, int F, long long ys, int binary, int chunks)
 {
     const int node = blockIdx.x / chunks, chunk = blockIdx.x % chunks;
-    const float mean = mean_buf[node], rstd = rstd_buf[node];
+    const BnStatistics stat = bn_statistics(sums, node, total_frames);
+    const float mean = stat.mean, rstd = stat.rstd;
+    if (chunk == 0 && threadIdx.x == 0) bn_record(stat, node, mean_out, rstd_out, running_mean, running_var, momentum);
     float *row = y + (size_t)node * ys;
     const int f0 = chunk * 4096;
     const int f1 = min(F, f0 + 4096);
@@ -636,21 +655,31 @@ k_dl6_backward_stats_from_y(const float *__restrict__ y, const float *__restrict
     if (threadIdx.x == 0) {
         double a = 0.0, b = 0.0;
         for (int w = 0; w < 8; ++w) { a += red[0][w]; b += red[1][w]; }
-        atomicAdd(sums + 2 * (size_t)node, a);
-        atomicAdd(sums + 2 * (size_t)node + 1, b);
+        if (chunks == 1) {
+            sums[2 * (size_t)node] = a;
+            sums[2 * (size_t)node + 1] = b;
+        } else {                                          // several chunks: the launcher has cleared the sums
+            atomicAdd(sums + 2 * (size_t)node, a);
+            atomicAdd(sums + 2 * (size_t)node + 1, b);
+        }
     }
+}
+
+__device__ __forceinline__ void bn_backward_finalize(const double *__restrict__ sums, int n, const float *__restrict__ mean_buf,
+                                                     const float *__restrict__ rstd_buf, float *dmean_out, float *dvar_out, long long total_frames)
+{
+    const float rF = 1.0f / (float)total_frames;
+    const float dstd = (float)sums[2 * (size_t)n], dmeanx = (float)sums[2 * (size_t)n + 1];
+    const float dvar = dstd * rstd_buf[n];
+    dvar_out[n]  = dvar;
+    dmean_out[n] = (dmeanx - (mean_buf[n] * dvar)) * rF;
 }
 
 __global__ void k_bn_backward_finalize(const double *__restrict__ sums, const float *__restrict__ mean_buf, const float *__restrict__ rstd_buf,
                                        float *dmean_out, float *dvar_out, int O, long long total_frames)
 {
     int n = blockIdx.x * blockDim.x + threadIdx.x;
-    if (n >= O) return;
-    const float rF = 1.0f / (float)total_frames;
-    const float dstd = (float)sums[2 * (size_t)n], dmeanx = (float)sums[2 * (size_t)n + 1];
-    const float dvar = dstd * rstd_buf[n];
-    dvar_out[n]  = dvar;
-    dmean_out[n] = (dmeanx - (mean_buf[n] * dvar)) * rF;
+    if (n < O) bn_backward_finalize(sums, n, mean_buf, rstd_buf, dmean_out, dvar_out, total_frames);
 }
 
 // dW / dx.  BN = true folds the batch-norm backward (DifferentiableLutN.h:1225-1258) in front of the LUT's.
@@ -771,7 +800,7 @@ k_lut6_backward(const BwdArgs a)
 //     launch.
 // The tile is wide (1024-2048 frames) to amortise that flush: measured, the extra L2 misses of a wide tile cost less than
 // flushing more often, because the kernel is issue-bound, not memory-bound.
-// dx rows must be zero on entry.
+// dx rows must be zero on entry (k_backward_prepare).
 // ---------------------------------------------------------------------------------------------
 constexpr int kBvStages     = 3;
 constexpr int kBvRowBytes   = kFramesPerIter * 4;                 // one row segment of a chunk
@@ -786,21 +815,42 @@ constexpr int kBvSmem       = kWarpsPerCta * kBvWarpBytes;
 static_assert(kBvSmem <= 227 * 1024, "one CTA per SM must fit");
 static_assert(6 * kBvRowBytes <= kBvTrBytes, "dx staging fits the transpose buffer");
 
-// Every node's table in the half-packed form of lut6_forward_keep_halves: 16 x (c[2k], c[2k+32], c[2k+1], c[2k+33]).
+// Everything the persistent backward wants done before it, in one launch: every node's table in the half-packed form of
+// lut6_forward_keep_halves (16 x (c[2k], c[2k+32], c[2k+1], c[2k+33])), cleared coefficient gradients, the node's dmean and dvar from the
+// batch sums (`sums` not null), and dx cleared by all threads of the grid with 128-bit stores (`zero` not null; a large cudaMemsetAsync
+// ran at about half of the copy bandwidth).
+struct BwdPrepare {
+    const float *W;
+    float4 *coef;
+    float2 *dC;
+    const double *sums;
+    const float *mean, *rstd;
+    float *dmean, *dvar;
+    float4 *zero;
+    size_t zero_quads;
+    long long total_frames;
+    int O, lut_binarize;
+};
+
 __global__ void __launch_bounds__(kWarpsPerCta * 32)
-k_table_halves(const float *__restrict__ W, float4 *__restrict__ coef, int O, int lut_binarize)
+k_backward_prepare(const BwdPrepare a)
 {
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
     const int node = blockIdx.x * kWarpsPerCta + warp;
-    if (node >= O) return;
-    float2 v = reinterpret_cast<const float2 *>(W + (size_t)node * 64)[lane];
-    if (lut_binarize) { v.x = v.x > 0.5f ? 1.0f : 0.0f; v.y = v.y > 0.5f ? 1.0f : 0.0f; }
-    v = table_to_coeffs(v, lane);
-    const float hx = __shfl_down_sync(kFull, v.x, 16), hy = __shfl_down_sync(kFull, v.y, 16);
-    if (lane < 16) coef[(size_t)node * 16 + lane] = make_float4(v.x, hx, v.y, hy);
+    if (node < a.O) {
+        float2 v = reinterpret_cast<const float2 *>(a.W + (size_t)node * 64)[lane];
+        if (a.lut_binarize) { v.x = v.x > 0.5f ? 1.0f : 0.0f; v.y = v.y > 0.5f ? 1.0f : 0.0f; }
+        v = table_to_coeffs(v, lane);
+        const float hx = __shfl_down_sync(kFull, v.x, 16), hy = __shfl_down_sync(kFull, v.y, 16);
+        if (lane < 16) a.coef[(size_t)node * 16 + lane] = make_float4(v.x, hx, v.y, hy);
+        a.dC[(size_t)node * 32 + lane] = make_float2(0.0f, 0.0f);
+        if (a.sums != nullptr && lane == 0) bn_backward_finalize(a.sums, node, a.mean, a.rstd, a.dmean, a.dvar, a.total_frames);
+    }
+    const float4 z = make_float4(0.0f, 0.0f, 0.0f, 0.0f);
+    for (size_t i = (size_t)blockIdx.x * blockDim.x + threadIdx.x; i < a.zero_quads; i += (size_t)gridDim.x * blockDim.x) a.zero[i] = z;
 }
 
-// dW += adjoint butterfly of the coefficient gradients (dC in the half-packed layout of k_table_halves); one warp per node.
+// dW += adjoint butterfly of the coefficient gradients (dC in the half-packed layout of k_backward_prepare); one warp per node.
 __global__ void __launch_bounds__(kWarpsPerCta * 32)
 k_coeff_grads_to_dw(const float4 *__restrict__ dC, float *__restrict__ dW, int O)
 {
@@ -1029,7 +1079,11 @@ static int check_common(const void *x, const void *y, const int *idx, const floa
 template <bool XBIT, int PHASE, bool YBIT>
 static int launch_forward(FwdArgs a, int max_tile, cudaStream_t st)
 {
-    if (a.O == 0 || a.F == 0) return BBCU_OK;
+    if (a.O == 0) return BBCU_OK;
+    if (a.F == 0) {
+        if (PHASE == PH_STATS) BB200_CUDA(cudaMemsetAsync(a.sums, 0, sizeof(double) * 2 * (size_t)a.O, st));
+        return BBCU_OK;
+    }
     a.groups = (a.O + kWarpsPerCta - 1) / kWarpsPerCta;
     // input count is not part of this ABI: between O (square layer) and 6*O rows are touched
     a.T = frame_tile(3LL * a.O, XBIT ? 1 : 32, a.groups, a.F, max_tile);
@@ -1051,15 +1105,17 @@ static int launch_forward(FwdArgs a, int max_tile, cudaStream_t st)
                 // slot 1 of the stream's scratch: slot 0 may hold the caller's batch-norm sums at the same time
                 float4 *coef = static_cast<float4 *>(stream_scratch(st, (size_t)a.O * kFpTabSlotBytes, 1));
                 if (coef != nullptr) {
-                    k_table_coeffs<<<a.groups, kWarpsPerCta * 32, 0, st>>>(a.W, coef, a.O, a.lut_binarize);
+                    k_table_coeffs<<<a.groups, kWarpsPerCta * 32, 0, st>>>(a.W, coef, a.sums, a.O, a.lut_binarize);
                     BB200_CUDA(cudaPeekAtLastError());
                     a.coef = coef;
                 }
             }
+            if (PHASE == PH_STATS && a.coef == nullptr) BB200_CUDA(cudaMemsetAsync(a.sums, 0, sizeof(double) * 2 * (size_t)a.O, st));
             kern<<<(unsigned)grid, kWarpsPerCta * 32, kFpSmem, st>>>(a, (a.F + a.T - 1) / a.T);
             return launch_status();
         }
     }
+    if (PHASE == PH_STATS) BB200_CUDA(cudaMemsetAsync(a.sums, 0, sizeof(double) * 2 * (size_t)a.O, st));
     const long long tiles = (a.F + a.T - 1) / a.T;
     const long long blocks = tiles * a.groups;
     BB200_REQUIRE(blocks < (1LL << 31), BBCU_ERR_TOO_LARGE);
@@ -1069,8 +1125,8 @@ static int launch_forward(FwdArgs a, int max_tile, cudaStream_t st)
 
 // The statistics half of the fp32 backward (the two batch-norm sums from a re-evaluated LUT value and dy) through the pipelined
 // forward kernel, which evaluates the tree at nearly twice the rate of k_lut6_backward_stats.  Returns false, having launched
-// nothing, when the rows are not 16-byte aligned or the shared-memory opt-in is refused; *rc is the launch status otherwise.
-// b.sums must be zero on entry.
+// nothing, when the rows are not 16-byte aligned or the shared-memory opt-in is refused; *rc is the launch status otherwise.  Clears
+// b.sums.
 static bool backward_stats_pipe(const BwdArgs &b, cudaStream_t st, int *rc, void *tmp = nullptr, size_t tmp_bytes = 0)
 {
     const bool aligned = ((reinterpret_cast<uintptr_t>(b.x) | reinterpret_cast<uintptr_t>(b.W) | reinterpret_cast<uintptr_t>(b.dy)) & 15) == 0 &&
@@ -1093,8 +1149,11 @@ static bool backward_stats_pipe(const BwdArgs &b, cudaStream_t st, int *rc, void
     float4 *coef = (tmp != nullptr && tmp_bytes >= need && (reinterpret_cast<uintptr_t>(tmp) & 15) == 0)
                        ? static_cast<float4 *>(tmp) : static_cast<float4 *>(stream_scratch(st, need, 1));
     if (coef != nullptr) {
-        k_table_coeffs<<<a.groups, kWarpsPerCta * 32, 0, st>>>(a.W, coef, a.O, a.lut_binarize);
+        k_table_coeffs<<<a.groups, kWarpsPerCta * 32, 0, st>>>(a.W, coef, a.sums, a.O, a.lut_binarize);
         a.coef = coef;
+    } else if (cudaMemsetAsync(a.sums, 0, sizeof(double) * 2 * (size_t)a.O, st) != cudaSuccess) {
+        *rc = launch_status();
+        return true;
     }
     kern<<<(unsigned)grid, kWarpsPerCta * 32, kFpSmem, st>>>(a, (a.F + a.T - 1) / a.T);
     *rc = launch_status();
@@ -1141,7 +1200,9 @@ static int backward_pipe_tile(long long rows, int groups, int F)
 
 // The persistent backward (k_lut6_backward_pipe); BBCU_ERR_NO_MEMORY when its scratch (512 bytes per node) cannot be had.
 // `tmp` / `tmp_bytes`: scratch handed in by the caller (the reference's dev_dx_tmp), used when it is large enough and 16-byte aligned.
-static int launch_backward_pipe(BwdArgs a, bool bn, int I, void *tmp, size_t tmp_bytes, cudaStream_t st)
+// Clears dx and, with `sums` (batch norm: the batch sums over total_frames), forms dmean and dvar.
+static int launch_backward_pipe(BwdArgs a, bool bn, int I, const double *sums, float *dmean_out, float *dvar_out, long long total_frames, void *tmp,
+                                size_t tmp_bytes, cudaStream_t st)
 {
     const size_t need = (size_t)a.O * 512;
     unsigned char *scratch = nullptr;
@@ -1163,35 +1224,20 @@ static int launch_backward_pipe(BwdArgs a, bool bn, int I, void *tmp, size_t tmp
     long long grid = device_info().sm_count;
     if (grid > n_items) grid = n_items;
     const int groups8 = (a.O + kWarpsPerCta - 1) / kWarpsPerCta;
-    k_table_halves<<<groups8, kWarpsPerCta * 32, 0, st>>>(a.W, coef, a.O, a.lut_binarize);
+    BwdPrepare pre = {};
+    pre.W = a.W; pre.coef = coef; pre.dC = reinterpret_cast<float2 *>(dC); pre.O = a.O; pre.lut_binarize = a.lut_binarize;
+    pre.sums = sums; pre.mean = a.mean; pre.rstd = a.rstd; pre.dmean = dmean_out; pre.dvar = dvar_out; pre.total_frames = total_frames;
+    pre.zero = reinterpret_cast<float4 *>(a.dx);
+    pre.zero_quads = (size_t)I * (size_t)a.dxs / 4;
+    long long fill = (long long)((pre.zero_quads + 1023) / 1024);
+    if (fill > 8LL * device_info().sm_count) fill = 8LL * device_info().sm_count;
+    k_backward_prepare<<<(unsigned)(fill > groups8 ? fill : groups8), kWarpsPerCta * 32, 0, st>>>(pre);
     BB200_CUDA(cudaPeekAtLastError());
-    BB200_CUDA(cudaMemsetAsync(dC, 0, (size_t)a.O * 256, st));
+    a.dmean = dmean_out; a.dvar = dvar_out;
     kern<<<(unsigned)grid, kWarpsPerCta * 32, kBvSmem, st>>>(a, coef, dC, n_tiles, n_full, n_last);
     BB200_CUDA(cudaPeekAtLastError());
     k_coeff_grads_to_dw<<<groups8, kWarpsPerCta * 32, 0, st>>>(reinterpret_cast<const float4 *>(dC), a.dW, a.O);
     return launch_status();
-}
-
-// Zero fill with 128-bit stores from a grid sized to the GPU.  A large cudaMemsetAsync ran at about half of the copy bandwidth
-// (8 GiB of dx in 2.7 ms); the clear is 6 % of a training step, so it gets a kernel.
-__global__ void __launch_bounds__(256)
-k_zero_fill(float4 *__restrict__ p, size_t n)
-{
-    const float4 z = make_float4(0.0f, 0.0f, 0.0f, 0.0f);
-    for (size_t i = (size_t)blockIdx.x * blockDim.x + threadIdx.x; i < n; i += (size_t)gridDim.x * blockDim.x) p[i] = z;
-}
-
-static int zero_async(void *ptr, size_t bytes, cudaStream_t st)
-{
-    if (bytes >= ((size_t)1 << 20) && (reinterpret_cast<uintptr_t>(ptr) & 15) == 0) {
-        const size_t n = bytes / 16;
-        k_zero_fill<<<(unsigned)(8 * device_info().sm_count), 256, 0, st>>>(static_cast<float4 *>(ptr), n);
-        BB200_CUDA(cudaPeekAtLastError());
-        if (bytes % 16) BB200_CUDA(cudaMemsetAsync(static_cast<unsigned char *>(ptr) + n * 16, 0, bytes % 16, st));
-        return BBCU_OK;
-    }
-    BB200_CUDA(cudaMemsetAsync(ptr, 0, bytes, st));
-    return BBCU_OK;
 }
 
 static SmallLayerArgs small_args(const float *x, const int *idx, const float *W, int F, long long fs, int lut_binarize, const void *p, const void *q,
@@ -1221,18 +1267,19 @@ static int backward_common(BwdArgs a, bool bn, long long total_frames, float *dm
                                                    dvar_out, a.gamma, a.beta, a.bias, I, a.O, a.F, a.dxs, total_frames, a.lut_binarize, st);
         if (rc != BBCU_ERR_NO_MEMORY) return rc;
     }
-    if (!XBIT && !a.binary && ext_sums == nullptr && a.xs == a.dxs && a.dys == a.dxs && total_frames == a.F && small_probability_layer(a.O, a.F)) {
+    if (!XBIT && !a.binary && ext_sums == nullptr && a.xs == a.dxs && a.dys == a.dxs && total_frames == a.F && small_probability_layer(a.O, a.F) &&
+        (bn || (long long)a.O * a.F <= kSmallProbability / 2)) {        // (without batch norm the persistent kernel has fewer launches around it)
         SmallLayerArgs s = small_args(static_cast<const float *>(a.x), a.idx, a.W, a.F, a.dxs, a.lut_binarize, a.dy, a.dx, nullptr);
         s.dy = a.dy; s.dx = a.dx; s.dW = a.dW; s.mean_in = a.mean; s.rstd_in = a.rstd; s.dmean = dmean_out; s.dvar = dvar_out;
         s.gamma = a.gamma; s.beta = a.beta;
         return small_backward(bn, s, I, a.O, st);
     }
     // dx starts from zero (the reference's CPU path: dx_buf.FillZero(), DifferentiableLutN.h:1159)
-    if (I > 0 && a.dxs > 0) {
-        const int rc = zero_async(a.dx, sizeof(float) * (size_t)I * a.dxs, st);
-        if (rc) return rc;
+    const size_t dx_bytes = sizeof(float) * (size_t)(I > 0 ? I : 0) * (size_t)(a.dxs > 0 ? a.dxs : 0);
+    if (a.O == 0 || a.F == 0) {
+        BB200_CUDA(cudaMemsetAsync(a.dx, 0, dx_bytes, st));
+        return BBCU_OK;
     }
-    if (a.O == 0 || a.F == 0) return BBCU_OK;
     a.groups = (a.O + kWarpsPerCta - 1) / kWarpsPerCta;
     const long long rows = (long long)(I < 6LL * a.O ? I : 6LL * a.O);
     // Wide tiles: a warp reduces its 64 dW accumulators across lanes once per (node, tile), about 250 instructions, so the
@@ -1249,28 +1296,31 @@ static int backward_common(BwdArgs a, bool bn, long long total_frames, float *dm
         if (ext_sums == nullptr) {
             double *sums = static_cast<double *>(stream_scratch(st, sizeof(double) * 2 * (size_t)a.O));
             BB200_REQUIRE(sums != nullptr, BBCU_ERR_NO_MEMORY);
-            BB200_CUDA(cudaMemsetAsync(sums, 0, sizeof(double) * 2 * (size_t)a.O, st));
             a.sums = sums;
             int rc = BBCU_OK;
             if (XBIT || !backward_stats_pipe(a, st, &rc, tmp, tmp_bytes)) {
+                BB200_CUDA(cudaMemsetAsync(sums, 0, sizeof(double) * 2 * (size_t)a.O, st));
                 k_lut6_backward_stats<XBIT><<<(unsigned)blocks, kWarpsPerCta * 32, 0, st>>>(a);
                 rc = launch_status();
             }
             if (rc) return rc;
             ext_sums = sums;
         }
-        k_bn_backward_finalize<<<(a.O + 255) / 256, 256, 0, st>>>(ext_sums, a.mean, a.rstd, dmean_out, dvar_out, a.O, total_frames);
-        BB200_CUDA(cudaPeekAtLastError());
-        a.dmean = dmean_out; a.dvar = dvar_out;
     }
     if (!XBIT) {
         // rows on 16-byte boundaries (the FrameBuffer layout gives them): the persistent kernel
         const bool aligned = ((reinterpret_cast<uintptr_t>(a.x) | reinterpret_cast<uintptr_t>(a.dy) | reinterpret_cast<uintptr_t>(a.dx) |
                                reinterpret_cast<uintptr_t>(a.dW)) & 15) == 0 && (a.xs % 4) == 0 && (a.dys % 4) == 0 && (a.dxs % 4) == 0;
         if (aligned) {
-            const int rc = launch_backward_pipe(a, bn, I, tmp, tmp_bytes, st);
+            const int rc = launch_backward_pipe(a, bn, I, bn ? ext_sums : nullptr, dmean_out, dvar_out, total_frames, tmp, tmp_bytes, st);
             if (rc != BBCU_ERR_NO_MEMORY) return rc;
         }
+    }
+    BB200_CUDA(cudaMemsetAsync(a.dx, 0, dx_bytes, st));
+    if (bn) {
+        k_bn_backward_finalize<<<(a.O + 255) / 256, 256, 0, st>>>(ext_sums, a.mean, a.rstd, dmean_out, dvar_out, a.O, total_frames);
+        BB200_CUDA(cudaPeekAtLastError());
+        a.dmean = dmean_out; a.dvar = dvar_out;
     }
     if (bn) k_lut6_backward<XBIT, true><<<(unsigned)blocks, kWarpsPerCta * 32, 0, st>>>(a);
     else    k_lut6_backward<XBIT, false><<<(unsigned)blocks, kWarpsPerCta * 32, 0, st>>>(a);
@@ -1383,13 +1433,13 @@ static int dl6_finalize_and_normalize(float *y, const double *sums, float *mean,
                                       int binary, cudaStream_t st)
 {
     if (O == 0) return BBCU_OK;
-    k_bn_finalize<<<(O + 255) / 256, 256, 0, st>>>(sums, mean, rstd, rmean, rvar, momentum, O, total_frames);
-    BB200_CUDA(cudaPeekAtLastError());
     if (y != nullptr && F > 0) {
         const int chunks = (F + 4095) / 4096;
         const long long blocks = (long long)O * chunks;
         BB200_REQUIRE(blocks < (1LL << 31), BBCU_ERR_TOO_LARGE);
-        k_bn_normalize_inplace<<<(unsigned)blocks, 256, 0, st>>>(y, mean, rstd, gamma, beta, F, ys, binary, chunks);
+        k_bn_normalize_inplace<<<(unsigned)blocks, 256, 0, st>>>(y, sums, mean, rstd, rmean, rvar, gamma, beta, momentum, total_frames, F, ys, binary, chunks);
+    } else {
+        k_bn_finalize<<<(O + 255) / 256, 256, 0, st>>>(sums, mean, rstd, rmean, rvar, momentum, O, total_frames);
     }
     return launch_status();
 }
@@ -1407,7 +1457,6 @@ int dl6_forward_stats(const float *x, float *y, const int *idx, const float *W, 
                                          unbinarize_bias, node_size, frame_size, frame_stride, lut_binarize, st);
         if (rc != BBCU_ERR_NO_MEMORY) return rc;
     }
-    BB200_CUDA(cudaMemsetAsync(dev_sums, 0, sizeof(double) * 2 * (size_t)node_size, st));
     FwdArgs a = {};
     a.x = x; a.y = y; a.idx = idx; a.W = W; a.sums = dev_sums; a.bias = unbinarize_bias;
     a.O = node_size; a.F = frame_size; a.xs = frame_stride; a.ys = frame_stride; a.lut_binarize = lut_binarize; a.binary = binary_mode;
@@ -1487,7 +1536,6 @@ extern "C" int bbcu_bit_fp32_DifferentiableLut6_ForwardTraining(const int *x, in
     if (rc != BBCU_ERR_NO_MEMORY) return rc;
     double *sums = static_cast<double *>(stream_scratch(st, sizeof(double) * 2 * (size_t)node_size));
     BB200_REQUIRE(sums != nullptr, BBCU_ERR_NO_MEMORY);
-    BB200_CUDA(cudaMemsetAsync(sums, 0, sizeof(double) * 2 * (size_t)node_size, st));
     FwdArgs a = {};
     a.x = x; a.ybits = reinterpret_cast<uint32_t *>(y); a.idx = idx; a.W = W; a.sums = sums; a.bias = unbinarize_bias;
     a.gamma = gamma; a.beta = beta;
@@ -1610,14 +1658,15 @@ extern "C" int bbcu_fp32_DifferentiableLut6_BackwardStats(const float *x, const 
                                          lut_binarize, st);
         if (rc != BBCU_ERR_NO_MEMORY) return rc;
     }
-    BB200_CUDA(cudaMemsetAsync(dev_sums, 0, sizeof(double) * 2 * (size_t)node_size, st));
-    if (node_size == 0 || frame_size == 0) return BBCU_OK;
+    if (node_size == 0) return BBCU_OK;
+    if (frame_size == 0) { BB200_CUDA(cudaMemsetAsync(dev_sums, 0, sizeof(double) * 2 * (size_t)node_size, st)); return BBCU_OK; }
     BwdArgs a = {};
     a.x = x; a.dy = dy; a.idx = idx; a.W = W; a.mean = mean; a.rstd = rstd; a.sums = dev_sums;
     a.gamma = gamma; a.beta = beta; a.bias = unbinarize_bias;
     a.O = node_size; a.F = frame_size; a.xs = frame_stride; a.dys = frame_stride; a.lut_binarize = lut_binarize; a.binary = binary_mode;
     a.groups = (a.O + kWarpsPerCta - 1) / kWarpsPerCta;
     if (backward_stats_pipe(a, st, &rc)) return rc;
+    BB200_CUDA(cudaMemsetAsync(dev_sums, 0, sizeof(double) * 2 * (size_t)node_size, st));
     a.T = frame_tile(3LL * a.O, 32, a.groups, a.F, 2048);
     const long long blocks = (long long)((a.F + a.T - 1) / a.T) * a.groups;
     BB200_REQUIRE(blocks < (1LL << 31), BBCU_ERR_TOO_LARGE);
@@ -1634,9 +1683,10 @@ extern "C" int bbcu_fp32_DifferentiableLut6_BackwardStatsFromOutput(const float 
     BB200_REQUIRE(binary_mode == 0, BBCU_ERR_BAD_SIZE);          // a binarised output does not carry the pre-activation value
     BB200_REQUIRE(frame_stride >= frame_size, BBCU_ERR_BAD_STRIDE);
     cudaStream_t st = as_stream(stream);
-    BB200_CUDA(cudaMemsetAsync(dev_sums, 0, sizeof(double) * 2 * (size_t)node_size, st));
-    if (node_size == 0 || frame_size == 0) return BBCU_OK;
+    if (node_size == 0) return BBCU_OK;
     const int chunks = (frame_size + 8191) / 8192;
+    if (chunks != 1) BB200_CUDA(cudaMemsetAsync(dev_sums, 0, sizeof(double) * 2 * (size_t)node_size, st));
+    if (frame_size == 0) return BBCU_OK;
     BB200_REQUIRE((long long)node_size * chunks < (1LL << 31), BBCU_ERR_TOO_LARGE);
     k_dl6_backward_stats_from_y<<<node_size * chunks, 256, 0, st>>>(y, dy, rstd, dev_sums, gamma, beta, frame_size, frame_stride, frame_stride,
                                                                     chunks);

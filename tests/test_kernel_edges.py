@@ -105,6 +105,12 @@ def test_small_probability_layers_edges(ops, I, O, F, stride):
     parity._dl6_fp32_check(ops, x, idx, W, dy, rng.random(O, dtype=np.float32), rng.random(O, dtype=np.float32) + 0.5, dict(binary=0, lut_binarize=0), stride)
 
 
+# above the one-launch range: persistent kernels (tile remainders, a short last group of nodes, one and several chunks of the statistics), rows that are not aligned
+@pytest.mark.parametrize("I,O,F,stride", [(6, 1, 4097, None), (33, 17, 4225, 4228), (33, 17, 4225, 4227), (700, 1025, 2049, None), (9, 5, 20011, None)])
+def test_large_probability_layers_edges(ops, I, O, F, stride):
+    test_small_probability_layers_edges(ops, I, O, F, stride)
+
+
 # one CTA (up to 2^15 target values) and the general form; Adam with the gradients cleared on the way, whole quads and a remainder
 @pytest.mark.parametrize("classes,frames", [(1, 1), (10, 129), (10, 3276), (10, 3277), (3, 20000)])
 def test_mean_loss_and_adam_update(ops, classes, frames):
