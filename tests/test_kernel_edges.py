@@ -129,3 +129,13 @@ def test_mean_loss_and_adam_update(ops, classes, frames):
         ops.Adam([Wd], [dWd]).update()
         port.adam_update(W, dW, np.zeros_like(W), np.zeros_like(W), np.ones(2, np.float32))
         assert np.abs(Wd.cpu().numpy() - W).max() <= 1e-6 and not dWd.any()
+
+
+# Im2Col by quads of pixels (filters 3 and 5 wide, one band and several, a short last band, every border) and bit Im2Col with several word columns
+# a block, several periods a warp, split blocks, windows beyond four and words without any
+@pytest.mark.parametrize("c,h,w,fh,fw,ys,xs,pad,F", [
+    (2, 5, 8, 3, 3, 1, 1, "same", 33), (3, 19, 12, 5, 5, 1, 1, "same", 70), (2, 9, 36, 3, 3, 1, 1, "valid", 31), (1, 20, 64, 3, 5, 1, 1, "same", 100),
+    (64, 8, 8, 3, 3, 1, 1, "same", 600), (40, 6, 8, 3, 3, 1, 1, "same", 300), (1, 4, 4, 1, 1, 1, 1, "same", 65), (5, 3, 7, 5, 4, 2, 1, "same", 290)])
+def test_im2col_quads_and_bit_columns(ops, c, h, w, fh, fw, ys, xs, pad, F):
+    import test_conv_lowering as lowering
+    lowering.test_im2col_bands_and_bit_words_against_oracle(c, h, w, fh, fw, ys, xs, pad, F)
