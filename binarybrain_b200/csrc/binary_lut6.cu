@@ -182,12 +182,12 @@ struct MuxTree<1, K, NW> {
 
 // ---------------------------------------------------------------------------------------------
 // Persistent, bulk-copy-pipelined variant (aligned rows; the launcher's default).
-// Work item = (word tile of 256 words, group of 8 nodes); CTA c takes items c, c + gridDim, ... so the CTAs in
-// flight sweep the node groups of one tile together and the tile's rows stay in L2.  Each warp owns one node of
-// the group and runs its own two-stage pipeline: lane 0 starts six 1 KiB bulk copies (one per gathered row) for
-// item j+2 as soon as item j has been read out of shared memory into registers, then the warp computes item j
-// while the copies of j+1 and j+2 are in flight.  No warp ever waits on a load it has only just issued, and no
-// CTA-wide barrier exists after set-up.
+// Work item = (word tile of 256 words, node) of one warp; the warps of the grid take the items in order, so that those in
+// flight sweep the nodes of one tile together and the tile's rows stay in L2.  (Items of a CTA and eight nodes left warps
+// idle where the nodes are no multiple of 8: 36 nodes x 2^20 frames 8.9 -> 8.1 us.)  Each warp runs its own two-stage
+// pipeline: its lanes start six 1 KiB bulk copies (one per gathered row) for item j+2 as soon as item j has been read out
+// of shared memory into registers, then the warp computes item j while the copies of j+1 and j+2 are in flight.  No warp
+// ever waits on a load it has only just issued, and no CTA-wide barrier exists after set-up.
 // ---------------------------------------------------------------------------------------------
 constexpr int kPipeCtas   = 2;                        // resident CTAs per SM
 constexpr int kPipeNW     = 8;                        // words per lane and item
@@ -202,14 +202,14 @@ static_assert(kBlWarps * kPipeStages * 8 <= kPipeBarBytes, "barrier block too sm
 
 // Position of a work item, advanced incrementally (item index + gridDim) so that no division runs per item.
 struct PipePos {
-    int tile, group;
+    int tile, node;
 };
 
-__device__ __forceinline__ PipePos pipe_advance(PipePos p, int dt, int dg, int groups)
+__device__ __forceinline__ PipePos pipe_advance(PipePos p, int dt, int dn, int nodes)
 {
-    p.group += dg;
+    p.node += dn;
     p.tile += dt;
-    if (p.group >= groups) { p.group -= groups; ++p.tile; }
+    if (p.node >= nodes) { p.node -= nodes; ++p.tile; }
     return p;
 }
 
@@ -225,9 +225,8 @@ __device__ __forceinline__ void pipe_issue(const BlArgs &a, PipePos pos, int row
     if (lane < 6) bulk_copy_g2s(stage + lane * kPipeWords, a.x + (size_t)row * a.stride + w0, bytes, bar);
 }
 
-__device__ __forceinline__ int pipe_row(const BlArgs &a, PipePos pos, int warp, int lane)
+__device__ __forceinline__ int pipe_row(const BlArgs &a, int node, int lane)
 {
-    const int node = min(pos.group * kBlWarps + warp, a.O - 1);
     return lane < 6 ? __ldg(a.idx + (size_t)node * 6 + lane) : 0;
 }
 
@@ -250,27 +249,25 @@ k_binary_lut6_pipe(const BlArgs a, int n_tiles, int *fault)
     }
     __syncwarp();
 
-    // items blockIdx, blockIdx + gridDim, ...: position of the current item and of the next two
-    const int step = (int)gridDim.x;
-    const int dt = step / a.groups, dg = step - dt * a.groups;
+    // items first, first + all warps, ...: position of the current item and of the next two
+    const int step = (int)gridDim.x * kBlWarps, first = (int)blockIdx.x * kBlWarps + warp;
+    const int dt = step / a.O, dn = step - dt * a.O;
     PipePos p0;
-    p0.tile  = (int)blockIdx.x / a.groups;
-    p0.group = (int)blockIdx.x - p0.tile * a.groups;
-    PipePos p1 = pipe_advance(p0, dt, dg, a.groups);
-    PipePos p2 = pipe_advance(p1, dt, dg, a.groups);
+    p0.tile = first / a.O;
+    p0.node = first - p0.tile * a.O;
+    PipePos p1 = pipe_advance(p0, dt, dn, a.O);
+    PipePos p2 = pipe_advance(p1, dt, dn, a.O);
 
-    if (p0.tile < n_tiles) pipe_issue(a, p0, pipe_row(a, p0, warp, lane), lane, my_rows, my_bar);
-    if (p1.tile < n_tiles) pipe_issue(a, p1, pipe_row(a, p1, warp, lane), lane, my_rows + 6 * kPipeWords, my_bar + 1);
-    int row2 = p2.tile < n_tiles ? pipe_row(a, p2, warp, lane) : 0;          // input rows of item k+2, one item ahead of their use
+    if (p0.tile < n_tiles) pipe_issue(a, p0, pipe_row(a, p0.node, lane), lane, my_rows, my_bar);
+    if (p1.tile < n_tiles) pipe_issue(a, p1, pipe_row(a, p1.node, lane), lane, my_rows + 6 * kPipeWords, my_bar + 1);
+    int row2 = p2.tile < n_tiles ? pipe_row(a, p2.node, lane) : 0;          // input rows of item k+2, one item ahead of their use
     uint32_t tword = 0;
-    if (p0.tile < n_tiles) tword = (uint32_t)__ldg(a.table + 2 * (size_t)min(p0.group * kBlWarps + warp, a.O - 1) + (lane >> 4));
+    if (p0.tile < n_tiles) tword = (uint32_t)__ldg(a.table + 2 * (size_t)p0.node + (lane >> 4));
 
     for (int k = 0; p0.tile < n_tiles; ++k) {
         const int s = k & 1;
         const uint32_t parity = (uint32_t)(k >> 1) & 1u;
         uint32_t *stage = my_rows + s * 6 * kPipeWords;
-        const int node = p0.group * kBlWarps + warp;
-        const bool store = node < a.O;
         const int w0 = p0.tile * kPipeWords;
         const int nw = min(kPipeWords, a.nwords - w0);
 
@@ -282,7 +279,7 @@ k_binary_lut6_pipe(const BlArgs a, int n_tiles, int *fault)
             __syncwarp();
         }
         const bool have_next = p1.tile < n_tiles;
-        if (have_next) tword = (uint32_t)__ldg(a.table + 2 * (size_t)min(p1.group * kBlWarps + warp, a.O - 1) + (lane >> 4));
+        if (have_next) tword = (uint32_t)__ldg(a.table + 2 * (size_t)p1.node + (lane >> 4));
 
         if (!mbar_wait(my_bar + s, parity)) {          // bounded: record the fault, let the other stage's copies land, leave
             if (lane == 0) atomicCAS(fault, 0, kFaultBarrierTimeout);
@@ -304,13 +301,13 @@ k_binary_lut6_pipe(const BlArgs a, int n_tiles, int *fault)
             proxy_fence_async();                        // reads above (generic proxy) before the refill (async proxy)
             pipe_issue(a, p2, row2, lane, stage, my_bar + s);
         }
-        const PipePos p3 = pipe_advance(p2, dt, dg, a.groups);
-        if (p3.tile < n_tiles) row2 = pipe_row(a, p3, warp, lane);
+        const PipePos p3 = pipe_advance(p2, dt, dn, a.O);
+        if (p3.tile < n_tiles) row2 = pipe_row(a, p3.node, lane);
         MuxTree<6, 0, kPipeNW>::eval(my_ab, xw, o);
-        uint32_t *yrow = a.y + (size_t)min(node, a.O - 1) * a.stride + w0;
+        uint32_t *yrow = a.y + (size_t)p0.node * a.stride + w0;
 #pragma unroll
         for (int h = 0; h < kPipeNW / 4; ++h)
-            if (store && w + 128 * h < nw) *reinterpret_cast<uint4 *>(yrow + w + 128 * h) = make_uint4(o[4 * h], o[4 * h + 1], o[4 * h + 2], o[4 * h + 3]);
+            if (w + 128 * h < nw) *reinterpret_cast<uint4 *>(yrow + w + 128 * h) = make_uint4(o[4 * h], o[4 * h + 1], o[4 * h + 2], o[4 * h + 3]);
 
         p0 = p1; p1 = p2; p2 = p3;
     }
@@ -416,15 +413,15 @@ k_binary_lut6_imm(const BlArgs a, int n_tiles)
 
     const int step = (int)gridDim.x;
     const int dt = step / a.groups, dg = step - dt * a.groups;
-    PipePos pi;                                        // copy side: two items ahead
+    PipePos pi;                                        // copy side: two items ahead (an item is a CTA's: `node` counts groups of nodes)
     pi.tile  = (int)blockIdx.x / a.groups;
-    pi.group = (int)blockIdx.x - pi.tile * a.groups;
+    pi.node = (int)blockIdx.x - pi.tile * a.groups;
     PipePos pc = pi;                                   // arithmetic side
-    int row_i = pi.tile < n_tiles ? pipe_row(a, pi, warp, lane) : 0;
+    int row_i = pi.tile < n_tiles ? pipe_row(a, min(pi.node * kBlWarps + warp, a.O - 1), lane) : 0;
     int row_n;
     {
         const PipePos t = pipe_advance(pi, dt, dg, a.groups);
-        row_n = t.tile < n_tiles ? pipe_row(a, t, warp, lane) : 0;
+        row_n = t.tile < n_tiles ? pipe_row(a, min(t.node * kBlWarps + warp, a.O - 1), lane) : 0;
     }
     int ist = 0;
     auto issue = [&]() {
@@ -443,7 +440,7 @@ k_binary_lut6_imm(const BlArgs a, int n_tiles)
             pi = pipe_advance(pi, dt, dg, a.groups);
             row_i = row_n;
             const PipePos t = pipe_advance(pi, dt, dg, a.groups);
-            row_n = t.tile < n_tiles ? pipe_row(a, t, warp, lane) : 0;
+            row_n = t.tile < n_tiles ? pipe_row(a, min(t.node * kBlWarps + warp, a.O - 1), lane) : 0;
         }
         cp_async_commit();
         ist ^= 1;
@@ -452,15 +449,15 @@ k_binary_lut6_imm(const BlArgs a, int n_tiles)
     issue();
 
     uint2 tab_n = make_uint2(0u, 0u);                   // the node's 64-bit table, one item ahead of its use
-    if (pc.tile < n_tiles) tab_n = __ldg(reinterpret_cast<const uint2 *>(a.table) + min(pc.group * kBlWarps + warp, a.O - 1));
+    if (pc.tile < n_tiles) tab_n = __ldg(reinterpret_cast<const uint2 *>(a.table) + min(pc.node * kBlWarps + warp, a.O - 1));
     int cst = 0;
     while (pc.tile < n_tiles) {
-        const int node = pc.group * kBlWarps + warp;
+        const int node = pc.node * kBlWarps + warp;
         const bool store = node < a.O;
         const int w0 = pc.tile * kImmWords;
         const uint2 tab = tab_n;
         const PipePos pn = pipe_advance(pc, dt, dg, a.groups);
-        if (pn.tile < n_tiles) tab_n = __ldg(reinterpret_cast<const uint2 *>(a.table) + min(pn.group * kBlWarps + warp, a.O - 1));
+        if (pn.tile < n_tiles) tab_n = __ldg(reinterpret_cast<const uint2 *>(a.table) + min(pn.node * kBlWarps + warp, a.O - 1));
 
         cp_async_wait<1>();                             // the copies of this item (this lane's own pieces) have landed
         const uint32_t *st = my + cst * 6 * kImmWords + 4 * lane;
