@@ -48,6 +48,7 @@ __device__ __forceinline__ uint32_t lut6_word(uint32_t x0, uint32_t x1, uint32_t
 __global__ void __launch_bounds__(kBlWarps * 32)
 k_binary_lut6(const BlArgs a)
 {
+    grid_dependency();
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
     const int tile = blockIdx.x / a.groups;
     const int node = (blockIdx.x % a.groups) * kBlWarps + warp;
@@ -109,6 +110,7 @@ __device__ __forceinline__ uint32_t lut6_word_imad(uint32_t x0, uint32_t x1, uin
 __global__ void __launch_bounds__(kBlWarps * 32)
 k_binary_lut6_2pipe(const BlArgs a)
 {
+    grid_dependency();
     __shared__ int2 s_ab[kBlWarps][32];
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
     const int tile = blockIdx.x / a.groups;
@@ -233,6 +235,7 @@ __device__ __forceinline__ int pipe_row(const BlArgs &a, int node, int lane)
 __global__ void __launch_bounds__(kBlWarps * 32, kPipeCtas)
 k_binary_lut6_pipe(const BlArgs a, int n_tiles, int *fault)
 {
+    grid_dependency();
     extern __shared__ __align__(128) unsigned char smem_raw[];
     uint32_t *s_rows = reinterpret_cast<uint32_t *>(smem_raw);                                   // [warp][stage][6][256]
     uint64_t *s_bar  = reinterpret_cast<uint64_t *>(smem_raw + kPipeRowsBytes);                   // [warp][stage]
@@ -407,6 +410,7 @@ __device__ __forceinline__ void lut6_words_by_immediates(uint32_t (&y)[16], cons
 __global__ void __launch_bounds__(kBlWarps * 32, 1)
 k_binary_lut6_imm(const BlArgs a, int n_tiles)
 {
+    grid_dependency();
     extern __shared__ __align__(128) unsigned char smem_raw[];
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
     uint32_t *my = reinterpret_cast<uint32_t *>(smem_raw) + (size_t)warp * kImmStages * 6 * kImmWords;
@@ -516,13 +520,13 @@ extern "C" int bbcu_bit_BinaryLut6_Forward(const int *x, int *y, const int *idx,
             BB200_REQUIRE(n_items < (1LL << 31) - 4096, BBCU_ERR_TOO_LARGE);      // 32-bit item arithmetic in the kernel
             long long grid = (long long)kPipeCtas * device_info().sm_count;
             if (grid > n_items) grid = n_items;
-            k_binary_lut6_pipe<<<(unsigned)grid, kBlWarps * 32, kPipeSmem, as_stream(stream)>>>(a, (a.nwords + kPipeWords - 1) / kPipeWords, fault);
+            launch(k_binary_lut6_pipe, (unsigned)grid, kBlWarps * 32, kPipeSmem, as_stream(stream), a, (a.nwords + kPipeWords - 1) / kPipeWords, fault);
             return launch_status();
         }
     }
     // aligned rows without the shared-memory opt-in (or without a fault word): the non-pipelined 128-bit kernel; otherwise word loads
-    if (vec) k_binary_lut6_2pipe<<<(unsigned)blocks, kBlWarps * 32, 0, as_stream(stream)>>>(a);
-    else     k_binary_lut6<<<(unsigned)blocks, kBlWarps * 32, 0, as_stream(stream)>>>(a);
+    if (vec) launch(k_binary_lut6_2pipe, (unsigned)blocks, kBlWarps * 32, 0, as_stream(stream), a);
+    else     launch(k_binary_lut6, (unsigned)blocks, kBlWarps * 32, 0, as_stream(stream), a);
     return launch_status();
 }
 
@@ -551,7 +555,7 @@ extern "C" int bbcu_bit_BinaryLut6_Forward_Lop3Immediate(const int *x, int *y, c
     BB200_REQUIRE(n_items < (1LL << 31) - 4096, BBCU_ERR_TOO_LARGE);
     long long grid = device_info().sm_count;
     if (grid > n_items) grid = n_items;
-    k_binary_lut6_imm<<<(unsigned)grid, kBlWarps * 32, kImmSmem, as_stream(stream)>>>(a, n_tiles);
+    launch(k_binary_lut6_imm, (unsigned)grid, kBlWarps * 32, kImmSmem, as_stream(stream), a, n_tiles);
     return launch_status();
 }
 

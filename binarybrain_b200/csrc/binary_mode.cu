@@ -41,6 +41,7 @@ __global__ void __launch_bounds__(kWarpsPerCta * 32)
 k_pattern_values(const float *__restrict__ W, float *__restrict__ Y, int *__restrict__ table, const float *__restrict__ mean_buf,
                  const float *__restrict__ var_buf, float gamma, float beta, float bias, int O, int lut_binarize)
 {
+    grid_dependency();
     __shared__ float4 s_tab[kWarpsPerCta][32];
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
     const int node = blockIdx.x * kWarpsPerCta + warp;
@@ -103,6 +104,7 @@ __global__ void __launch_bounds__(kWarpsPerCta * 32)
 k_pattern_histogram(const uint32_t *__restrict__ x, const int *__restrict__ idx, uint32_t *__restrict__ hist, int O, int F, long long xs, int groups,
                     int tile_words)
 {
+    grid_dependency();
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
     const int tile = blockIdx.x / groups;
     const int node = (blockIdx.x % groups) * kWarpsPerCta + warp;
@@ -137,6 +139,7 @@ __global__ void __launch_bounds__(kWarpsPerCta * 32)
 k_dl6_bit_train_finalize(const float *__restrict__ Y, const uint32_t *__restrict__ hist, int *__restrict__ table, float *mean_out, float *rstd_out,
                          float *running_mean, float *running_var, float gamma, float beta, float momentum, int O, int F)
 {
+    grid_dependency();
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
     const int node = blockIdx.x * kWarpsPerCta + warp;
     if (node >= O) return;
@@ -167,6 +170,7 @@ k_dl6_bit_train_finalize(const float *__restrict__ Y, const uint32_t *__restrict
 // BinaryLut6 leaves the bits past the last frame as its inputs make them; these layers clear them.
 __global__ void k_clear_tail_bits(uint32_t *y, int O, int F, long long ys)
 {
+    grid_dependency();
     const int node = blockIdx.x * blockDim.x + threadIdx.x;
     if (node >= O) return;
     y[(size_t)node * ys + (F >> 5)] &= (1u << (F & 31)) - 1u;
@@ -181,6 +185,7 @@ __global__ void __launch_bounds__(kWarpsPerCta * 32)
 k_bit_gather_forward(const uint32_t *__restrict__ x, float *__restrict__ y, const int *__restrict__ idx, const float *__restrict__ Y, int O, int F,
                      long long xs, long long ys, int groups, int tile_words)
 {
+    grid_dependency();
     __shared__ float s_val[kWarpsPerCta][64];
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
     const int tile = blockIdx.x / groups;
@@ -275,6 +280,7 @@ __device__ __forceinline__ float4 load_frames(const float *row, long long f, int
 __global__ void __launch_bounds__(kWarpsPerCta * 32)
 k_pack_bits(const float *__restrict__ x, uint32_t *__restrict__ bits, int I, int F, long long xs, long long ws, int runs)
 {
+    grid_dependency();
     const int lane = threadIdx.x & 31;
     const long long unit = (long long)blockIdx.x * kWarpsPerCta + (threadIdx.x >> 5);
     const int row = (int)(unit / runs), run = (int)(unit - (long long)row * runs);
@@ -347,6 +353,7 @@ template <bool XF32, bool BN>
 __global__ void __launch_bounds__(kPsWarps * 32)
 k_pattern_sums(const BitBwdArgs a)
 {
+    grid_dependency();
     extern __shared__ __align__(16) unsigned char smem_raw[];
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
     const int tile = blockIdx.x / a.groups;
@@ -439,6 +446,7 @@ k_pattern_sums(const BitBwdArgs a)
 // ---- the consumers of every input row, as lists of 8 node + input number
 __global__ void k_edge_count(const int *__restrict__ idx, int *count, int edges)
 {
+    grid_dependency();
     const int e = blockIdx.x * blockDim.x + threadIdx.x;
     if (e < edges) atomicAdd(count + idx[e], 1);
 }
@@ -446,6 +454,7 @@ __global__ void k_edge_count(const int *__restrict__ idx, int *count, int edges)
 // room for every row's list, in no particular order: `total` is a bump pointer, advanced once per warp
 __global__ void k_edge_room(const int *__restrict__ count, int *cursor, int *total, int I)
 {
+    grid_dependency();
     const int i = blockIdx.x * blockDim.x + threadIdx.x, lane = threadIdx.x & 31;
     const int n = i < I ? count[i] : 0;
     int at = n;
@@ -463,6 +472,7 @@ __global__ void k_edge_room(const int *__restrict__ count, int *cursor, int *tot
 // afterwards cursor[i] is the end of row i's list
 __global__ void k_edge_fill(const int *__restrict__ idx, int *cursor, int *list, int edges)
 {
+    grid_dependency();
     const int e = blockIdx.x * blockDim.x + threadIdx.x;
     if (e < edges) list[atomicAdd(cursor + idx[e], 1)] = e + 2 * (e / 6);
 }
@@ -535,6 +545,7 @@ template <bool BN, int NC>
 __global__ void __launch_bounds__(kWarpsPerCta * 32, 4)
 k_pattern_gather(const BitBwdArgs a)
 {
+    grid_dependency();
     extern __shared__ __align__(16) unsigned char smem_raw[];           // split > 1: float4 [split][NC][32]
     float4 *s_part = reinterpret_cast<float4 *>(smem_raw);
     const int part = threadIdx.x >> 5, lane = threadIdx.x & 31;
@@ -633,6 +644,7 @@ __device__ __forceinline__ void store_edge_tables(float *etab, int lane, const f
 __global__ void __launch_bounds__(kWarpsPerCta * 32)
 k_pattern_derivatives(const float *__restrict__ W, float *__restrict__ etab, float bias, int O, int lut_binarize)
 {
+    grid_dependency();
     __shared__ float4 s_tab[kWarpsPerCta][16];
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
     const int node = blockIdx.x * kWarpsPerCta + warp;
@@ -648,6 +660,7 @@ __global__ void __launch_bounds__(kWarpsPerCta * 32)
 k_pattern_masks(const float *__restrict__ W, uint2 *__restrict__ mask, const float *__restrict__ mean_buf, const float *__restrict__ rstd_buf, float gamma,
                 float beta, float bias, int O, int lut_binarize)
 {
+    grid_dependency();
     __shared__ float4 s_tab[kWarpsPerCta][16];
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
     const int node = blockIdx.x * kWarpsPerCta + warp;
@@ -677,6 +690,7 @@ k_bit_backward_finalize(const float *__restrict__ hdy, const uint32_t *__restric
                         float *__restrict__ etab, float2 *__restrict__ ntab, float *dW, const float *__restrict__ mean_buf, const float *__restrict__ rstd_buf, float *dmean_out, float *dvar_out, float gamma,
                         float beta, float bias, int O, float rF, int lut_binarize, double *sums_out, const double *__restrict__ sums_in)
 {
+    grid_dependency();
     __shared__ float4 s_tab[BN ? kWarpsPerCta : 1][16];
     __shared__ float s_hg[kWarpsPerCta][64];
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
@@ -750,6 +764,7 @@ template <int PASS>
 __global__ void __launch_bounds__(kWarpsPerCta * 32)
 k_f32_binary_forward(const F32BinArgs a)
 {
+    grid_dependency();
     __shared__ float    s_val[kWarpsPerCta][64];
     __shared__ unsigned s_cnt[kWarpsPerCta][64];
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
@@ -831,6 +846,7 @@ k_f32_binary_forward(const F32BinArgs a)
 __global__ void __launch_bounds__(kWarpsPerCta * 32)
 k_counts_to_sums(const float *__restrict__ Y, const uint32_t *__restrict__ hist, double *__restrict__ sums, int O)
 {
+    grid_dependency();
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
     const int node = blockIdx.x * kWarpsPerCta + warp;
     if (node >= O) return;
@@ -886,6 +902,7 @@ template <bool XBIT>
 __global__ void __launch_bounds__(kWarpsPerCta * 32)
 k_small_binary_forward(const SmallBinArgs a)
 {
+    grid_dependency();
     __shared__ float4 s_tab[32];
     __shared__ unsigned s_cnt[64];
     __shared__ unsigned s_table[2];
@@ -974,6 +991,7 @@ template <bool XBIT, bool BN>
 __global__ void __launch_bounds__(kWarpsPerCta * 32)
 k_small_binary_backward(const SmallBinArgs a)
 {
+    grid_dependency();
     __shared__ float4 s_tab[16];
     __shared__ float s_hdy[64], s_hg[64];
     __shared__ unsigned s_cnt[64];
@@ -1150,7 +1168,7 @@ int run_binary_lut(const int *x, int *y, const int *idx, const int *table, int O
     int rc = bbcu_bit_BinaryLut6_Forward(x, y, idx, table, O, F, stride, reinterpret_cast<bbcu_stream_t>(st));
     if (rc) return rc;
     if (F & 31) {
-        k_clear_tail_bits<<<(O + 255) / 256, 256, 0, st>>>(reinterpret_cast<uint32_t *>(y), O, F, stride);
+        launch(k_clear_tail_bits, (O + 255) / 256, 256, 0, st, reinterpret_cast<uint32_t *>(y), O, F, stride);
         return launch_status();
     }
     return BBCU_OK;
@@ -1167,8 +1185,8 @@ int bit_forward_by_table(bool with_bn, const int *x, int *y, const int *idx, con
     Scratch s;
     if (!carve(s, O, st)) return BBCU_ERR_NO_MEMORY;
     const int blocks = (O + kWarpsPerCta - 1) / kWarpsPerCta;
-    if (with_bn) k_pattern_values<kTableNorm><<<blocks, kWarpsPerCta * 32, 0, st>>>(W, nullptr, s.table, rmean, rvar, gamma, beta, bias, O, lut_binarize);
-    else         k_pattern_values<kTableRaw><<<blocks, kWarpsPerCta * 32, 0, st>>>(W, nullptr, s.table, nullptr, nullptr, 0.0f, 0.0f, bias, O, lut_binarize);
+    if (with_bn) launch(k_pattern_values<kTableNorm>, blocks, kWarpsPerCta * 32, 0, st, W, nullptr, s.table, rmean, rvar, gamma, beta, bias, O, lut_binarize);
+    else         launch(k_pattern_values<kTableRaw>, blocks, kWarpsPerCta * 32, 0, st, W, nullptr, s.table, nullptr, nullptr, 0.0f, 0.0f, bias, O, lut_binarize);
     BB200_CUDA(cudaPeekAtLastError());
     return run_binary_lut(x, y, idx, s.table, O, F, stride, st);
 }
@@ -1182,13 +1200,13 @@ int dl6_bit_forward_training_by_table(const int *x, int *y, const int *idx, cons
         SmallBinArgs a = {};
         a.x = x; a.y = y; a.idx = idx; a.W = W; a.mean = mean; a.rstd = rstd; a.running_mean = rmean; a.running_var = rvar;
         a.gamma = gamma; a.beta = beta; a.momentum = momentum; a.bias = bias; a.F = F; a.lut_binarize = lut_binarize; a.xs = stride; a.ys = stride;
-        k_small_binary_forward<true><<<O, small_threads(F), 0, st>>>(a);
+        launch(k_small_binary_forward<true>, O, small_threads(F), 0, st, a);
         return launch_status();
     }
     Scratch s;
     if (!carve(s, O, st)) return BBCU_ERR_NO_MEMORY;
     const int groups = (O + kWarpsPerCta - 1) / kWarpsPerCta;
-    k_pattern_values<kTableNone><<<groups, kWarpsPerCta * 32, 0, st>>>(W, s.Y, nullptr, nullptr, nullptr, 0.0f, 0.0f, bias, O, lut_binarize);
+    launch(k_pattern_values<kTableNone>, groups, kWarpsPerCta * 32, 0, st, W, s.Y, nullptr, nullptr, nullptr, 0.0f, 0.0f, bias, O, lut_binarize);
     BB200_CUDA(cudaPeekAtLastError());
     BB200_CUDA(cudaMemsetAsync(s.hist, 0, (size_t)O * 256, st));
     // word tiles: wide enough to amortise the 64-counter reduction (about 400 instructions per warp), narrow enough to fill the GPU
@@ -1197,10 +1215,10 @@ int dl6_bit_forward_training_by_table(const int *x, int *y, const int *idx, cons
     while (tile_words > 32 && (long long)groups * ((words + tile_words - 1) / tile_words) < 2LL * device_info().sm_count) tile_words /= 2;
     const long long blocks = (long long)groups * ((words + tile_words - 1) / tile_words);
     BB200_REQUIRE(blocks < (1LL << 31), BBCU_ERR_TOO_LARGE);
-    k_pattern_histogram<<<(unsigned)blocks, kWarpsPerCta * 32, 0, st>>>(reinterpret_cast<const uint32_t *>(x), idx, s.hist, O, F, stride, groups,
+    launch(k_pattern_histogram, (unsigned)blocks, kWarpsPerCta * 32, 0, st, reinterpret_cast<const uint32_t *>(x), idx, s.hist, O, F, stride, groups,
                                                                        tile_words);
     BB200_CUDA(cudaPeekAtLastError());
-    k_dl6_bit_train_finalize<<<groups, kWarpsPerCta * 32, 0, st>>>(s.Y, s.hist, s.table, mean, rstd, rmean, rvar, gamma, beta, momentum, O, F);
+    launch(k_dl6_bit_train_finalize, groups, kWarpsPerCta * 32, 0, st, s.Y, s.hist, s.table, mean, rstd, rmean, rvar, gamma, beta, momentum, O, F);
     BB200_CUDA(cudaPeekAtLastError());
     return run_binary_lut(x, y, idx, s.table, O, F, stride, st);
 }
@@ -1213,14 +1231,14 @@ int bit_fp32_forward_by_table(const int *x, float *y, const int *idx, const floa
     Scratch s;
     if (!carve(s, O, st)) return BBCU_ERR_NO_MEMORY;
     const int groups = (O + kWarpsPerCta - 1) / kWarpsPerCta;
-    k_pattern_values<kTableNone><<<groups, kWarpsPerCta * 32, 0, st>>>(W, s.Y, nullptr, nullptr, nullptr, 0.0f, 0.0f, bias, O, lut_binarize);
+    launch(k_pattern_values<kTableNone>, groups, kWarpsPerCta * 32, 0, st, W, s.Y, nullptr, nullptr, nullptr, 0.0f, 0.0f, bias, O, lut_binarize);
     BB200_CUDA(cudaPeekAtLastError());
     // frame tiles as in the other LUT kernels: the tile's input rows stay in L2 while all nodes consume them
     const int tf = frame_tile(3LL * O, 1, groups, F, 1 << 20);
     const int tile_words = ((tf + 1023) / 1024) * 32;
     const long long blocks = (long long)groups * (((F + 31) / 32 + tile_words - 1) / tile_words);
     BB200_REQUIRE(blocks < (1LL << 31), BBCU_ERR_TOO_LARGE);
-    k_bit_gather_forward<<<(unsigned)blocks, kWarpsPerCta * 32, 0, st>>>(reinterpret_cast<const uint32_t *>(x), y, idx, s.Y, O, F, xs, ys, groups,
+    launch(k_bit_gather_forward, (unsigned)blocks, kWarpsPerCta * 32, 0, st, reinterpret_cast<const uint32_t *>(x), y, idx, s.Y, O, F, xs, ys, groups,
                                                                         tile_words);
     return launch_status();
 }
@@ -1239,7 +1257,7 @@ int f32_binary_forward_by_table(int mode, const float *x, float *y, const int *i
         SmallBinArgs a = {};
         a.x = x; a.y = y; a.idx = idx; a.W = W; a.mean = mean; a.rstd = rstd; a.running_mean = rmean; a.running_var = rvar;
         a.gamma = gamma; a.beta = beta; a.momentum = momentum; a.bias = bias; a.F = F; a.lut_binarize = lut_binarize; a.xs = fs; a.ys = fs; a.vec = aligned;
-        k_small_binary_forward<false><<<O, small_threads(F), 0, st>>>(a);
+        launch(k_small_binary_forward<false>, O, small_threads(F), 0, st, a);
         return launch_status();
     }
     if (!aligned) return BBCU_ERR_NO_MEMORY;
@@ -1258,37 +1276,37 @@ int f32_binary_forward_by_table(int mode, const float *x, float *y, const int *i
     const long long blocks = (long long)a.groups * ((F + a.tile_frames - 1) / a.tile_frames);
     BB200_REQUIRE(blocks < (1LL << 31), BBCU_ERR_TOO_LARGE);
     if (mode == 0) {
-        k_pattern_values<kTableNone><<<a.groups, threads, 0, st>>>(W, s.Y, nullptr, nullptr, nullptr, 0.0f, 0.0f, bias, O, lut_binarize);
+        launch(k_pattern_values<kTableNone>, a.groups, threads, 0, st, W, s.Y, nullptr, nullptr, nullptr, 0.0f, 0.0f, bias, O, lut_binarize);
         BB200_CUDA(cudaPeekAtLastError());
-        k_f32_binary_forward<kPassDirect><<<(unsigned)blocks, threads, 0, st>>>(a);
+        launch(k_f32_binary_forward<kPassDirect>, (unsigned)blocks, threads, 0, st, a);
         return launch_status();
     }
     if (mode == 3) {          // first half of a sharded training forward: raw values into y, per-rank sums (mean doubles as the sums pointer)
-        k_pattern_values<kTableNone><<<a.groups, threads, 0, st>>>(W, s.Y, nullptr, nullptr, nullptr, 0.0f, 0.0f, bias, O, lut_binarize);
+        launch(k_pattern_values<kTableNone>, a.groups, threads, 0, st, W, s.Y, nullptr, nullptr, nullptr, 0.0f, 0.0f, bias, O, lut_binarize);
         BB200_CUDA(cudaPeekAtLastError());
         BB200_CUDA(cudaMemsetAsync(s.hist, 0, (size_t)O * 256, st));
-        k_f32_binary_forward<kPassStats><<<(unsigned)blocks, threads, 0, st>>>(a);
+        launch(k_f32_binary_forward<kPassStats>, (unsigned)blocks, threads, 0, st, a);
         BB200_CUDA(cudaPeekAtLastError());
-        k_counts_to_sums<<<a.groups, threads, 0, st>>>(s.Y, s.hist, reinterpret_cast<double *>(mean), O);
+        launch(k_counts_to_sums, a.groups, threads, 0, st, s.Y, s.hist, reinterpret_cast<double *>(mean), O);
         return launch_status();
     }
     if (mode == 1) {
-        k_pattern_values<kTableNorm><<<a.groups, threads, 0, st>>>(W, nullptr, s.table, rmean, rvar, gamma, beta, bias, O, lut_binarize);
+        launch(k_pattern_values<kTableNorm>, a.groups, threads, 0, st, W, nullptr, s.table, rmean, rvar, gamma, beta, bias, O, lut_binarize);
         BB200_CUDA(cudaPeekAtLastError());
         a.table = s.table;
-        k_f32_binary_forward<kPassDirect><<<(unsigned)blocks, threads, 0, st>>>(a);
+        launch(k_f32_binary_forward<kPassDirect>, (unsigned)blocks, threads, 0, st, a);
         return launch_status();
     }
-    k_pattern_values<kTableNone><<<a.groups, threads, 0, st>>>(W, s.Y, nullptr, nullptr, nullptr, 0.0f, 0.0f, bias, O, lut_binarize);
+    launch(k_pattern_values<kTableNone>, a.groups, threads, 0, st, W, s.Y, nullptr, nullptr, nullptr, 0.0f, 0.0f, bias, O, lut_binarize);
     BB200_CUDA(cudaPeekAtLastError());
     BB200_CUDA(cudaMemsetAsync(s.hist, 0, (size_t)O * 256, st));
     a.pat = s.pat;
-    k_f32_binary_forward<kPassCount><<<(unsigned)blocks, threads, 0, st>>>(a);
+    launch(k_f32_binary_forward<kPassCount>, (unsigned)blocks, threads, 0, st, a);
     BB200_CUDA(cudaPeekAtLastError());
-    k_dl6_bit_train_finalize<<<a.groups, threads, 0, st>>>(s.Y, s.hist, s.table, mean, rstd, rmean, rvar, gamma, beta, momentum, O, F);
+    launch(k_dl6_bit_train_finalize, a.groups, threads, 0, st, s.Y, s.hist, s.table, mean, rstd, rmean, rvar, gamma, beta, momentum, O, F);
     BB200_CUDA(cudaPeekAtLastError());
     a.table = s.table;
-    k_f32_binary_forward<kPassOutput><<<(unsigned)blocks, threads, 0, st>>>(a);
+    launch(k_f32_binary_forward<kPassOutput>, (unsigned)blocks, threads, 0, st, a);
     return launch_status();
 }
 
@@ -1332,15 +1350,15 @@ bool input_side(BitBwdArgs &a, int I, bool pack, cudaStream_t st)
     int *total = count + I, *cursor = total + 1, *list = cursor + I;
     a.edge_count = count; a.edge_end = cursor; a.edges = list;
     cudaMemsetAsync(count, 0, ((size_t)I + 1) * sizeof(int), st);
-    k_edge_count<<<(edges + 255) / 256, 256, 0, st>>>(a.idx, count, edges);
-    k_edge_room<<<(I + 255) / 256, 256, 0, st>>>(count, cursor, total, I);
-    k_edge_fill<<<(edges + 255) / 256, 256, 0, st>>>(a.idx, cursor, list, edges);
+    launch(k_edge_count, (edges + 255) / 256, 256, 0, st, a.idx, count, edges);
+    launch(k_edge_room, (I + 255) / 256, 256, 0, st, count, cursor, total, I);
+    launch(k_edge_fill, (edges + 255) / 256, 256, 0, st, a.idx, cursor, list, edges);
     if (pack) {
         uint32_t *bits = reinterpret_cast<uint32_t *>(reinterpret_cast<unsigned char *>(count) + list_bytes);
         const int runs = (int)((ws + 31) / 32);
         const long long blocks = ((long long)I * runs + kWarpsPerCta - 1) / kWarpsPerCta;
         if (blocks >= (1LL << 31)) return false;
-        k_pack_bits<<<(unsigned)blocks, kWarpsPerCta * 32, 0, st>>>(reinterpret_cast<const float *>(a.x), bits, I, a.F, a.xs, ws, runs);
+        launch(k_pack_bits, (unsigned)blocks, kWarpsPerCta * 32, 0, st, reinterpret_cast<const float *>(a.x), bits, I, a.F, a.xs, ws, runs);
         a.x = bits;
         a.xs = ws;
     }
@@ -1367,7 +1385,7 @@ int launch_pattern_sums(BitBwdArgs a, bool bn, cudaStream_t st)
     const int smem = kPsWarps * 64 * 32 * (int)(bn ? sizeof(PatternSlot<true>) : sizeof(PatternSlot<false>));
     auto kern = bn ? k_pattern_sums<XF32, true> : k_pattern_sums<XF32, false>;
     BB200_REQUIRE(allow_big_smem(kern, smem), BBCU_ERR_NO_MEMORY);
-    kern<<<(unsigned)blocks, kPsWarps * 32, smem, st>>>(a);
+    launch(kern, (unsigned)blocks, kPsWarps * 32, smem, st, a);
     return launch_status();
 }
 
@@ -1387,7 +1405,7 @@ int launch_pattern_gather(BitBwdArgs a, bool bn, cudaStream_t st)
     const int smem = a.split > 1 ? a.split * nc * 32 * (int)sizeof(float4) : 0;
     auto kern = bn ? (nc == 4 ? k_pattern_gather<true, 4> : nc == 2 ? k_pattern_gather<true, 2> : k_pattern_gather<true, 1>)
                    : (nc == 4 ? k_pattern_gather<false, 4> : nc == 2 ? k_pattern_gather<false, 2> : k_pattern_gather<false, 1>);
-    kern<<<(unsigned)blocks, a.split * 32, smem, st>>>(a);
+    launch(kern, (unsigned)blocks, a.split * 32, smem, st, a);
     return launch_status();
 }
 
@@ -1407,7 +1425,7 @@ int bit_backward_by_table(bool bn, bool x_is_fp32, const void *x, const float *d
         BB200_CUDA(cudaMemsetAsync(dx, 0, sizeof(float) * (size_t)I * (size_t)fs, st));
         auto kern = x_is_fp32 ? (bn ? k_small_binary_backward<false, true> : k_small_binary_backward<false, false>)
                               : (bn ? k_small_binary_backward<true, true> : k_small_binary_backward<true, false>);
-        kern<<<O, small_threads(F), 0, st>>>(a);
+        launch(kern, O, small_threads(F), 0, st, a);
         return launch_status();
     }
     BitBwdArgs a;
@@ -1415,14 +1433,14 @@ int bit_backward_by_table(bool bn, bool x_is_fp32, const void *x, const float *d
     BB200_CUDA(cudaPeekAtLastError());
     a.dx = dx;
     const unsigned blocks = (unsigned)((O + kWarpsPerCta - 1) / kWarpsPerCta), threads = kWarpsPerCta * 32;
-    if (bn) k_pattern_masks<<<blocks, threads, 0, st>>>(W, a.mask, mean, rstd, gamma, beta, bias, O, lut_binarize);
-    else    k_pattern_derivatives<<<blocks, threads, 0, st>>>(W, a.etab, bias, O, lut_binarize);
+    if (bn) launch(k_pattern_masks, blocks, threads, 0, st, W, a.mask, mean, rstd, gamma, beta, bias, O, lut_binarize);
+    else    launch(k_pattern_derivatives, blocks, threads, 0, st, W, a.etab, bias, O, lut_binarize);
     BB200_CUDA(cudaPeekAtLastError());
     const int rc = launch_pattern_sums<false>(a, bn, st);
     if (rc) return rc;
-    if (bn) k_bit_backward_finalize<true><<<blocks, threads, 0, st>>>(a.hdy, a.hist, a.mask, W, a.etab, a.ntab, dW, mean, rstd, dmean_out, dvar_out, gamma, beta,
+    if (bn) launch(k_bit_backward_finalize<true>, blocks, threads, 0, st, a.hdy, a.hist, a.mask, W, a.etab, a.ntab, dW, mean, rstd, dmean_out, dvar_out, gamma, beta,
                                                                      bias, O, 1.0f / (float)F, lut_binarize, nullptr, nullptr);
-    else    k_bit_backward_finalize<false><<<blocks, threads, 0, st>>>(a.hdy, nullptr, nullptr, nullptr, nullptr, nullptr, dW, nullptr, nullptr, nullptr, nullptr,
+    else    launch(k_bit_backward_finalize<false>, blocks, threads, 0, st, a.hdy, nullptr, nullptr, nullptr, nullptr, nullptr, dW, nullptr, nullptr, nullptr, nullptr,
                                                                       0.0f, 0.0f, bias, O, 0.0f, lut_binarize, nullptr, nullptr);
     BB200_CUDA(cudaPeekAtLastError());
     return launch_pattern_gather(a, bn, st);
@@ -1439,11 +1457,11 @@ int bit_backward_stats_by_table(const float *x, const float *dy, const int *idx,
     BitBwdArgs a;
     if (!backward_setup(a, x, dy, idx, O, F, fs, fs, st)) return BBCU_ERR_NO_MEMORY;
     const unsigned blocks = (unsigned)((O + kWarpsPerCta - 1) / kWarpsPerCta), threads = kWarpsPerCta * 32;
-    k_pattern_masks<<<blocks, threads, 0, st>>>(W, a.mask, mean, rstd, gamma, beta, bias, O, lut_binarize);
+    launch(k_pattern_masks, blocks, threads, 0, st, W, a.mask, mean, rstd, gamma, beta, bias, O, lut_binarize);
     BB200_CUDA(cudaPeekAtLastError());
     int rc = launch_pattern_sums<true>(a, true, st);
     if (rc) return rc;
-    k_bit_backward_finalize<true><<<blocks, threads, 0, st>>>(a.hdy, a.hist, a.mask, W, nullptr, nullptr, nullptr, mean, rstd, nullptr, nullptr, gamma, beta, bias,
+    launch(k_bit_backward_finalize<true>, blocks, threads, 0, st, a.hdy, a.hist, a.mask, W, nullptr, nullptr, nullptr, mean, rstd, nullptr, nullptr, gamma, beta, bias,
                                                              O, 0.0f, lut_binarize, sums, nullptr);
     rc = launch_status();
     if (rc == BBCU_OK) {
@@ -1474,13 +1492,13 @@ int bit_backward_apply_by_table(const float *x, const float *dy, float *dx, cons
     BB200_CUDA(cudaPeekAtLastError());
     const unsigned blocks = (unsigned)((O + kWarpsPerCta - 1) / kWarpsPerCta), threads = kWarpsPerCta * 32;
     if (!have) {
-        k_pattern_masks<<<blocks, threads, 0, st>>>(W, a.mask, mean, rstd, gamma, beta, bias, O, lut_binarize);
+        launch(k_pattern_masks, blocks, threads, 0, st, W, a.mask, mean, rstd, gamma, beta, bias, O, lut_binarize);
         BB200_CUDA(cudaPeekAtLastError());
         const int rc = launch_pattern_sums<false>(a, true, st);
         if (rc) return rc;
     }
     a.dx = dx;
-    k_bit_backward_finalize<true><<<blocks, threads, 0, st>>>(a.hdy, a.hist, a.mask, W, a.etab, a.ntab, dW, mean, rstd, dmean_out, dvar_out, gamma, beta, bias,
+    launch(k_bit_backward_finalize<true>, blocks, threads, 0, st, a.hdy, a.hist, a.mask, W, a.etab, a.ntab, dW, mean, rstd, dmean_out, dvar_out, gamma, beta, bias,
                                                              O, 1.0f / (float)total_frames, lut_binarize, nullptr, sums);
     BB200_CUDA(cudaPeekAtLastError());
     return launch_pattern_gather(a, true, st);

@@ -85,6 +85,7 @@ constexpr int kIm2ColTiles = 4;
 __global__ void __launch_bounds__(256)
 k_im2col_forward_f32(const float *__restrict__ x, float *__restrict__ y, Im2ColGeom g, float border_value, int p_tiles, int f_tiles)
 {
+    grid_dependency();
     __shared__ float tile[kIm2ColTiles][32][33];
     const int tx = threadIdx.x, ty = threadIdx.y;
     int b = blockIdx.x;
@@ -128,6 +129,7 @@ k_im2col_forward_f32(const float *__restrict__ x, float *__restrict__ y, Im2ColG
 __global__ void __launch_bounds__(256)
 k_im2col_backward_f32(const float *__restrict__ dy, float *__restrict__ dx, Im2ColGeom g, int q_tiles, int f_tiles)
 {
+    grid_dependency();
     __shared__ float tile[32][33];
     const int tx = threadIdx.x, ty = threadIdx.y;
     int b = blockIdx.x;
@@ -200,6 +202,7 @@ __global__ void __launch_bounds__(256)
 k_im2col_forward_band_f32(const float *__restrict__ x, float *__restrict__ y, Im2ColGeom g, float border_value, int R, int rows_in, int bands,
                           int f_tiles)
 {
+    grid_dependency();
     extern __shared__ __align__(16) unsigned char band_smem[];
     float *tile = reinterpret_cast<float *>(band_smem);                                   // [rows_in * in_w][kBandPitch]
     int *src = reinterpret_cast<int *>(tile + ((size_t)rows_in * g.in_w + 1) * kBandPitch);  // [taps][R * out_w], then [taps] flags
@@ -286,6 +289,7 @@ k_im2col_forward_band_f32(const float *__restrict__ x, float *__restrict__ y, Im
 __global__ void __launch_bounds__(256)
 k_im2col_backward_band_f32(const float *__restrict__ dy, float *__restrict__ dx, Im2ColGeom g, int R, int bands, int f_tiles)
 {
+    grid_dependency();
     extern __shared__ __align__(16) unsigned char band_smem[];
     float *tile = reinterpret_cast<float *>(band_smem);                                   // [R * in_w][kBandPitch]
     int *src = reinterpret_cast<int *>(tile + (size_t)R * g.in_w * kBandPitch);            // [taps][R * in_w]: output pixel, or -1
@@ -379,6 +383,7 @@ template <int FW>
 __global__ void __launch_bounds__(256)
 k_im2col_forward_quads_f32(const float *__restrict__ x, float *__restrict__ y, Im2ColGeom g, float border_value, int R, int bands, int f_tiles)
 {
+    grid_dependency();
     extern __shared__ __align__(16) float quad_tile[];                        // [32 frames][rows of the band with the filter's halo][out_w + 4]
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
     int b = blockIdx.x;
@@ -434,6 +439,7 @@ template <int FW>
 __global__ void __launch_bounds__(256)
 k_im2col_backward_quads_f32(const float *__restrict__ dy, float *__restrict__ dx, Im2ColGeom g, int R, int bands, int f_tiles)
 {
+    grid_dependency();
     extern __shared__ __align__(16) float quad_tile[];                        // [32 frames][R * in_w]
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
     int b = blockIdx.x;
@@ -502,6 +508,7 @@ constexpr int kBitColumns = 8;
 __global__ void __launch_bounds__(256)
 k_im2col_forward_bit(const uint32_t *__restrict__ x, uint32_t *__restrict__ y, Im2ColGeom g, int groups, int g_tiles, int in_words, int w_tiles)
 {
+    grid_dependency();
     __shared__ uint32_t tile[kBitColumns][32][33];                // [word column][input frame j][pixel group]
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
     int b = blockIdx.x;
@@ -546,6 +553,7 @@ constexpr unsigned kPieceOverflow = 0xffffffffu;
 __global__ void __launch_bounds__(256)
 k_im2col_bit_pieces(Im2ColGeom g, int period_words, int2 *__restrict__ pieces)
 {
+    grid_dependency();
     const int lane = threadIdx.x & 31;
     const int e = blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5);
     const int taps = g.filter_h * g.filter_w;
@@ -594,6 +602,7 @@ __global__ void __launch_bounds__(384, 3)
 k_im2col_forward_bit_words(const uint32_t *__restrict__ x, uint32_t *__restrict__ y, Im2ColGeom g, const int2 *__restrict__ pieces, int period_words,
                            int period_frames, int qw, int in_words, long long out_words, int runs, int splits, int columns, int column_groups)
 {
+    grid_dependency();
     extern __shared__ uint32_t bit_rows[];                        // [column][32 frames][qw + 2]: one zero word before and after every row
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, warps = blockDim.x >> 5;
     int blk = blockIdx.x;
@@ -710,6 +719,7 @@ k_im2col_forward_bit_words(const uint32_t *__restrict__ x, uint32_t *__restrict_
 __global__ void __launch_bounds__(256)
 k_im2col_forward_bit_any(const uint32_t *__restrict__ x, uint32_t *__restrict__ y, Im2ColGeom g, int out_words, int out_nodes)
 {
+    grid_dependency();
     const long long t = (long long)blockIdx.x * blockDim.x + threadIdx.x;
     if (t >= (long long)out_words * out_nodes) return;
     const int on = (int)(t / out_words), wo = (int)(t % out_words);
@@ -739,6 +749,7 @@ __global__ void __launch_bounds__(256)
 k_col2im_f32(const float *__restrict__ src, float *__restrict__ dst, int hw, int out_frames, long long col_fs, long long img_fs, int xy_tiles,
              int f_tiles)
 {
+    grid_dependency();
     __shared__ float tile[kCol2ImTile][kCol2ImTile + 1];
     const int tx = threadIdx.x & 63, ty = threadIdx.x >> 6;
     int b = blockIdx.x;
@@ -781,6 +792,7 @@ __global__ void __launch_bounds__(256)
 k_col2im_forward_bit(const uint32_t *__restrict__ x, uint32_t *__restrict__ y, int hw, int out_frames, long long in_fs, long long out_fs,
                      int groups, int w_tiles, int out_words, long long in_words)
 {
+    grid_dependency();
     __shared__ uint32_t tile[32][33];                             // [pixel k][output word]
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
     int b = blockIdx.x;
@@ -819,6 +831,7 @@ template <int V>
 __global__ void __launch_bounds__(256)
 k_maxpool_forward_f32(const float *__restrict__ x, float *__restrict__ y, int *__restrict__ argmax, PoolGeom g, long long fs)
 {
+    grid_dependency();
     const int f = (blockIdx.x * blockDim.x + threadIdx.x) * V;
     if (f >= g.frames) return;
     const bool full = f + V <= g.frames;
@@ -865,6 +878,7 @@ k_maxpool_forward_f32(const float *__restrict__ x, float *__restrict__ y, int *_
 __global__ void __launch_bounds__(256)
 k_maxpool_forward_bit(const uint32_t *__restrict__ x, uint32_t *__restrict__ y, PoolGeom g, long long fs, int words)
 {
+    grid_dependency();
     const int w = blockIdx.x * blockDim.x + threadIdx.x;
     if (w >= words) return;
     for (int on = blockIdx.y * blockDim.y + threadIdx.y; on < g.c_size * g.out_h * g.out_w; on += gridDim.y * blockDim.y) {
@@ -888,6 +902,7 @@ template <bool XBITS, int V>
 __global__ void __launch_bounds__(256)
 k_maxpool_backward(const void *__restrict__ sel, const float *__restrict__ dy, float *__restrict__ dx, PoolGeom g, long long sel_fs, long long fs)
 {
+    grid_dependency();
     const int f = (blockIdx.x * blockDim.x + threadIdx.x) * V;
     if (f >= g.frames) return;
     const bool full = f + V <= g.frames;
@@ -1026,7 +1041,7 @@ extern "C" int bbcu_fp32_Im2Col_Forward(const float *dev_x_buf, float *dev_y_buf
             BB200_REQUIRE(blocks < (1LL << 31), BBCU_ERR_TOO_LARGE);
             auto kern = filter_w_size == 3 ? k_im2col_forward_quads_f32<3> : k_im2col_forward_quads_f32<5>;
             if (allow_big_smem(kern, kBandSmemLimit)) {
-                kern<<<(unsigned)blocks, 256, smem, as_stream(stream)>>>(dev_x_buf, dev_y_buf, g, border_value, (int)R, bands, f_tiles);
+                launch(kern, (unsigned)blocks, 256, smem, as_stream(stream), dev_x_buf, dev_y_buf, g, border_value, (int)R, bands, f_tiles);
                 return launch_status();
             }
         }
@@ -1050,7 +1065,7 @@ extern "C" int bbcu_fp32_Im2Col_Forward(const float *dev_x_buf, float *dev_y_buf
             BB200_REQUIRE(blocks < (1LL << 31), BBCU_ERR_TOO_LARGE);
             const int smem = (int)smem_of(R);
             BB200_REQUIRE(allow_big_smem(k_im2col_forward_band_f32, kBandSmemLimit), BBCU_ERR_NO_MEMORY);
-            k_im2col_forward_band_f32<<<(unsigned)blocks, 256, smem, as_stream(stream)>>>(dev_x_buf, dev_y_buf, g, border_value, R, (int)rows_in_of(R),
+            launch(k_im2col_forward_band_f32, (unsigned)blocks, 256, smem, as_stream(stream), dev_x_buf, dev_y_buf, g, border_value, R, (int)rows_in_of(R),
                                                                                        bands, f_tiles);
             return launch_status();
         }
@@ -1059,7 +1074,7 @@ extern "C" int bbcu_fp32_Im2Col_Forward(const float *dev_x_buf, float *dev_y_buf
     const int p_tiles = (int)((P + 32 * kIm2ColTiles - 1) / (32 * kIm2ColTiles));
     const long long blocks = out_nodes * p_tiles * f_tiles;
     BB200_REQUIRE(blocks < (1LL << 31), BBCU_ERR_TOO_LARGE);
-    k_im2col_forward_f32<<<(unsigned)blocks, dim3(32, 8), 0, as_stream(stream)>>>(dev_x_buf, dev_y_buf, g, border_value, p_tiles, f_tiles);
+    launch(k_im2col_forward_f32, (unsigned)blocks, dim3(32, 8), 0, as_stream(stream), dev_x_buf, dev_y_buf, g, border_value, p_tiles, f_tiles);
     return launch_status();
 }
 
@@ -1090,7 +1105,7 @@ extern "C" int bbcu_bit_Im2Col_Forward(const int *dev_x_buf, int *dev_y_buf, int
             int2 *pieces = static_cast<int2 *>(stream_scratch(as_stream(stream), table_bytes, 2));
             if (pieces != nullptr) {
                 const int entries = taps * period_words;
-                k_im2col_bit_pieces<<<(entries + 7) / 8, 256, 0, as_stream(stream)>>>(g, period_words, pieces);
+                launch(k_im2col_bit_pieces, (entries + 7) / 8, 256, 0, as_stream(stream), g, period_words, pieces);
                 BB200_CUDA(cudaPeekAtLastError());
                 const long long out_words = ((long long)input_frame_size * P + 31) / 32;
                 // A warp per tap where there are enough taps, up to 12 a block.  As many columns a block, up to 8 and 48 KiB, as leave two blocks
@@ -1107,7 +1122,7 @@ extern "C" int bbcu_bit_Im2Col_Forward(const int *dev_x_buf, int *dev_y_buf, int
                 splits = splits > gcd ? gcd : splits;
                 const long long per_block = (long long)warps / (taps < warps ? taps : warps);       // units a tap needs to keep the warps busy
                 const int runs = (int)(splits * per_block > gcd ? gcd : splits * per_block);
-                k_im2col_forward_bit_words<<<(unsigned)(blocks * splits), 32 * warps, smem * columns, as_stream(stream)>>>(
+                launch(k_im2col_forward_bit_words, (unsigned)(blocks * splits), 32 * warps, smem * columns, as_stream(stream),
                     x, y, g, pieces, period_words, period_frames, qw, in_words, out_words, runs, (int)splits, columns, column_groups);
                 return launch_status();
             }
@@ -1118,12 +1133,12 @@ extern "C" int bbcu_bit_Im2Col_Forward(const int *dev_x_buf, int *dev_y_buf, int
         const int w_tiles = (in_words + kBitColumns - 1) / kBitColumns;
         const long long blocks = out_nodes * w_tiles * g_tiles;
         BB200_REQUIRE(blocks < (1LL << 31), BBCU_ERR_TOO_LARGE);
-        k_im2col_forward_bit<<<(unsigned)blocks, 256, 0, as_stream(stream)>>>(x, y, g, groups, g_tiles, in_words, w_tiles);
+        launch(k_im2col_forward_bit, (unsigned)blocks, 256, 0, as_stream(stream), x, y, g, groups, g_tiles, in_words, w_tiles);
     } else {
         const long long out_words = ((long long)input_frame_size * P + 31) / 32;
         const long long blocks = (out_words * out_nodes + 255) / 256;
         BB200_REQUIRE(blocks < (1LL << 31), BBCU_ERR_TOO_LARGE);
-        k_im2col_forward_bit_any<<<(unsigned)blocks, 256, 0, as_stream(stream)>>>(x, y, g, (int)out_words, (int)out_nodes);
+        launch(k_im2col_forward_bit_any, (unsigned)blocks, 256, 0, as_stream(stream), x, y, g, (int)out_words, (int)out_nodes);
     }
     return launch_status();
 }
@@ -1153,7 +1168,7 @@ extern "C" int bbcu_fp32_Im2Col_Backward(const float *dev_dy_buf, float *dev_dx_
             BB200_REQUIRE(blocks < (1LL << 31), BBCU_ERR_TOO_LARGE);
             auto kern = filter_w_size == 3 ? k_im2col_backward_quads_f32<3> : k_im2col_backward_quads_f32<5>;
             if (allow_big_smem(kern, kBandSmemLimit)) {
-                kern<<<(unsigned)blocks, 256, smem, as_stream(stream)>>>(dev_dy_buf, dev_dx_buf, g, (int)R, bands, f_tiles);
+                launch(kern, (unsigned)blocks, 256, smem, as_stream(stream), dev_dy_buf, dev_dx_buf, g, (int)R, bands, f_tiles);
                 return launch_status();
             }
         }
@@ -1169,14 +1184,14 @@ extern "C" int bbcu_fp32_Im2Col_Backward(const float *dev_dy_buf, float *dev_dx_
             const long long blocks = (long long)input_c_size * bands * f_tiles;
             BB200_REQUIRE(blocks < (1LL << 31), BBCU_ERR_TOO_LARGE);
             BB200_REQUIRE(allow_big_smem(k_im2col_backward_band_f32, kBandSmemLimit), BBCU_ERR_NO_MEMORY);
-            k_im2col_backward_band_f32<<<(unsigned)blocks, 256, (int)(per_row * R), as_stream(stream)>>>(dev_dy_buf, dev_dx_buf, g, R, bands, f_tiles);
+            launch(k_im2col_backward_band_f32, (unsigned)blocks, 256, (int)(per_row * R), as_stream(stream), dev_dy_buf, dev_dx_buf, g, R, bands, f_tiles);
             return launch_status();
         }
     }
     const int q_tiles = (input_w_size * input_h_size + 31) / 32;
     const long long blocks = (long long)input_c_size * q_tiles * f_tiles;
     BB200_REQUIRE(blocks < (1LL << 31), BBCU_ERR_TOO_LARGE);
-    k_im2col_backward_f32<<<(unsigned)blocks, dim3(32, 8), 0, as_stream(stream)>>>(dev_dy_buf, dev_dx_buf, g, q_tiles, f_tiles);
+    launch(k_im2col_backward_f32, (unsigned)blocks, dim3(32, 8), 0, as_stream(stream), dev_dy_buf, dev_dx_buf, g, q_tiles, f_tiles);
     return launch_status();
 }
 
@@ -1199,7 +1214,7 @@ static int col2im_f32(const float *src, float *dst, int w, int h, int c, int col
     const int hw = w * h, xy_tiles = (hw + kCol2ImTile - 1) / kCol2ImTile, f_tiles = (out_frames + kCol2ImTile - 1) / kCol2ImTile;
     const long long blocks = (long long)c * xy_tiles * f_tiles;
     BB200_REQUIRE(blocks < (1LL << 31), BBCU_ERR_TOO_LARGE);
-    k_col2im_f32<FORWARD><<<(unsigned)blocks, 256, 0, st>>>(src, dst, hw, out_frames, col_fs, img_fs, xy_tiles, f_tiles);
+    launch(k_col2im_f32<FORWARD>, (unsigned)blocks, 256, 0, st, src, dst, hw, out_frames, col_fs, img_fs, xy_tiles, f_tiles);
     return launch_status();
 }
 
@@ -1230,7 +1245,7 @@ extern "C" int bbcu_bit_Col2Im_Forward(const int *dev_x_buf, int *dev_y_buf, int
     const long long in_words = ((long long)output_frame_size * hw + 31) / 32;
     const long long blocks = (long long)c_size * groups * w_tiles;
     BB200_REQUIRE(blocks < (1LL << 31), BBCU_ERR_TOO_LARGE);
-    k_col2im_forward_bit<<<(unsigned)blocks, 256, 0, as_stream(stream)>>>(x, y, hw, output_frame_size, input_frame_stride, output_frame_stride, groups,
+    launch(k_col2im_forward_bit, (unsigned)blocks, 256, 0, as_stream(stream), x, y, hw, output_frame_size, input_frame_stride, output_frame_stride, groups,
                                                                          w_tiles, out_words, in_words);
     return launch_status();
 }
@@ -1263,8 +1278,8 @@ extern "C" int bbcu_fp32_MaxPooling_Forward(const float *dev_x_buf, float *dev_y
                                                reinterpret_cast<uintptr_t>(dev_argmax_buf)) & 15) == 0;
     const int per = vec ? 4 : 1;
     const dim3 block = pool_block((frame_size + per - 1) / per), grid = pool_grid((frame_size + per - 1) / per, g, block);
-    if (vec) k_maxpool_forward_f32<4><<<grid, block, 0, as_stream(stream)>>>(dev_x_buf, dev_y_buf, dev_argmax_buf, g, frame_stride);
-    else     k_maxpool_forward_f32<1><<<grid, block, 0, as_stream(stream)>>>(dev_x_buf, dev_y_buf, dev_argmax_buf, g, frame_stride);
+    if (vec) launch(k_maxpool_forward_f32<4>, grid, block, 0, as_stream(stream), dev_x_buf, dev_y_buf, dev_argmax_buf, g, frame_stride);
+    else     launch(k_maxpool_forward_f32<1>, grid, block, 0, as_stream(stream), dev_x_buf, dev_y_buf, dev_argmax_buf, g, frame_stride);
     return launch_status();
 }
 
@@ -1279,7 +1294,7 @@ extern "C" int bbcu_bit_MaxPooling_Forward(const int *dev_x_buf, int *dev_y_buf,
     const PoolGeom g = make_pool(filter_h_size, filter_w_size, input_w_size, input_h_size, output_w_size, output_h_size, c_size, frame_size);
     const int words = (frame_size + 31) / 32;
     const dim3 block = pool_block(words), grid = pool_grid(words, g, block);
-    k_maxpool_forward_bit<<<grid, block, 0, as_stream(stream)>>>(reinterpret_cast<const uint32_t *>(dev_x_buf), reinterpret_cast<uint32_t *>(dev_y_buf), g,
+    launch(k_maxpool_forward_bit, grid, block, 0, as_stream(stream), reinterpret_cast<const uint32_t *>(dev_x_buf), reinterpret_cast<uint32_t *>(dev_y_buf), g,
                                                               frame_stride, words);
     return launch_status();
 }
@@ -1298,8 +1313,8 @@ extern "C" int bbcu_fp32_MaxPooling_Backward(const int *dev_argmax_buf, const fl
                                                reinterpret_cast<uintptr_t>(dev_dx_buf)) & 15) == 0;
     const int per = vec ? 4 : 1;
     const dim3 block = pool_block((frame_size + per - 1) / per), grid = pool_grid((frame_size + per - 1) / per, g, block);
-    if (vec) k_maxpool_backward<false, 4><<<grid, block, 0, as_stream(stream)>>>(dev_argmax_buf, dev_dy_buf, dev_dx_buf, g, frame_stride, frame_stride);
-    else     k_maxpool_backward<false, 1><<<grid, block, 0, as_stream(stream)>>>(dev_argmax_buf, dev_dy_buf, dev_dx_buf, g, frame_stride, frame_stride);
+    if (vec) launch(k_maxpool_backward<false, 4>, grid, block, 0, as_stream(stream), dev_argmax_buf, dev_dy_buf, dev_dx_buf, g, frame_stride, frame_stride);
+    else     launch(k_maxpool_backward<false, 1>, grid, block, 0, as_stream(stream), dev_argmax_buf, dev_dy_buf, dev_dx_buf, g, frame_stride, frame_stride);
     return launch_status();
 }
 
@@ -1317,7 +1332,7 @@ extern "C" int bbcu_bit_fp32_MaxPooling_Backward(const int *dev_x_buf, const flo
     const bool vec = backward_frame_stride % 4 == 0 && ((reinterpret_cast<uintptr_t>(dev_dy_buf) | reinterpret_cast<uintptr_t>(dev_dx_buf)) & 15) == 0;
     const int per = vec ? 4 : 1;
     const dim3 block = pool_block((frame_size + per - 1) / per), grid = pool_grid((frame_size + per - 1) / per, g, block);
-    if (vec) k_maxpool_backward<true, 4><<<grid, block, 0, as_stream(stream)>>>(dev_x_buf, dev_dy_buf, dev_dx_buf, g, forward_frame_stride, backward_frame_stride);
-    else     k_maxpool_backward<true, 1><<<grid, block, 0, as_stream(stream)>>>(dev_x_buf, dev_dy_buf, dev_dx_buf, g, forward_frame_stride, backward_frame_stride);
+    if (vec) launch(k_maxpool_backward<true, 4>, grid, block, 0, as_stream(stream), dev_x_buf, dev_dy_buf, dev_dx_buf, g, forward_frame_stride, backward_frame_stride);
+    else     launch(k_maxpool_backward<true, 1>, grid, block, 0, as_stream(stream), dev_x_buf, dev_dy_buf, dev_dx_buf, g, forward_frame_stride, backward_frame_stride);
     return launch_status();
 }

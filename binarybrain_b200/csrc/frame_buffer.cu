@@ -13,6 +13,7 @@ constexpr int kFbChunk = 4096;        // words per CTA
 __global__ void __launch_bounds__(256)
 k_frame_buffer_copy(int *__restrict__ dst, const int *__restrict__ src, int frame_words, long long dst_stride, long long src_stride, int chunks, int vec)
 {
+    grid_dependency();
     const int node = blockIdx.x / chunks, chunk = blockIdx.x % chunks;
     int *d = dst + (size_t)node * dst_stride;
     const int *s = src + (size_t)node * src_stride;
@@ -40,6 +41,7 @@ __global__ void __launch_bounds__(256)
 k_conv_bit_to_real(const uint32_t *__restrict__ x, float *__restrict__ y, float value0, float value1, int frame_size, long long x_stride,
                    long long y_stride, int chunks, int vec)
 {
+    grid_dependency();
     const int node = blockIdx.x / chunks, chunk = blockIdx.x % chunks;
     const uint32_t *xr = x + (size_t)node * x_stride;
     float *yr = y + (size_t)node * y_stride;
@@ -78,7 +80,7 @@ extern "C" int bbcu_int32_FrameBufferCopy(int *dev_dst_buf, const int *dev_src_b
     const int vec = ((reinterpret_cast<uintptr_t>(dst) | reinterpret_cast<uintptr_t>(src)) & 15) == 0 && dst_frame_stride % 4 == 0 && src_frame_stride % 4 == 0;
     const int chunks = (frame_size + kFbChunk - 1) / kFbChunk;
     BB200_REQUIRE((long long)node_size * chunks < (1LL << 31), BBCU_ERR_TOO_LARGE);
-    k_frame_buffer_copy<<<node_size * chunks, 256, 0, as_stream(stream)>>>(dst, src, frame_size, dst_frame_stride, src_frame_stride, chunks, vec);
+    launch(k_frame_buffer_copy, node_size * chunks, 256, 0, as_stream(stream), dst, src, frame_size, dst_frame_stride, src_frame_stride, chunks, vec);
     return launch_status();
 }
 
@@ -92,7 +94,7 @@ extern "C" int bbcu_fp32_ConvBitToReal(const int *dev_x_buf, float *dev_y_buf, f
     const int vec = (reinterpret_cast<uintptr_t>(dev_y_buf) & 15) == 0 && y_frame_stride % 4 == 0;
     const int chunks = (frame_size + kFbChunk - 1) / kFbChunk;
     BB200_REQUIRE((long long)node_size * chunks < (1LL << 31), BBCU_ERR_TOO_LARGE);
-    k_conv_bit_to_real<<<node_size * chunks, 256, 0, as_stream(stream)>>>(reinterpret_cast<const uint32_t *>(dev_x_buf), dev_y_buf, value0, value1,
+    launch(k_conv_bit_to_real, node_size * chunks, 256, 0, as_stream(stream), reinterpret_cast<const uint32_t *>(dev_x_buf), dev_y_buf, value0, value1,
                                                                            frame_size, x_frame_stride, y_frame_stride, chunks, vec);
     return launch_status();
 }

@@ -57,6 +57,7 @@ __device__ __forceinline__ double softmax_frame(const float *__restrict__ y, con
 __global__ void k_softmax_cross_entropy(const float *__restrict__ y, const float *__restrict__ t, float *dy, double *loss_buf, float t_sum,
                                         int pix_size, int ch_size, int F, long long stride)
 {
+    grid_dependency();
     const int f = blockIdx.x * blockDim.x + threadIdx.x;
     if (f < F) loss_buf[f] = softmax_frame(y, t, dy, t_sum, pix_size, ch_size, f, stride);
 }
@@ -65,6 +66,7 @@ __global__ void __launch_bounds__(1024)
 k_softmax_cross_entropy_one(const float *__restrict__ y, const float *__restrict__ t, float *dy, double *loss, int pix_size, int ch_size, int F,
                             long long stride)
 {
+    grid_dependency();
     __shared__ double red[32];
     double s = 0.0;
     for (int row = threadIdx.x / 128; row < pix_size * ch_size; row += blockDim.x / 128)
@@ -79,6 +81,7 @@ k_softmax_cross_entropy_one(const float *__restrict__ y, const float *__restrict
 __global__ void __launch_bounds__(256)
 k_target_sum(const float *__restrict__ t, double *work, int rows, int F, long long stride)
 {
+    grid_dependency();
     __shared__ double red[8];
     double s = 0.0;
     for (int row = blockIdx.y; row < rows; row += gridDim.y)
@@ -91,6 +94,7 @@ __global__ void __launch_bounds__(128)
 k_softmax_cross_entropy_sums(const float *__restrict__ y, const float *__restrict__ t, float *dy, double *work, int pix_size, int ch_size, int F,
                              long long stride)
 {
+    grid_dependency();
     __shared__ double red[4];
     const int f = blockIdx.x * blockDim.x + threadIdx.x;
     double l = f < F ? softmax_frame(y, t, dy, (float)work[0], pix_size, ch_size, f, stride) : 0.0;
@@ -98,13 +102,14 @@ k_softmax_cross_entropy_sums(const float *__restrict__ y, const float *__restric
     if (threadIdx.x == 0) atomicAdd(work + 1, l);
 }
 
-__global__ void k_mean_loss(const double *__restrict__ work, double *loss) { *loss = -work[1] / work[0]; }
+__global__ void k_mean_loss(const double *__restrict__ work, double *loss) { grid_dependency(); *loss = -work[1] / work[0]; }
 
 // dy = grad_reduction * (y - t);  loss_buf[block % loss_buf_size] += sum (y - t)^2 * loss_reduction  (NaN terms skipped)
 __global__ void __launch_bounds__(256)
 k_mean_squared_error(const float *__restrict__ y, const float *__restrict__ t, float *dy, double *loss_buf, int loss_buf_size, int F,
                      long long stride, float grad_reduction, double loss_reduction, int chunks)
 {
+    grid_dependency();
     __shared__ double red[8];
     const int node = blockIdx.x / chunks, chunk = blockIdx.x % chunks;
     const size_t row = (size_t)node * stride;
@@ -130,6 +135,7 @@ k_mean_squared_error(const float *__restrict__ y, const float *__restrict__ t, f
 // y[o] = mean_i x[out_nodes * i + o]    /    dx[out_nodes * i + o] = dy[o] / mux
 __global__ void k_reduce_forward(const float *__restrict__ x, float *y, int out_nodes, int mux, int F, long long xs, long long ys)
 {
+    grid_dependency();
     const int f = blockIdx.x * blockDim.x + threadIdx.x;
     const int o = blockIdx.y;
     if (f >= F) return;
@@ -140,6 +146,7 @@ __global__ void k_reduce_forward(const float *__restrict__ x, float *y, int out_
 
 __global__ void k_reduce_backward(const float *__restrict__ dy, float *dx, int out_nodes, int mux, int F, long long dys, long long dxs)
 {
+    grid_dependency();
     const int f = blockIdx.x * blockDim.x + threadIdx.x;
     const int o = blockIdx.y;
     if (f >= F) return;
@@ -158,7 +165,7 @@ extern "C" int bbcu_fp32_LossSoftmaxCrossEntropy(const float *y, const float *t,
     BB200_REQUIRE(pix_size > 0 && ch_size > 0 && frame_size >= 0, BBCU_ERR_BAD_SIZE);
     BB200_REQUIRE(frame_stride >= frame_size, BBCU_ERR_BAD_STRIDE);
     if (frame_size == 0) return BBCU_OK;
-    k_softmax_cross_entropy<<<(frame_size + 127) / 128, 128, 0, as_stream(stream)>>>(y, t, dy, loss_buf, t_sum, pix_size, ch_size, frame_size,
+    launch(k_softmax_cross_entropy, (frame_size + 127) / 128, 128, 0, as_stream(stream), y, t, dy, loss_buf, t_sum, pix_size, ch_size, frame_size,
                                                                                    frame_stride);
     return launch_status();
 }
@@ -172,7 +179,7 @@ extern "C" int bbcu_fp32_LossSoftmaxCrossEntropyMean(const float *y, const float
     cudaStream_t st = as_stream(stream);
     const long long rows = (long long)pix_size * ch_size;
     if (rows * frame_size <= kOneCta) {
-        k_softmax_cross_entropy_one<<<1, 1024, 0, st>>>(y, t, dy, loss, pix_size, ch_size, frame_size, frame_stride);
+        launch(k_softmax_cross_entropy_one, 1, 1024, 0, st, y, t, dy, loss, pix_size, ch_size, frame_size, frame_stride);
         return launch_status();
     }
     double *work = static_cast<double *>(stream_scratch(st, 2 * sizeof(double)));
@@ -180,11 +187,11 @@ extern "C" int bbcu_fp32_LossSoftmaxCrossEntropyMean(const float *y, const float
     BB200_REQUIRE(rows < (1LL << 31), BBCU_ERR_TOO_LARGE);
     BB200_CUDA(cudaMemsetAsync(work, 0, 2 * sizeof(double), st));
     const unsigned bx = (unsigned)((frame_size + 2047) / 2048);
-    k_target_sum<<<dim3(bx, (unsigned)(rows < 64 ? rows : 64)), 256, 0, st>>>(t, work, (int)rows, frame_size, frame_stride);
+    launch(k_target_sum, dim3(bx, (unsigned)(rows < 64 ? rows : 64)), 256, 0, st, t, work, (int)rows, frame_size, frame_stride);
     BB200_CUDA(cudaPeekAtLastError());
-    k_softmax_cross_entropy_sums<<<(frame_size + 127) / 128, 128, 0, st>>>(y, t, dy, work, pix_size, ch_size, frame_size, frame_stride);
+    launch(k_softmax_cross_entropy_sums, (frame_size + 127) / 128, 128, 0, st, y, t, dy, work, pix_size, ch_size, frame_size, frame_stride);
     BB200_CUDA(cudaPeekAtLastError());
-    k_mean_loss<<<1, 1, 0, st>>>(work, loss);
+    launch(k_mean_loss, 1, 1, 0, st, work, loss);
     return launch_status();
 }
 
@@ -198,7 +205,7 @@ extern "C" int bbcu_fp32_LossMeanSquaredError(const float *y, const float *t, fl
     if (node_size == 0 || frame_size == 0) return BBCU_OK;
     const int chunks = (frame_size + 8191) / 8192;
     BB200_REQUIRE((long long)node_size * chunks < (1LL << 31), BBCU_ERR_TOO_LARGE);
-    k_mean_squared_error<<<node_size * chunks, 256, 0, as_stream(stream)>>>(y, t, dy, loss_buf, loss_buf_size, frame_size, frame_stride,
+    launch(k_mean_squared_error, node_size * chunks, 256, 0, as_stream(stream), y, t, dy, loss_buf, loss_buf_size, frame_size, frame_stride,
                                                                           grad_reduction, loss_reduction, chunks);
     return launch_status();
 }
@@ -211,7 +218,7 @@ extern "C" int bbcu_fp32_Reduce_Forward(const float *x, float *y, int input_node
                   output_node_size <= 65535, BBCU_ERR_BAD_SIZE);
     BB200_REQUIRE(x_frame_stride >= frame_size && y_frame_stride >= frame_size, BBCU_ERR_BAD_STRIDE);
     if (frame_size == 0) return BBCU_OK;
-    k_reduce_forward<<<dim3((frame_size + 255) / 256, output_node_size), 256, 0, as_stream(stream)>>>(
+    launch(k_reduce_forward, dim3((frame_size + 255) / 256, output_node_size), 256, 0, as_stream(stream),
         x, y, output_node_size, input_node_size / output_node_size, frame_size, x_frame_stride, y_frame_stride);
     return launch_status();
 }
@@ -224,7 +231,7 @@ extern "C" int bbcu_fp32_Reduce_Backward(const float *dy, float *dx, int input_n
                   output_node_size <= 65535, BBCU_ERR_BAD_SIZE);
     BB200_REQUIRE(dy_frame_stride >= frame_size && dx_frame_stride >= frame_size, BBCU_ERR_BAD_STRIDE);
     if (frame_size == 0) return BBCU_OK;
-    k_reduce_backward<<<dim3((frame_size + 255) / 256, output_node_size), 256, 0, as_stream(stream)>>>(
+    launch(k_reduce_backward, dim3((frame_size + 255) / 256, output_node_size), 256, 0, as_stream(stream),
         dy, dx, output_node_size, input_node_size / output_node_size, frame_size, dy_frame_stride, dx_frame_stride);
     return launch_status();
 }

@@ -121,6 +121,7 @@ template <bool XBIT, int PHASE, bool YBIT>
 __global__ void __launch_bounds__(kWarpsPerCta * 32, kFwdCtas)
 k_lut6_forward(const FwdArgs a)
 {
+    grid_dependency();
     __shared__ float4 s_tab[kWarpsPerCta][32];
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
     const int tile = blockIdx.x / a.groups;
@@ -291,6 +292,7 @@ __device__ __forceinline__ void fp_issue(const FwdArgs &a, FpPos pos, bool exist
 __global__ void __launch_bounds__(kWarpsPerCta * 32)
 k_table_coeffs(const float *__restrict__ W, float4 *__restrict__ coef, double *__restrict__ sums, int O, int lut_binarize)
 {
+    grid_dependency();
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
     const int node = blockIdx.x * kWarpsPerCta + warp;
     if (node >= O) return;
@@ -305,6 +307,7 @@ template <int PHASE, bool BINARY>            // BINARY: the layer's binary mode,
 __global__ void __launch_bounds__(kWarpsPerCta * 32, kFpCtas)
 k_lut6_forward_pipe(const FwdArgs a, int n_tiles)
 {
+    grid_dependency();
     extern __shared__ __align__(128) unsigned char smem_raw[];
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
     unsigned char *my_stages = smem_raw + (size_t)warp * kFpStages * kFpStageBytes;
@@ -492,6 +495,7 @@ __device__ __forceinline__ void bn_record(const BnStatistics &s, int n, float *m
 __global__ void k_bn_finalize(const double *__restrict__ sums, float *mean_out, float *rstd_out, float *running_mean, float *running_var,
                               float momentum, int O, long long total_frames)
 {
+    grid_dependency();
     int n = blockIdx.x * blockDim.x + threadIdx.x;
     if (n < O) bn_record(bn_statistics(sums, n, total_frames), n, mean_out, rstd_out, running_mean, running_var, momentum);
 }
@@ -502,6 +506,7 @@ __global__ void __launch_bounds__(256)
 k_bn_normalize_inplace(float *y, const double *__restrict__ sums, float *mean_out, float *rstd_out, float *running_mean, float *running_var, float gamma,
                        float beta, float momentum, long long total_frames, int F, long long ys, int binary, int chunks)
 {
+    grid_dependency();
     const int node = blockIdx.x / chunks, chunk = blockIdx.x % chunks;
     const BnStatistics stat = bn_statistics(sums, node, total_frames);
     const float mean = stat.mean, rstd = stat.rstd;
@@ -572,6 +577,7 @@ template <bool XBIT>
 __global__ void __launch_bounds__(kWarpsPerCta * 32, 3)
 k_lut6_backward_stats(const BwdArgs a)
 {
+    grid_dependency();
     __shared__ float4 s_tab[kWarpsPerCta][16];
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
     const int tile = blockIdx.x / a.groups;
@@ -621,6 +627,7 @@ __global__ void __launch_bounds__(256)
 k_dl6_backward_stats_from_y(const float *__restrict__ y, const float *__restrict__ dy, const float *__restrict__ rstd_buf, double *sums,
                             float gamma, float beta, int F, long long ys, long long dys, int chunks)
 {
+    grid_dependency();
     __shared__ double red[2][8];
     const int node = blockIdx.x / chunks, chunk = blockIdx.x % chunks;
     const float *yr = y + (size_t)node * ys;
@@ -678,6 +685,7 @@ __device__ __forceinline__ void bn_backward_finalize(const double *__restrict__ 
 __global__ void k_bn_backward_finalize(const double *__restrict__ sums, const float *__restrict__ mean_buf, const float *__restrict__ rstd_buf,
                                        float *dmean_out, float *dvar_out, int O, long long total_frames)
 {
+    grid_dependency();
     int n = blockIdx.x * blockDim.x + threadIdx.x;
     if (n < O) bn_backward_finalize(sums, n, mean_buf, rstd_buf, dmean_out, dvar_out, total_frames);
 }
@@ -690,6 +698,7 @@ template <bool XBIT, bool BN>
 __global__ void __launch_bounds__(kWarpsPerCta * 32, 1)
 k_lut6_backward(const BwdArgs a)
 {
+    grid_dependency();
     __shared__ float4 s_tab[kWarpsPerCta][16];
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
     const int tile = blockIdx.x / a.groups;
@@ -835,6 +844,7 @@ struct BwdPrepare {
 __global__ void __launch_bounds__(kWarpsPerCta * 32)
 k_backward_prepare(const BwdPrepare a)
 {
+    grid_dependency();
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
     const int node = blockIdx.x * kWarpsPerCta + warp;
     if (node < a.O) {
@@ -854,6 +864,7 @@ k_backward_prepare(const BwdPrepare a)
 __global__ void __launch_bounds__(kWarpsPerCta * 32)
 k_coeff_grads_to_dw(const float4 *__restrict__ dC, float *__restrict__ dW, int O)
 {
+    grid_dependency();
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
     const int node = blockIdx.x * kWarpsPerCta + warp;
     if (node >= O) return;
@@ -889,6 +900,7 @@ template <bool BN, bool BINARY>
 __global__ void __launch_bounds__(kWarpsPerCta * 32, 1)
 k_lut6_backward_pipe(const BwdArgs a, const float4 *__restrict__ coef, float *__restrict__ dC, int n_tiles, int n_full, int n_last)
 {
+    grid_dependency();
     extern __shared__ __align__(128) unsigned char smem_raw[];
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
     unsigned char *my = smem_raw + (size_t)warp * kBvWarpBytes;
@@ -1105,13 +1117,13 @@ static int launch_forward(FwdArgs a, int max_tile, cudaStream_t st)
                 // slot 1 of the stream's scratch: slot 0 may hold the caller's batch-norm sums at the same time
                 float4 *coef = static_cast<float4 *>(stream_scratch(st, (size_t)a.O * kFpTabSlotBytes, 1));
                 if (coef != nullptr) {
-                    k_table_coeffs<<<a.groups, kWarpsPerCta * 32, 0, st>>>(a.W, coef, a.sums, a.O, a.lut_binarize);
+                    launch(k_table_coeffs, a.groups, kWarpsPerCta * 32, 0, st, a.W, coef, a.sums, a.O, a.lut_binarize);
                     BB200_CUDA(cudaPeekAtLastError());
                     a.coef = coef;
                 }
             }
             if (PHASE == PH_STATS && a.coef == nullptr) BB200_CUDA(cudaMemsetAsync(a.sums, 0, sizeof(double) * 2 * (size_t)a.O, st));
-            kern<<<(unsigned)grid, kWarpsPerCta * 32, kFpSmem, st>>>(a, (a.F + a.T - 1) / a.T);
+            launch(kern, (unsigned)grid, kWarpsPerCta * 32, kFpSmem, st, a, (a.F + a.T - 1) / a.T);
             return launch_status();
         }
     }
@@ -1119,7 +1131,7 @@ static int launch_forward(FwdArgs a, int max_tile, cudaStream_t st)
     const long long tiles = (a.F + a.T - 1) / a.T;
     const long long blocks = tiles * a.groups;
     BB200_REQUIRE(blocks < (1LL << 31), BBCU_ERR_TOO_LARGE);
-    k_lut6_forward<XBIT, PHASE, YBIT><<<(unsigned)blocks, kWarpsPerCta * 32, 0, st>>>(a);
+    launch(k_lut6_forward<XBIT, PHASE, YBIT>, (unsigned)blocks, kWarpsPerCta * 32, 0, st, a);
     return launch_status();
 }
 
@@ -1149,13 +1161,13 @@ static bool backward_stats_pipe(const BwdArgs &b, cudaStream_t st, int *rc, void
     float4 *coef = (tmp != nullptr && tmp_bytes >= need && (reinterpret_cast<uintptr_t>(tmp) & 15) == 0)
                        ? static_cast<float4 *>(tmp) : static_cast<float4 *>(stream_scratch(st, need, 1));
     if (coef != nullptr) {
-        k_table_coeffs<<<a.groups, kWarpsPerCta * 32, 0, st>>>(a.W, coef, a.sums, a.O, a.lut_binarize);
+        launch(k_table_coeffs, a.groups, kWarpsPerCta * 32, 0, st, a.W, coef, a.sums, a.O, a.lut_binarize);
         a.coef = coef;
     } else if (cudaMemsetAsync(a.sums, 0, sizeof(double) * 2 * (size_t)a.O, st) != cudaSuccess) {
         *rc = launch_status();
         return true;
     }
-    kern<<<(unsigned)grid, kWarpsPerCta * 32, kFpSmem, st>>>(a, (a.F + a.T - 1) / a.T);
+    launch(kern, (unsigned)grid, kWarpsPerCta * 32, kFpSmem, st, a, (a.F + a.T - 1) / a.T);
     *rc = launch_status();
     return true;
 }
@@ -1231,12 +1243,12 @@ static int launch_backward_pipe(BwdArgs a, bool bn, int I, const double *sums, f
     pre.zero_quads = (size_t)I * (size_t)a.dxs / 4;
     long long fill = (long long)((pre.zero_quads + 1023) / 1024);
     if (fill > 8LL * device_info().sm_count) fill = 8LL * device_info().sm_count;
-    k_backward_prepare<<<(unsigned)(fill > groups8 ? fill : groups8), kWarpsPerCta * 32, 0, st>>>(pre);
+    launch(k_backward_prepare, (unsigned)(fill > groups8 ? fill : groups8), kWarpsPerCta * 32, 0, st, pre);
     BB200_CUDA(cudaPeekAtLastError());
     a.dmean = dmean_out; a.dvar = dvar_out;
-    kern<<<(unsigned)grid, kWarpsPerCta * 32, kBvSmem, st>>>(a, coef, dC, n_tiles, n_full, n_last);
+    launch(kern, (unsigned)grid, kWarpsPerCta * 32, kBvSmem, st, a, coef, dC, n_tiles, n_full, n_last);
     BB200_CUDA(cudaPeekAtLastError());
-    k_coeff_grads_to_dw<<<groups8, kWarpsPerCta * 32, 0, st>>>(reinterpret_cast<const float4 *>(dC), a.dW, a.O);
+    launch(k_coeff_grads_to_dw, groups8, kWarpsPerCta * 32, 0, st, reinterpret_cast<const float4 *>(dC), a.dW, a.O);
     return launch_status();
 }
 
@@ -1300,7 +1312,7 @@ static int backward_common(BwdArgs a, bool bn, long long total_frames, float *dm
             int rc = BBCU_OK;
             if (XBIT || !backward_stats_pipe(a, st, &rc, tmp, tmp_bytes)) {
                 BB200_CUDA(cudaMemsetAsync(sums, 0, sizeof(double) * 2 * (size_t)a.O, st));
-                k_lut6_backward_stats<XBIT><<<(unsigned)blocks, kWarpsPerCta * 32, 0, st>>>(a);
+                launch(k_lut6_backward_stats<XBIT>, (unsigned)blocks, kWarpsPerCta * 32, 0, st, a);
                 rc = launch_status();
             }
             if (rc) return rc;
@@ -1318,12 +1330,12 @@ static int backward_common(BwdArgs a, bool bn, long long total_frames, float *dm
     }
     BB200_CUDA(cudaMemsetAsync(a.dx, 0, dx_bytes, st));
     if (bn) {
-        k_bn_backward_finalize<<<(a.O + 255) / 256, 256, 0, st>>>(ext_sums, a.mean, a.rstd, dmean_out, dvar_out, a.O, total_frames);
+        launch(k_bn_backward_finalize, (a.O + 255) / 256, 256, 0, st, ext_sums, a.mean, a.rstd, dmean_out, dvar_out, a.O, total_frames);
         BB200_CUDA(cudaPeekAtLastError());
         a.dmean = dmean_out; a.dvar = dvar_out;
     }
-    if (bn) k_lut6_backward<XBIT, true><<<(unsigned)blocks, kWarpsPerCta * 32, 0, st>>>(a);
-    else    k_lut6_backward<XBIT, false><<<(unsigned)blocks, kWarpsPerCta * 32, 0, st>>>(a);
+    if (bn) launch(k_lut6_backward<XBIT, true>, (unsigned)blocks, kWarpsPerCta * 32, 0, st, a);
+    else    launch(k_lut6_backward<XBIT, false>, (unsigned)blocks, kWarpsPerCta * 32, 0, st, a);
     return launch_status();
 }
 
@@ -1437,9 +1449,9 @@ static int dl6_finalize_and_normalize(float *y, const double *sums, float *mean,
         const int chunks = (F + 4095) / 4096;
         const long long blocks = (long long)O * chunks;
         BB200_REQUIRE(blocks < (1LL << 31), BBCU_ERR_TOO_LARGE);
-        k_bn_normalize_inplace<<<(unsigned)blocks, 256, 0, st>>>(y, sums, mean, rstd, rmean, rvar, gamma, beta, momentum, total_frames, F, ys, binary, chunks);
+        launch(k_bn_normalize_inplace, (unsigned)blocks, 256, 0, st, y, sums, mean, rstd, rmean, rvar, gamma, beta, momentum, total_frames, F, ys, binary, chunks);
     } else {
-        k_bn_finalize<<<(O + 255) / 256, 256, 0, st>>>(sums, mean, rstd, rmean, rvar, momentum, O, total_frames);
+        launch(k_bn_finalize, (O + 255) / 256, 256, 0, st, sums, mean, rstd, rmean, rvar, momentum, O, total_frames);
     }
     return launch_status();
 }
@@ -1670,7 +1682,7 @@ extern "C" int bbcu_fp32_DifferentiableLut6_BackwardStats(const float *x, const 
     a.T = frame_tile(3LL * a.O, 32, a.groups, a.F, 2048);
     const long long blocks = (long long)((a.F + a.T - 1) / a.T) * a.groups;
     BB200_REQUIRE(blocks < (1LL << 31), BBCU_ERR_TOO_LARGE);
-    k_lut6_backward_stats<false><<<(unsigned)blocks, kWarpsPerCta * 32, 0, st>>>(a);
+    launch(k_lut6_backward_stats<false>, (unsigned)blocks, kWarpsPerCta * 32, 0, st, a);
     return launch_status();
 }
 
@@ -1688,7 +1700,7 @@ extern "C" int bbcu_fp32_DifferentiableLut6_BackwardStatsFromOutput(const float 
     if (chunks != 1) BB200_CUDA(cudaMemsetAsync(dev_sums, 0, sizeof(double) * 2 * (size_t)node_size, st));
     if (frame_size == 0) return BBCU_OK;
     BB200_REQUIRE((long long)node_size * chunks < (1LL << 31), BBCU_ERR_TOO_LARGE);
-    k_dl6_backward_stats_from_y<<<node_size * chunks, 256, 0, st>>>(y, dy, rstd, dev_sums, gamma, beta, frame_size, frame_stride, frame_stride,
+    launch(k_dl6_backward_stats_from_y, node_size * chunks, 256, 0, st, y, dy, rstd, dev_sums, gamma, beta, frame_size, frame_stride, frame_stride,
                                                                     chunks);
     return launch_status();
 }

@@ -33,6 +33,7 @@ template <int MODE>
 __global__ void __launch_bounds__(kWarpsPerCta * 32)
 k_lut6_small_forward(const SmallLayerArgs a)
 {
+    grid_dependency();
     extern __shared__ __align__(16) float s_raw[];                                             // kSmallTrain: the node's raw values
     __shared__ float4 s_tab[32];
     __shared__ double s_sum[kWarpsPerCta][2];
@@ -134,6 +135,7 @@ template <bool BN>
 __global__ void __launch_bounds__(kWarpsPerCta * 32, 1)
 k_lut6_small_backward(const SmallLayerArgs a)
 {
+    grid_dependency();
     __shared__ float4 s_tab[16];
     __shared__ double s_sum[kWarpsPerCta][2];
     __shared__ float s_stat[2];
@@ -268,11 +270,11 @@ int small_forward(int mode, const SmallLayerArgs &a, int O, cudaStream_t st)
     const unsigned threads = threads_for(a.F);
     if (mode == kSmallTrain) {
         const int round = 4 * (int)threads;
-        k_lut6_small_forward<kSmallTrain><<<O, threads, (a.F + round - 1) / round * round * (int)sizeof(float), st>>>(a);
+        launch(k_lut6_small_forward<kSmallTrain>, O, threads, (a.F + round - 1) / round * round * (int)sizeof(float), st, a);
     } else if (mode == kSmallInfer) {
-        k_lut6_small_forward<kSmallInfer><<<O, threads, 0, st>>>(a);
+        launch(k_lut6_small_forward<kSmallInfer>, O, threads, 0, st, a);
     } else {
-        k_lut6_small_forward<kSmallPlain><<<O, threads, 0, st>>>(a);
+        launch(k_lut6_small_forward<kSmallPlain>, O, threads, 0, st, a);
     }
     return launch_status();
 }
@@ -280,8 +282,8 @@ int small_forward(int mode, const SmallLayerArgs &a, int O, cudaStream_t st)
 int small_backward(bool bn, const SmallLayerArgs &a, int I, int O, cudaStream_t st)
 {
     BB200_CUDA(cudaMemsetAsync(a.dx, 0, sizeof(float) * (size_t)I * (size_t)a.fs, st));
-    if (bn) k_lut6_small_backward<true><<<O, threads_for(a.F), 0, st>>>(a);
-    else    k_lut6_small_backward<false><<<O, threads_for(a.F), 0, st>>>(a);
+    if (bn) launch(k_lut6_small_backward<true>, O, threads_for(a.F), 0, st, a);
+    else    launch(k_lut6_small_backward<false>, O, threads_for(a.F), 0, st, a);
     return launch_status();
 }
 

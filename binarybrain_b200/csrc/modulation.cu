@@ -19,6 +19,7 @@ __global__ void __launch_bounds__(256)
 k_real_to_binary_bit(const float *__restrict__ x, uint32_t *y, const float *__restrict__ th, unsigned depth_mod, unsigned frame_mod, float lo,
                      float hi, unsigned point_size, unsigned x_frame_size, long long xs, long long ys, long long ths)
 {
+    grid_dependency();
     const unsigned node = blockIdx.y;                                  // output node = (input_depth * depth_mod + d) * point_size + p
     const unsigned out_frames = x_frame_size * frame_mod;
     unsigned of = blockIdx.x * kR2bFrames + threadIdx.x;               // output frame = fi * frame_mod + f
@@ -71,6 +72,7 @@ template <bool XBIT>
 __global__ void __launch_bounds__(256)
 k_binary_to_real_forward(const void *x, float *y, int node_mux, int frame_mux, int y_nodes, long long xs, int y_frames, long long ys)
 {
+    grid_dependency();
     __shared__ int s_cnt[32 * kB2rSteps];                              // counts of a run of input frames
     __shared__ int s_out[32];
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
@@ -113,6 +115,7 @@ __global__ void __launch_bounds__(256)
 k_binary_to_real_backward(const float *__restrict__ dy, float *dx, int node_mux, int frame_mux, int y_nodes, long long xs, int y_frames, long long ys,
                           int vec)
 {
+    grid_dependency();
     const long long x_frames = (long long)y_frames * frame_mux;
     const long long xf = 4 * ((long long)blockIdx.x * blockDim.x + threadIdx.x);
     const int xn = blockIdx.y;
@@ -154,7 +157,7 @@ extern "C" int bbcu_bit_fp32_RealToBinary_Forward(const float *x, int *y, const 
     BB200_REQUIRE(dev_thresholds == nullptr || (unsigned long long)threshold_frame_stride >= out_frames, BBCU_ERR_BAD_STRIDE);
     if (out_frames == 0 || out_nodes == 0) return BBCU_OK;
     BB200_REQUIRE(out_nodes <= 65535, BBCU_ERR_TOO_LARGE);
-    k_real_to_binary_bit<<<dim3((unsigned)((out_frames + kR2bFrames - 1) / kR2bFrames), (unsigned)out_nodes), 256, 0, as_stream(stream)>>>(
+    launch(k_real_to_binary_bit, dim3((unsigned)((out_frames + kR2bFrames - 1) / kR2bFrames), (unsigned)out_nodes), 256, 0, as_stream(stream),
         x, reinterpret_cast<uint32_t *>(y), dev_thresholds, depth_modulation_size, frame_modulation_size, input_range_lo, input_range_hi, point_size,
         x_frame_size, x_frame_stride, y_frame_stride, threshold_frame_stride);
     return launch_status();
@@ -174,7 +177,7 @@ extern "C" int bbcu_bit_fp32_BinaryToReal_Forward(const int *x, float *y, int no
 {
     int rc = b2r_check(x, y, node_mux_size, frame_mux_size, y_node_size, x_frame_stride, y_frame_size, y_frame_stride, true);
     if (rc || y_frame_size == 0) return rc;
-    k_binary_to_real_forward<true><<<dim3((y_frame_size + 31) / 32, y_node_size), 256, 0, as_stream(stream)>>>(
+    launch(k_binary_to_real_forward<true>, dim3((y_frame_size + 31) / 32, y_node_size), 256, 0, as_stream(stream),
         x, y, node_mux_size, frame_mux_size, y_node_size, x_frame_stride, y_frame_size, y_frame_stride);
     return launch_status();
 }
@@ -184,7 +187,7 @@ extern "C" int bbcu_fp32_BinaryToReal_Forward(const float *x, float *y, int node
 {
     int rc = b2r_check(x, y, node_mux_size, frame_mux_size, y_node_size, x_frame_stride, y_frame_size, y_frame_stride, false);
     if (rc || y_frame_size == 0) return rc;
-    k_binary_to_real_forward<false><<<dim3((y_frame_size + 31) / 32, y_node_size), 256, 0, as_stream(stream)>>>(
+    launch(k_binary_to_real_forward<false>, dim3((y_frame_size + 31) / 32, y_node_size), 256, 0, as_stream(stream),
         x, y, node_mux_size, frame_mux_size, y_node_size, x_frame_stride, y_frame_size, y_frame_stride);
     return launch_status();
 }
@@ -196,7 +199,7 @@ extern "C" int bbcu_fp32_BinaryToReal_Backward(const float *dy, float *dx, int n
     if (rc || y_frame_size == 0) return rc;
     const long long xf = (long long)y_frame_size * frame_mux_size;
     const int vec = (reinterpret_cast<uintptr_t>(dx) & 15) == 0 && x_frame_stride % 4 == 0;
-    k_binary_to_real_backward<<<dim3((unsigned)((xf + 1023) / 1024), y_node_size * node_mux_size), 256, 0, as_stream(stream)>>>(
+    launch(k_binary_to_real_backward, dim3((unsigned)((xf + 1023) / 1024), y_node_size * node_mux_size), 256, 0, as_stream(stream),
         dy, dx, node_mux_size, frame_mux_size, y_node_size, x_frame_stride, y_frame_size, y_frame_stride, vec);
     return launch_status();
 }

@@ -46,6 +46,7 @@ __device__ __forceinline__ void for_each_frame(int f0, int f1, bool vec, Fn fn)
 __global__ void __launch_bounds__(256)
 k_sbn_stats(const float *__restrict__ x, double *sums, int F, long long xs, int chunks)
 {
+    grid_dependency();
     __shared__ double red[8];
     const int node = blockIdx.x / chunks, chunk = blockIdx.x % chunks;
     const float *row = x + (size_t)node * xs;
@@ -69,6 +70,7 @@ k_sbn_stats(const float *__restrict__ x, double *sums, int F, long long xs, int 
 __global__ void k_sbn_finalize(const double *__restrict__ sums, float *mean_out, float *rstd_out, float *running_mean, float *running_var,
                                float momentum, int O, int F)
 {
+    grid_dependency();
     int n = blockIdx.x * blockDim.x + threadIdx.x;
     if (n >= O) return;
     const double m = sums[2 * (size_t)n] / (double)F;
@@ -88,6 +90,7 @@ __global__ void __launch_bounds__(256)
 k_sbn_apply(const float *__restrict__ x, float *y, const float *__restrict__ a_buf, const float *__restrict__ b_buf,
             float gamma, float beta, int F, long long xs, int chunks, int mode)
 {
+    grid_dependency();
     const int node = blockIdx.x / chunks, chunk = blockIdx.x % chunks;
     const float *row = x + (size_t)node * xs;
     float *out = y + (size_t)node * xs;
@@ -120,6 +123,7 @@ __global__ void __launch_bounds__(256)
 k_sbn_backward_stats(const float *__restrict__ x, const float *__restrict__ dy, const float *__restrict__ mean_buf,
                      const float *__restrict__ rstd_buf, double *sums, float gamma, int F, long long xs, long long dys, int chunks)
 {
+    grid_dependency();
     __shared__ double red[8];
     const int node = blockIdx.x / chunks, chunk = blockIdx.x % chunks;
     const float *xr = x + (size_t)node * xs;
@@ -152,6 +156,7 @@ k_sbn_backward_apply(const float *__restrict__ x, const float *__restrict__ dy, 
                      const float *__restrict__ rstd_buf, const double *__restrict__ sums, float gamma, float rF, int F,
                      long long xs, long long dys, int chunks)
 {
+    grid_dependency();
     const int node = blockIdx.x / chunks, chunk = blockIdx.x % chunks;
     const float *xr = x + (size_t)node * xs;
     const float *gr = dy + (size_t)node * dys;
@@ -179,11 +184,13 @@ k_sbn_backward_apply(const float *__restrict__ x, const float *__restrict__ dy, 
 // ------------------------------------------------------------------------------------------- element-wise
 __global__ void k_clamp(float *dst, const float *__restrict__ src, float lo, float hi, int n)
 {
+    grid_dependency();
     for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x) dst[i] = fmaxf(lo, fminf(hi, src[i]));
 }
 
 __global__ void k_set(float *dst, float a, int n)
 {
+    grid_dependency();
     for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x) dst[i] = a;
 }
 
@@ -194,6 +201,7 @@ __global__ void __launch_bounds__(256)
 k_adam(const int *__restrict__ size_table, float *const *params, float *const *grads, float *const *m_tab, float *const *v_tab, float lr_t,
        float beta1, float beta2)
 {
+    grid_dependency();
     const int t = blockIdx.y;
     const int n = size_table[t];
     float *p = params[t], *m = m_tab[t], *v = v_tab[t], *g = grads[t];
@@ -250,11 +258,11 @@ extern "C" int bbcu_fp32_StochasticBatchNormalization_ForwardTraining(const floa
     BB200_REQUIRE(sums != nullptr, BBCU_ERR_NO_MEMORY);
     BB200_CUDA(cudaMemsetAsync(sums, 0, sizeof(double) * 2 * (size_t)node_size, st));
     const int chunks = (frame_size + kChunk - 1) / kChunk;
-    k_sbn_stats<<<node_size * chunks, 256, 0, st>>>(x, sums, frame_size, frame_stride, chunks);
+    launch(k_sbn_stats, node_size * chunks, 256, 0, st, x, sums, frame_size, frame_stride, chunks);
     BB200_CUDA(cudaPeekAtLastError());
-    k_sbn_finalize<<<(node_size + 255) / 256, 256, 0, st>>>(sums, mean, rstd, rmean, rvar, momentum, node_size, frame_size);
+    launch(k_sbn_finalize, (node_size + 255) / 256, 256, 0, st, sums, mean, rstd, rmean, rvar, momentum, node_size, frame_size);
     BB200_CUDA(cudaPeekAtLastError());
-    k_sbn_apply<<<node_size * chunks, 256, 0, st>>>(x, y, mean, rstd, gamma, beta, frame_size, frame_stride, chunks, 0);
+    launch(k_sbn_apply, node_size * chunks, 256, 0, st, x, y, mean, rstd, gamma, beta, frame_size, frame_stride, chunks, 0);
     return launch_status();
 }
 
@@ -267,7 +275,7 @@ extern "C" int bbcu_fp32_StochasticBatchNormalization_ReForward(const float *x, 
     BB200_REQUIRE_PTR(mean); BB200_REQUIRE_PTR(rstd);
     if (node_size == 0 || frame_size == 0) return BBCU_OK;
     const int chunks = (frame_size + kChunk - 1) / kChunk;
-    k_sbn_apply<<<node_size * chunks, 256, 0, as_stream(stream)>>>(x, y, mean, rstd, gamma, beta, frame_size, frame_stride, chunks, 0);
+    launch(k_sbn_apply, node_size * chunks, 256, 0, as_stream(stream), x, y, mean, rstd, gamma, beta, frame_size, frame_stride, chunks, 0);
     return launch_status();
 }
 
@@ -280,7 +288,7 @@ extern "C" int bbcu_fp32_StochasticBatchNormalization_ForwardInference(const flo
     BB200_REQUIRE_PTR(rmean); BB200_REQUIRE_PTR(rvar);
     if (node_size == 0 || frame_size == 0) return BBCU_OK;
     const int chunks = (frame_size + kChunk - 1) / kChunk;
-    k_sbn_apply<<<node_size * chunks, 256, 0, as_stream(stream)>>>(x, y, rmean, rvar, gamma, beta, frame_size, frame_stride, chunks, 1);
+    launch(k_sbn_apply, node_size * chunks, 256, 0, as_stream(stream), x, y, rmean, rvar, gamma, beta, frame_size, frame_stride, chunks, 1);
     return launch_status();
 }
 
@@ -298,9 +306,9 @@ extern "C" int bbcu_fp32_StochasticBatchNormalization_Backward(const float *x, c
     BB200_REQUIRE(sums != nullptr, BBCU_ERR_NO_MEMORY);
     BB200_CUDA(cudaMemsetAsync(sums, 0, sizeof(double) * 2 * (size_t)node_size, st));
     const int chunks = (frame_size + kChunk - 1) / kChunk;
-    k_sbn_backward_stats<<<node_size * chunks, 256, 0, st>>>(x, dy, mean, rstd, sums, gamma, frame_size, x_frame_stride, frame_stride, chunks);
+    launch(k_sbn_backward_stats, node_size * chunks, 256, 0, st, x, dy, mean, rstd, sums, gamma, frame_size, x_frame_stride, frame_stride, chunks);
     BB200_CUDA(cudaPeekAtLastError());
-    k_sbn_backward_apply<<<node_size * chunks, 256, 0, st>>>(x, dy, dx, mean, rstd, sums, gamma, reciprocal_frame_size, frame_size,
+    launch(k_sbn_backward_apply, node_size * chunks, 256, 0, st, x, dy, dx, mean, rstd, sums, gamma, reciprocal_frame_size, frame_size,
                                                            x_frame_stride, frame_stride, chunks);
     return launch_status();
 }
@@ -311,7 +319,7 @@ extern "C" int bbcu_fp32_Vector_clamp(float *dst, const float *src, float lo, fl
     BB200_REQUIRE(size >= 0, BBCU_ERR_BAD_SIZE);
     if (size == 0) return BBCU_OK;
     int blocks = (size + 255) / 256; if (blocks > 4096) blocks = 4096;
-    k_clamp<<<blocks, 256, 0, as_stream(stream)>>>(dst, src, lo, hi, size);
+    launch(k_clamp, blocks, 256, 0, as_stream(stream), dst, src, lo, hi, size);
     return launch_status();
 }
 
@@ -321,7 +329,7 @@ extern "C" int bbcu_fp32_Vector_set(float *dst, float a, int size, bbcu_stream_t
     BB200_REQUIRE(size >= 0, BBCU_ERR_BAD_SIZE);
     if (size == 0) return BBCU_OK;
     int blocks = (size + 255) / 256; if (blocks > 4096) blocks = 4096;
-    k_set<<<blocks, 256, 0, as_stream(stream)>>>(dst, a, size);
+    launch(k_set, blocks, 256, 0, as_stream(stream), dst, a, size);
     return launch_status();
 }
 
@@ -332,7 +340,7 @@ static int adam(bool clear, int size, const int *size_table, float *const *param
     BB200_REQUIRE(size >= 0 && size <= 65535, BBCU_ERR_BAD_SIZE);
     if (size == 0) return BBCU_OK;
     auto kern = clear ? k_adam<true> : k_adam<false>;
-    kern<<<dim3(296, size), 256, 0, as_stream(stream)>>>(size_table, params, grads, m_tab, v_tab, lr_t, beta1, beta2);
+    launch(kern, dim3(296, size), 256, 0, as_stream(stream), size_table, params, grads, m_tab, v_tab, lr_t, beta1, beta2);
     return launch_status();
 }
 
