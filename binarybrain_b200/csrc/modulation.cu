@@ -62,31 +62,31 @@ k_real_to_binary_bit(const float *__restrict__ x, uint32_t *y, const float *__re
 }
 
 // y[f][n] = mean over i < node_mux, j < frame_mux of bit x[f * frame_mux + j][n + i * y_nodes]
-// Block = one output node x 32 output frames, i.e. 32 * frame_mux consecutive input frames of node_mux rows; its eight warps share
-// the rows, a lane counts its input frames (lane + 32 m) over the warp's rows in registers, and the counts meet in shared
+// Block = one output node x 32 output frames, i.e. 32 * frame_mux consecutive input frames of node_mux rows; its warps (8 to 32, a row
+// each while there are enough: there are few blocks, and 13 rows one after the other took a warp 14 us for 1020 x 1792 -> 10 x 256, 8.6 us now) share the rows, a lane counts its input frames (lane + 32 m) over the warp's rows in registers, and the counts meet in shared
 // memory.  The counts are whole numbers, so the order of addition does not show.  (One thread per output value walked its node_mux *
 // frame_mux inputs alone: 1020 x 1792 -> 10 x 256 took 43 us on 2560 threads; the rows are 7.3 MB.)
 constexpr int kB2rSteps = 8;
 
 template <bool XBIT>
-__global__ void __launch_bounds__(256)
+__global__ void __launch_bounds__(1024)
 k_binary_to_real_forward(const void *x, float *y, int node_mux, int frame_mux, int y_nodes, long long xs, int y_frames, long long ys)
 {
     grid_dependency();
     __shared__ int s_cnt[32 * kB2rSteps];                              // counts of a run of input frames
     __shared__ int s_out[32];
-    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, warps = blockDim.x >> 5;
     const int n = blockIdx.y, f0 = blockIdx.x * 32;
     const long long x_begin = (long long)f0 * frame_mux, x_end = (long long)min(y_frames, f0 + 32) * frame_mux;
     if (threadIdx.x < 32) s_out[threadIdx.x] = 0;
     for (int m0 = 0; m0 < frame_mux; m0 += kB2rSteps) {
         const int m_end = min(kB2rSteps, frame_mux - m0);
-        s_cnt[threadIdx.x] = 0;
+        if (threadIdx.x < 32 * kB2rSteps) s_cnt[threadIdx.x] = 0;
         __syncthreads();
         int acc[kB2rSteps];
 #pragma unroll
         for (int m = 0; m < kB2rSteps; ++m) acc[m] = 0;
-        for (int i = warp; i < node_mux; i += 8) {
+        for (int i = warp; i < node_mux; i += warps) {
             const size_t row = (size_t)(n + (size_t)i * y_nodes) * xs;
 #pragma unroll
             for (int m = 0; m < kB2rSteps; ++m) {
@@ -172,12 +172,14 @@ static int b2r_check(const void *x, const void *y, int node_mux, int frame_mux, 
     return BBCU_OK;
 }
 
+static int b2r_threads(int node_mux) { return 32 * (node_mux < 8 ? 8 : node_mux > 32 ? 32 : node_mux); }
+
 extern "C" int bbcu_bit_fp32_BinaryToReal_Forward(const int *x, float *y, int node_mux_size, int frame_mux_size, int y_node_size,
                                                   int x_frame_stride, int y_frame_size, int y_frame_stride, bbcu_stream_t stream)
 {
     int rc = b2r_check(x, y, node_mux_size, frame_mux_size, y_node_size, x_frame_stride, y_frame_size, y_frame_stride, true);
     if (rc || y_frame_size == 0) return rc;
-    launch(k_binary_to_real_forward<true>, dim3((y_frame_size + 31) / 32, y_node_size), 256, 0, as_stream(stream),
+    launch(k_binary_to_real_forward<true>, dim3((y_frame_size + 31) / 32, y_node_size), b2r_threads(node_mux_size), 0, as_stream(stream),
         x, y, node_mux_size, frame_mux_size, y_node_size, x_frame_stride, y_frame_size, y_frame_stride);
     return launch_status();
 }
@@ -187,7 +189,7 @@ extern "C" int bbcu_fp32_BinaryToReal_Forward(const float *x, float *y, int node
 {
     int rc = b2r_check(x, y, node_mux_size, frame_mux_size, y_node_size, x_frame_stride, y_frame_size, y_frame_stride, false);
     if (rc || y_frame_size == 0) return rc;
-    launch(k_binary_to_real_forward<false>, dim3((y_frame_size + 31) / 32, y_node_size), 256, 0, as_stream(stream),
+    launch(k_binary_to_real_forward<false>, dim3((y_frame_size + 31) / 32, y_node_size), b2r_threads(node_mux_size), 0, as_stream(stream),
         x, y, node_mux_size, frame_mux_size, y_node_size, x_frame_stride, y_frame_size, y_frame_stride);
     return launch_status();
 }
