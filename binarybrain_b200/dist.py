@@ -64,20 +64,19 @@ class ShardedDifferentiableLut6:
 
     def forward(self, x, frames, total_frames, y=None):
         """x: this rank's [n_in, stride] shard with `frames` valid frames; total_frames: frames of the whole step."""
-        if y is None:
-            y = torch.empty((self.n_out, x.shape[1]), dtype=torch.float32, device=x.device)
         # One rank needs no exchange point: the unsplit operators, which take the per-pattern table route in binary mode and run a small
         # layer in one launch.  (A large layer in probability mode keeps the split operators, whose backward reads the saved output.)
         self._fused = (hasattr(self.ops, "differentiable_lut6_forward_training") and self.world == 1 and
                        (self.binary or (frames == total_frames and frames <= self.ops.SMALL_FRAMES and
                                         frames * self.n_out <= self.ops.SMALL_NODE_FRAMES)))
         if self._fused:
-            _, mean, rstd = self.ops.differentiable_lut6_forward_training(x, self.idx, self.W, self.running_mean, self.running_var, frames, y=y,
-                                                                         gamma=self.gamma, beta=self.beta, momentum=self.momentum,
-                                                                         lut_binarize=self.lut_binarize, binary=self.binary)
-            self.mean, self.rstd = mean, rstd
+            y, self.mean, self.rstd = self.ops.differentiable_lut6_forward_training(
+                x, self.idx, self.W, self.running_mean, self.running_var, frames, y=y, gamma=self.gamma, beta=self.beta, momentum=self.momentum,
+                lut_binarize=self.lut_binarize, binary=self.binary)
             self._x, self._frames, self._total, self._y = x, frames, total_frames, None
             return y
+        if y is None:
+            y = torch.empty((self.n_out, x.shape[1]), dtype=torch.float32, device=x.device)
         self.ops.dl6_forward_stats(x, self.idx, self.W, frames, y, self.sums, lut_binarize=self.lut_binarize, binary=self.binary)
         self._allreduce(self.sums)
         self.ops.dl6_forward_normalize(y, self.sums, self.mean, self.rstd, self.running_mean, self.running_var, frames, total_frames,
@@ -91,13 +90,12 @@ class ShardedDifferentiableLut6:
     def backward(self, dy, dx=None):
         """Returns dx for this rank's frames; dW (local partial) is all-reduced asynchronously -- call wait_grad() before using it."""
         x, frames, total = self._x, self._frames, self._total
-        if dx is None:
-            dx = torch.empty((self.n_in, dy.shape[1]), dtype=torch.float32, device=dy.device)
         kw = dict(gamma=self.gamma, beta=self.beta, lut_binarize=self.lut_binarize, binary=self.binary)
         if getattr(self, "_fused", False):
-            self.ops.differentiable_lut6_backward(x, dy, self.idx, self.W, self.dW, self.mean, self.rstd, self.n_in, frames, dx=dx, **kw)
             self._x = None
-            return dx
+            return self.ops.differentiable_lut6_backward(x, dy, self.idx, self.W, self.dW, self.mean, self.rstd, self.n_in, frames, dx=dx, **kw)
+        if dx is None:
+            dx = torch.empty((self.n_in, dy.shape[1]), dtype=torch.float32, device=dy.device)
         if self._y is not None and self._y.shape[1] == dy.shape[1]:
             self.ops.dl6_backward_stats_from_output(self._y, dy, self.rstd, frames, self.sums, gamma=self.gamma, beta=self.beta)
         else:

@@ -139,7 +139,9 @@ def differentiable_lut6_backward(x, dy, idx, W, dW, mean, rstd, n_in, frames, dx
     O = idx.shape[0]
     if dx is None:
         dx = _n.empty_f32(dy, n_in, dy.shape[1])
-    dmean, dvar = _n.vector_f32(dy, O), _n.vector_f32(dy, O)
+    scratch = _n.vector_f32(dy, 2 * O)
+    dmean = scratch.data_ptr()
+    dvar = dmean + 4 * O
     if x.dtype == torch.float32:
         assert x.shape[1] == dy.shape[1]
         _n.bbcu_fp32_DifferentiableLut6_Backward(x, dy, dx, dx_tmp, idx, 0, W, dW, mean, rstd, dmean, dvar, gamma, beta, bias, 0, n_in, O, frames,
