@@ -1335,6 +1335,15 @@ bool backward_setup(BitBwdArgs &a, const void *x, const float *dy, const int *id
     return true;
 }
 
+bool pack_bits(const float *x, uint32_t *bits, int I, int F, long long xs, long long ws, cudaStream_t st)
+{
+    const int runs = (int)((ws + 31) / 32);
+    const long long blocks = ((long long)I * runs + kWarpsPerCta - 1) / kWarpsPerCta;
+    if (blocks >= (1LL << 31)) return false;
+    launch(k_pack_bits, (unsigned)blocks, kWarpsPerCta * 32, 0, st, x, bits, I, F, xs, ws, runs);
+    return true;
+}
+
 // Slot 3 of the stream's scratch: consumer lists, and the bits of the I fp32 rows when `pack`.
 bool input_side(BitBwdArgs &a, int I, bool pack, cudaStream_t st)
 {
@@ -1355,10 +1364,7 @@ bool input_side(BitBwdArgs &a, int I, bool pack, cudaStream_t st)
     launch(k_edge_fill, (edges + 255) / 256, 256, 0, st, a.idx, cursor, list, edges);
     if (pack) {
         uint32_t *bits = reinterpret_cast<uint32_t *>(reinterpret_cast<unsigned char *>(count) + list_bytes);
-        const int runs = (int)((ws + 31) / 32);
-        const long long blocks = ((long long)I * runs + kWarpsPerCta - 1) / kWarpsPerCta;
-        if (blocks >= (1LL << 31)) return false;
-        launch(k_pack_bits, (unsigned)blocks, kWarpsPerCta * 32, 0, st, reinterpret_cast<const float *>(a.x), bits, I, a.F, a.xs, ws, runs);
+        if (!pack_bits(reinterpret_cast<const float *>(a.x), bits, I, a.F, a.xs, ws, st)) return false;
         a.x = bits;
         a.xs = ws;
     }
@@ -1410,6 +1416,29 @@ int launch_pattern_gather(BitBwdArgs a, bool bn, cudaStream_t st)
 }
 
 }   // namespace
+
+// Training forward in binary mode by way of the bit operators: pack the rows, count patterns and evaluate truth tables on bits, expand the
+// output.  Per node-frame that moves 4 bytes of y (and 4 per input row and frame) against the 24 + 1 that the per-node passes of
+// f32_binary_forward_by_table() read through L2: 8192 x 8192 nodes x 16384 frames 360 -> 302 us, 90 of them the packing.  So it is taken up to
+// two input rows a node.
+int f32_binary_forward_packed(const float *x, float *y, const int *idx, const float *W, float *mean, float *rstd, float *rmean, float *rvar,
+                              float gamma, float beta, float momentum, float bias, int I, int O, int F, long long fs, int lut_binarize,
+                              cudaStream_t st)
+{
+    if (small_layer(O, F) || I < 1 || I > 2LL * O) return BBCU_ERR_NO_MEMORY;
+    const long long ws = ((long long)F + 127) / 128 * 4;                // whole 16-byte pieces
+    const size_t x_bytes = (size_t)I * (size_t)ws * 4, y_bytes = (size_t)O * (size_t)ws * 4;
+    if (x_bytes + y_bytes > ((size_t)1 << 30)) return BBCU_ERR_NO_MEMORY;
+    uint32_t *xb = static_cast<uint32_t *>(stream_scratch(st, x_bytes + y_bytes, 3));
+    if (xb == nullptr) return BBCU_ERR_NO_MEMORY;
+    int *yb = reinterpret_cast<int *>(xb + (size_t)I * (size_t)ws);
+    if (!pack_bits(x, xb, I, F, fs, ws, st)) return BBCU_ERR_NO_MEMORY;
+    BB200_CUDA(cudaPeekAtLastError());
+    const int rc = dl6_bit_forward_training_by_table(reinterpret_cast<const int *>(xb), yb, idx, W, mean, rstd, rmean, rvar, gamma, beta, momentum, bias,
+                                                     O, F, (int)ws, lut_binarize, st);
+    if (rc) return rc;
+    return bbcu_fp32_ConvBitToReal(yb, y, 0.0f, 1.0f, O, F, (int)ws, (int)fs, reinterpret_cast<bbcu_stream_t>(st));
+}
 
 // Backward of the bit-input layers (StochasticLut6: bn = false; DifferentiableLut6: bn = true); writes all of dx's I rows.
 int bit_backward_by_table(bool bn, bool x_is_fp32, const void *x, const float *dy, float *dx, const int *idx, const float *W, float *dW,

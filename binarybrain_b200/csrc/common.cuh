@@ -70,6 +70,10 @@ int bit_backward_apply_by_table(const float *x, const float *dy, float *dx, cons
                                 const float *rstd, const double *sums, float *dmean_out, float *dvar_out, float gamma, float beta, float bias, int I,
                                 int O, int F, long long fs, long long total_frames, int lut_binarize, cudaStream_t st);
 
+// The training forward of a binary-mode layer on I fp32 rows through packed rows; declines (small layers, I > 2 O, no scratch) like the others.
+int f32_binary_forward_packed(const float *x, float *y, const int *idx, const float *W, float *mean, float *rstd, float *rmean, float *rvar,
+                              float gamma, float beta, float momentum, float bias, int I, int O, int F, long long fs, int lut_binarize,
+                              cudaStream_t st);
 int f32_binary_forward_by_table(int mode, const float *x, float *y, const int *idx, const float *W, float *mean, float *rstd, float *rmean,
                                 float *rvar, float gamma, float beta, float momentum, float bias, int O, int F, long long fs, int lut_binarize,
                                 cudaStream_t st);

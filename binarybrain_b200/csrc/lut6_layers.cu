@@ -1497,6 +1497,24 @@ extern "C" int bbcu_fp32_DifferentiableLut6_ForwardNormalize(float *y, const dou
                                       total_frame_size, binary_mode, as_stream(stream));
 }
 
+extern "C" int bbcu_fp32_DifferentiableLut6_ForwardTrainingRows(const float *x, float *y, const int *idx, const float *W, float *mean, float *rstd,
+                                                                float *rmean, float *rvar, float gamma, float beta, float momentum,
+                                                                float unbinarize_bias, int input_node_size, int node_size, int frame_size,
+                                                                int frame_stride, int lut_binarize, int binary_mode, bbcu_stream_t stream)
+{
+    BB200_REQUIRE(input_node_size >= 0, BBCU_ERR_BAD_SIZE);
+    if (binary_mode && node_size > 0 && frame_size > 0 && mean != nullptr && rstd != nullptr && rmean != nullptr && rvar != nullptr) {
+        int rc = check_common(x, y, idx, W, node_size, frame_size, frame_stride);
+        if (rc) return rc;
+        BB200_REQUIRE(frame_stride >= frame_size, BBCU_ERR_BAD_STRIDE);
+        rc = f32_binary_forward_packed(x, y, idx, W, mean, rstd, rmean, rvar, gamma, beta, momentum, unbinarize_bias, input_node_size, node_size,
+                                       frame_size, frame_stride, lut_binarize, as_stream(stream));
+        if (rc != BBCU_ERR_NO_MEMORY) return rc;
+    }
+    return bbcu_fp32_DifferentiableLut6_ForwardTraining(x, y, idx, W, mean, rstd, rmean, rvar, gamma, beta, momentum, unbinarize_bias, node_size,
+                                                        frame_size, frame_stride, lut_binarize, binary_mode, stream);
+}
+
 extern "C" int bbcu_fp32_DifferentiableLut6_ForwardTraining(const float *x, float *y, const int *idx, const float *W, float *mean, float *rstd,
                                                             float *rmean, float *rvar, float gamma, float beta, float momentum,
                                                             float unbinarize_bias, int node_size, int frame_size, int frame_stride,

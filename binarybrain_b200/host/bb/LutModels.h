@@ -520,10 +520,10 @@ public:
             } else {
                 BB_ASSERT(xs == ys);
                 if (train) {
-                    BBCU_CHECK(bbcu_fp32_DifferentiableLut6_ForwardTraining(
+                    BBCU_CHECK(bbcu_fp32_DifferentiableLut6_ForwardTrainingRows(
                         (float const *)x_buf.LockDeviceMemoryConst(), (float *)y_buf.LockDeviceMemory(true), idx, this->m_W->DevConst(), m_mean.Dev(true),
-                        m_rstd.Dev(true), m_running_mean.Dev(), m_running_var.Dev(), m_gamma, m_beta, m_momentum, this->m_unbinarize_bias, O, F, ys,
-                        this->m_lut_binarize, this->m_binary_mode, st));
+                        m_rstd.Dev(true), m_running_mean.Dev(), m_running_var.Dev(), m_gamma, m_beta, m_momentum, this->m_unbinarize_bias, (int)x_buf.GetNodeSize(),
+                        O, F, ys, this->m_lut_binarize, this->m_binary_mode, st));
                     // probability mode: the backward takes its batch-norm sums from this output (8 bytes per node-frame) instead of
                     // evaluating the LUT a second time; the buffer is the one the next layer holds anyway
                     m_y_stack.push_back(this->m_binary_mode ? FrameBuffer() : y_buf);

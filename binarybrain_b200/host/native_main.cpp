@@ -142,7 +142,7 @@ PyObject *scalar_f64(PyObject *, PyObject *const *o, Py_ssize_t n) { return empt
 
 #define BB200_OPERATORS(X)                                                                                                                    \
     X(bbcu_fp32_StochasticLut6_Forward) X(bbcu_bit_fp32_StochasticLut6_Forward) X(bbcu_bit_bit_fp32_StochasticLut6_Forward)                   \
-    X(bbcu_fp32_StochasticLut6_Backward) X(bbcu_bit_fp32_StochasticLut6_Backward) X(bbcu_fp32_DifferentiableLut6_ForwardTraining)             \
+    X(bbcu_fp32_StochasticLut6_Backward) X(bbcu_bit_fp32_StochasticLut6_Backward) X(bbcu_fp32_DifferentiableLut6_ForwardTrainingRows)         \
     X(bbcu_bit_fp32_DifferentiableLut6_ForwardTraining) X(bbcu_fp32_DifferentiableLut6_ForwardInference)                                      \
     X(bbcu_bit_fp32_DifferentiableLut6_ForwardInference) X(bbcu_fp32_DifferentiableLut6_Backward) X(bbcu_bit_fp32_DifferentiableLut6_Backward) \
     X(bbcu_fp32_DifferentiableLut6_ForwardStats) X(bbcu_fp32_DifferentiableLut6_ForwardNormalize) X(bbcu_fp32_DifferentiableLut6_BackwardStats) \

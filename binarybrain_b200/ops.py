@@ -107,8 +107,8 @@ def differentiable_lut6_forward_training(x, idx, W, running_mean, running_var, f
     if x.dtype == torch.float32:
         if y is None:
             y = _n.empty_f32(x, O, x.shape[1])
-        _n.bbcu_fp32_DifferentiableLut6_ForwardTraining(x, y, idx, W, mean, rstd, running_mean, running_var, gamma, beta, momentum, bias, O, frames,
-                                                        x.shape[1], int(lut_binarize), int(binary))
+        _n.bbcu_fp32_DifferentiableLut6_ForwardTrainingRows(x, y, idx, W, mean, rstd, running_mean, running_var, gamma, beta, momentum, bias,
+                                                            x.shape[0], O, frames, x.shape[1], int(lut_binarize), int(binary))
     else:
         _chk(x, torch.int32, "x")
         if y is None:

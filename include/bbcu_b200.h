@@ -342,6 +342,14 @@ int bbcu_fp32_DifferentiableLut6_BackwardFromOutput(const float *dev_x_buf, cons
                                                     int input_node_size, int output_node_size, int frame_size, int frame_stride, int lut_binarize,
                                                     bbcu_stream_t stream);
 
+/* Additive: bbcu_fp32_DifferentiableLut6_ForwardTraining for callers that know how many rows x has (the reference's operator is not
+ * told).  Same results; a large layer in binary mode then packs its input rows to bits once instead of reading six fp32 rows per node. */
+int bbcu_fp32_DifferentiableLut6_ForwardTrainingRows(const float *dev_x_buf, float *dev_y_buf, const int *dev_input_index, const float *dev_W,
+                                                     float *dev_mean_buf, float *dev_rstd_buf, float *dev_running_mean_buf,
+                                                     float *dev_running_var_buf, float gamma, float beta, float momentum, float unbinarize_bias,
+                                                     int input_node_size, int node_size, int frame_size, int frame_stride, int lut_binarize,
+                                                     int binary_mode, bbcu_stream_t stream);
+
 /* ------------------------------------------------------------------ Additive: a training forward that allocates nothing.
  * No counterpart in the reference.  Same arguments and results as bbcu_fp32_DifferentiableLut6_ForwardTraining, for callers that
  * cannot tolerate a cudaMalloc inside the call (a pre-planned device-memory budget, or a latency path that must not take

@@ -89,6 +89,12 @@ def test_two_valued_layers_edges(ops, I, O, F, stride):
     assert err(host_fp32(dx, F), dx_w) <= parity.BN_GRAD_FACTOR * parity.TOL * amp and err(dW.cpu().numpy(), dW_w) <= parity.BN_GRAD_FACTOR * parity.TOL * amp
 
 
+# above the one-launch range, fp32 rows packed for the forward (up to two input rows a node) and not
+@pytest.mark.parametrize("I,O,F,stride", [(700, 1025, 2049, None), (70, 40, 4129, 4131), (60, 33, 70001, None), (1300, 513, 4200, None)])
+def test_large_two_valued_layers_edges(ops, I, O, F, stride):
+    test_two_valued_layers_edges(ops, I, O, F, stride)
+
+
 # probability mode, one launch per direction: one warp, ragged and whole warps, eight warps and several rounds, unaligned rows, the largest
 @pytest.mark.parametrize("I,O,F,stride", [(6, 1, 1, None), (9, 5, 3, 4), (33, 70, 128, None), (50, 31, 129, 131), (30, 40, 1025, None), (12, 8, 4096, 4099),
                                           (700, 512, 4096, None)])
