@@ -249,7 +249,7 @@ struct BitBwdArgs {
     float *hdy;                         // [O][64] sums of dy per pattern
     uint32_t *hist;                     // [O][64] pattern counts
     uint2 *mask;                        // [O] hard-tanh masks of the 64 patterns (batch norm only)
-    uint16_t *pat;                      // [O][ps] doubled patterns p | p << 6, bit 15: the mask passes
+    uint8_t *pat;                       // [O][ps] patterns, bit 7: the mask passes
     float *etab;                        // [6 O][64] look-up tables, see k_bit_backward_finalize
     float2 *ntab;                       // [O] gamma rstd, dvar bias / F
     const int *edge_end, *edge_count, *edges;      // consumers of every input row (8 node + input number)
@@ -311,25 +311,25 @@ constexpr int kPsWarps = 4;
 template <bool BN> struct PatternSlot { float s; uint32_t n; };      // n: count, bit 31: the pattern's mask bit
 template <> struct PatternSlot<false> { float s; };
 
-// Adds four frames (patterns one per byte, frames from `live` on do not count) to a lane's column; returns their doubled patterns with the
-// mask bits, which come with the slots.
+// Adds four frames (patterns one per byte, frames from `live` on do not count) to a lane's column; returns the patterns with their mask
+// bits, which come with the slots.
 template <bool BN>
-__device__ __forceinline__ uint2 pattern_columns_add(PatternSlot<BN> *mine, uint32_t p4, const float4 &g, int live)
+__device__ __forceinline__ uint32_t pattern_columns_add(PatternSlot<BN> *mine, uint32_t p4, const float4 &g, int live)
 {
     const float gv[4] = {g.x, g.y, g.z, g.w};
-    uint32_t q[2] = {__byte_perm(p4, 0u, 0x4140) * 65u, __byte_perm(p4, 0u, 0x4342) * 65u};
+    uint32_t q4 = p4;
 #pragma unroll
     for (int i = 0; i < 4; ++i) {
         PatternSlot<BN> *slot = mine + 32 * __byte_perm(p4, 0u, 0x4440 + i);
         PatternSlot<BN> v = *slot;
         v.s += gv[i];
         if constexpr (BN) {
-            q[i >> 1] |= i & 1 ? v.n & 0x80000000u : (v.n >> 16) & 0x8000u;
+            q4 |= (v.n >> (24 - 8 * i)) & (0x80u << (8 * i));
             v.n += i < live ? 1u : 0u;
         }
         *slot = v;
     }
-    return make_uint2(q[0], q[1]);
+    return q4;
 }
 
 // adds the 32 columns of every pattern: lane l returns patterns l and l + 32
@@ -372,7 +372,7 @@ k_pattern_sums(const BitBwdArgs a)
 #pragma unroll
     for (int j = 0; j < 6; ++j) rows[j] = a.x + (size_t)__ldg(a.idx + (size_t)node * 6 + j) * a.xs;
     const float *dyrow = a.dy + (size_t)node * a.fs;
-    uint16_t *prow = a.pat + (size_t)node * a.ps;
+    uint8_t *prow = a.pat + (size_t)node * a.ps;
     const int f_begin = tile * a.tile_frames, f_end = min(a.F, f_begin + a.tile_frames);
 
     int f = f_begin + 4 * lane;
@@ -396,7 +396,7 @@ k_pattern_sums(const BitBwdArgs a)
             if (k < steps) {
 #pragma unroll
                 for (int c = 0; c < NC; ++c)
-                    *reinterpret_cast<uint2 *>(prow + f + k * kStep + 128 * c) = pattern_columns_add<BN>(mine, pattern_bytes(b.w[c], lane), b.dy[c], 4);
+                    *reinterpret_cast<uint32_t *>(prow + f + k * kStep + 128 * c) = pattern_columns_add<BN>(mine, pattern_bytes(b.w[c], lane), b.dy[c], 4);
             }
         };
         Set s0, s1;
@@ -424,7 +424,7 @@ k_pattern_sums(const BitBwdArgs a)
             for (int j = 0; j < 6; ++j) w[j] = __ldg(rows[j] + (f >> 5));
             p4 = pattern_bytes(w, lane);
         }
-        *reinterpret_cast<uint2 *>(prow + f) = pattern_columns_add<BN>(mine, p4, load_frames(dyrow, f, a.F, a.vec), a.F - f);      // rows of pat are padded
+        *reinterpret_cast<uint32_t *>(prow + f) = pattern_columns_add<BN>(mine, p4, load_frames(dyrow, f, a.F, a.vec), a.F - f);      // rows of pat are padded
     }
     __syncwarp();
     float s[2];
@@ -488,10 +488,12 @@ __device__ __forceinline__ uint32_t prmt(uint32_t v)
 // dx_i(f) = sum over the consumers (node o, input j) of row i of g_o(f) D_j[p_o(f)], frames from F on 0.  A CTA is one row and NC
 // chunks of 128 frames; `split` warps share the consumers (rows with many of them, or few rows).  One warp per CTA otherwise, because
 // the number of consumers varies from row to row and a CTA of several rows waits for the longest.
-// The tables of a consumer live in registers, one entry per lane, and a look-up is a shuffle whose source lane is a field of the doubled
-// pattern: bits j+1 .. j+5 are the other five inputs, bit j+6 is input j.  With batch norm g is put together here, ten
-// instructions per consumer and 32 frames in all, which is what bounds the kernel; writing g out once and reading it back would
-// leave three, but costs 10 bytes per node-frame of HBM traffic.
+// The tables of a consumer live in registers, one entry per lane, and a look-up is a shuffle whose source lane is the pattern rotated by
+// j + 1 (the rotation serves the patterns of four frames at once): bits 0 .. 4 are the other five inputs, bit 5 is input j.  No single
+// resource is exhausted (8192 x 8192 nodes x 8192 frames under ncu: issue 69 %, L1 68 %, logic pipe 59 %, a third of the stalls on L2
+// loads, 27 warps per SM): two shuffles, 5 bytes and 16 instructions per consumer and frame.  With batch norm g is put together here;
+// writing g out once and reading it back would spare a shuffle and six instructions, but costs 10 bytes per node-frame of HBM traffic.
+// Several rows one after the other in a CTA keep more tiles in flight than L2 holds (8 rows: 509 -> 617 us for 16384 frames).
 template <bool BN, int NC, bool WHOLE>
 __device__ __forceinline__ void pattern_gather(const BitBwdArgs &a, int row, int part, int f0, int lane, float (&acc)[NC][4])
 {
@@ -507,32 +509,34 @@ __device__ __forceinline__ void pattern_gather(const BitBwdArgs &a, int row, int
         const float2 gs = BN ? __ldg(a.ntab + node) : make_float2(1.0f, 0.0f);
         const uint32_t minus_slope = __float_as_uint(-gs.y);
         const float *dyrow = a.dy + (size_t)node * a.fs;
-        const uint16_t *prow = a.pat + (size_t)node * a.ps;
+        const uint8_t *prow = a.pat + (size_t)node * a.ps;
+        const uint32_t low = ((1u << (5 - j)) - 1u) * 0x01010101u;        // bits that the rotation takes from the left of their byte
         float4 dyq[NC];
-        uint2 q2[NC];
+        uint32_t q4[NC];
 #pragma unroll
         for (int c = 0; c < NC; ++c) {
             const int f = f0 + 128 * c;
             if (WHOLE) {
                 dyq[c] = __ldg(reinterpret_cast<const float4 *>(dyrow + f));
-                q2[c] = __ldg(reinterpret_cast<const uint2 *>(prow + f));
+                q4[c] = __ldg(reinterpret_cast<const uint32_t *>(prow + f));
             } else {
                 dyq[c] = load_frames(dyrow, f, a.F, a.vec);
-                q2[c] = f < a.F ? __ldg(reinterpret_cast<const uint2 *>(prow + f)) : make_uint2(0u, 0u);
+                q4[c] = f < a.F ? __ldg(reinterpret_cast<const uint32_t *>(prow + f)) : 0u;
             }
         }
 #pragma unroll
         for (int c = 0; c < NC; ++c) {
             const float dyv[4] = {dyq[c].x, dyq[c].y, dyq[c].z, dyq[c].w};
+            const uint32_t rot = ((q4[c] >> (j + 1)) & low) | ((q4[c] << (5 - j)) & ~low);        // (bits 6 and 7 of the bytes: anything)
 #pragma unroll
             for (int i = 0; i < 4; ++i) {
-                const uint32_t q = i < 2 ? q2[c].x : q2[c].y;
-                const uint32_t r = q >> (j + 1 + 16 * (i & 1));
+                const uint32_t r = rot >> (8 * i);
                 const float d = __shfl_sync(kFull, D, r);
                 float g = dyv[i];
                 if (BN) {
-                    const float slope = __uint_as_float(((r << 26) & 0x80000000u) ^ minus_slope);      // +slope where input j is set
-                    const uint32_t pass = i & 1 ? prmt<0xbbbb>(q) : prmt<0x9999>(q);                   // bit 15 of the frame's half, replicated
+                    const float slope = __uint_as_float(((rot << (26 - 8 * i)) & 0x80000000u) ^ minus_slope);      // +slope where input j is set
+                    const uint32_t pass = i == 0 ? prmt<0x8888>(q4[c]) : i == 1 ? prmt<0x9999>(q4[c])               // bit 7 of the frame's byte, replicated
+                                        : i == 2 ? prmt<0xaaaa>(q4[c]) : prmt<0xbbbb>(q4[c]);
                     g = fmaf(__uint_as_float(__float_as_uint(g) & pass), gs.x, fmaf(slope, d, __shfl_sync(kFull, base, r)));
                 }
                 acc[c][i] = fmaf(g, d, acc[c][i]);
@@ -621,7 +625,7 @@ __device__ __forceinline__ void eval_pattern_pair(const float4 *tab2, int lane, 
 }
 
 // The look-up tables of a node's six edges, 64 floats each: D_j for the 32 values of the other five bits -- entry m belongs to the
-// patterns whose bits j+1 .. j+5 (mod 6) are m, a field of the doubled pattern p | p << 6 -- and, with batch norm, the part of
+// patterns whose bits j+1 .. j+5 (mod 6) are m, the low bits of the pattern rotated by j + 1 -- and, with batch norm, the part of
 // dmean + Y[p] dvar / F that does not depend on bit j (the rest is +-D_j times dvar bias / F).
 template <bool BN>
 __device__ __forceinline__ void store_edge_tables(float *etab, int lane, const float (&y)[2], const float (&d)[2][6], float dmean, float dvar_rF)
@@ -1319,9 +1323,9 @@ bool backward_setup(BitBwdArgs &a, const void *x, const float *dy, const int *id
 {
     const long long ps = ((long long)F + 127) / 128 * 128;
     const size_t tables = (size_t)O * (6 * 64 * sizeof(float) + sizeof(float2) + sizeof(uint2));
-    if ((size_t)O * (size_t)ps > ((size_t)1 << 32)) return false;        // 8 GiB of patterns at most
+    if ((size_t)O * (size_t)ps > ((size_t)1 << 32)) return false;        // 4 GiB of patterns at most
     Scratch s;
-    if (!carve(s, O, st, ((tables + 255) & ~(size_t)255) + (size_t)O * (size_t)ps * sizeof(uint16_t))) return false;
+    if (!carve(s, O, st, ((tables + 255) & ~(size_t)255) + (size_t)O * (size_t)ps)) return false;
     a = BitBwdArgs{};
     a.x = static_cast<const uint32_t *>(x); a.dy = dy; a.idx = idx;
     a.hist = s.hist;
@@ -1329,7 +1333,7 @@ bool backward_setup(BitBwdArgs &a, const void *x, const float *dy, const int *id
     a.etab = reinterpret_cast<float *>(s.pat);
     a.ntab = reinterpret_cast<float2 *>(a.etab + (size_t)O * 6 * 64);
     a.mask = reinterpret_cast<uint2 *>(a.ntab + O);
-    a.pat = reinterpret_cast<uint16_t *>(s.pat + ((tables + 255) & ~(size_t)255));
+    a.pat = s.pat + ((tables + 255) & ~(size_t)255);
     a.O = O; a.F = F; a.xs = xs; a.fs = fs; a.ps = ps;
     a.vec = (reinterpret_cast<uintptr_t>(dy) & 15) == 0 && fs % 4 == 0;
     return true;
@@ -1395,7 +1399,7 @@ int launch_pattern_sums(BitBwdArgs a, bool bn, cudaStream_t st)
     return launch_status();
 }
 
-// dx.  The tile is 512 frames (the tables of a consumer are loaded once per tile) unless the dy and pattern rows of such a tile, 6
+// dx.  The tile is 512 frames (the tables of a consumer are loaded once per tile) unless the dy and pattern rows of such a tile, 5
 // bytes per node and frame, exceed two thirds of L2, or the GPU would run short of warps.
 int launch_pattern_gather(BitBwdArgs a, bool bn, cudaStream_t st)
 {
@@ -1403,7 +1407,7 @@ int launch_pattern_gather(BitBwdArgs a, bool bn, cudaStream_t st)
     const DeviceInfo &di = device_info();
     const long long fan = (6LL * a.O + a.I - 1) / a.I;                                // consumers per row, on average
     int nc = 4;
-    while (nc > 1 && (6LL * a.O * 128 * nc > (long long)(di.l2_bytes / 3 * 2) || (long long)a.I * ((a.fs + 128 * nc - 1) / (128 * nc)) < 16LL * di.sm_count)) nc /= 2;
+    while (nc > 1 && (5LL * a.O * 128 * nc > (long long)(di.l2_bytes / 3 * 2) || (long long)a.I * ((a.fs + 128 * nc - 1) / (128 * nc)) < 16LL * di.sm_count)) nc /= 2;
     const long long blocks = (long long)a.I * ((a.fs + 128 * nc - 1) / (128 * nc));
     BB200_REQUIRE(blocks < (1LL << 31), BBCU_ERR_TOO_LARGE);
     a.split = 1;
