@@ -22,6 +22,7 @@
 #include "common.cuh"
 #include "async_copy.cuh"
 #include "bit_transpose.cuh"
+#include "grid_clear.cuh"
 #include "lut6_core.cuh"
 
 namespace bb200 {
@@ -993,7 +994,7 @@ k_small_binary_forward(const SmallBinArgs a)
 // Backward (BN: batch-normalised layer): the arithmetic of k_bit_backward_finalize and k_pattern_gather.
 template <bool XBIT, bool BN>
 __global__ void __launch_bounds__(kWarpsPerCta * 32)
-k_small_binary_backward(const SmallBinArgs a)
+k_small_binary_backward(const SmallBinArgs a, const GridClear clear)
 {
     grid_dependency();
     __shared__ float4 s_tab[16];
@@ -1033,6 +1034,7 @@ k_small_binary_backward(const SmallBinArgs a)
             store_edge_tables<false>(s_edge, lane, y, d, 0.0f, 0.0f);
         }
     }
+    grid_clear_slices(clear);
     __syncthreads();
     const float *dyrow = a.dy + (size_t)node * a.fs;
     const int step = 4 * (int)blockDim.x;
@@ -1075,6 +1077,7 @@ k_small_binary_backward(const SmallBinArgs a)
         float *dst = a.dW + (size_t)node * 64 + 2 * lane;
         dst[0] += gw.x;
         dst[1] += gw.y;
+        if (lane == 0) grid_clear_wait(clear);
     }
     __syncthreads();
     float D[6], base[6];
@@ -1455,10 +1458,12 @@ int bit_backward_by_table(bool bn, bool x_is_fp32, const void *x, const float *d
         a.x = x; a.dy = dy; a.dx = dx; a.idx = idx; a.W = W; a.dW = dW; a.mean_in = mean; a.rstd_in = rstd; a.dmean = dmean_out; a.dvar = dvar_out;
         a.gamma = gamma; a.beta = beta; a.bias = bias; a.F = F; a.lut_binarize = lut_binarize; a.xs = xs; a.fs = fs;
         a.vec = ((reinterpret_cast<uintptr_t>(dy) | reinterpret_cast<uintptr_t>(dx) | (x_is_fp32 ? reinterpret_cast<uintptr_t>(x) : 0)) & 15) == 0 && fs % 4 == 0;
-        BB200_CUDA(cudaMemsetAsync(dx, 0, sizeof(float) * (size_t)I * (size_t)fs, st));
+        GridClear clear;
+        const int rcc = grid_clear_setup(clear, dx, (size_t)I * (size_t)fs, st);
+        if (rcc) return rcc;
         auto kern = x_is_fp32 ? (bn ? k_small_binary_backward<false, true> : k_small_binary_backward<false, false>)
                               : (bn ? k_small_binary_backward<true, true> : k_small_binary_backward<true, false>);
-        launch(kern, O, small_threads(F), 0, st, a);
+        launch(kern, O, small_threads(F), 0, st, a, clear);
         return launch_status();
     }
     BitBwdArgs a;

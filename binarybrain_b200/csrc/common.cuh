@@ -33,8 +33,12 @@ const DeviceInfo &device_info();
 // kScratchSlots independent blocks, for callers whose scratch is alive at the same time (slot 0: batch-norm
 // sums, slot 1: per-node coefficient / pattern tables of the LUT operators, slot 2: the piece table of the bit Im2Col,
 // slot 3: fp32 rows packed to bits).
-constexpr int kScratchSlots = 4;
+constexpr int kScratchSlots = 5;
 void *stream_scratch(cudaStream_t stream, size_t bytes, int slot = 0);
+
+// 64 counters of the stream (slot 4), zeroed when they are made; a kernel that uses them leaves them zero.  nullptr when they cannot be had,
+// and for the per-thread default stream, whose one handle stands for a stream of every thread.
+unsigned *stream_counters(cudaStream_t stream);
 
 // Pass 1 of the DifferentiableLut6 training forward (raw LUT values into y, fp64 sums per node); with may_allocate = false
 // it takes nothing from the heap or the stream scratch.

@@ -12,6 +12,7 @@
 #include "common.cuh"
 #include "async_copy.cuh"
 #include "lut6_core.cuh"
+#include "grid_clear.cuh"
 
 namespace bb200 {
 
@@ -133,7 +134,7 @@ k_lut6_small_forward(const SmallLayerArgs a)
 // dx must be zero on entry; dW is accumulated into.
 template <bool BN>
 __global__ void __launch_bounds__(kWarpsPerCta * 32, 1)
-k_lut6_small_backward(const SmallLayerArgs a)
+k_lut6_small_backward(const SmallLayerArgs a, const GridClear clear)
 {
     grid_dependency();
     __shared__ float4 s_tab[16];
@@ -159,6 +160,7 @@ k_lut6_small_backward(const SmallLayerArgs a)
     };
     fetch(f);
     if (warp == 0) stage_table_halves(s_tab, a.W, node, lane, a.lut_binarize);
+    grid_clear_slices(clear);
     float mean = 0.0f, rstd = 0.0f, dmean = 0.0f, dvar = 0.0f;
     const float rF = 1.0f / (float)a.F;
     if (BN) { mean = a.mean_in[node]; rstd = a.rstd_in[node]; }
@@ -195,11 +197,16 @@ k_lut6_small_backward(const SmallLayerArgs a)
             a.dmean[node] = dm;
             s_stat[0] = dm;
             s_stat[1] = dv;
+            grid_clear_wait(clear);
         }
         __syncthreads();
         dmean = s_stat[0];
         dvar = s_stat[1];
         if (a.F > step) fetch(f);                                                              // more than one round: start over
+    }
+    if (!BN) {
+        if (threadIdx.x == 0) grid_clear_wait(clear);
+        __syncthreads();
     }
     size_t out[6];
 #pragma unroll
@@ -281,9 +288,11 @@ int small_forward(int mode, const SmallLayerArgs &a, int O, cudaStream_t st)
 
 int small_backward(bool bn, const SmallLayerArgs &a, int I, int O, cudaStream_t st)
 {
-    BB200_CUDA(cudaMemsetAsync(a.dx, 0, sizeof(float) * (size_t)I * (size_t)a.fs, st));
-    if (bn) launch(k_lut6_small_backward<true>, O, threads_for(a.F), 0, st, a);
-    else    launch(k_lut6_small_backward<false>, O, threads_for(a.F), 0, st, a);
+    GridClear clear;
+    const int rc = grid_clear_setup(clear, a.dx, (size_t)I * (size_t)a.fs, st);
+    if (rc) return rc;
+    if (bn) launch(k_lut6_small_backward<true>, O, threads_for(a.F), 0, st, a, clear);
+    else    launch(k_lut6_small_backward<false>, O, threads_for(a.F), 0, st, a, clear);
     return launch_status();
 }
 

@@ -130,6 +130,8 @@ int *fault_word()
     return it->second;
 }
 
+constexpr int kCounterSlot = 4;
+
 void *stream_scratch(cudaStream_t stream, size_t bytes, int slot)
 {
     if (slot < 0 || slot >= kScratchSlots) return nullptr;
@@ -146,6 +148,11 @@ void *stream_scratch(cudaStream_t stream, size_t bytes, int slot)
     // the heap only after the stream has drained)
     void *fresh = bbcu_LocalHeap_Malloc(bytes);
     if (!fresh) return nullptr;
+    if (slot == kCounterSlot && cudaMemsetAsync(fresh, 0, bytes, stream) != cudaSuccess) {
+        cudaGetLastError();
+        bbcu_LocalHeap_Free(fresh);
+        return nullptr;
+    }
     void *old = nullptr;
     {
         std::lock_guard<std::mutex> g(p.mu);
@@ -158,6 +165,11 @@ void *stream_scratch(cudaStream_t stream, size_t bytes, int slot)
         bbcu_LocalHeap_Free(old);
     }
     return fresh;
+}
+
+unsigned *stream_counters(cudaStream_t stream)
+{
+    return stream == cudaStreamPerThread ? nullptr : static_cast<unsigned *>(stream_scratch(stream, 256, kCounterSlot));
 }
 
 }   // namespace bb200
