@@ -506,11 +506,7 @@ extern "C" int bbcu_bit_BinaryLut6_Forward(const int *x, int *y, const int *idx,
     // 128-bit path: rows start 16-byte aligned and whole uint4 groups fit inside the row stride
     const bool vec = (frame_stride % 4 == 0) && ((reinterpret_cast<uintptr_t>(x) & 15) == 0) && ((reinterpret_cast<uintptr_t>(y) & 15) == 0);
     if (vec) a.nwords = (a.nwords + 3) & ~3;
-    // word tile: frame_tile() counts in frames; a word is 32 of them
-    const int tf = frame_tile(2LL * node_size, 1, a.groups, a.nwords * 32, 1024 * 32);
-    a.Tw = ((tf / 32 + 127) / 128) * 128;
-    const long long blocks = (long long)((a.nwords + a.Tw - 1) / a.Tw) * a.groups;
-    BB200_REQUIRE(blocks < (1LL << 31), BBCU_ERR_TOO_LARGE);
+    a.Tw = 0;
     if (vec) {
         // persistent pipeline: two CTAs per SM, each walking (tile, node group) items
         const bool attr_ok = allow_big_smem(k_binary_lut6_pipe, kPipeSmem);
@@ -524,6 +520,11 @@ extern "C" int bbcu_bit_BinaryLut6_Forward(const int *x, int *y, const int *idx,
             return launch_status();
         }
     }
+    // word tile: frame_tile() counts in frames; a word is 32 of them
+    const int tf = frame_tile(2LL * node_size, 1, a.groups, a.nwords * 32, 1024 * 32);
+    a.Tw = ((tf / 32 + 127) / 128) * 128;
+    const long long blocks = (long long)((a.nwords + a.Tw - 1) / a.Tw) * a.groups;
+    BB200_REQUIRE(blocks < (1LL << 31), BBCU_ERR_TOO_LARGE);
     // aligned rows without the shared-memory opt-in (or without a fault word): the non-pipelined 128-bit kernel; otherwise word loads
     if (vec) launch(k_binary_lut6_2pipe, (unsigned)blocks, kBlWarps * 32, 0, as_stream(stream), a);
     else     launch(k_binary_lut6, (unsigned)blocks, kBlWarps * 32, 0, as_stream(stream), a);

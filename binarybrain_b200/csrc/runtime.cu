@@ -104,9 +104,13 @@ int frame_tile(long long rows_touched, int bits_per_row_frame, int node_groups, 
     t = (t / kFramesPerIterHost) * kFramesPerIterHost;
     if (t < kFramesPerIterHost) t = kFramesPerIterHost;
     if (t > max_tile) t = max_tile;
-    // keep at least ~4 CTAs per SM in flight while the tile is still wider than one iteration
-    const long long want_ctas = 4LL * di.sm_count;
-    while (t > kFramesPerIterHost && (long long)node_groups * ((frame_size + t - 1) / t) < want_ctas) t -= kFramesPerIterHost;
+    // keep at least ~4 CTAs per SM in flight while the tile is still wider than one iteration: the widest tile with at least `tiles` of them
+    const long long tiles = (4LL * di.sm_count + node_groups - 1) / (node_groups > 0 ? node_groups : 1);
+    if (tiles > 1) {
+        long long widest = (frame_size - 1LL) / (tiles - 1) / kFramesPerIterHost * kFramesPerIterHost;
+        if (widest < kFramesPerIterHost) widest = kFramesPerIterHost;
+        if (t > widest) t = widest;
+    }
     return (int)t;
 }
 
