@@ -317,6 +317,43 @@ k_binary_lut6_pipe(const BlArgs a, int n_tiles, int *fault)
 }
 
 // ---------------------------------------------------------------------------------------------
+// One word of one node per thread: the smallest calls, where the pipeline's set-up and its eight words a lane are most of the time.
+// Bound by latency: wiring, then the six words, then the tree with the table's bits spread to masks on the way (about 200 operations).
+// ---------------------------------------------------------------------------------------------
+template <int L, int K>
+struct WordTree {
+    static __device__ __forceinline__ uint32_t eval(uint32_t t0, uint32_t t1, const uint32_t (&x)[6])
+    {
+        const uint32_t lo = WordTree<L - 1, 2 * K>::eval(t0, t1, x), hi = WordTree<L - 1, 2 * K + 1>::eval(t0, t1, x);
+        return (lo & ~x[L - 1]) | (hi & x[L - 1]);
+    }
+};
+
+template <int K>
+struct WordTree<0, K> {              // table bit K in all 32 positions
+    static __device__ __forceinline__ uint32_t eval(uint32_t t0, uint32_t t1, const uint32_t (&)[6])
+    {
+        return (uint32_t)((int)((K < 32 ? t0 : t1) << (31 - (K & 31))) >> 31);
+    }
+};
+
+constexpr int kWordThreads = 128;
+
+__global__ void __launch_bounds__(kWordThreads)
+k_binary_lut6_words(const BlArgs a)
+{
+    grid_dependency();
+    const unsigned t = blockIdx.x * kWordThreads + threadIdx.x, words = (unsigned)a.nwords;
+    const unsigned node = t / words, w = t - node * words;
+    if (node >= (unsigned)a.O) return;
+    const uint32_t t0 = (uint32_t)__ldg(a.table + 2 * (size_t)node), t1 = (uint32_t)__ldg(a.table + 2 * (size_t)node + 1);
+    uint32_t x[6];
+#pragma unroll
+    for (int j = 0; j < 6; ++j) x[j] = __ldg(a.x + (size_t)__ldg(a.idx + (size_t)node * 6 + j) * a.stride + w);
+    a.y[(size_t)node * a.stride + w] = WordTree<6, 0>::eval(t0, t1, x);
+}
+
+// ---------------------------------------------------------------------------------------------
 // Truth-table-immediate variant (aligned rows).
 // lop3.b32 evaluates ANY three-input boolean function in one instruction, the function being an 8-bit immediate.  Byte b of a
 // node's 64-bit table is exactly the function of (x0, x1, x2) that applies where x3 + 2 x4 + 4 x5 = b, so a word costs eight lop3
@@ -507,6 +544,13 @@ extern "C" int bbcu_bit_BinaryLut6_Forward(const int *x, int *y, const int *idx,
     const bool vec = (frame_stride % 4 == 0) && ((reinterpret_cast<uintptr_t>(x) & 15) == 0) && ((reinterpret_cast<uintptr_t>(y) & 15) == 0);
     if (vec) a.nwords = (a.nwords + 3) & ~3;
     a.Tw = 0;
+    // Up to half a wave of threads with a word each (1024 nodes x 200 frames 3.4 -> 2.0 us, 4096 x 1024 7.0 -> 3.0, 1024 x 4096 3.4 -> 2.9; at
+    // 512 x 10000, a little above, both take 3.5).
+    const long long node_words = (long long)node_size * a.nwords;
+    if (node_words <= 1024LL * device_info().sm_count) {
+        launch(k_binary_lut6_words, (unsigned)((node_words + kWordThreads - 1) / kWordThreads), kWordThreads, 0, as_stream(stream), a);
+        return launch_status();
+    }
     if (vec) {
         // persistent pipeline: two CTAs per SM, each walking (tile, node group) items
         const bool attr_ok = allow_big_smem(k_binary_lut6_pipe, kPipeSmem);

@@ -38,6 +38,23 @@ def test_modulation_edges(ops, nodes, frames, mod, depth, points):
     assert np.abs(host_fp32(dx, frames * mod) - port.binary_to_real_backward(dy, rows, mod)).max() <= 1e-7
 
 
+# a word per thread and, above 1024 x 148 words, the pipeline: one word, no whole quad of words, unaligned rows, nodes that fill no CTA
+@pytest.mark.parametrize("n_in,n_out,frames,stride", [(6, 1, 1, 1), (9, 7, 129, 5), (300, 420, 200, 8), (64, 4736, 1024, 32), (64, 4737, 1024, 32), (50, 37, 131073, 4100),
+                                                      (50, 37, 131073, 4099)])
+def test_binary_lut6_words_and_pipeline(ops, n_in, n_out, frames, stride):
+    import torch
+    from gpu_util import dev, wiring
+    rng = np.random.default_rng(n_out)
+    words = (frames + 31) // 32
+    x = rng.integers(-2**31, 2**31, (n_in, stride), dtype=np.int64).astype(np.int32)
+    idx, table = wiring(rng, n_in, n_out), rng.integers(-2**31, 2**31, (n_out, 2), dtype=np.int64).astype(np.int32)
+    y = ops.binary_lut6_forward(dev(x), dev(idx), dev(table), frames, y=torch.zeros((n_out, stride), dtype=torch.int32, device="cuda"))
+    want = port.binary_lut6_forward(x.view(np.uint32), idx, table, frames)
+    live = np.full(words, 0xffffffff, np.uint32)
+    live[-1] >>= words * 32 - frames
+    assert ((y.cpu().numpy().view(np.uint32)[:, :words] ^ want[:, :words]) & live == 0).all()
+
+
 # one chunk, a first and a last chunk only, full-width chunks with a one-word remainder
 @pytest.mark.parametrize("n_in,n_out,words,spare", [(9, 7, 1, 0), (700, 400, 130, 30), (4096, 64, 257, 31), (1024, 1100, 1793, 5)])
 def test_binary_lut6_host_chunks(ops, n_in, n_out, words, spare):
