@@ -544,10 +544,12 @@ extern "C" int bbcu_bit_BinaryLut6_Forward(const int *x, int *y, const int *idx,
     const bool vec = (frame_stride % 4 == 0) && ((reinterpret_cast<uintptr_t>(x) & 15) == 0) && ((reinterpret_cast<uintptr_t>(y) & 15) == 0);
     if (vec) a.nwords = (a.nwords + 3) & ~3;
     a.Tw = 0;
-    // Up to half a wave of threads with a word each (1024 nodes x 200 frames 3.4 -> 2.0 us, 4096 x 1024 7.0 -> 3.0, 1024 x 4096 3.4 -> 2.9; at
-    // 512 x 10000, a little above, both take 3.5).
-    const long long node_words = (long long)node_size * a.nwords;
-    if (node_words <= 1024LL * device_info().sm_count) {
+    // A word per thread while that is at most a quarter of what the pipeline's rounds of warps could take in 256-word tiles: a round costs
+    // the same whether its tiles are full or not (1024 nodes x 200 frames 3.4 -> 2.0 us, 1024 x 4096 3.4 -> 2.9, 4096 x 2048 7.0 -> 4.4,
+    // 10000 x 2048 13.2 -> 8.5; at 512 x 10000 both take 3.5, and 384 x 65536 is 10.1 against 6.0).
+    const long long node_words = (long long)node_size * a.nwords, warps = (long long)kPipeCtas * kBlWarps * device_info().sm_count;
+    const long long rounds = ((long long)node_size * ((a.nwords + kPipeWords - 1) / kPipeWords) + warps - 1) / warps;
+    if (node_words <= 1024LL * device_info().sm_count * rounds && node_words < (1LL << 31) - kWordThreads) {
         launch(k_binary_lut6_words, (unsigned)((node_words + kWordThreads - 1) / kWordThreads), kWordThreads, 0, as_stream(stream), a);
         return launch_status();
     }

@@ -38,8 +38,8 @@ def test_modulation_edges(ops, nodes, frames, mod, depth, points):
     assert np.abs(host_fp32(dx, frames * mod) - port.binary_to_real_backward(dy, rows, mod)).max() <= 1e-7
 
 
-# a word per thread and, above 1024 x 148 words, the pipeline: one word, no whole quad of words, unaligned rows, nodes that fill no CTA
-@pytest.mark.parametrize("n_in,n_out,frames,stride", [(6, 1, 1, 1), (9, 7, 129, 5), (300, 420, 200, 8), (64, 4736, 1024, 32), (64, 4737, 1024, 32), (50, 37, 131073, 4100),
+# a word per thread and, above 1024 x 148 words a round of 256-word tiles, the pipeline: one word, no whole quad of words, unaligned rows, nodes that fill no CTA
+@pytest.mark.parametrize("n_in,n_out,frames,stride", [(6, 1, 1, 1), (9, 7, 129, 5), (300, 420, 200, 8), (64, 4736, 1024, 32), (64, 4737, 1024, 32), (64, 600, 8100, 256), (50, 37, 131073, 4100),
                                                       (50, 37, 131073, 4099)])
 def test_binary_lut6_words_and_pipeline(ops, n_in, n_out, frames, stride):
     import torch
