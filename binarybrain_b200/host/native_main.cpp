@@ -61,7 +61,16 @@ template <class T> bool parse(PyObject *o, T &v)
     if constexpr (std::is_pointer_v<T>) {
         if (o == Py_None) { v = nullptr; return true; }
         if (THPVariable_Check(o)) {
-            v = reinterpret_cast<T>(const_cast<void *>(static_cast<const void *>(THPVariable_Unpack(o).const_data_ptr())));
+            // an operator that may write through the pointer needs the tensor's own memory: mutable_data_ptr() gives a lazily cloned
+            // tensor its copy, where const_data_ptr() would have the operator write into the tensor it was cloned from
+            const at::Tensor &t = THPVariable_Unpack(o);
+            try {
+                if constexpr (std::is_const_v<std::remove_pointer_t<T>>) v = static_cast<T>(t.const_data_ptr());
+                else v = static_cast<T>(t.mutable_data_ptr());
+            } catch (const std::exception &e) {
+                PyErr_SetString(PyExc_RuntimeError, e.what());
+                return false;
+            }
             return true;
         }
         v = reinterpret_cast<T>(PyLong_AsVoidPtr(o));
