@@ -37,7 +37,8 @@ constexpr int kScratchSlots = 5;
 void *stream_scratch(cudaStream_t stream, size_t bytes, int slot = 0);
 
 // 64 counters of the stream (slot 4), zeroed when they are made; a kernel that uses them leaves them zero.  nullptr when they cannot be had,
-// and for the per-thread default stream, whose one handle stands for a stream of every thread.
+// for the per-thread default stream, whose one handle stands for a stream of every thread, and for a stream that is being captured: the
+// graph may be launched on any stream, beside kernels of this one, and the zeroing would only be a node of the graph.
 unsigned *stream_counters(cudaStream_t stream);
 
 // Pass 1 of the DifferentiableLut6 training forward (raw LUT values into y, fp64 sums per node); with may_allocate = false

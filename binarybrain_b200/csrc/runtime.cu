@@ -173,7 +173,11 @@ void *stream_scratch(cudaStream_t stream, size_t bytes, int slot)
 
 unsigned *stream_counters(cudaStream_t stream)
 {
-    return stream == cudaStreamPerThread ? nullptr : static_cast<unsigned *>(stream_scratch(stream, 256, kCounterSlot));
+    if (stream == cudaStreamPerThread) return nullptr;
+    cudaStreamCaptureStatus capture = cudaStreamCaptureStatusNone;
+    if (cudaStreamIsCapturing(stream, &capture) != cudaSuccess) { cudaGetLastError(); return nullptr; }
+    if (capture != cudaStreamCaptureStatusNone) return nullptr;
+    return static_cast<unsigned *>(stream_scratch(stream, 256, kCounterSlot));
 }
 
 }   // namespace bb200
