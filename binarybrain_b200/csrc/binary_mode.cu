@@ -884,8 +884,8 @@ k_counts_to_sums(const float *__restrict__ Y, const uint32_t *__restrict__ hist,
 // Where a layer has up to a million or two node-frames, the kernels above take a few microseconds each and the launches between them take as
 // long again.  Here one CTA is one node with all of its frames (1 to 8 warps): tables, counts, statistics and output without
 // leaving the SM.  The rows are read twice (the second time from L1 or L2), counts and sums go through shared-memory atomics, and the
-// backward scatters dx with reductions in L2 (36 clocks per SM, warp and 32 frames; dx must be zero on entry) -- which is why larger layers
-// do not come here: see small_layer().
+// backward scatters dx, which it clears first (grid_clear.cuh), with reductions in L2 (36 clocks per SM, warp and 32 frames) -- which is
+// why larger layers do not come here: see small_layer().
 
 struct SmallBinArgs {
     const void *x;                      // fp32 rows, or bit rows
@@ -1096,7 +1096,8 @@ k_small_binary_backward(const SmallBinArgs a, const GridClear clear)
         float *dst = a.dW + (size_t)node * 64 + 2 * lane;
         dst[0] += gw.x;
         dst[1] += gw.y;
-        if (lane == 0) grid_clear_wait(clear);
+        __syncwarp();
+        if (lane == 0) grid_clear_wait(clear, a.dW + (size_t)node * 64, s_edge, 6 * 64);
     }
     __syncthreads();
     float D[6], base[6];

@@ -3,8 +3,9 @@
 //
 // The buffer is cut into slices of kClearSlice floats.  Every CTA, when it starts, claims slices until none is left, so that a slice is
 // always in the hands of a CTA that runs, whichever CTAs the GPU has room for; before its first addition a CTA waits until all slices are
-// cleared.  That wait therefore ends without any CTA that has not started; it is bounded all the same.  The last CTA to pass it resets the
-// counters for the next kernel of the stream, which touches them after its grid_dependency() only.
+// cleared.  That wait therefore ends without any CTA that has not started; it is bounded all the same, and a CTA whose wait has run out
+// records the fault and makes its gradients NaN.  The last CTA to pass the wait resets the counters for the next kernel of the stream, which
+// touches them after its grid_dependency() only.
 #pragma once
 
 #include "common.cuh"
@@ -60,19 +61,25 @@ __device__ __forceinline__ void grid_clear_slices(const GridClear &c)
     }
 }
 
-// One thread of the CTA, once; a barrier of the CTA has to follow before the first addition.
-__device__ __forceinline__ void grid_clear_wait(const GridClear &c)
+// One thread of the CTA, once; a barrier of the CTA has to follow before the first addition.  Where the buffer is not cleared after a second or
+// so, what follows is no gradient: the 64 table gradients of the CTA's node and the `n` floats of `factors`, shared memory that every addition
+// to the buffer is multiplied by, become NaN.  (Leaving the kernel instead cost the ordinary call 1 us: the branch, and loads held back by it.)
+__device__ __forceinline__ void grid_clear_wait(const GridClear &c, float *dW_row, float *factors, int n)
 {
     if (c.dst == nullptr) return;
     const unsigned slices = (unsigned)((c.floats + kClearSlice - 1) / kClearSlice);
     unsigned done = 0;
     int tries = 0;
-    for (; tries < (1 << 22); ++tries) {                      // (a second or more)
+    for (; tries < (1 << 20); ++tries) {
         asm volatile("ld.acquire.gpu.global.u32 %0, [%1];" : "=r"(done) : "l"(c.counters + 1) : "memory");
         if (done >= slices) break;
         __nanosleep(64);
     }
-    if (done < slices) atomicCAS(c.fault, 0, kFaultBarrierTimeout);
+    if (done < slices) {
+        atomicCAS(c.fault, 0, kFaultBarrierTimeout);
+        for (int i = 0; i < 64; ++i) dW_row[i] = __int_as_float(0x7fffffff);
+        for (int i = 0; i < n; ++i) factors[i] = __int_as_float(0x7fffffff);
+    }
     __threadfence();
     if (atomicAdd(c.counters + 2, 1u) == gridDim.x - 1) {     // nobody looks at the counters any more
         c.counters[0] = 0u;

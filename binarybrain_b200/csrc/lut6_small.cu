@@ -131,7 +131,7 @@ k_lut6_small_forward(const SmallLayerArgs a)
     }
 }
 
-// dx must be zero on entry; dW is accumulated into.
+// dx is cleared on the way (`clear`), or by the launcher; dW is accumulated into.
 template <bool BN>
 __global__ void __launch_bounds__(kWarpsPerCta * 32, 1)
 k_lut6_small_backward(const SmallLayerArgs a, const GridClear clear)
@@ -197,7 +197,7 @@ k_lut6_small_backward(const SmallLayerArgs a, const GridClear clear)
             a.dmean[node] = dm;
             s_stat[0] = dm;
             s_stat[1] = dv;
-            grid_clear_wait(clear);
+            grid_clear_wait(clear, a.dW + (size_t)node * 64, &s_tab[0].x, 64);
         }
         __syncthreads();
         dmean = s_stat[0];
@@ -205,7 +205,7 @@ k_lut6_small_backward(const SmallLayerArgs a, const GridClear clear)
         if (a.F > step) fetch(f);                                                              // more than one round: start over
     }
     if (!BN) {
-        if (threadIdx.x == 0) grid_clear_wait(clear);
+        if (threadIdx.x == 0) grid_clear_wait(clear, a.dW + (size_t)node * 64, &s_tab[0].x, 64);
         __syncthreads();
     }
     size_t out[6];

@@ -89,3 +89,31 @@ def test_first_call_of_a_stream_is_captured(binary):
             eager.backward()
     torch.cuda.synchronize()
     assert eager.correct() and captured.correct()
+
+
+@pytest.mark.parametrize("binary", [False, True])
+def test_a_wait_that_runs_out_shows_in_the_gradients(binary):
+    """The stream's counters say that every slice has been taken by somebody, and none is ever reported cleared: each block gives up after its
+    bounded wait, and the fault word and all that it adds to say so.  The next call is as if nothing had been."""
+    import torch
+    from binarybrain_b200 import abi
+    layer, stream = Layer(5, binary), torch.cuda.Stream()
+    assert abi.lib().bbcu_b200_device_fault() == 0
+    counters = heap_block_of(0.0)
+    with torch.cuda.stream(stream):
+        layer.poison()
+        layer.backward()                                                  # makes the stream's counters, of that block
+    torch.cuda.synchronize()
+    assert layer.correct()
+    with torch.cuda.stream(stream):
+        layer.poison()
+        abi.call("bbcu_fp32_Vector_set", counters, 1.0, 1, stream.cuda_stream)      # (slices claimed: the bits of 1.0f)
+        layer.backward()
+    torch.cuda.synchronize()
+    assert abi.lib().bbcu_b200_device_fault() == 1
+    assert torch.isnan(layer.dW).all() and torch.isnan(layer.dx[layer.idx.unique().long(), :F]).all()
+    with torch.cuda.stream(stream):
+        layer.poison()
+        layer.backward()
+    torch.cuda.synchronize()
+    assert layer.correct() and abi.lib().bbcu_b200_device_fault() == 0
