@@ -984,7 +984,7 @@ class OptimizerAdam
     std::vector<std::shared_ptr<Tensor>> m_params, m_grads, m_m, m_v;
     Tensor_<std::int32_t> m_sizes;
     Tensor_<std::int64_t> m_tables;             // addresses of the parameters, gradients and both moments, one row each
-    std::vector<std::int64_t> m_addresses;      // what m_tables holds
+    std::vector<std::int64_t> m_uploaded;       // what m_tables and m_sizes hold
     float m_lr, m_beta1, m_beta2, m_b1, m_b2;
 
 public:
@@ -1017,21 +1017,21 @@ private:
     void Apply(bool clear_grads)
     {
         if (m_params.empty()) return;
-        // the tables go up when they are new or an address has changed (a tensor was resized), not on every step
+        // the tables go up when they are new or a tensor was resized (which need not change its address), not on every step
         const std::size_t n = m_params.size();
-        std::vector<std::int64_t> now(4 * n);
+        std::vector<std::int64_t> now(5 * n);
         for (std::size_t i = 0; i < n; ++i) {
             now[i] = (std::int64_t)m_params[i]->Dev();    now[n + i] = (std::int64_t)m_grads[i]->Dev();
             now[2 * n + i] = (std::int64_t)m_m[i]->Dev(); now[3 * n + i] = (std::int64_t)m_v[i]->Dev();
+            now[4 * n + i] = (std::int64_t)m_params[i]->GetSize();
+            BB_ASSERT(m_grads[i]->GetSize() >= m_params[i]->GetSize() && m_m[i]->GetSize() >= m_params[i]->GetSize());
         }
-        if (now != m_addresses) {
-            std::vector<std::int32_t> sizes(n);
-            for (std::size_t i = 0; i < n; ++i) sizes[i] = (std::int32_t)m_params[i]->GetSize();
+        if (now != m_uploaded) {
             m_sizes.Resize((index_t)n);
-            m_sizes.FromVector(sizes);
+            m_sizes.FromVector(std::vector<std::int32_t>(now.begin() + 4 * n, now.end()));
             m_tables.Resize((index_t)(4 * n));
-            m_tables.FromVector(now);
-            m_addresses = now;
+            m_tables.FromVector(std::vector<std::int64_t>(now.begin(), now.begin() + 4 * n));
+            m_uploaded = now;
         }
         auto table = [&](std::size_t k) { return (float *const *)(m_tables.DevConst() + k * n); };
         const float lr_t = m_lr * std::sqrt(1.0f - m_b2) / (1.0f - m_b1);

@@ -34,3 +34,16 @@ def test_host_example_runs(tmp_path):
     out = _build(tmp_path)
     r = subprocess.run([str(out)], capture_output=True, text=True, timeout=300)
     assert r.returncode == 0, (r.stdout + r.stderr)[-2000:]
+
+
+def test_adam_follows_a_parameter_that_is_resized_in_place(tmp_path):
+    cxx = shutil.which("g++")
+    if cxx is None:
+        pytest.skip("no g++")
+    out = tmp_path / "adam_resized_parameter"
+    r = subprocess.run([cxx, "-std=c++17", "-O1", os.path.join(ROOT, "tests", "adam_resized_parameter.cpp"), "-o", str(out),
+                        "-I" + os.path.join(ROOT, "binarybrain_b200", "host"), "-I" + os.path.join(ROOT, "include"),
+                        "-I" + os.path.join(os.environ.get("CUDA_HOME", "/usr/local/cuda"), "include")], capture_output=True, text=True, timeout=600)
+    assert r.returncode == 0, r.stderr[-3000:]
+    r = subprocess.run([str(out)], capture_output=True, text=True, timeout=60)
+    assert r.returncode == 0 and r.stdout == "ok\n", (r.stdout + r.stderr)[-2000:]
