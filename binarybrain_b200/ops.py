@@ -100,10 +100,11 @@ def stochastic_lut6_backward(x, dy, idx, W, dW, n_in, frames, dx=None, binary=Fa
 
 # ------------------------------------------------------------------------------------------ DifferentiableLut6
 def differentiable_lut6_forward_training(x, idx, W, running_mean, running_var, frames, y=None, gamma=0.3, beta=0.5, momentum=0.9,
-                                         bias=BIAS, lut_binarize=False, binary=True):
-    """Returns (y, mean, rstd); running_mean / running_var are updated in place.  Bit x gives bit y."""
+                                         bias=BIAS, lut_binarize=False, binary=True, mean=None, rstd=None):
+    """Returns (y, mean, rstd), in `mean` and `rstd` where they are given; running_mean / running_var are updated in place.  Bit x gives bit y."""
     O = idx.shape[0]
-    mean, rstd = _n.vector_f32(x, O), _n.vector_f32(x, O)
+    mean = _n.vector_f32(x, O) if mean is None else mean
+    rstd = _n.vector_f32(x, O) if rstd is None else rstd
     if x.dtype == torch.float32:
         if y is None:
             y = _n.empty_f32(x, O, x.shape[1])

@@ -161,3 +161,25 @@ def test_unsharded_layer_on_one_rank_enters_no_collective(tmp_path):
     p = port.dl6_forward_train(x, idx, W, np.zeros(O), np.ones(O), binary=0)
     r = np.load(out.format(0))
     assert np.abs(r["y"] - p["y"]).max() <= 1e-4 * max(1.0, 0.3 * float(p["rstd"].max()))
+
+
+def test_small_layers_statistics_stay_in_the_same_tensors():
+    """A layer whose step is not split hands its own mean and rstd to the unsplit operator, so that what a caller holds of them does not go stale."""
+    from binarybrain_b200.dist import ShardedDifferentiableLut6
+
+    class UnsplitOps(HostOps):
+        SMALL_FRAMES = SMALL_NODE_FRAMES = 1 << 20
+
+        def differentiable_lut6_forward_training(self, x, idx, W, running_mean, running_var, frames, mean=None, rstd=None, y=None, **kw):
+            mean = torch.empty(idx.shape[0]) if mean is None else mean
+            rstd = torch.empty(idx.shape[0]) if rstd is None else rstd
+            mean.fill_(float(x.mean()))
+            rstd.fill_(1.0)
+            return torch.zeros(idx.shape[0], x.shape[1]), mean, rstd
+
+    I, O, F, idx, W, x, dy = _case()
+    layer = ShardedDifferentiableLut6(torch.from_numpy(idx), torch.from_numpy(W), I, ops=UnsplitOps(), binary=False, sharded=False)
+    mean, rstd = layer.mean, layer.rstd
+    for scale in (1.0, 0.5):
+        layer.forward(torch.from_numpy(x) * scale, F, F)
+        assert layer.mean is mean and layer.rstd is rstd and torch.allclose(mean, torch.tensor(float((torch.from_numpy(x) * scale).mean())))
