@@ -1447,13 +1447,26 @@ int launch_pattern_gather(BitBwdArgs a, bool bn, cudaStream_t st)
 
 // Training forward in binary mode by way of the bit operators: pack the rows, count patterns and evaluate truth tables on bits, expand the
 // output.  Per node-frame that moves 4 bytes of y (and 4 per input row and frame) against the 24 + 1 that the per-node passes of
-// f32_binary_forward_by_table() read through L2: 8192 x 8192 nodes x 16384 frames 360 -> 302 us, 90 of them the packing.  So it is taken up to
-// two input rows a node.
+// f32_binary_forward_by_table() read through L2, for two launches more, a reduction of 64 counters per node that costs about as much as 1500
+// frames, and packing that grows with the rows.  Measured on B200 (220 layers of 2^22 to 2^27 node-frames, 256 to 40000 frames and 0.25 to 3
+// rows a node; packed / by node): 8192 nodes x 16384 frames 292 / 368 us with a row a node, 377 / 412 with two, 422 / 430 with two and a
+// half; 8192 x 4096 125 / 121 with two; 4096 x 4096 63.2 / 62.4 with one and a half; 1024 x 4096 25.7 / 21.3 with one; 30000 x 300 107 / 58;
+// 23000 x 780 105 / 85; 20676 x 1164 112 / 103.  With the rule below a layer takes 0.5 % longer than with the better of the two, on average
+// (always by node 6 %, packed up to two rows a node whatever the size 14 %).
+static bool packed_forward_pays(int I, int O, int F, long long fs, bool aligned)
+{
+    const long long node_frames = (long long)O * F;
+    if (!aligned || (long long)O * fs > (1LL << 30)) return I <= 2LL * O;              // by node declines these
+    if (node_frames >= 3LL << 24) return F >= 1024 && I <= 2LL * O;                    // rows of fp32 frames no longer stay in L2
+    return node_frames >= 1LL << 23 && F >= 3072 && 2LL * I <= 3LL * O;
+}
+
 int f32_binary_forward_packed(const float *x, float *y, const int *idx, const float *W, float *mean, float *rstd, float *rmean, float *rvar,
                               float gamma, float beta, float momentum, float bias, int I, int O, int F, long long fs, int lut_binarize,
                               cudaStream_t st)
 {
-    if (small_layer(O, F) || I < 1 || I > 2LL * O) return BBCU_ERR_NO_MEMORY;
+    const bool aligned = ((reinterpret_cast<uintptr_t>(x) | reinterpret_cast<uintptr_t>(y)) & 15) == 0 && fs % 4 == 0;
+    if (small_layer(O, F) || I < 1 || !packed_forward_pays(I, O, F, fs, aligned)) return BBCU_ERR_NO_MEMORY;
     const long long ws = ((long long)F + 127) / 128 * 4;                // whole 16-byte pieces
     const size_t x_bytes = (size_t)I * (size_t)ws * 4, y_bytes = (size_t)O * (size_t)ws * 4;
     if (x_bytes + y_bytes > ((size_t)1 << 30)) return BBCU_ERR_NO_MEMORY;

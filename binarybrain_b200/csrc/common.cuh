@@ -75,7 +75,7 @@ int bit_backward_apply_by_table(const float *x, const float *dy, float *dx, cons
                                 const float *rstd, const double *sums, float *dmean_out, float *dvar_out, float gamma, float beta, float bias, int I,
                                 int O, int F, long long fs, long long total_frames, int lut_binarize, cudaStream_t st);
 
-// The training forward of a binary-mode layer on I fp32 rows through packed rows; declines (small layers, I > 2 O, no scratch) like the others.
+// The training forward of a binary-mode layer on I fp32 rows through packed rows; declines (layers where it does not pay, no scratch) like the others.
 int f32_binary_forward_packed(const float *x, float *y, const int *idx, const float *W, float *mean, float *rstd, float *rmean, float *rvar,
                               float gamma, float beta, float momentum, float bias, int I, int O, int F, long long fs, int lut_binarize,
                               cudaStream_t st);

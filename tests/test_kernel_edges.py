@@ -106,7 +106,7 @@ def test_two_valued_layers_edges(ops, I, O, F, stride):
     assert err(host_fp32(dx, F), dx_w) <= parity.BN_GRAD_FACTOR * parity.TOL * amp and err(dW.cpu().numpy(), dW_w) <= parity.BN_GRAD_FACTOR * parity.TOL * amp
 
 
-# above the one-launch range, fp32 rows packed for the forward (up to two input rows a node) and not
+# above the one-launch range; the forward by node, and (rows that are not aligned) by way of packed rows
 @pytest.mark.parametrize("I,O,F,stride", [(700, 1025, 2049, None), (70, 40, 4129, 4131), (60, 33, 70001, None), (1300, 513, 4200, None)])
 def test_large_two_valued_layers_edges(ops, I, O, F, stride):
     test_two_valued_layers_edges(ops, I, O, F, stride)
@@ -179,3 +179,44 @@ def test_layer_keeps_its_statistics_tensors(ops, O, F):
         want = port.dl6_forward_train(x, idx, W, np.zeros(O), np.ones(O), binary=0)
         assert layer.mean is mean and layer.rstd is rstd
         assert np.abs(mean.cpu().numpy() - want["mean"]).max() <= 1e-6 and np.abs(rstd.cpu().numpy() / want["rstd"] - 1).max() <= 1e-4
+
+
+# Training forward of a binary-mode layer on fp32 frames: the rows go through bits, or the frames through per-node passes, by a rule on the
+# sizes.  Both sides of each of its lines; which way a call went shows in the scratch it asked the heap for.  The entry point that is not
+# told the number of rows always takes the per-node passes, and the two ways agree in every bit.
+@pytest.mark.parametrize("I,O,F,stride,packed", [
+    (1, 2731, 3072, None, True), (1, 2730, 3072, None, False), (1, 2732, 3071, None, False), (4096, 2731, 3072, None, True), (4097, 2731, 3072, None, False),
+    (12288, 12288, 4096, None, True), (24576, 12288, 4096, None, True), (24577, 12288, 4096, None, False), (12287, 12287, 4096, None, True),
+    (24574, 12287, 4096, None, False), (49152, 49152, 1024, None, True), (49201, 49201, 1023, None, False), (140, 70, 30001, 30003, True)])
+def test_binary_training_forward_by_bits_or_by_node(ops, I, O, F, stride, packed):
+    import torch
+    from binarybrain_b200 import abi
+    L = abi.lib()
+    g = torch.Generator(device="cuda").manual_seed(I + O)
+    stride = ops.fp32_stride(F) if stride is None else stride
+    x = torch.rand((I, stride), device="cuda", generator=g)
+    idx = torch.randint(0, I, (O, 6), device="cuda", generator=g, dtype=torch.int32)
+    W = torch.rand((O, 64), device="cuda", generator=g)
+
+    def run(rows):
+        y, s = torch.full((O, stride), -1.0, device="cuda"), [torch.ones(O, device="cuda") for _ in range(4)]
+        torch.cuda.synchronize()
+        L.bbcu_LocalHeap_GarbageCollect()
+        before = L.bbcu_LocalHeap_GetAllocatedSize()
+        args = [y.data_ptr(), idx.data_ptr(), W.data_ptr(), *[t.data_ptr() for t in s], 0.3, 0.5, 0.9, 0.25] + ([I] if rows else []) + [O, F, stride, 0, 1, None]
+        abi.call("bbcu_fp32_DifferentiableLut6_ForwardTraining" + ("Rows" if rows else ""), x.data_ptr(), *args)
+        torch.cuda.synchronize()
+        return y[:, :F], s, L.bbcu_LocalHeap_GetAllocatedSize() - before
+
+    def block(n):
+        return (n + 511) // 512 * 512
+
+    words, tables = (F + 127) // 128 * 4, 776 * O
+    y, s, scratch = run(True)
+    want = block((I + O) * words * 4) + block((tables + 255) // 256 * 256) if packed else block((tables + 255) // 256 * 256 + O * stride)
+    assert scratch == want
+    y2, s2, _ = run(False)
+    if stride % 4 == 0:
+        assert torch.equal(y, y2) and all(torch.equal(a, b) for a, b in zip(s, s2))
+    else:                                                # per-frame kernel: sums of the values instead of counts of the patterns
+        assert float((y != y2).float().mean()) < 1e-3 and all(torch.allclose(a, b, rtol=1e-4) for a, b in zip(s, s2))
