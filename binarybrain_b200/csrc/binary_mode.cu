@@ -272,8 +272,11 @@ struct BitBwdArgs {
     uint8_t *pat;                       // [O][ps] patterns, bit 7: the mask passes
     float *etab;                        // [6 O][64] look-up tables, see k_bit_backward_finalize
     float2 *ntab;                       // [O] gamma rstd, dvar bias / F
-    const int *edge_end, *edge_count, *edges;      // consumers of every input row (8 node + input number)
-    int I, O, F, groups, tile_frames, tiles, split;
+    const int *edge_end, *edge_count, *edges;      // consumers of every input row (8 node + input number); count: negative for heavy rows
+    const int2 *heavy;                  // chunks of the rows with more than heavy_from consumers: row, first consumer; heavy_count[0] of them
+    const int *heavy_count;
+    int heavy_from, heavy_chunk, heavy_ctas;
+    int I, O, F, groups, tile_frames, tiles, nc, split;
     int vec;                            // dy and dx (and fp32 x) rows start on 16-byte boundaries
     long long xs, fs, ps;               // word stride of x, float stride of dy / dx, stride of pat
 };
@@ -471,8 +474,9 @@ __global__ void k_edge_count(const int *__restrict__ idx, int *count, int edges)
     if (e < edges) atomicAdd(count + idx[e], 1);
 }
 
-// room for every row's list, in no particular order: `total` is a bump pointer, advanced once per warp
-__global__ void k_edge_room(const int *__restrict__ count, int *cursor, int *total, int I)
+// room for every row's list, in no particular order: `total` is a bump pointer, advanced once per warp; and the chunks of heavy rows,
+// whose count is negated
+__global__ void k_edge_room(int *count, int *cursor, int *total, int I, int2 *heavy, int *heavy_count, int heavy_from, int heavy_chunk)
 {
     grid_dependency();
     const int i = blockIdx.x * blockDim.x + threadIdx.x, lane = threadIdx.x & 31;
@@ -487,14 +491,25 @@ __global__ void k_edge_room(const int *__restrict__ count, int *cursor, int *tot
     if (lane == 31) base = atomicAdd(total, at);
     base = __shfl_sync(kFull, base, 31);
     if (i < I) cursor[i] = base + at - n;
+    if (n > heavy_from) {
+        const int chunks = (n + heavy_chunk - 1) / heavy_chunk, first = atomicAdd(heavy_count, chunks);
+        for (int k = 0; k < chunks; ++k) heavy[first + k] = make_int2(i, k * heavy_chunk);
+        count[i] = -n;
+    }
 }
 
-// afterwards cursor[i] is the end of row i's list
-__global__ void k_edge_fill(const int *__restrict__ idx, int *cursor, int *list, int edges)
+// afterwards cursor[i] is the end of row i's list; dx of the heavy rows, which several CTAs add to, is cleared
+__global__ void k_edge_fill(const int *__restrict__ idx, int *cursor, int *list, int edges, const int2 *__restrict__ heavy,
+                            const int *__restrict__ heavy_count, float *dx, long long fs)
 {
     grid_dependency();
-    const int e = blockIdx.x * blockDim.x + threadIdx.x;
+    const int e = blockIdx.x * blockDim.x + threadIdx.x, chunks = heavy_count[0];
     if (e < edges) list[atomicAdd(cursor + idx[e], 1)] = e + 2 * (e / 6);
+    for (int k = 0; k < chunks; ++k) {
+        const int2 h = heavy[k];
+        if (h.y == 0)
+            for (long long f = e; f < fs; f += (long long)gridDim.x * blockDim.x) dx[(size_t)h.x * fs + f] = 0.0f;
+    }
 }
 
 template <unsigned SEL>
@@ -507,7 +522,9 @@ __device__ __forceinline__ uint32_t prmt(uint32_t v)
 
 // dx_i(f) = sum over the consumers (node o, input j) of row i of g_o(f) D_j[p_o(f)], frames from F on 0.  A CTA is one row and NC
 // chunks of 128 frames; `split` warps share the consumers (rows with many of them, or few rows).  One warp per CTA otherwise, because
-// the number of consumers varies from row to row and a CTA of several rows waits for the longest.
+// the number of consumers varies from row to row and a CTA of several rows waits for the longest.  Rows with far more consumers than the
+// average (more than heavy_from) would hold up the whole pass as one CTA's loop: the first heavy_ctas CTAs take them, in chunks of
+// consumers, and add the chunks' sums to the row, which k_edge_fill has cleared.
 // The tables of a consumer live in registers, one entry per lane, and a look-up is a shuffle whose source lane is the pattern rotated by
 // j + 1 (the rotation serves the patterns of four frames at once): bits 0 .. 4 are the other five inputs, bit 5 is input j.  No single
 // resource is exhausted (8192 x 8192 nodes x 8192 frames under ncu: issue 69 %, L1 68 %, logic pipe 59 %, a third of the stalls on L2
@@ -515,10 +532,8 @@ __device__ __forceinline__ uint32_t prmt(uint32_t v)
 // writing g out once and reading it back would spare a shuffle and six instructions, but costs 10 bytes per node-frame of HBM traffic.
 // Several rows one after the other in a CTA keep more tiles in flight than L2 holds (8 rows: 509 -> 617 us for 16384 frames).
 template <bool BN, int NC, bool WHOLE>
-__device__ __forceinline__ void pattern_gather(const BitBwdArgs &a, int row, int part, int f0, int lane, float (&acc)[NC][4])
+__device__ __forceinline__ void pattern_gather(const BitBwdArgs &a, const int *list, int n, int part, int f0, int lane, float (&acc)[NC][4])
 {
-    const int n = __ldg(a.edge_count + row);
-    const int *list = a.edges + (__ldg(a.edge_end + row) - n);
     int e_n = part < n ? __ldg(list + part) : 0;
     for (int k = part; k < n; k += a.split) {
         const int node = e_n >> 3, j = e_n & 7;
@@ -565,24 +580,22 @@ __device__ __forceinline__ void pattern_gather(const BitBwdArgs &a, int row, int
     }
 }
 
-template <bool BN, int NC>
-__global__ void __launch_bounds__(kWarpsPerCta * 32, 4)
-k_pattern_gather(const BitBwdArgs a)
+// The sum over `n` consumers for one tile of a row, written (ADD: added) to dx by the CTA's first warp; nothing where n is negative (a heavy
+// row.  Asking that first, instead of before the store, costs every CTA a wait for n: 811 -> 816 us for 8192 x 8192 nodes x 16384 frames.)
+template <bool BN, int NC, bool ADD>
+__device__ __forceinline__ void gather_tile(const BitBwdArgs &a, int row, const int *list, int n, int tile, float4 *s_part)
 {
-    grid_dependency();
-    extern __shared__ __align__(16) unsigned char smem_raw[];           // split > 1: float4 [split][NC][32]
-    float4 *s_part = reinterpret_cast<float4 *>(smem_raw);
     const int part = threadIdx.x >> 5, lane = threadIdx.x & 31;
-    const int tile = blockIdx.x / a.I, row = blockIdx.x - tile * a.I;
     const int f_begin = tile * (128 * NC), f0 = f_begin + 4 * lane;
     float acc[NC][4];
 #pragma unroll
     for (int c = 0; c < NC; ++c)
 #pragma unroll
         for (int i = 0; i < 4; ++i) acc[c][i] = 0.0f;
-    if (a.vec && f_begin + 128 * NC <= a.F) pattern_gather<BN, NC, true>(a, row, part, f0, lane, acc);
-    else if (f_begin < a.F)                 pattern_gather<BN, NC, false>(a, row, part, f0, lane, acc);
+    if (a.vec && f_begin + 128 * NC <= a.F) pattern_gather<BN, NC, true>(a, list, n, part, f0, lane, acc);
+    else if (f_begin < a.F)                 pattern_gather<BN, NC, false>(a, list, n, part, f0, lane, acc);
     if (a.split > 1) {
+        if (ADD) __syncthreads();                                       // (the tile before has been read)
 #pragma unroll
         for (int c = 0; c < NC; ++c) s_part[(part * NC + c) * 32 + lane] = make_float4(acc[c][0], acc[c][1], acc[c][2], acc[c][3]);
         __syncthreads();
@@ -594,6 +607,7 @@ k_pattern_gather(const BitBwdArgs a)
                 acc[c][0] += v.x; acc[c][1] += v.y; acc[c][2] += v.z; acc[c][3] += v.w;
             }
     }
+    if (!ADD && n < 0) return;
     float *out = a.dx + (size_t)row * a.fs;
 #pragma unroll
     for (int c = 0; c < NC; ++c) {
@@ -602,13 +616,48 @@ k_pattern_gather(const BitBwdArgs a)
         for (int i = 0; i < 4; ++i)
             if (f + i >= a.F) acc[c][i] = 0.0f;
         if (a.vec && f + 3 < a.fs) {
-            *reinterpret_cast<float4 *>(out + f) = make_float4(acc[c][0], acc[c][1], acc[c][2], acc[c][3]);
+            if (ADD) red_add_v4(out + f, acc[c][0], acc[c][1], acc[c][2], acc[c][3]);
+            else     *reinterpret_cast<float4 *>(out + f) = make_float4(acc[c][0], acc[c][1], acc[c][2], acc[c][3]);
         } else {
 #pragma unroll
             for (int i = 0; i < 4; ++i)
-                if (f + i < a.fs) out[f + i] = acc[c][i];
+                if (f + i < a.fs) {
+                    if (ADD) atomicAdd(out + f + i, acc[c][i]);
+                    else     out[f + i] = acc[c][i];
+                }
         }
     }
+}
+
+// The chunks of the heavy rows, one (tile, chunk) after another; tiles of 256 frames at most, for which the registers of the ordinary path do.
+template <bool BN, int NC>
+__device__ __forceinline__ void gather_heavy(const BitBwdArgs &a, float4 *s_part)
+{
+    constexpr int HC = NC > 2 ? 2 : NC;
+    const int chunks = __ldg(a.heavy_count), items = chunks * ((a.F + 128 * HC - 1) / (128 * HC));
+    for (int item = blockIdx.x; item < items; item += a.heavy_ctas) {
+        const int tile = item / chunks;
+        const int2 h = __ldg(a.heavy + (item - tile * chunks));
+        const int n = -__ldg(a.edge_count + h.x);
+        gather_tile<BN, HC, true>(a, h.x, a.edges + (__ldg(a.edge_end + h.x) - n + h.y), min(n - h.y, a.heavy_chunk), tile, s_part);
+    }
+}
+
+template <bool BN, int NC>
+__global__ void __launch_bounds__(kWarpsPerCta * 32, 4)
+k_pattern_gather(const BitBwdArgs a)
+{
+    grid_dependency();
+    extern __shared__ __align__(16) unsigned char smem_raw[];           // split > 1: float4 [split][NC][32]
+    float4 *s_part = reinterpret_cast<float4 *>(smem_raw);
+    const int block = (int)blockIdx.x - a.heavy_ctas;
+    if (block < 0) {
+        gather_heavy<BN, NC>(a, s_part);
+        return;
+    }
+    const int tile = block / a.I, row = block - tile * a.I;
+    const int n = __ldg(a.edge_count + row);
+    gather_tile<BN, NC, false>(a, row, a.edges + (__ldg(a.edge_end + row) - n), n, tile, s_part);
 }
 
 // Per-pattern gradient sums -> table-entry gradients: for every input, (a, b) -> (a hi + b lo, a lo + b hi) with hi = 0.5 + bias,
@@ -1372,26 +1421,51 @@ bool pack_bits(const float *x, uint32_t *bits, int I, int F, long long xs, long 
     return true;
 }
 
-// Slot 3 of the stream's scratch: consumer lists, and the bits of the I fp32 rows when `pack`.
+// How k_pattern_gather divides its work.  The tile is 512 frames (the tables of a consumer are loaded once per tile) unless the dy and
+// pattern rows of such a tile, 5 bytes per node and frame, exceed two thirds of L2, or the GPU would run short of warps.  The warps of a
+// CTA are chosen by the average number of consumers of a row; a row with more than eight times the average, and more than 64, is heavy.
+// Backward of 8192 x 8192 nodes x 16384 frames: even wiring 811 us; one row feeding every node 7210 as the loop of one CTA per tile, 2765 / 990 /
+// 886 with 1 / 4 / 8 CTAs per SM for the chunks (which cost nothing where there are none).  2048 x 2048 x 2048: 66; 1035, 95 / 72 / 72.
+void gather_shape(BitBwdArgs &a)
+{
+    const DeviceInfo &di = device_info();
+    const long long fan = (6LL * a.O + a.I - 1) / a.I;
+    int nc = 4;
+    while (nc > 1 && (5LL * a.O * 128 * nc > (long long)(di.l2_bytes / 3 * 2) || (long long)a.I * ((a.fs + 128 * nc - 1) / (128 * nc)) < 16LL * di.sm_count)) nc /= 2;
+    a.nc = nc;
+    a.tiles = (int)((a.fs + 128 * nc - 1) / (128 * nc));
+    const long long blocks = (long long)a.I * a.tiles;
+    a.split = 1;
+    while (a.split < kWarpsPerCta && (fan >= 32LL * a.split || (fan >= 4LL * a.split && blocks * a.split < 8LL * di.sm_count))) a.split *= 2;
+    const long long heavy_from = 8 * fan > 64 ? 8 * fan : 64;
+    a.heavy_from = (int)(heavy_from < (1 << 30) ? heavy_from : 1 << 30);
+    a.heavy_chunk = 32 * a.split <= a.heavy_from / 2 ? 32 * a.split : a.heavy_from / 2;
+    a.heavy_ctas = 8 * di.sm_count;
+}
+
+// Slot 3 of the stream's scratch: consumer lists, the chunks of heavy rows, and the bits of the I fp32 rows when `pack`.
 bool input_side(BitBwdArgs &a, int I, bool pack, cudaStream_t st)
 {
     if (I == 0) return false;
     a.I = I;
+    gather_shape(a);
     const int edges = 6 * a.O;
     const long long ws = (a.F + 31) / 32;
-    const size_t list_bytes = ((2 * (size_t)I + 1 + (size_t)edges) * sizeof(int) + 255) & ~(size_t)255;
+    // a heavy row has more than heavy_from >= 2 heavy_chunk consumers, so its chunks number at most 3 / 2 of its consumers over heavy_chunk
+    const size_t heavy_most = (size_t)edges / (size_t)a.heavy_chunk * 3 / 2 + 2;
+    const size_t list_bytes = (heavy_most * sizeof(int2) + (2 * (size_t)I + 2 + (size_t)edges) * sizeof(int) + 255) & ~(size_t)255;
     const size_t bit_bytes = pack ? (size_t)I * (size_t)ws * 4 : 0;
     if (bit_bytes > ((size_t)1 << 30)) return false;
-    int *count = static_cast<int *>(stream_scratch(st, list_bytes + bit_bytes, 3));
-    if (count == nullptr) return false;
-    int *total = count + I, *cursor = total + 1, *list = cursor + I;
-    a.edge_count = count; a.edge_end = cursor; a.edges = list;
-    cudaMemsetAsync(count, 0, ((size_t)I + 1) * sizeof(int), st);
+    int2 *heavy = static_cast<int2 *>(stream_scratch(st, list_bytes + bit_bytes, 3));
+    if (heavy == nullptr) return false;
+    int *count = reinterpret_cast<int *>(heavy + heavy_most), *total = count + I, *heavy_count = total + 1, *cursor = heavy_count + 1, *list = cursor + I;
+    a.edge_count = count; a.edge_end = cursor; a.edges = list; a.heavy = heavy; a.heavy_count = heavy_count;
+    cudaMemsetAsync(count, 0, ((size_t)I + 2) * sizeof(int), st);
     launch(k_edge_count, (edges + 255) / 256, 256, 0, st, a.idx, count, edges);
-    launch(k_edge_room, (I + 255) / 256, 256, 0, st, count, cursor, total, I);
-    launch(k_edge_fill, (edges + 255) / 256, 256, 0, st, a.idx, cursor, list, edges);
+    launch(k_edge_room, (I + 255) / 256, 256, 0, st, count, cursor, total, I, heavy, heavy_count, a.heavy_from, a.heavy_chunk);
+    launch(k_edge_fill, (edges + 255) / 256, 256, 0, st, a.idx, cursor, list, edges, heavy, heavy_count, a.dx, a.fs);
     if (pack) {
-        uint32_t *bits = reinterpret_cast<uint32_t *>(reinterpret_cast<unsigned char *>(count) + list_bytes);
+        uint32_t *bits = reinterpret_cast<uint32_t *>(reinterpret_cast<unsigned char *>(heavy) + list_bytes);
         if (!pack_bits(reinterpret_cast<const float *>(a.x), bits, I, a.F, a.xs, ws, st)) return false;
         a.x = bits;
         a.xs = ws;
@@ -1423,19 +1497,12 @@ int launch_pattern_sums(BitBwdArgs a, bool bn, cudaStream_t st)
     return launch_status();
 }
 
-// dx.  The tile is 512 frames (the tables of a consumer are loaded once per tile) unless the dy and pattern rows of such a tile, 5
-// bytes per node and frame, exceed two thirds of L2, or the GPU would run short of warps.
 int launch_pattern_gather(BitBwdArgs a, bool bn, cudaStream_t st)
 {
     a.vec = a.vec && (reinterpret_cast<uintptr_t>(a.dx) & 15) == 0;
-    const DeviceInfo &di = device_info();
-    const long long fan = (6LL * a.O + a.I - 1) / a.I;                                // consumers per row, on average
-    int nc = 4;
-    while (nc > 1 && (5LL * a.O * 128 * nc > (long long)(di.l2_bytes / 3 * 2) || (long long)a.I * ((a.fs + 128 * nc - 1) / (128 * nc)) < 16LL * di.sm_count)) nc /= 2;
-    const long long blocks = (long long)a.I * ((a.fs + 128 * nc - 1) / (128 * nc));
+    const int nc = a.nc;
+    const long long blocks = (long long)a.I * a.tiles + a.heavy_ctas;
     BB200_REQUIRE(blocks < (1LL << 31), BBCU_ERR_TOO_LARGE);
-    a.split = 1;
-    while (a.split < kWarpsPerCta && (fan >= 32LL * a.split || (fan >= 4LL * a.split && blocks * a.split < 8LL * di.sm_count))) a.split *= 2;
     const int smem = a.split > 1 ? a.split * nc * 32 * (int)sizeof(float4) : 0;
     auto kern = bn ? (nc == 4 ? k_pattern_gather<true, 4> : nc == 2 ? k_pattern_gather<true, 2> : k_pattern_gather<true, 1>)
                    : (nc == 4 ? k_pattern_gather<false, 4> : nc == 2 ? k_pattern_gather<false, 2> : k_pattern_gather<false, 1>);
@@ -1501,9 +1568,10 @@ int bit_backward_by_table(bool bn, bool x_is_fp32, const void *x, const float *d
         return launch_status();
     }
     BitBwdArgs a;
-    if (!backward_setup(a, x, dy, idx, O, F, xs, fs, st) || !input_side(a, I, x_is_fp32, st)) return BBCU_ERR_NO_MEMORY;
-    BB200_CUDA(cudaPeekAtLastError());
+    if (!backward_setup(a, x, dy, idx, O, F, xs, fs, st)) return BBCU_ERR_NO_MEMORY;
     a.dx = dx;
+    if (!input_side(a, I, x_is_fp32, st)) return BBCU_ERR_NO_MEMORY;
+    BB200_CUDA(cudaPeekAtLastError());
     const unsigned blocks = (unsigned)((O + kWarpsPerCta - 1) / kWarpsPerCta), threads = kWarpsPerCta * 32;
     if (bn) launch(k_pattern_masks, blocks, threads, 0, st, W, a.mask, mean, rstd, gamma, beta, bias, O, lut_binarize);
     else    launch(k_pattern_derivatives, blocks, threads, 0, st, W, a.etab, bias, O, lut_binarize);
@@ -1560,6 +1628,7 @@ int bit_backward_apply_by_table(const float *x, const float *dy, float *dx, cons
     }
     BitBwdArgs a;
     if (!backward_setup(a, x, dy, idx, O, F, fs, fs, st)) return BBCU_ERR_NO_MEMORY;      // the same block as before (and it forgets the record)
+    a.dx = dx;
     if (!input_side(a, I, !have, st)) return BBCU_ERR_NO_MEMORY;
     BB200_CUDA(cudaPeekAtLastError());
     const unsigned blocks = (unsigned)((O + kWarpsPerCta - 1) / kWarpsPerCta), threads = kWarpsPerCta * 32;
@@ -1569,7 +1638,6 @@ int bit_backward_apply_by_table(const float *x, const float *dy, float *dx, cons
         const int rc = launch_pattern_sums<false>(a, true, st);
         if (rc) return rc;
     }
-    a.dx = dx;
     launch(k_bit_backward_finalize<true>, blocks, threads, 0, st, a.hdy, a.hist, a.mask, W, a.etab, a.ntab, dW, mean, rstd, dmean_out, dvar_out, gamma, beta, bias,
                                                              O, 1.0f / (float)total_frames, lut_binarize, nullptr, sums);
     BB200_CUDA(cudaPeekAtLastError());

@@ -220,3 +220,34 @@ def test_binary_training_forward_by_bits_or_by_node(ops, I, O, F, stride, packed
         assert torch.equal(y, y2) and all(torch.equal(a, b) for a, b in zip(s, s2))
     else:                                                # per-frame kernel: sums of the values instead of counts of the patterns
         assert float((y != y2).float().mean()) < 1e-3 and all(torch.allclose(a, b, rtol=1e-4) for a, b in zip(s, s2))
+
+
+# Two-valued inputs, uneven wiring: row 0 feeds every node and row 1 every other one, far more than the average (rows of several chunks of
+# consumers, shared by blocks that add to dx), beside rows without any consumer.  One warp and several a block, tiles of 128 frames and more,
+# rows that are not aligned.
+@pytest.mark.parametrize("I,O,F,stride", [(2400, 150, 4200, None), (2400, 80, 4097, 4099), (60, 330, 4099, 4099), (60, 330, 4100, None), (9, 8, 4100, None)])
+def test_two_valued_backward_uneven_wiring(ops, I, O, F, stride):
+    import torch
+    from gpu_util import dev, dev_bits, dev_fp32, err, host_fp32
+    rng = np.random.default_rng(I + O + F)
+    idx = np.stack([rng.permutation(np.arange(2, I))[:6] for _ in range(O)]).astype(np.int32)
+    idx[:, 3] = 0
+    idx[::2, 5] = 1
+    W = np.clip(rng.normal(0.5, 0.25, (O, 64)), 0, 1).astype(np.float32)
+    x, dy = rng.random((I, F), dtype=np.float32), rng.standard_normal((O, F), dtype=np.float32)
+    xb = pack_bits(x > 0.5)
+    dx_w, dW_w = port.sl6_backward(x, dy, idx, W, I, binary=1)
+    p = port.dl6_forward_train(xb, idx, W, np.zeros(O), np.ones(O), frames=F)
+    amp = max(1.0, 0.3 * float(p["rstd"].max()))
+    dy_n = np.where(parity._edges(p["y_pre"], amp), np.float32(0), dy).astype(np.float32)
+    dxn_w, dWn_w = port.dl6_backward(xb, dy_n, idx, W, p["mean"], p["rstd"], I)
+    for src in (dev_fp32(x, stride), dev_bits(xb, F)):
+        dW = torch.zeros((O, 64), device="cuda")
+        dx = torch.full((I, ops.fp32_stride(F) if stride is None else stride), 7.0, device="cuda")
+        ops.stochastic_lut6_backward(src, dev_fp32(dy, stride), dev(idx), dev(W), dW, I, F, dx=dx, binary=True)
+        assert err(host_fp32(dx, F), dx_w) <= parity.TOL and err(dW.cpu().numpy(), dW_w) <= parity.TOL and not dx[:, F:].any()
+        dW.zero_()
+        dx.fill_(7.0)
+        ops.differentiable_lut6_backward(src, dev_fp32(dy_n, stride), dev(idx), dev(W), dW, dev(p["mean"]), dev(p["rstd"]), I, F, dx=dx, binary=True)
+        tol = parity.BN_GRAD_FACTOR * parity.TOL * amp
+        assert err(host_fp32(dx, F), dxn_w) <= tol and err(dW.cpu().numpy(), dWn_w) <= tol and not dx[:, F:].any()
