@@ -11,9 +11,11 @@
 namespace bb200 {
 
 // The mean loss over frames in one go: work[0] = sum of all targets, work[1] = sum of the per-frame losses, *loss = -work[1] / work[0].
-// Up to kOneCta target values a single CTA does everything in one launch (ten classes x 512 frames: a read of the target sum by the
-// host, three reductions and a kernel took 58 us of host time); above, the sums go through `work`, which the caller clears.
-constexpr int kOneCta = 1 << 15;
+// Up to kOneCta target values a single CTA does everything in one launch; above, three kernels share it and the sums go through `work`, which
+// the caller clears (the clear and the launches are 14 us whatever the size).  One CTA / general on B200: 10 classes 8192 values 8.9 / 14.0 us,
+// 16384 13.5 / 14.0, 24576 18.7 / 14.1, 32768 24.0 / 14.1; 2 classes 8192 9.5 / 13.9, 16384 16.1 / 13.7; 100 classes 16384 34.2 / 39.0, 24576
+// 42.5 / 40.8.  (Before there was either, a read of the target sum by the host, three reductions and a kernel took 58 us of host time.)
+constexpr int kOneCta = 1 << 14;
 
 __device__ __forceinline__ double cta_sum(double v, double *red)
 {

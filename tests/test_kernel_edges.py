@@ -134,7 +134,7 @@ def test_large_probability_layers_edges(ops, I, O, F, stride):
     test_small_probability_layers_edges(ops, I, O, F, stride)
 
 
-# one CTA (up to 2^15 target values) and the general form; Adam with the gradients cleared on the way, whole quads and a remainder
+# one CTA (up to 2^14 target values) and the general form; Adam with the gradients cleared on the way, whole quads and a remainder
 @pytest.mark.parametrize("classes,frames", [(1, 1), (10, 129), (10, 3276), (10, 3277), (3, 20000)])
 def test_mean_loss_and_adam_update(ops, classes, frames):
     import torch
@@ -251,3 +251,9 @@ def test_two_valued_backward_uneven_wiring(ops, I, O, F, stride):
         ops.differentiable_lut6_backward(src, dev_fp32(dy_n, stride), dev(idx), dev(W), dW, dev(p["mean"]), dev(p["rstd"]), I, F, dx=dx, binary=True)
         tol = parity.BN_GRAD_FACTOR * parity.TOL * amp
         assert err(host_fp32(dx, F), dxn_w) <= tol and err(dW.cpu().numpy(), dWn_w) <= tol and not dx[:, F:].any()
+
+
+# the largest call of one CTA and the smallest of the general form
+@pytest.mark.parametrize("classes,frames", [(4, 4096), (10, 1638), (10, 1639)])
+def test_mean_loss_at_the_line(ops, classes, frames):
+    test_mean_loss_and_adam_update(ops, classes, frames)
