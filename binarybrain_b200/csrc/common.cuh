@@ -94,7 +94,7 @@ struct SmallLayerArgs {
     int F, lut_binarize, vec;
     long long fs;
 };
-constexpr long long kSmallProbability = 1LL << 21;       // node-frames, see small_probability_layer()
+constexpr long long kSmallProbability = BBCU_B200_SMALL_NODE_FRAMES;       // see small_probability_layer()
 bool small_probability_layer(int O, int F);
 int small_forward(int mode, const SmallLayerArgs &a, int O, cudaStream_t st);
 int small_backward(bool bn, const SmallLayerArgs &a, int I, int O, cudaStream_t st);

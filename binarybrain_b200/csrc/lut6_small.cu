@@ -270,7 +270,7 @@ unsigned threads_for(int F) { return 32u * (unsigned)(F > 128 * kWarpsPerCta ? k
 // Measured on B200 against the persistent kernels, training forward / batch-normalised backward of a layer: 360 nodes x 100 frames 6 / 9 us
 // (18 / 33), 1024 x 512 10 / 21 (20 / 46), 4096 x 512 24 / 60 (34 / 80), 2048 x 1000 27 / 72 (33 / 81; 64 from the saved output): even at
 // 2^21 node-frames.  A CTA works through its node's frames alone, hence the limit on those (64 x 11000: 16 / 39 against 21 / 49).
-bool small_probability_layer(int O, int F) { return O > 0 && F > 0 && (long long)O * F <= kSmallProbability && F <= 4096; }
+bool small_probability_layer(int O, int F) { return O > 0 && F > 0 && (long long)O * F <= kSmallProbability && F <= BBCU_B200_SMALL_FRAMES; }
 
 int small_forward(int mode, const SmallLayerArgs &a, int O, cudaStream_t st)
 {

@@ -187,4 +187,13 @@ PyModuleDef g_module = {PyModuleDef_HEAD_INIT, "_native", "bbcu_* operators on t
 
 }   // namespace
 
-PyMODINIT_FUNC PyInit__native() { return PyModule_Create(&g_module); }
+PyMODINIT_FUNC PyInit__native()
+{
+    PyObject *m = PyModule_Create(&g_module);
+    if (!m) return nullptr;
+    if (PyModule_AddIntConstant(m, "SMALL_NODE_FRAMES", BBCU_B200_SMALL_NODE_FRAMES) || PyModule_AddIntConstant(m, "SMALL_FRAMES", BBCU_B200_SMALL_FRAMES)) {
+        Py_DECREF(m);
+        return nullptr;
+    }
+    return m;
+}

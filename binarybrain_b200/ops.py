@@ -13,8 +13,13 @@ from . import abi
 BIAS = 0.25   # unbinarize_bias of the reference's layers (include/bb/DifferentiableLutN.h:63)
 
 
-# A layer of at most this many node-frames and frames runs in one launch per direction when its operators are called unsplit.
-SMALL_NODE_FRAMES, SMALL_FRAMES = 1 << 21, 4096
+def __getattr__(name):
+    """SMALL_NODE_FRAMES, SMALL_FRAMES: a layer of at most this many node-frames and frames runs in one launch per direction when its
+    operators are called unsplit.  The numbers are the library's (include/bbcu_b200.h), looked up once."""
+    if name in ("SMALL_NODE_FRAMES", "SMALL_FRAMES"):
+        from . import _native
+        return globals().setdefault(name, getattr(_native, name))
+    raise AttributeError(f"module {__name__!r} has no attribute {name!r}")
 
 
 class _Native:

@@ -56,6 +56,11 @@ typedef void *bbcu_stream_t;
 #define BBCU_ERR_NO_MEMORY     (-5)
 #define BBCU_ERR_TOO_LARGE     (-6)
 
+/* A layer in probability mode of at most this many node-frames and this many frames runs in one launch per direction when its operators are
+ * called unsplit. */
+#define BBCU_B200_SMALL_NODE_FRAMES (1 << 21)
+#define BBCU_B200_SMALL_FRAMES      4096
+
 /* Human-readable text for a return value of any function below. */
 const char *bbcu_b200_error_string(int status);
 /* ABI version of this library (bumped when a signature changes). */

@@ -31,6 +31,14 @@ def test_a_tensor_without_memory_is_an_error(native):
             native.bbcu_fp32_Vector_clamp(*args, 0.0, 1.0, 0, 0)
 
 
+def test_the_small_layer_limits_are_those_of_the_library(native):
+    from binarybrain_b200 import ops
+    assert (ops.SMALL_NODE_FRAMES, ops.SMALL_FRAMES) == (native.SMALL_NODE_FRAMES, native.SMALL_FRAMES) == (1 << 21, 4096)
+    assert "SMALL_FRAMES" in vars(ops)                                   # looked up once
+    with pytest.raises(AttributeError):
+        ops.SMALL_LAYERS
+
+
 @pytest.mark.gpu
 def test_a_lazily_cloned_output_leaves_its_twin_alone():
     import torch
