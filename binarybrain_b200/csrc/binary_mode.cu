@@ -1205,13 +1205,32 @@ struct Scratch {
 };
 
 // What the statistics half of a frame-sharded backward left in a stream's scratch (pattern counts, per-pattern dy sums, pattern
-// bytes), so that the apply half that follows it on the same stream need not repeat that pass.  Any other use of the scratch
-// forgets it; the apply half checks every field and redoes the pass when something differs.
+// bytes and masks), so that the apply half that follows it on the same stream need not repeat that pass.  It holds while nobody has been
+// handed the block (`ticket`), within one capture of the stream or outside of any (`capture`), and for the same call; the apply half
+// redoes the pass when something differs.
 struct PassOneRecord {
-    const void *x = nullptr, *dy = nullptr, *W = nullptr, *mean = nullptr, *rstd = nullptr;
-    int O = 0, F = 0;
-    long long fs = 0;
+    const void *x, *dy, *idx, *W, *mean, *rstd;
+    float gamma, beta, bias;
+    int O, F, lut_binarize;
+    long long fs;
+    unsigned long long ticket, capture;
+    bool operator==(const PassOneRecord &r) const
+    {
+        return x == r.x && dy == r.dy && idx == r.idx && W == r.W && mean == r.mean && rstd == r.rstd && gamma == r.gamma && beta == r.beta && bias == r.bias &&
+               O == r.O && F == r.F && lut_binarize == r.lut_binarize && fs == r.fs && ticket == r.ticket && capture == r.capture;
+    }
 };
+// what such a record reads at this moment; ticket 0 when the stream cannot be asked
+PassOneRecord pass_one(const void *x, const void *dy, const void *idx, const void *W, const void *mean, const void *rstd, float gamma, float beta, float bias,
+                       int O, int F, int lut_binarize, long long fs, cudaStream_t st)
+{
+    cudaStreamCaptureStatus status = cudaStreamCaptureStatusNone;
+    unsigned long long capture = 0;
+    const bool known = cudaStreamGetCaptureInfo(st, &status, &capture) == cudaSuccess;
+    if (!known) cudaGetLastError();
+    return PassOneRecord{x, dy, idx, W, mean, rstd, gamma, beta, bias, O, F, lut_binarize, fs, known ? stream_scratch_ticket(st, 1) : 0,
+                         status == cudaStreamCaptureStatusActive ? capture : 0};
+}
 std::mutex g_record_mu;
 std::map<std::pair<int, cudaStream_t>, PassOneRecord> g_records;
 
@@ -1224,10 +1243,6 @@ std::pair<int, cudaStream_t> record_key(cudaStream_t st)
 
 bool carve(Scratch &s, int O, cudaStream_t st, size_t extra = 0)
 {
-    {
-        std::lock_guard<std::mutex> g(g_record_mu);
-        g_records.erase(record_key(st));
-    }
     const size_t per_node = 64 * 4 + 64 * 4 + 8 + 64 * 4;        // Y, pattern counts, truth table, per-pattern dy sums
     const size_t fixed = (per_node * (size_t)O + 255) & ~(size_t)255;
     unsigned char *base = static_cast<unsigned char *>(stream_scratch(st, fixed + extra, 1));
@@ -1443,8 +1458,9 @@ void gather_shape(BitBwdArgs &a)
     a.heavy_ctas = 8 * di.sm_count;
 }
 
-// Slot 3 of the stream's scratch: consumer lists, the chunks of heavy rows, and the bits of the I fp32 rows when `pack`.
-bool input_side(BitBwdArgs &a, int I, bool pack, cudaStream_t st)
+// Slot 3 of the stream's scratch: consumer lists, the chunks of heavy rows, and the bits of the I rows where x is fp32.  The block is the same
+// size when they need not be packed, so that a call after which that is known does not have to grow it.
+bool input_side(BitBwdArgs &a, int I, bool x_is_fp32, bool packed, cudaStream_t st)
 {
     if (I == 0) return false;
     a.I = I;
@@ -1454,8 +1470,11 @@ bool input_side(BitBwdArgs &a, int I, bool pack, cudaStream_t st)
     // a heavy row has more than heavy_from >= 2 heavy_chunk consumers, so its chunks number at most 3 / 2 of its consumers over heavy_chunk
     const size_t heavy_most = (size_t)edges / (size_t)a.heavy_chunk * 3 / 2 + 2;
     const size_t list_bytes = (heavy_most * sizeof(int2) + (2 * (size_t)I + 2 + (size_t)edges) * sizeof(int) + 255) & ~(size_t)255;
-    const size_t bit_bytes = pack ? (size_t)I * (size_t)ws * 4 : 0;
-    if (bit_bytes > ((size_t)1 << 30)) return false;
+    size_t bit_bytes = x_is_fp32 ? (size_t)I * (size_t)ws * 4 : 0;
+    if (bit_bytes > ((size_t)1 << 30)) {
+        if (!packed) return false;
+        bit_bytes = 0;
+    }
     int2 *heavy = static_cast<int2 *>(stream_scratch(st, list_bytes + bit_bytes, 3));
     if (heavy == nullptr) return false;
     int *count = reinterpret_cast<int *>(heavy + heavy_most), *total = count + I, *heavy_count = total + 1, *cursor = heavy_count + 1, *list = cursor + I;
@@ -1464,7 +1483,7 @@ bool input_side(BitBwdArgs &a, int I, bool pack, cudaStream_t st)
     launch(k_edge_count, (edges + 255) / 256, 256, 0, st, a.idx, count, edges);
     launch(k_edge_room, (I + 255) / 256, 256, 0, st, count, cursor, total, I, heavy, heavy_count, a.heavy_from, a.heavy_chunk);
     launch(k_edge_fill, (edges + 255) / 256, 256, 0, st, a.idx, cursor, list, edges, heavy, heavy_count, a.dx, a.fs);
-    if (pack) {
+    if (x_is_fp32 && !packed) {
         uint32_t *bits = reinterpret_cast<uint32_t *>(reinterpret_cast<unsigned char *>(heavy) + list_bytes);
         if (!pack_bits(reinterpret_cast<const float *>(a.x), bits, I, a.F, a.xs, ws, st)) return false;
         a.x = bits;
@@ -1570,7 +1589,7 @@ int bit_backward_by_table(bool bn, bool x_is_fp32, const void *x, const float *d
     BitBwdArgs a;
     if (!backward_setup(a, x, dy, idx, O, F, xs, fs, st)) return BBCU_ERR_NO_MEMORY;
     a.dx = dx;
-    if (!input_side(a, I, x_is_fp32, st)) return BBCU_ERR_NO_MEMORY;
+    if (!input_side(a, I, x_is_fp32, false, st)) return BBCU_ERR_NO_MEMORY;
     BB200_CUDA(cudaPeekAtLastError());
     const unsigned blocks = (unsigned)((O + kWarpsPerCta - 1) / kWarpsPerCta), threads = kWarpsPerCta * 32;
     if (bn) launch(k_pattern_masks, blocks, threads, 0, st, W, a.mask, mean, rstd, gamma, beta, bias, O, lut_binarize);
@@ -1605,8 +1624,7 @@ int bit_backward_stats_by_table(const float *x, const float *dy, const int *idx,
                                                              O, 0.0f, lut_binarize, sums, nullptr);
     rc = launch_status();
     if (rc == BBCU_OK) {
-        PassOneRecord r;
-        r.x = x; r.dy = dy; r.W = W; r.mean = mean; r.rstd = rstd; r.O = O; r.F = F; r.fs = fs;
+        const PassOneRecord r = pass_one(x, dy, idx, W, mean, rstd, gamma, beta, bias, O, F, lut_binarize, fs, st);
         std::lock_guard<std::mutex> g(g_record_mu);
         g_records[record_key(st)] = r;
     }
@@ -1619,17 +1637,18 @@ int bit_backward_apply_by_table(const float *x, const float *dy, float *dx, cons
                                 const float *rstd, const double *sums, float *dmean_out, float *dvar_out, float gamma, float beta, float bias, int I,
                                 int O, int F, long long fs, long long total_frames, int lut_binarize, cudaStream_t st)
 {
+    const PassOneRecord now = pass_one(x, dy, idx, W, mean, rstd, gamma, beta, bias, O, F, lut_binarize, fs, st);
     bool have = false;
     {
         std::lock_guard<std::mutex> g(g_record_mu);
         auto it = g_records.find(record_key(st));
-        have = it != g_records.end() && it->second.x == x && it->second.dy == dy && it->second.W == W && it->second.mean == mean && it->second.rstd == rstd &&
-               it->second.O == O && it->second.F == F && it->second.fs == fs;
+        have = it != g_records.end() && now.ticket != 0 && it->second == now;
+        if (it != g_records.end()) g_records.erase(it);
     }
     BitBwdArgs a;
-    if (!backward_setup(a, x, dy, idx, O, F, fs, fs, st)) return BBCU_ERR_NO_MEMORY;      // the same block as before (and it forgets the record)
+    if (!backward_setup(a, x, dy, idx, O, F, fs, fs, st)) return BBCU_ERR_NO_MEMORY;      // the same block as before
     a.dx = dx;
-    if (!input_side(a, I, !have, st)) return BBCU_ERR_NO_MEMORY;
+    if (!input_side(a, I, true, have, st)) return BBCU_ERR_NO_MEMORY;
     BB200_CUDA(cudaPeekAtLastError());
     const unsigned blocks = (unsigned)((O + kWarpsPerCta - 1) / kWarpsPerCta), threads = kWarpsPerCta * 32;
     if (!have) {

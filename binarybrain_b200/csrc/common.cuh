@@ -36,6 +36,10 @@ const DeviceInfo &device_info();
 constexpr int kScratchSlots = 5;
 void *stream_scratch(cudaStream_t stream, size_t bytes, int slot = 0);
 
+// A number that is another one after every request for the stream's block (0: it has none).  A caller that leaves something in the block for
+// a later call of its own compares it: equal means that nobody has been handed the block since.
+unsigned long long stream_scratch_ticket(cudaStream_t stream, int slot);
+
 // 64 counters of the stream (slot 4), zeroed when they are made; a kernel that uses them leaves them zero.  nullptr when they cannot be had,
 // for the per-thread default stream, whose one handle stands for a stream of every thread, and for a stream that is being captured: the
 // graph may be launched on any stream, beside kernels of this one, and the zeroing would only be a node of the graph.

@@ -29,7 +29,9 @@ struct Pool {
     std::unordered_map<void *, size_t> live;          // ptr -> block size
     std::multimap<size_t, void *> cached;             // block size -> ptr
     size_t live_bytes = 0, cached_bytes = 0, max_alloc = 0, byte_limit = 0;
-    std::map<std::pair<cudaStream_t, int>, std::pair<void *, size_t>> scratch;     // (stream, slot) -> block
+    struct Scratch { void *ptr; size_t bytes; unsigned long long ticket; };
+    std::map<std::pair<cudaStream_t, int>, Scratch> scratch;                       // (stream, slot) -> block
+    unsigned long long tickets = 0;                                                // requests for scratch blocks so far
 };
 
 std::mutex g_pools_mu;
@@ -145,7 +147,10 @@ void *stream_scratch(cudaStream_t stream, size_t bytes, int slot)
     {
         std::lock_guard<std::mutex> g(p.mu);
         auto it = p.scratch.find(key);
-        if (it != p.scratch.end() && it->second.second >= bytes) return it->second.first;
+        if (it != p.scratch.end() && it->second.bytes >= bytes) {
+            it->second.ticket = ++p.tickets;
+            return it->second.ptr;
+        }
     }
     // grow: the old block goes back to the heap cache (work already enqueued on it is stream-ordered
     // before anything a later owner enqueues only if that owner uses the same stream, so hand it to
@@ -161,14 +166,22 @@ void *stream_scratch(cudaStream_t stream, size_t bytes, int slot)
     {
         std::lock_guard<std::mutex> g(p.mu);
         auto it = p.scratch.find(key);
-        if (it != p.scratch.end()) old = it->second.first;
-        p.scratch[key] = std::make_pair(fresh, bytes);
+        if (it != p.scratch.end()) old = it->second.ptr;
+        p.scratch[key] = Pool::Scratch{fresh, bytes, ++p.tickets};
     }
     if (old) {
         cudaStreamSynchronize(stream);
         bbcu_LocalHeap_Free(old);
     }
     return fresh;
+}
+
+unsigned long long stream_scratch_ticket(cudaStream_t stream, int slot)
+{
+    Pool &p = pool_of_current_device();
+    std::lock_guard<std::mutex> g(p.mu);
+    auto it = p.scratch.find(std::make_pair(stream, slot));
+    return it != p.scratch.end() ? it->second.ticket : 0;
 }
 
 unsigned *stream_counters(cudaStream_t stream)
@@ -350,7 +363,7 @@ extern "C" void bbcu_LocalHeap_GarbageCollect(void)
     std::vector<void *> scratch;
     {
         std::lock_guard<std::mutex> g(p.mu);
-        for (auto &kv : p.scratch) scratch.push_back(kv.second.first);
+        for (auto &kv : p.scratch) scratch.push_back(kv.second.ptr);
         p.scratch.clear();
     }
     if (!scratch.empty()) cudaDeviceSynchronize();

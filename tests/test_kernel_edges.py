@@ -257,3 +257,51 @@ def test_two_valued_backward_uneven_wiring(ops, I, O, F, stride):
 @pytest.mark.parametrize("classes,frames", [(4, 4096), (10, 1638), (10, 1639)])
 def test_mean_loss_at_the_line(ops, classes, frames):
     test_mean_loss_and_adam_update(ops, classes, frames)
+
+
+# The apply half of a frame-sharded binary-mode backward uses what the statistics half left in the stream's scratch, unless something else has
+# used or released that scratch in between, or the call is another one.
+@pytest.mark.parametrize("between", ["nothing", "another layer", "garbage collection", "another gamma", "captured"])
+def test_apply_half_after_the_scratch_was_used(ops, between):
+    import torch
+    from binarybrain_b200 import abi
+    from gpu_util import dev, dev_fp32, wiring
+    rng = np.random.default_rng(17)
+    I, O, F = 40, 30, 700
+    x, dy, idx = dev_fp32(rng.random((I, F))), dev_fp32(rng.standard_normal((O, F))), dev(wiring(rng, I, O))
+    W = dev(np.clip(rng.normal(0.5, 0.25, (O, 64)), 0, 1).astype(np.float32))
+    mean, rstd = torch.full((O,), 0.5, device="cuda"), torch.full((O,), 4.0, device="cuda")
+    sums, dx, dW = torch.zeros((O, 2), dtype=torch.float64, device="cuda"), torch.empty_like(x), torch.zeros_like(W)
+    gamma = 0.1 if between == "another gamma" else 0.3
+
+    def apply(dx, dW):
+        return ops.dl6_backward_apply(x, dy, dx, idx, W, dW, mean, rstd, sums, I, F, F, gamma=gamma)
+
+    ops.dl6_backward_stats(x, dy, idx, W, mean, rstd, F, sums)
+    abi.lib().bbcu_LocalHeap_GarbageCollect()                              # nothing of the statistics half is left
+    want_dW = W.new_zeros(O, 64)
+    want_dx = apply(torch.empty_like(x), want_dW)
+    if between == "captured":
+        side, graph = torch.cuda.Stream(), torch.cuda.CUDAGraph()
+        side.wait_stream(torch.cuda.current_stream())
+        with torch.cuda.stream(side):
+            ops.dl6_backward_stats(x, dy, idx, W, mean, rstd, F, sums)
+            apply(dx, dW)
+            ops.dl6_backward_stats(x, dy, idx, W, mean, rstd, F, sums)     # outside of the graph: nothing that a replay could count on
+        torch.cuda.synchronize()
+        with torch.cuda.graph(graph, stream=side):
+            apply(dx, dW)
+        with torch.cuda.stream(side):
+            ops.dl6_backward_stats(x, torch.zeros_like(dy), idx, W, mean, rstd, F, torch.zeros_like(sums))
+            dx.fill_(7.0)
+            dW.zero_()
+            graph.replay()
+        torch.cuda.synchronize()
+    else:
+        ops.dl6_backward_stats(x, dy, idx, W, mean, rstd, F, sums)
+        if between == "another layer":
+            ops.stochastic_lut6_forward(dev_fp32(rng.random((I, 40000))), dev(wiring(rng, I, 60)), torch.rand((60, 64), device="cuda"), 40000)
+        if between == "garbage collection":
+            abi.lib().bbcu_LocalHeap_GarbageCollect()
+        apply(dx, dW)
+    assert torch.allclose(dx, want_dx, rtol=1e-5, atol=1e-5) and torch.allclose(dW, want_dW, rtol=1e-5, atol=1e-4)
