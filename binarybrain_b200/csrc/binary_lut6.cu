@@ -554,7 +554,7 @@ extern "C" int bbcu_bit_BinaryLut6_Forward(const int *x, int *y, const int *idx,
         return launch_status();
     }
     if (vec) {
-        // persistent pipeline: two CTAs per SM, each walking (tile, node group) items
+        // persistent pipeline: two CTAs per SM, each warp of which walks (tile, node) items
         const bool attr_ok = allow_big_smem(k_binary_lut6_pipe, kPipeSmem);
         int *fault = fault_word();
         if (attr_ok && fault != nullptr) {

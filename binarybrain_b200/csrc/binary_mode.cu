@@ -372,6 +372,7 @@ __device__ __forceinline__ void pattern_columns_reduce(const PatternSlot<BN> *sl
     }
 }
 
+// XF32 (the statistics half of a sharded backward, always batch-normalised): the patterns come from fp32 rows.
 template <bool XF32, bool BN>
 __global__ void __launch_bounds__(kPsWarps * 32)
 k_pattern_sums(const BitBwdArgs a)
@@ -760,8 +761,9 @@ k_pattern_masks(const float *__restrict__ W, uint2 *__restrict__ mask, const flo
 template <bool BN>
 __global__ void __launch_bounds__(kWarpsPerCta * 32)
 k_bit_backward_finalize(const float *__restrict__ hdy, const uint32_t *__restrict__ hist, const uint2 *__restrict__ mask, const float *__restrict__ W,
-                        float *__restrict__ etab, float2 *__restrict__ ntab, float *dW, const float *__restrict__ mean_buf, const float *__restrict__ rstd_buf, float *dmean_out, float *dvar_out, float gamma,
-                        float beta, float bias, int O, float rF, int lut_binarize, double *sums_out, const double *__restrict__ sums_in)
+                        float *__restrict__ etab, float2 *__restrict__ ntab, float *dW, const float *__restrict__ mean_buf,
+                        const float *__restrict__ rstd_buf, float *dmean_out, float *dvar_out, float gamma, float beta, float bias, int O, float rF,
+                        int lut_binarize, double *sums_out, const double *__restrict__ sums_in)
 {
     grid_dependency();
     __shared__ float4 s_tab[BN ? kWarpsPerCta : 1][16];
@@ -1510,7 +1512,8 @@ int launch_pattern_sums(BitBwdArgs a, bool bn, cudaStream_t st)
         if (bn) BB200_CUDA(cudaMemsetAsync(a.hist, 0, (size_t)a.O * 256, st));
     }
     const int smem = kPsWarps * 64 * 32 * (int)(bn ? sizeof(PatternSlot<true>) : sizeof(PatternSlot<false>));
-    auto kern = bn ? k_pattern_sums<XF32, true> : k_pattern_sums<XF32, false>;
+    void (*kern)(BitBwdArgs) = k_pattern_sums<XF32, true>;
+    if constexpr (!XF32) { if (!bn) kern = k_pattern_sums<false, false>; }
     BB200_REQUIRE(allow_big_smem(kern, smem), BBCU_ERR_NO_MEMORY);
     launch(kern, (unsigned)blocks, kPsWarps * 32, smem, st, a);
     return launch_status();

@@ -807,7 +807,7 @@ k_lut6_backward(const BwdArgs a)
 //     (16 stores, 32 loads and 32 packed adds per lane instead of 62 shuffles with two selects each) and leave as one 8-byte
 //     reduction per lane into the coefficient-gradient scratch dC, which k_coeff_grads_to_dw maps to table gradients once per
 //     launch.
-// The tile is wide (1024-2048 frames) to amortise that flush: measured, the extra L2 misses of a wide tile cost less than
+// The tile is wide (512-2048 frames, backward_pipe_tile()) to amortise that flush: measured, the extra L2 misses of a wide tile cost less than
 // flushing more often, because the kernel is issue-bound, not memory-bound.
 // dx rows must be zero on entry (k_backward_prepare).
 // ---------------------------------------------------------------------------------------------

@@ -6,8 +6,9 @@
 // statistics and output -- or batch sums, gradients and the table gradient -- without leaving the SM.  Bound by latency (wiring, then
 // rows, then the reductions), not by throughput, so larger layers do not come here (small_probability_layer()).
 //
-// The arithmetic per frame is that of the persistent kernels, operation for operation (lut6_core.cuh), so a layer gives the same LUT
-// values whichever way it runs.  Semantics: include/bb/DifferentiableLutN.h:747-905 (forward), :1157-1266 (backward),
+// The LUT evaluation and its reverse pass are those of the persistent kernels (lut6_core.cuh), so a layer gives the same LUT values whichever
+// way it runs; the batch-norm gradient is rounded differently (three products and two sums here, two fused multiply-adds there), and the sums
+// over frames are taken in another order.  Semantics: include/bb/DifferentiableLutN.h:747-905 (forward), :1157-1266 (backward),
 // include/bb/StochasticLutN.h:512-559, :668-752.
 #include "common.cuh"
 #include "async_copy.cuh"

@@ -68,10 +68,11 @@ k_real_to_binary_bit(const float *__restrict__ x, uint32_t *y, const float *__re
 }
 
 // y[f][n] = mean over i < node_mux, j < frame_mux of bit x[f * frame_mux + j][n + i * y_nodes]
-// Block = one output node x 32 output frames, i.e. 32 * frame_mux consecutive input frames of node_mux rows; its warps (8 to 32, a row
-// each while there are enough: there are few blocks, and 13 rows one after the other took a warp 14 us for 1020 x 1792 -> 10 x 256, 8.6 us now) share the rows, a lane counts its input frames (lane + 32 m) over the warp's rows in registers, and the counts meet in shared
-// memory.  The counts are whole numbers, so the order of addition does not show.  (One thread per output value walked its node_mux *
-// frame_mux inputs alone: 1020 x 1792 -> 10 x 256 took 43 us on 2560 threads; the rows are 7.3 MB.)
+// Block = one output node x 32 output frames, i.e. 32 * frame_mux consecutive input frames of node_mux rows; its warps share the rows, a
+// lane counts its input frames (lane + 32 m) over the warp's rows in registers, and the counts meet in shared memory.  The counts are whole
+// numbers, so the order of addition does not show.  (One thread per output value walked its node_mux * frame_mux inputs alone: 1020 x 1792 ->
+// 10 x 256 took 43 us on 2560 threads; the rows are 7.3 MB.)  8 to 32 warps, a row each while there are enough: there are few blocks, and 13
+// rows one after the other took a warp 14 us for that size, 8.6 us now.
 constexpr int kB2rSteps = 8;
 
 template <bool XBIT>

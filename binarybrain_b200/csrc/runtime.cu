@@ -232,6 +232,7 @@ extern "C" int bbcu_b200_device_fault(void)
 namespace bb200 {
 __global__ void k_selftest_wait_expiry(int *fault, int attempts)
 {
+    grid_dependency();
     __shared__ uint64_t bar;
     if (threadIdx.x == 0) {
         mbar_init(&bar, 1);
@@ -251,7 +252,7 @@ extern "C" int bbcu_b200_selftest_wait_expiry(bbcu_stream_t stream)
 {
     int *w = fault_word();
     if (w == nullptr) return BBCU_ERR_NO_DEVICE;
-    k_selftest_wait_expiry<<<1, 32, 0, as_stream(stream)>>>(w, 2000);
+    launch(k_selftest_wait_expiry, 1, 32, 0, as_stream(stream), w, 2000);
     return launch_status();
 }
 

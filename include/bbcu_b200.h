@@ -24,10 +24,10 @@
  *   - scratch: the fp32 backward operators use the caller's dev_dx_tmp when it is given, 16-byte aligned and at least 512 bytes
  *     per output node.  Otherwise, and for the operators whose reference signature carries no scratch, the LUT operators keep
  *     per-stream work areas in the device heap below: per-node sums, coefficient and pattern tables (at most ~3 KiB per output
- *     node), the lists of the consumers of every input row (32 bytes per node) and, for two-valued inputs, the patterns of the frames (backward:
- *     2 bytes per node-frame; forward of DifferentiableLut6 in binary mode on fp32 frames: 1) and fp32 rows packed to bits; when
- *     these would exceed 8 GiB (forward: 1 GiB) the operator runs its scratch-free kernels instead.  The first call on a
- *     stream allocates them, later calls reuse them, and bbcu_LocalHeap_GarbageCollect releases them.
+ *     node), the lists of the consumers of every input row (about 26 bytes per node and 8 per row) and, for two-valued inputs, the patterns of
+ *     the frames (a byte per node-frame) and fp32 rows packed to bits.  When the patterns would exceed 4 GiB (training forward of
+ *     DifferentiableLut6 in binary mode on fp32 frames: 1 GiB) or the packed rows 1 GiB, the operator runs its scratch-free kernels instead.  The
+ *     first call on a stream allocates them, later calls reuse them, and bbcu_LocalHeap_GarbageCollect releases them.
  *     ..._ForwardTraining_NoAlloc is the variant that never allocates.
  *
  * Results follow the reference's CPU branches (the header-only path in include/bb), which is what
@@ -66,8 +66,9 @@ const char *bbcu_b200_error_string(int status);
 /* ABI version of this library (bumped when a signature changes). */
 int bbcu_b200_abi_version(void);
 /* Synchronises the current device and returns the first fault code one of this library's kernels recorded since the last call
- * (0 = none, 1 = a bounded wait on an asynchronous copy expired, -1 = the query itself failed).  Kernels never trap or spin
- * forever: a wait that does not complete is abandoned, recorded here, and the kernel returns. */
+ * (0 = none, 1 = a bounded wait expired, -1 = the query itself failed).  Kernels never trap or spin forever: a wait that does not complete
+ * is abandoned and recorded here, and the kernel returns.  (A wait on an asynchronous copy leaves the outputs that it was for unwritten; one of
+ * the small layers' backward on the clearing of dx makes the gradients of its node NaN.) */
 int bbcu_b200_device_fault(void);
 /* Self-test of that path: one warp waits, with a small attempt limit, on a barrier that nothing completes, gives up, records fault
  * code 1 and returns (nothing hangs, nothing faults); bbcu_b200_device_fault() then reports 1 once. */
@@ -348,7 +349,8 @@ int bbcu_fp32_DifferentiableLut6_BackwardFromOutput(const float *dev_x_buf, cons
                                                     bbcu_stream_t stream);
 
 /* Additive: bbcu_fp32_DifferentiableLut6_ForwardTraining for callers that know how many rows x has (the reference's operator is not
- * told).  Same results; a large layer in binary mode then packs its input rows to bits once instead of reading six fp32 rows per node. */
+ * told).  Same results; a layer in binary mode then packs its input rows to bits once, where that is faster, instead of reading six fp32 rows
+ * per node. */
 int bbcu_fp32_DifferentiableLut6_ForwardTrainingRows(const float *dev_x_buf, float *dev_y_buf, const int *dev_input_index, const float *dev_W,
                                                      float *dev_mean_buf, float *dev_rstd_buf, float *dev_running_mean_buf,
                                                      float *dev_running_var_buf, float gamma, float beta, float momentum, float unbinarize_bias,
