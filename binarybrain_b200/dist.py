@@ -70,11 +70,10 @@ class ShardedDifferentiableLut6:
                        (self.binary or (frames == total_frames and frames <= self.ops.SMALL_FRAMES and
                                         frames * self.n_out <= self.ops.SMALL_NODE_FRAMES)))
         if self._fused:
-            # the statistics of a probability-mode layer stay in the same two tensors whatever its size; in binary mode every step has its own
-            keep = {} if self.binary else {"mean": self.mean, "rstd": self.rstd}
-            y, self.mean, self.rstd = self.ops.differentiable_lut6_forward_training(
+            # the statistics stay in the same two tensors, as with the split operators
+            y, _, _ = self.ops.differentiable_lut6_forward_training(
                 x, self.idx, self.W, self.running_mean, self.running_var, frames, y=y, gamma=self.gamma, beta=self.beta, momentum=self.momentum,
-                lut_binarize=self.lut_binarize, binary=self.binary, **keep)
+                lut_binarize=self.lut_binarize, binary=self.binary, mean=self.mean, rstd=self.rstd)
             self._x, self._frames, self._total, self._y = x, frames, total_frames, None
             return y
         if y is None:

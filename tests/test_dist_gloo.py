@@ -163,7 +163,8 @@ def test_unsharded_layer_on_one_rank_enters_no_collective(tmp_path):
     assert np.abs(r["y"] - p["y"]).max() <= 1e-4 * max(1.0, 0.3 * float(p["rstd"].max()))
 
 
-def test_small_layers_statistics_stay_in_the_same_tensors():
+@pytest.mark.parametrize("binary", [False, True])
+def test_unsplit_layers_statistics_stay_in_the_same_tensors(binary):
     """A layer whose step is not split hands its own mean and rstd to the unsplit operator, so that what a caller holds of them does not go stale."""
     from binarybrain_b200.dist import ShardedDifferentiableLut6
 
@@ -178,7 +179,7 @@ def test_small_layers_statistics_stay_in_the_same_tensors():
             return torch.zeros(idx.shape[0], x.shape[1]), mean, rstd
 
     I, O, F, idx, W, x, dy = _case()
-    layer = ShardedDifferentiableLut6(torch.from_numpy(idx), torch.from_numpy(W), I, ops=UnsplitOps(), binary=False, sharded=False)
+    layer = ShardedDifferentiableLut6(torch.from_numpy(idx), torch.from_numpy(W), I, ops=UnsplitOps(), binary=binary, sharded=False)
     mean, rstd = layer.mean, layer.rstd
     for scale in (1.0, 0.5):
         layer.forward(torch.from_numpy(x) * scale, F, F)

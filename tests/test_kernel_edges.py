@@ -164,19 +164,20 @@ def test_im2col_quads_and_bit_columns(ops, c, h, w, fh, fw, ys, xs, pad, F):
     lowering.test_im2col_bands_and_bit_words_against_oracle(c, h, w, fh, fw, ys, xs, pad, F)
 
 
-# a layer of one launch and one of the split operators; the second step's frames are other ones
+# a layer of one launch and one of several (in probability mode: of the split operators); the second step's frames are other ones
+@pytest.mark.parametrize("binary", [False, True])
 @pytest.mark.parametrize("O,F", [(20, 300), (20, 4200)])
-def test_layer_keeps_its_statistics_tensors(ops, O, F):
+def test_layer_keeps_its_statistics_tensors(ops, O, F, binary):
     from binarybrain_b200.dist import ShardedDifferentiableLut6
     from gpu_util import dev, dev_fp32, wiring
     rng = np.random.default_rng(F)
     idx, W = wiring(rng, 30, O), np.clip(rng.normal(0.5, 0.25, (O, 64)), 0, 1).astype(np.float32)
-    layer = ShardedDifferentiableLut6(dev(idx), dev(W), 30, sharded=False)
+    layer = ShardedDifferentiableLut6(dev(idx), dev(W), 30, sharded=False, binary=binary)
     mean, rstd = layer.mean, layer.rstd
     for _ in range(2):
         x = rng.random((30, F), dtype=np.float32)
         layer.forward(dev_fp32(x), F, F)
-        want = port.dl6_forward_train(x, idx, W, np.zeros(O), np.ones(O), binary=0)
+        want = port.dl6_forward_train(x, idx, W, np.zeros(O), np.ones(O), binary=int(binary))
         assert layer.mean is mean and layer.rstd is rstd
         assert np.abs(mean.cpu().numpy() - want["mean"]).max() <= 1e-6 and np.abs(rstd.cpu().numpy() / want["rstd"] - 1).max() <= 1e-4
 
