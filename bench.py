@@ -46,14 +46,15 @@ SM_CLOCK_HZ = 1.965e9                # clocks.max.sm of the B200s of this pool
 # Algorithmic work per node-frame (one LUT evaluation) of the kernels the rooflines are quoted on, counted for the 63-interpolation
 # tree: forward 126 flops; backward 126 (recomputed forward) + 63 x 5 (reverse pass) + 64 (table-gradient sums) = 505.
 FLOPS_FWD, FLOPS_BWD = 126.0, 505.0
-# what the centred-polynomial kernels issue instead: 63 FMA forward; backward 31 + 1 FMA forward halves, 41 packed FMA + 40 packed
-# mul/add + 7 scalar operations in the reverse pass, 12 for input conditioning
-FLOPS_FWD_EXECUTED, FLOPS_BWD_EXECUTED = 126.0 + 12.0, 379.0
+# what the centred-polynomial kernels issue instead (a packed FMA is four): 63 FMA forward; backward 31 packed FMA and one scalar in the
+# forward halves, 47 packed FMA, 27 packed products and sums and 7 scalar operations in the reverse pass; 12 for conditioning the inputs
+FLOPS_FWD_EXECUTED, FLOPS_BWD_EXECUTED = 126.0 + 12.0, 4.0 * (31 + 47) + 2.0 * (1 + 27) + 7.0 + 12.0
 # dram__bytes_read.sum + dram__bytes_write.sum of one k_binary_lut6_pipe launch: ncu on a 131072-frame launch; traffic grows with frames
-NCU_BL6_TRAFFIC_BYTES_PER_FRAME = (449.7e6 + 244.6e6) / 131072
-# the same for one k_lut6_backward_pipe<BN> launch on a 65536 -> 65536 x 4096-frame layer: 11.379 GB read + 5.201 GB written for 2.68e8
-# node-frames; the tile width does not depend on the frame count, so the traffic grows in proportion to the frames of a launch
-NCU_BWD_TRAFFIC_BYTES_PER_NF = (11.379342e9 + 5.201327e9) / (65536 * 4096)
+NCU_BL6_TRAFFIC_BYTES_PER_FRAME = (457.5e6 + 244.4e6) / 131072
+# the same for one k_lut6_backward_pipe<BN> launch on a 65536 -> 65536 x 4096-frame layer: 12.325 GB read + 5.616 GB written for 2.68e8
+# node-frames.  backward_pipe_tile() gives this layer 1408-frame tiles at 4096, 8192, 16384 and 32768 frames alike, so the traffic grows in
+# proportion to the frames of a launch
+NCU_BWD_TRAFFIC_BYTES_PER_NF = (12.325492e9 + 5.616424e9) / (65536 * 4096)
 
 
 def measured_peaks():
@@ -653,17 +654,18 @@ def operators_section(torch, ops, steps):
         "sl6_forward_bit_fp32": (lambda: ops.stochastic_lut6_forward(xb, idx, W, F, y=yf), nf, 4.125, 0.0),       # per-pattern value lookup
         # bit in, bit out: evaluated as a BinaryLut6 forward with a per-node truth table (no per-frame fp32 tree), so the bound is HBM
         "sl6_forward_bit_bit": (lambda: ops.stochastic_lut6_forward(xbb, idx, W, FB, y=ybb, bit_output=True), nfb, 0.25, 0.0),
-        "sl6_backward_bit": (lambda: ops.stochastic_lut6_backward(xb, dy, idx, W, dW, I, F, dx=dx), nf, 8.125, 505.0),
+        "sl6_backward_bit": (lambda: ops.stochastic_lut6_backward(xb, dy, idx, W, dW, I, F, dx=dx), nf, 8.125, 0.0),
         "dl6_forward_training_bit": (dl_bit_fwd, nfb, 0.375, 0.0),      # x read twice (pattern histogram, then the table forward)
         "dl6_forward_inference_bit": (lambda: ops.differentiable_lut6_forward_inference(xbb, idx, W, rm, rv, FB, y=ybb), nfb, 0.25, 0.0),
         "dl6_forward_inference_fp32": (lambda: ops.differentiable_lut6_forward_inference(xf, idx, W, rm, rv, F, y=yf, binary=False), nf, 8.0, 136.0),
-        "dl6_backward_bit": (lambda: ops.differentiable_lut6_backward(xb, dy, idx, W, dW, st["mean"], st["rstd"], I, F, dx=dx), nf, 12.125, 651.0),
-        # binary mode on fp32 frames (the reference's default mode): forward by the fp32 tree, backward through the per-pattern tables
-        "dl6_forward_training_fp32_binary": (dl_binary_fwd, nf, 13.0, 0.0),     # x read, pattern byte written and read, y written
+        "dl6_backward_bit": (lambda: ops.differentiable_lut6_backward(xb, dy, idx, W, dW, st["mean"], st["rstd"], I, F, dx=dx), nf, 8.125, 0.0),
+        # binary mode on fp32 frames (the reference's default mode): per-pattern tables both ways, like the bit-input operators above, whose backward
+        # evaluates no tree per frame either: the bytes are the bound
+        "dl6_forward_training_fp32_binary": (dl_binary_fwd, nf, 8.0, 0.0),      # x read, y written
         "sl6_forward_fp32_binary": (lambda: ops.stochastic_lut6_forward(xf, idx, W, F, y=yf, binary=True), nf, 8.0, 0.0),
         "dl6_backward_fp32_binary": (lambda: ops.differentiable_lut6_backward(xf, dy, idx, W, dW, st["bmean"], st["brstd"], I, F, dx=dx, binary=True),
-                                     nf, 24.0, 651.0),
-        "sl6_backward_fp32_binary": (lambda: ops.stochastic_lut6_backward(xf, dy, idx, W, dW, I, F, dx=dx, binary=True), nf, 12.0, 505.0),
+                                     nf, 12.0, 0.0),
+        "sl6_backward_fp32_binary": (lambda: ops.stochastic_lut6_backward(xf, dy, idx, W, dW, I, F, dx=dx, binary=True), nf, 12.0, 0.0),
         "sbn_forward_training": (sbn_fwd, nf, 12.0, 8.0),
         "sbn_backward": (lambda: ops.stochastic_bn_backward(xf, dy, st["smean"], st["srstd"], F), nf, 20.0, 12.0),
         "adam_update": (lambda: adam.update(), 8.0 * 65536 * 64, 32.0, 12.0),      # W, m, v read and written, dW read, then cleared (Update = Step + ZeroGrad)

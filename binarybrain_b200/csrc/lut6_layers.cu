@@ -792,8 +792,8 @@ k_lut6_backward(const BwdArgs a)
 // Work item = (frame tile of a.T frames, group of 8 nodes), walked in tile-major order by one CTA per SM; each warp owns one node
 // of the group.  What the kernel is bound by: an SM sub-partition issues one instruction per clock and a packed f32x2
 // instruction takes two issue slots (measured: 32 packed FMAs take 65 clocks per warp, and scalar FMAs, logic ops or anything
-// else issued beside them add their own clocks in full), so the time is the weighted instruction count -- 106 packed (212
-// slots) + about 100 others per frame -- over the issue rate.  Everything here is about the "others":
+// else issued beside them add their own clocks in full), so the time is the weighted instruction count -- 105 packed (210
+// slots) + 109 others per frame with batch norm -- over the issue rate.  Everything here is about the "others":
 //   * the per-node table arrives ready to use (k_backward_prepare has converted every table once per launch);
 //   * global -> shared: a warp streams its item in 128-frame chunks through a three-stage ring; every lane copies 16 bytes (four
 //     consecutive frames) of each of the six input rows and of dy with cp.async, two chunks ahead of the arithmetic, so the
