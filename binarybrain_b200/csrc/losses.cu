@@ -180,13 +180,12 @@ extern "C" int bbcu_fp32_LossSoftmaxCrossEntropyMean(const float *y, const float
     BB200_REQUIRE(frame_stride >= frame_size, BBCU_ERR_BAD_STRIDE);
     cudaStream_t st = as_stream(stream);
     const long long rows = (long long)pix_size * ch_size;
-    if (rows * frame_size <= kOneCta) {
+    BB200_REQUIRE(rows < (1LL << 31), BBCU_ERR_TOO_LARGE);
+    double *work = rows * frame_size <= kOneCta ? nullptr : static_cast<double *>(stream_scratch(st, 2 * sizeof(double)));
+    if (work == nullptr) {                                    // (a heap that declines it: slower, not an error)
         launch(k_softmax_cross_entropy_one, 1, 1024, 0, st, y, t, dy, loss, pix_size, ch_size, frame_size, frame_stride);
         return launch_status();
     }
-    double *work = static_cast<double *>(stream_scratch(st, 2 * sizeof(double)));
-    BB200_REQUIRE(work != nullptr, BBCU_ERR_NO_MEMORY);
-    BB200_REQUIRE(rows < (1LL << 31), BBCU_ERR_TOO_LARGE);
     BB200_CUDA(cudaMemsetAsync(work, 0, 2 * sizeof(double), st));
     const unsigned bx = (unsigned)((frame_size + 2047) / 2048);
     launch(k_target_sum, dim3(bx, (unsigned)(rows < 64 ? rows : 64)), 256, 0, st, t, work, (int)rows, frame_size, frame_stride);

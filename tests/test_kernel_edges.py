@@ -260,6 +260,20 @@ def test_mean_loss_at_the_line(ops, classes, frames):
     test_mean_loss_and_adam_update(ops, classes, frames)
 
 
+def test_mean_loss_without_scratch(ops):
+    """A heap that has nothing left to give: the one block takes calls of the general form too."""
+    import torch
+    from binarybrain_b200 import abi
+    torch.cuda.synchronize()
+    abi.lib().bbcu_LocalHeap_GarbageCollect()
+    abi.lib().bbcu_LocalHeap_SetByteLimit(1)
+    try:
+        test_mean_loss_and_adam_update(ops, 10, 3277)
+        assert abi.lib().bbcu_LocalHeap_GetAllocatedSize() == 0
+    finally:
+        abi.lib().bbcu_LocalHeap_SetByteLimit(0)
+
+
 # The apply half of a frame-sharded binary-mode backward uses what the statistics half left in the stream's scratch, unless something else has
 # used or released that scratch in between, or the call is another one.
 @pytest.mark.parametrize("between", ["nothing", "another layer", "garbage collection", "another gamma", "captured"])
