@@ -41,8 +41,8 @@ TRAIN_GLOBAL_BATCH = 32768           # frames per step over all GPUs (8 GiB per 
 CPU_TRAIN_SAMPLE_FRAMES = 8          # the reference's DifferentiableLutN backward is a serial loop over nodes (~2e5 node-frames/s)
 BL6_NODES = 16384
 BL6_FRAMES = 1 << 20
-FALLBACK_HBM_GBS = 6650.0            # the pool's earlier measurement, used only when MEASURED_PEAKS.json is absent
-SM_CLOCK_HZ = 1.965e9                # clocks.max.sm of the B200s of this pool
+FALLBACK_HBM_GBS = 6650.0            # an earlier measurement, used only when MEASURED_PEAKS.json is absent
+SM_CLOCK_HZ = 1.965e9                # clocks.max.sm of the B200s measured on
 # Algorithmic work per node-frame (one LUT evaluation) of the kernels the rooflines are quoted on, counted for the 63-interpolation
 # tree: forward 126 flops; backward 126 (recomputed forward) + 63 x 5 (reverse pass) + 64 (table-gradient sums) = 505.
 FLOPS_FWD, FLOPS_BWD = 126.0, 505.0

@@ -1,7 +1,7 @@
 """TEST INFRASTRUCTURE ONLY: numpy front-ends of the CPU oracle.
 
 Only ``tests/``, ``__graft_entry__.smoke()`` and the CPU-baseline legs of ``bench.py`` may import
-this package, and only as the checker.  The product (``binarybrain_b200``) never does.
+this package, and only as the oracle.  The product (``binarybrain_b200``) never does.
 
 ``port``  : oracle/lut6_oracle.c, the plain-C restatement of the reference's CPU arithmetic.
 ``ref``   : oracle/_ref/libbbref.so, the unmodified reference headers behind oracle/ref_driver.cpp
