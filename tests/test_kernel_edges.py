@@ -266,10 +266,11 @@ def test_mean_loss_without_scratch(ops):
     from binarybrain_b200 import abi
     torch.cuda.synchronize()
     abi.lib().bbcu_LocalHeap_GarbageCollect()
+    others = abi.lib().bbcu_LocalHeap_GetAllocatedSize()                   # (what earlier tests in this process still hold)
     abi.lib().bbcu_LocalHeap_SetByteLimit(1)
     try:
         test_mean_loss_and_adam_update(ops, 10, 3277)
-        assert abi.lib().bbcu_LocalHeap_GetAllocatedSize() == 0
+        assert abi.lib().bbcu_LocalHeap_GetAllocatedSize() == others
     finally:
         abi.lib().bbcu_LocalHeap_SetByteLimit(0)
 
