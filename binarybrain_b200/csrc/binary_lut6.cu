@@ -10,6 +10,8 @@
 // contiguous bytes of each of its six rows per iteration; CTAs of consecutive node groups share a
 // word tile so the tile's input rows stay in L2 for the ~6 nodes that read each of them.
 
+#include <type_traits>
+
 #include "common.cuh"
 #include "async_copy.cuh"
 
@@ -358,169 +360,236 @@ k_binary_lut6_words(const BlArgs a)
 // lop3.b32 evaluates ANY three-input boolean function in one instruction, the function being an 8-bit immediate.  Byte b of a
 // node's 64-bit table is exactly the function of (x0, x1, x2) that applies where x3 + 2 x4 + 4 x5 = b, so a word costs eight lop3
 // with the table bytes as immediates and seven selects on x3, x4, x5: 15 logic operations instead of 63.  The immediates are
-// instruction text, so each table byte is dispatched through one indexed branch (brx.idx) into 256 case bodies that hold the
-// lop3 for all 16 words of a lane; the byte is warp-uniform (one node per warp), so the branch never diverges and its cost --
-// the branch and the instruction fetch of a cold case body -- is spread over 16 words.  The eight partial results are folded as
-// a binary counter does (s0 waits for its odd neighbour, s1 for the next pair, s2 for the upper half).  The whole per-item
-// evaluation is one asm statement: branch targets must be labels of the block that holds the table, and mutable PTX registers
-// keep the partial results in place across the eight trips.
-// Operands: %0-%15 y, %16-%31 x0, %32-%47 x1, %48-%63 x2, %64-%79 x3, %80-%95 x4, %96-%111 x5, %112 / %113 the table words.
-// Staging: every lane copies, with cp.async, the 16-byte pieces of the six rows that it will itself read, two items ahead
-// (two-stage ring per warp): no barrier and no cross-lane dependence.
+// instruction text, so each table byte is dispatched through an indexed branch (brx.idx) into 256 case bodies that hold the
+// lop3 for all eight words of a lane; they return to one tail, which goes by the byte's position and folds the partial results as
+// a binary counter does.  The byte is warp-uniform (one node per warp): the branches never diverge.  (Returning by a second indexed branch
+// took 16 % longer.)
+// What bounds it is the fetch of case bodies that are cold, and that is shared: four warps of a CTA -- one on every scheduler -- take
+// neighbouring segments of the same node at the same time.  Registers only, clocks per word and scheduler, 28 warps per SM: every warp
+// its own node 169, two sharing one 112, four 65, seven (all of a scheduler) 56, all 28 46, and four with two segments each 57; the
+// multiplexer tree of k_binary_lut6_pipe takes 106 whatever is shared.
+// The bodies write one set of registers, which costs four moves a word: with a second set of bodies for the odd bytes, 80 KiB of code in all,
+// fetching them bounds the kernel again (1000 nodes x 2^20 frames 130 us instead of 92).  16384 x 2^20: 1951 -> 1483 us, 5000 x 2^20 609 -> 414,
+// 216 x 2^20 30.3 -> 22.7; 46 instructions and 93 clocks per word and scheduler (of 127), issue 0.5, the rest latency of branches, fetches and
+// shared memory at 20 warps per SM (24 do not leave it the registers: 110 us instead of 92).
+// %0-%7 x0 and the result, %8-%15 x1, %16-%23 x2, %24 / %25 the table words, %26 the lane's first piece of x3 in shared memory; x3, x4 and x5 are
+// read there when they are needed (24 registers fewer).
 // ---------------------------------------------------------------------------------------------
-constexpr int kImmNW     = 16;                         // words per lane and item (four 128-bit pieces per row)
-constexpr int kImmWords  = 32 * kImmNW;                // words per row segment and item
-constexpr int kImmStages = 2;
-constexpr int kImmStageBytes = 6 * kImmWords * 4;
-constexpr int kImmSmem   = kBlWarps * kImmStages * kImmStageBytes;
-static_assert(kImmSmem <= 227 * 1024, "one CTA per SM must fit");
+constexpr int kImmGroup  = 4;                          // warps that share a node
+constexpr int kImmWarps  = 20;
+constexpr int kImmTile   = kImmGroup * kPipeWords;     // words of a work item, 256 for each warp of the group
+// dynamic shared memory, per warp: [x0..x2: 3 x 256 words][x3..x5: 2 x 3 x 256 words]
+constexpr int kImmHalf   = 3 * kPipeWords;
+constexpr int kImmSmem   = kImmWarps * 3 * kImmHalf * 4;
+static_assert(kPipeWords == 256 && kImmSmem <= 227 * 1024, "the row distance is in the code below; one CTA per SM");
 
 #define BB200_LOPS(imm) \
-    "lop3.b32 p0, %48, %32, %16, " imm ";\n\t" "lop3.b32 p1, %49, %33, %17, " imm ";\n\t" "lop3.b32 p2, %50, %34, %18, " imm ";\n\t" "lop3.b32 p3, %51, %35, %19, " imm ";\n\t" \
-    "lop3.b32 p4, %52, %36, %20, " imm ";\n\t" "lop3.b32 p5, %53, %37, %21, " imm ";\n\t" "lop3.b32 p6, %54, %38, %22, " imm ";\n\t" "lop3.b32 p7, %55, %39, %23, " imm ";\n\t" \
-    "lop3.b32 p8, %56, %40, %24, " imm ";\n\t" "lop3.b32 p9, %57, %41, %25, " imm ";\n\t" "lop3.b32 p10, %58, %42, %26, " imm ";\n\t" "lop3.b32 p11, %59, %43, %27, " imm ";\n\t" \
-    "lop3.b32 p12, %60, %44, %28, " imm ";\n\t" "lop3.b32 p13, %61, %45, %29, " imm ";\n\t" "lop3.b32 p14, %62, %46, %30, " imm ";\n\t" "lop3.b32 p15, %63, %47, %31, " imm ";\n\t"
-#define BB200_CASE(h, l) "T" #h #l ":\n\t" BB200_LOPS("0x" #h #l) "bra.uni TEND;\n\t"
+    "lop3.b32 p0, %16, %8, %0, " imm ";\n\tlop3.b32 p1, %17, %9, %1, " imm ";\n\tlop3.b32 p2, %18, %10, %2, " imm ";\n\tlop3.b32 p3, %19, %11, %3, " imm ";\n\t" \
+    "lop3.b32 p4, %20, %12, %4, " imm ";\n\tlop3.b32 p5, %21, %13, %5, " imm ";\n\tlop3.b32 p6, %22, %14, %6, " imm ";\n\tlop3.b32 p7, %23, %15, %7, " imm ";\n\t"
+#define BB200_CASE(h, l) "T" #h #l ":\n\t" BB200_LOPS("0x" #h #l) "bra.uni TAIL;\n\t"
 #define BB200_ROW(h)                                                                                                                        \
     BB200_CASE(h, 0) BB200_CASE(h, 1) BB200_CASE(h, 2) BB200_CASE(h, 3) BB200_CASE(h, 4) BB200_CASE(h, 5) BB200_CASE(h, 6) BB200_CASE(h, 7) \
     BB200_CASE(h, 8) BB200_CASE(h, 9) BB200_CASE(h, A) BB200_CASE(h, B) BB200_CASE(h, C) BB200_CASE(h, D) BB200_CASE(h, E) BB200_CASE(h, F)
 #define BB200_TGT(h)                                                                                                                        \
     "T" #h "0, T" #h "1, T" #h "2, T" #h "3, T" #h "4, T" #h "5, T" #h "6, T" #h "7, T" #h "8, T" #h "9, T" #h "A, T" #h "B, T" #h "C, T" #h "D, T" #h "E, T" #h "F"
+// on to the case of the lowest byte of tw
+#define BB200_DISPATCH "and.b32 byte, tw, 255;\n\tshr.u32 tw, tw, 8;\n\tbrx.idx byte, TBL;\n\t"
+#define BB200_KEEP "mov.u32 a0, p0;\n\tmov.u32 a1, p1;\n\tmov.u32 a2, p2;\n\tmov.u32 a3, p3;\n\tmov.u32 a4, p4;\n\tmov.u32 a5, p5;\n\tmov.u32 a6, p6;\n\tmov.u32 a7, p7;\n\t"
+// a row of the lane's words: u = row at `at` (second half at `at2`); d = u ? hi : lo
+#define BB200_LOAD(at, at2) "ld.shared.v4.u32 {u0, u1, u2, u3}, [%26+" at "];\n\tld.shared.v4.u32 {u4, u5, u6, u7}, [%26+" at2 "];\n\t"
+#define BB200_LOAD3 BB200_LOAD("0", "512")
+#define BB200_LOAD4 BB200_LOAD("1024", "1536")
+#define BB200_LOAD5 BB200_LOAD("2048", "2560")
+#define BB200_SELECT(d, hi, lo)                                                                                                              \
+    "lop3.b32 " d "0, u0, " hi "0, " lo "0, 0xCA;\n\tlop3.b32 " d "1, u1, " hi "1, " lo "1, 0xCA;\n\tlop3.b32 " d "2, u2, " hi "2, " lo "2, 0xCA;\n\t" \
+    "lop3.b32 " d "3, u3, " hi "3, " lo "3, 0xCA;\n\tlop3.b32 " d "4, u4, " hi "4, " lo "4, 0xCA;\n\tlop3.b32 " d "5, u5, " hi "5, " lo "5, 0xCA;\n\t" \
+    "lop3.b32 " d "6, u6, " hi "6, " lo "6, 0xCA;\n\tlop3.b32 " d "7, u7, " hi "7, " lo "7, 0xCA;\n\t"
 
-// y[w] = table[x0[w] + 2 x1[w] + 4 x2[w] + 8 x3[w] + 16 x4[w] + 32 x5[w]] bitwise, for the 16 words of a lane
-__device__ __forceinline__ void lut6_words_by_immediates(uint32_t (&y)[16], const uint32_t (&x)[6][16], uint32_t table_lo, uint32_t table_hi)
+// x[0][w] = table[x0[w] + 2 x1[w] + 4 x2[w] + 8 x3[w] + 16 x4[w] + 32 x5[w]] bitwise, for the 8 words of a lane
+__device__ __forceinline__ void lut6_words_by_immediates(uint32_t (&x)[3][8], uint32_t table_lo, uint32_t table_hi, uint32_t upper)
 {
     asm volatile(
         "{\n\t"
-        ".reg .u32 p<16>, s0_<16>, s1_<16>, s2_<16>, t<16>;\n\t"
-        ".reg .u32 b, byte, sh, tw, c;\n\t"
+        ".reg .u32 p<8>, a<8>, b<8>, c<8>, u<8>;\n\t"
+        ".reg .u32 byte, tw, i, t;\n\t"
         ".reg .pred q;\n\t"
-        "mov.u32 b, 0;\n\t"
-        "LOOP:\n\t"
-        "setp.lt.u32 q, b, 4;\n\t"
-        "selp.u32 tw, %112, %113, q;\n\t"
-        "and.b32 sh, b, 3;\n\t"
-        "shl.b32 sh, sh, 3;\n\t"
-        "shr.u32 byte, tw, sh;\n\t"
-        "and.b32 byte, byte, 255;\n\t"
         "TBL: .branchtargets " BB200_TGT(0) ", " BB200_TGT(1) ", " BB200_TGT(2) ", " BB200_TGT(3) ", " BB200_TGT(4) ", " BB200_TGT(5) ", "
         BB200_TGT(6) ", " BB200_TGT(7) ", " BB200_TGT(8) ", " BB200_TGT(9) ", " BB200_TGT(A) ", " BB200_TGT(B) ", " BB200_TGT(C) ", "
         BB200_TGT(D) ", " BB200_TGT(E) ", " BB200_TGT(F) ";\n\t"
-        "brx.idx byte, TBL;\n\t"
+        "mov.u32 i, 0;\n\t"
+        "mov.u32 tw, %24;\n\t"
+        BB200_DISPATCH
         BB200_ROW(0) BB200_ROW(1) BB200_ROW(2) BB200_ROW(3) BB200_ROW(4) BB200_ROW(5) BB200_ROW(6) BB200_ROW(7)
         BB200_ROW(8) BB200_ROW(9) BB200_ROW(A) BB200_ROW(B) BB200_ROW(C) BB200_ROW(D) BB200_ROW(E) BB200_ROW(F)
-        "TEND:\n\t"
-        "and.b32 c, b, 1;\n\t"
-        "setp.ne.u32 q, c, 0;\n\t"
+        "TAIL:\n\t"
+        "and.b32 t, i, 1;\n\t"
+        "setp.ne.u32 q, t, 0;\n\t"
         "@q bra.uni ODD;\n\t"
-        "mov.u32 s0_0, p0;\n\tmov.u32 s0_1, p1;\n\tmov.u32 s0_2, p2;\n\tmov.u32 s0_3, p3;\n\tmov.u32 s0_4, p4;\n\tmov.u32 s0_5, p5;\n\tmov.u32 s0_6, p6;\n\tmov.u32 s0_7, p7;\n\tmov.u32 s0_8, p8;\n\tmov.u32 s0_9, p9;\n\tmov.u32 s0_10, p10;\n\tmov.u32 s0_11, p11;\n\tmov.u32 s0_12, p12;\n\tmov.u32 s0_13, p13;\n\tmov.u32 s0_14, p14;\n\tmov.u32 s0_15, p15;\n\t"
-        "bra.uni NEXT;\n\t"
+        BB200_KEEP
+        BB200_LOAD3
+        "add.u32 i, i, 1;\n\t"
+        BB200_DISPATCH
         "ODD:\n\t"
-        "lop3.b32 t0, %64, p0, s0_0, 0xCA;\n\tlop3.b32 t1, %65, p1, s0_1, 0xCA;\n\tlop3.b32 t2, %66, p2, s0_2, 0xCA;\n\tlop3.b32 t3, %67, p3, s0_3, 0xCA;\n\tlop3.b32 t4, %68, p4, s0_4, 0xCA;\n\tlop3.b32 t5, %69, p5, s0_5, 0xCA;\n\tlop3.b32 t6, %70, p6, s0_6, 0xCA;\n\tlop3.b32 t7, %71, p7, s0_7, 0xCA;\n\tlop3.b32 t8, %72, p8, s0_8, 0xCA;\n\tlop3.b32 t9, %73, p9, s0_9, 0xCA;\n\tlop3.b32 t10, %74, p10, s0_10, 0xCA;\n\tlop3.b32 t11, %75, p11, s0_11, 0xCA;\n\tlop3.b32 t12, %76, p12, s0_12, 0xCA;\n\tlop3.b32 t13, %77, p13, s0_13, 0xCA;\n\tlop3.b32 t14, %78, p14, s0_14, 0xCA;\n\tlop3.b32 t15, %79, p15, s0_15, 0xCA;\n\t"
-        "and.b32 c, b, 2;\n\t"
-        "setp.ne.u32 q, c, 0;\n\t"
+        "and.b32 t, i, 2;\n\t"
+        "setp.ne.u32 q, t, 0;\n\t"
         "@q bra.uni PAIR;\n\t"
-        "mov.u32 s1_0, t0;\n\tmov.u32 s1_1, t1;\n\tmov.u32 s1_2, t2;\n\tmov.u32 s1_3, t3;\n\tmov.u32 s1_4, t4;\n\tmov.u32 s1_5, t5;\n\tmov.u32 s1_6, t6;\n\tmov.u32 s1_7, t7;\n\tmov.u32 s1_8, t8;\n\tmov.u32 s1_9, t9;\n\tmov.u32 s1_10, t10;\n\tmov.u32 s1_11, t11;\n\tmov.u32 s1_12, t12;\n\tmov.u32 s1_13, t13;\n\tmov.u32 s1_14, t14;\n\tmov.u32 s1_15, t15;\n\t"
-        "bra.uni NEXT;\n\t"
+        BB200_SELECT("b", "p", "a")
+        "add.u32 i, i, 1;\n\t"
+        BB200_DISPATCH
         "PAIR:\n\t"
-        "lop3.b32 t0, %80, t0, s1_0, 0xCA;\n\tlop3.b32 t1, %81, t1, s1_1, 0xCA;\n\tlop3.b32 t2, %82, t2, s1_2, 0xCA;\n\tlop3.b32 t3, %83, t3, s1_3, 0xCA;\n\tlop3.b32 t4, %84, t4, s1_4, 0xCA;\n\tlop3.b32 t5, %85, t5, s1_5, 0xCA;\n\tlop3.b32 t6, %86, t6, s1_6, 0xCA;\n\tlop3.b32 t7, %87, t7, s1_7, 0xCA;\n\tlop3.b32 t8, %88, t8, s1_8, 0xCA;\n\tlop3.b32 t9, %89, t9, s1_9, 0xCA;\n\tlop3.b32 t10, %90, t10, s1_10, 0xCA;\n\tlop3.b32 t11, %91, t11, s1_11, 0xCA;\n\tlop3.b32 t12, %92, t12, s1_12, 0xCA;\n\tlop3.b32 t13, %93, t13, s1_13, 0xCA;\n\tlop3.b32 t14, %94, t14, s1_14, 0xCA;\n\tlop3.b32 t15, %95, t15, s1_15, 0xCA;\n\t"
-        "and.b32 c, b, 4;\n\t"
-        "setp.ne.u32 q, c, 0;\n\t"
-        "@q bra.uni TOP;\n\t"
-        "mov.u32 s2_0, t0;\n\tmov.u32 s2_1, t1;\n\tmov.u32 s2_2, t2;\n\tmov.u32 s2_3, t3;\n\tmov.u32 s2_4, t4;\n\tmov.u32 s2_5, t5;\n\tmov.u32 s2_6, t6;\n\tmov.u32 s2_7, t7;\n\tmov.u32 s2_8, t8;\n\tmov.u32 s2_9, t9;\n\tmov.u32 s2_10, t10;\n\tmov.u32 s2_11, t11;\n\tmov.u32 s2_12, t12;\n\tmov.u32 s2_13, t13;\n\tmov.u32 s2_14, t14;\n\tmov.u32 s2_15, t15;\n\t"
-        "bra.uni NEXT;\n\t"
-        "TOP:\n\t"
-        "lop3.b32 %0, %96, t0, s2_0, 0xCA;\n\tlop3.b32 %1, %97, t1, s2_1, 0xCA;\n\tlop3.b32 %2, %98, t2, s2_2, 0xCA;\n\tlop3.b32 %3, %99, t3, s2_3, 0xCA;\n\tlop3.b32 %4, %100, t4, s2_4, 0xCA;\n\tlop3.b32 %5, %101, t5, s2_5, 0xCA;\n\tlop3.b32 %6, %102, t6, s2_6, 0xCA;\n\tlop3.b32 %7, %103, t7, s2_7, 0xCA;\n\tlop3.b32 %8, %104, t8, s2_8, 0xCA;\n\tlop3.b32 %9, %105, t9, s2_9, 0xCA;\n\tlop3.b32 %10, %106, t10, s2_10, 0xCA;\n\tlop3.b32 %11, %107, t11, s2_11, 0xCA;\n\tlop3.b32 %12, %108, t12, s2_12, 0xCA;\n\tlop3.b32 %13, %109, t13, s2_13, 0xCA;\n\tlop3.b32 %14, %110, t14, s2_14, 0xCA;\n\tlop3.b32 %15, %111, t15, s2_15, 0xCA;\n\t"
-        "NEXT:\n\t"
-        "add.u32 b, b, 1;\n\t"
-        "setp.lt.u32 q, b, 8;\n\t"
-        "@q bra.uni LOOP;\n\t"
+        BB200_SELECT("p", "p", "a")
+        BB200_LOAD4
+        "setp.eq.u32 q, i, 7;\n\t"
+        "@q bra.uni LAST;\n\t"
+        BB200_SELECT("c", "p", "b")
+        "mov.u32 tw, %25;\n\t"
+        "mov.u32 i, 4;\n\t"
+        BB200_DISPATCH
+        "LAST:\n\t"
+        BB200_SELECT("p", "p", "b")
+        BB200_LOAD5
+        BB200_SELECT("%", "p", "c")
         "}"
-        : "=&r"(y[0]), "=&r"(y[1]), "=&r"(y[2]), "=&r"(y[3]), "=&r"(y[4]), "=&r"(y[5]), "=&r"(y[6]), "=&r"(y[7]), "=&r"(y[8]), "=&r"(y[9]), "=&r"(y[10]), "=&r"(y[11]), "=&r"(y[12]), "=&r"(y[13]), "=&r"(y[14]), "=&r"(y[15])
-        : "r"(x[0][0]), "r"(x[0][1]), "r"(x[0][2]), "r"(x[0][3]), "r"(x[0][4]), "r"(x[0][5]), "r"(x[0][6]), "r"(x[0][7]), "r"(x[0][8]), "r"(x[0][9]), "r"(x[0][10]), "r"(x[0][11]), "r"(x[0][12]), "r"(x[0][13]), "r"(x[0][14]), "r"(x[0][15]), "r"(x[1][0]), "r"(x[1][1]), "r"(x[1][2]), "r"(x[1][3]), "r"(x[1][4]), "r"(x[1][5]), "r"(x[1][6]), "r"(x[1][7]), "r"(x[1][8]), "r"(x[1][9]), "r"(x[1][10]), "r"(x[1][11]), "r"(x[1][12]), "r"(x[1][13]), "r"(x[1][14]), "r"(x[1][15]), "r"(x[2][0]), "r"(x[2][1]), "r"(x[2][2]), "r"(x[2][3]), "r"(x[2][4]), "r"(x[2][5]), "r"(x[2][6]), "r"(x[2][7]), "r"(x[2][8]), "r"(x[2][9]), "r"(x[2][10]), "r"(x[2][11]), "r"(x[2][12]), "r"(x[2][13]), "r"(x[2][14]), "r"(x[2][15]), "r"(x[3][0]), "r"(x[3][1]), "r"(x[3][2]), "r"(x[3][3]), "r"(x[3][4]), "r"(x[3][5]), "r"(x[3][6]), "r"(x[3][7]), "r"(x[3][8]), "r"(x[3][9]), "r"(x[3][10]), "r"(x[3][11]), "r"(x[3][12]), "r"(x[3][13]), "r"(x[3][14]), "r"(x[3][15]), "r"(x[4][0]), "r"(x[4][1]), "r"(x[4][2]), "r"(x[4][3]), "r"(x[4][4]), "r"(x[4][5]), "r"(x[4][6]), "r"(x[4][7]), "r"(x[4][8]), "r"(x[4][9]), "r"(x[4][10]), "r"(x[4][11]), "r"(x[4][12]), "r"(x[4][13]), "r"(x[4][14]), "r"(x[4][15]), "r"(x[5][0]), "r"(x[5][1]), "r"(x[5][2]), "r"(x[5][3]), "r"(x[5][4]), "r"(x[5][5]), "r"(x[5][6]), "r"(x[5][7]), "r"(x[5][8]), "r"(x[5][9]), "r"(x[5][10]), "r"(x[5][11]), "r"(x[5][12]), "r"(x[5][13]), "r"(x[5][14]), "r"(x[5][15]), "r"(table_lo), "r"(table_hi));
+        : "+r"(x[0][0]), "+r"(x[0][1]), "+r"(x[0][2]), "+r"(x[0][3]), "+r"(x[0][4]), "+r"(x[0][5]), "+r"(x[0][6]), "+r"(x[0][7])
+        : "r"(x[1][0]), "r"(x[1][1]), "r"(x[1][2]), "r"(x[1][3]), "r"(x[1][4]), "r"(x[1][5]), "r"(x[1][6]), "r"(x[1][7]),
+          "r"(x[2][0]), "r"(x[2][1]), "r"(x[2][2]), "r"(x[2][3]), "r"(x[2][4]), "r"(x[2][5]), "r"(x[2][6]), "r"(x[2][7]),
+          "r"(table_lo), "r"(table_hi), "r"(upper)
+        : "memory");
 }
 #undef BB200_LOPS
 #undef BB200_CASE
 #undef BB200_ROW
 #undef BB200_TGT
+#undef BB200_DISPATCH
+#undef BB200_KEEP
+#undef BB200_SELECT
+#undef BB200_LOAD
+#undef BB200_LOAD3
+#undef BB200_LOAD4
+#undef BB200_LOAD5
 
-__global__ void __launch_bounds__(kBlWarps * 32, 1)
-k_binary_lut6_imm(const BlArgs a, int n_tiles)
+// Persistent: a group of four warps takes (tile of 1024 words, node) items in tile-major order, each warp a segment of 256 words.  x0..x2 go to
+// registers at the start of an item, and the copies of the next item's follow at once; x3..x5 are used from shared memory, in two buffers.
+// Every lane copies, with cp.async, the 16-byte pieces that it will itself read: no barrier and no cross-lane dependence.
+__global__ void __launch_bounds__(kImmWarps * 32, 1)
+k_binary_lut6_imm(const BlArgs a)
 {
     grid_dependency();
     extern __shared__ __align__(128) unsigned char smem_raw[];
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-    uint32_t *my = reinterpret_cast<uint32_t *>(smem_raw) + (size_t)warp * kImmStages * 6 * kImmWords;
-
-    const int step = (int)gridDim.x;
-    const int dt = step / a.groups, dg = step - dt * a.groups;
-    PipePos pi;                                        // copy side: two items ahead (an item is a CTA's: `node` counts groups of nodes)
-    pi.tile  = (int)blockIdx.x / a.groups;
-    pi.node = (int)blockIdx.x - pi.tile * a.groups;
-    PipePos pc = pi;                                   // arithmetic side
-    int row_i = pi.tile < n_tiles ? pipe_row(a, min(pi.node * kBlWarps + warp, a.O - 1), lane) : 0;
-    int row_n;
-    {
-        const PipePos t = pipe_advance(pi, dt, dg, a.groups);
-        row_n = t.tile < n_tiles ? pipe_row(a, min(t.node * kBlWarps + warp, a.O - 1), lane) : 0;
-    }
-    int ist = 0;
-    auto issue = [&]() {
-        if (pi.tile < n_tiles) {
-            const int w0 = pi.tile * kImmWords + 4 * lane;
-            uint32_t *st = my + ist * 6 * kImmWords + 4 * lane;
-#pragma unroll
-            for (int j = 0; j < 6; ++j) {
-                const uint32_t *src = a.x + (size_t)__shfl_sync(0xffffffffu, row_i, j) * a.stride + w0;
-#pragma unroll
-                for (int h = 0; h < kImmNW / 4; ++h) {
-                    const bool in_row = w0 + 128 * h < a.nwords;
-                    cp_async16(st + j * kImmWords + 128 * h, in_row ? src + 128 * h : a.x, in_row);
-                }
+    constexpr int kGroups = kImmWarps / kImmGroup;
+    const int segment = (warp % kImmGroup) * kPipeWords;
+    const uint32_t lower = smem_addr(smem_raw) + (uint32_t)warp * 3 * kImmHalf * 4 + 16 * lane, upper = lower + kImmHalf * 4;
+    const int tiles = a.nwords > segment ? (a.nwords - segment - 1) / kImmTile + 1 : 0;      // tiles that have words for this warp, and
+    const int whole = (a.nwords + kImmTile - kPipeWords - segment) / kImmTile;               // those in which it has all 256
+    const int step = (int)gridDim.x * kGroups, first = (int)blockIdx.x * kGroups + warp / kImmGroup;
+    // A node's run is a.Tw tiles (a power of two); the runs of a group are `first`, first + step, ...
+    const int dt = step / a.O, dn = step - dt * a.O, last = a.Tw - 1;
+    auto advance = [&](PipePos p) {
+        if ((p.tile & last) != last && p.tile + 1 < tiles) {
+            ++p.tile;
+            return p;
+        }
+        p.tile = (p.tile & ~last) + dt * a.Tw;
+        p.node += dn;
+        if (p.node >= a.O) { p.node -= a.O; p.tile += a.Tw; }
+        return p;
+    };
+    PipePos p0;
+    p0.tile = first / a.O;
+    p0.node = first - p0.tile * a.O;
+    p0.tile *= a.Tw;
+    // three rows, from input `J` on, of item p to `dst`; lane j of `row` holds the item's input row j
+    const uint32_t row_bytes = (uint32_t)a.stride * 4u;
+    const uint64_t mine = (uint64_t)__cvta_generic_to_global(a.x) + (uint64_t)(segment + 4 * lane) * 4;
+    auto issue = [&](const PipePos &p, int row, auto j_tag, uint32_t dst) {
+        constexpr int J = decltype(j_tag)::value;
+        if (p.tile < tiles) {
+            const uint64_t base = mine + (uint64_t)(uint32_t)p.tile * (kImmTile * 4);
+            const uint64_t s0 = base + (uint64_t)(uint32_t)__shfl_sync(0xffffffffu, row, J) * row_bytes,
+                           s1 = base + (uint64_t)(uint32_t)__shfl_sync(0xffffffffu, row, J + 1) * row_bytes,
+                           s2 = base + (uint64_t)(uint32_t)__shfl_sync(0xffffffffu, row, J + 2) * row_bytes;
+            if (p.tile < whole) {
+                cp_async16_at<0, 0>(dst, s0); cp_async16_at<512, 512>(dst, s0);
+                cp_async16_at<1024, 0>(dst, s1); cp_async16_at<1536, 512>(dst, s1);
+                cp_async16_at<2048, 0>(dst, s2); cp_async16_at<2560, 512>(dst, s2);
+            } else {
+                const int w0 = p.tile * kImmTile + segment + 4 * lane;
+                if (w0 < a.nwords) { cp_async16_at<0, 0>(dst, s0); cp_async16_at<1024, 0>(dst, s1); cp_async16_at<2048, 0>(dst, s2); }
+                if (w0 + 128 < a.nwords) { cp_async16_at<512, 512>(dst, s0); cp_async16_at<1536, 512>(dst, s1); cp_async16_at<2560, 512>(dst, s2); }
             }
-            pi = pipe_advance(pi, dt, dg, a.groups);
-            row_i = row_n;
-            const PipePos t = pipe_advance(pi, dt, dg, a.groups);
-            row_n = t.tile < n_tiles ? pipe_row(a, min(t.node * kBlWarps + warp, a.O - 1), lane) : 0;
         }
         cp_async_commit();
-        ist ^= 1;
     };
-    issue();
-    issue();
-
-    uint2 tab_n = make_uint2(0u, 0u);                   // the node's 64-bit table, one item ahead of its use
-    if (pc.tile < n_tiles) tab_n = __ldg(reinterpret_cast<const uint2 *>(a.table) + min(pc.node * kBlWarps + warp, a.O - 1));
-    int cst = 0;
-    while (pc.tile < n_tiles) {
-        const int node = pc.node * kBlWarps + warp;
-        const bool store = node < a.O;
-        const int w0 = pc.tile * kImmWords;
-        const uint2 tab = tab_n;
-        const PipePos pn = pipe_advance(pc, dt, dg, a.groups);
-        if (pn.tile < n_tiles) tab_n = __ldg(reinterpret_cast<const uint2 *>(a.table) + min(pn.node * kBlWarps + warp, a.O - 1));
-
-        cp_async_wait<1>();                             // the copies of this item (this lane's own pieces) have landed
-        const uint32_t *st = my + cst * 6 * kImmWords + 4 * lane;
-        cst ^= 1;
-        uint32_t x[6][kImmNW], y[kImmNW];
+    using Lo = std::integral_constant<int, 0>;
+    using Hi = std::integral_constant<int, 3>;
+    PipePos p1 = advance(p0);
+    int row1 = 0, row2 = 0;                              // input rows of items k + 1 and k + 2 (lanes 0..5)
+    uint2 table = make_uint2(0u, 0u);
+    {
+        const int row0 = p0.tile < tiles ? pipe_row(a, p0.node, lane) : 0;
+        if (p1.tile < tiles) row1 = pipe_row(a, p1.node, lane);
+        issue(p0, row0, Hi{}, upper);
+        issue(p0, row0, Lo{}, lower);
+        issue(p1, row1, Hi{}, upper + kImmHalf * 4);
+    }
+    if (p0.tile < tiles) table = make_uint2((uint32_t)__ldg(a.table + 2 * (size_t)p0.node), (uint32_t)__ldg(a.table + 2 * (size_t)p0.node + 1));
+    PipePos p2 = advance(p1);
+    if (p2.tile < tiles) row2 = pipe_row(a, p2.node, lane);
+    uint32_t buf = upper;
+    while (p0.tile < tiles) {
+        cp_async_wait<1>();                              // all but the newest copies, which are item k + 1's x3..x5
+        uint32_t x[3][8];
 #pragma unroll
-        for (int j = 0; j < 6; ++j) {
+        for (int j = 0; j < 3; ++j) {
 #pragma unroll
-            for (int h = 0; h < kImmNW / 4; ++h) {
-                const uint4 v = *reinterpret_cast<const uint4 *>(st + j * kImmWords + 128 * h);
-                x[j][4 * h] = v.x; x[j][4 * h + 1] = v.y; x[j][4 * h + 2] = v.z; x[j][4 * h + 3] = v.w;
-            }
+            for (int h = 0; h < 2; ++h)
+                asm volatile("ld.shared.v4.u32 {%0, %1, %2, %3}, [%4];" : "=r"(x[j][4 * h]), "=r"(x[j][4 * h + 1]), "=r"(x[j][4 * h + 2]), "=r"(x[j][4 * h + 3])
+                             : "r"(lower + 1024 * j + 512 * h) : "memory");
         }
-        issue();                                        // refills the stage just read (each lane overwrites only what it has read itself)
-        lut6_words_by_immediates(y, x, tab.x, tab.y);
-        uint32_t *yrow = a.y + (size_t)min(node, a.O - 1) * a.stride + w0 + 4 * lane;
+        issue(p1, row1, Lo{}, lower);
+        const uint2 tab = table;
+        if (p1.tile < tiles) table = make_uint2((uint32_t)__ldg(a.table + 2 * (size_t)p1.node), (uint32_t)__ldg(a.table + 2 * (size_t)p1.node + 1));
+        lut6_words_by_immediates(x, tab.x, tab.y, buf);
+        issue(p2, row2, Hi{}, buf);
+        buf = buf == upper ? upper + kImmHalf * 4 : upper;
+        const int w = p0.tile * kImmTile + segment + 4 * lane;
+        uint32_t *yrow = a.y + (size_t)p0.node * a.stride + w;
 #pragma unroll
-        for (int h = 0; h < kImmNW / 4; ++h)
-            if (store && w0 + 4 * lane + 128 * h < a.nwords) *reinterpret_cast<uint4 *>(yrow + 128 * h) = make_uint4(y[4 * h], y[4 * h + 1], y[4 * h + 2], y[4 * h + 3]);
-        pc = pn;
+        for (int h = 0; h < 2; ++h)
+            if (w + 128 * h < a.nwords) *reinterpret_cast<uint4 *>(yrow + 128 * h) = make_uint4(x[0][4 * h], x[0][4 * h + 1], x[0][4 * h + 2], x[0][4 * h + 3]);
+        p0 = p1; p1 = p2; row1 = row2;
+        p2 = advance(p2);
+        if (p2.tile < tiles) row2 = pipe_row(a, p2.node, lane);
     }
     cp_async_wait<0>();
+}
+
+// Rounds of the persistent grid that the call takes (a round: every group of every SM one tile of a node).
+long long imm_rounds(const BlArgs &a)
+{
+    const long long groups = (long long)(kImmWarps / kImmGroup) * device_info().sm_count;
+    return ((a.nwords + kImmTile - 1) / kImmTile * (long long)a.O + groups - 1) / groups;
+}
+
+// Tiles that a group takes of a node before the next node.  Two halve the case bodies to fetch, but the rows of both, 8 KiB a node, have to stay
+// in L2, and they make the rounds coarser: 8192 nodes x 2^20 frames 982 us by k_binary_lut6_pipe, 727 with one tile, 668 with two, 796 with
+// four; 20000 x 2^18 606, 467, 479, 618; 318 x 56770 (one round) 4.5, 4.6, 5.9, 5.9.
+int imm_run(const BlArgs &a) { return imm_rounds(a) >= 8 && 2LL * kImmTile * 4 * a.O <= (long long)(device_info().l2_bytes / 10 * 9) ? 2 : 1; }
+
+// What the kernel's 32-bit arithmetic can take.
+bool imm_fits(const BlArgs &a)
+{
+    return a.stride < (1 << 30) && ((long long)a.nwords / kImmTile + 2) * a.O < (1LL << 31) - 65536 && allow_big_smem(k_binary_lut6_imm, kImmSmem);
+}
+
+int launch_immediate(BlArgs a, cudaStream_t st)
+{
+    a.Tw = imm_run(a);
+    const long long tiles = (a.nwords + kImmTile - 1) / kImmTile, runs = (tiles + a.Tw - 1) / a.Tw * a.O, groups = kImmWarps / kImmGroup;
+    const long long grid = (runs + groups - 1) / groups;
+    launch(k_binary_lut6_imm, (unsigned)(grid < device_info().sm_count ? grid : device_info().sm_count), kImmWarps * 32, kImmSmem, st, a);
+    return launch_status();
 }
 
 }   // namespace bb200
@@ -553,6 +622,13 @@ extern "C" int bbcu_bit_BinaryLut6_Forward(const int *x, int *y, const int *idx,
         launch(k_binary_lut6_words, (unsigned)((node_words + kWordThreads - 1) / kWordThreads), kWordThreads, 0, as_stream(stream), a);
         return launch_status();
     }
+    // The table bytes as immediates where the rounds of its grid (four warps and 1024 words each) are hardly more than those of the pipeline (a warp and
+    // 256 words), which take a little longer: at 1.05 times as many both sides are even (22916 nodes x 71132 frames 202 / 200 us, 4164 x 32966, at
+    // 1.33, 23.9 / 26.5); below three rounds neither wins, and its cold case bodies cost up to 0.5 us.
+    if (vec) {
+        const long long rounds_pipe = ((long long)((a.nwords + kPipeWords - 1) / kPipeWords) * node_size + warps - 1) / warps;
+        if (rounds_pipe >= 3 && 20 * imm_rounds(a) <= 21 * rounds_pipe && imm_fits(a)) return launch_immediate(a, as_stream(stream));
+    }
     if (vec) {
         // persistent pipeline: two CTAs per SM, each warp of which walks (tile, node) items
         const bool attr_ok = allow_big_smem(k_binary_lut6_pipe, kPipeSmem);
@@ -577,10 +653,8 @@ extern "C" int bbcu_bit_BinaryLut6_Forward(const int *x, int *y, const int *idx,
     return launch_status();
 }
 
-// The same operator through the truth-table-immediate kernel (k_binary_lut6_imm).  Kept as an entry point of its own because it is the
-// formulation with the fewest logic operations (15 per word against 63) and nevertheless the slower one on B200 -- its case
-// bodies are fetched cold from the instruction cache on every dispatch -- so that the comparison stays measurable.  Rows must be
-// 16-byte aligned (stride a multiple of 4 words, aligned base pointers).
+// The same operator through the truth-table-immediate kernel whatever the size.  Rows must be 16-byte aligned (stride a multiple of 4 words,
+// aligned base pointers).
 extern "C" int bbcu_bit_BinaryLut6_Forward_Lop3Immediate(const int *x, int *y, const int *idx, const int *table, int node_size, int frame_size,
                                                          int frame_stride, bbcu_stream_t stream)
 {
@@ -594,16 +668,10 @@ extern "C" int bbcu_bit_BinaryLut6_Forward_Lop3Immediate(const int *x, int *y, c
     a.x = reinterpret_cast<const uint32_t *>(x); a.y = reinterpret_cast<uint32_t *>(y); a.idx = idx; a.table = table;
     a.O = node_size; a.stride = frame_stride;
     a.nwords = ((frame_size + 31) / 32 + 3) & ~3;
-    a.groups = (node_size + kBlWarps - 1) / kBlWarps;
-    a.Tw = kImmWords;
-    BB200_REQUIRE(allow_big_smem(k_binary_lut6_imm, kImmSmem), BBCU_ERR_TOO_LARGE);
-    const int n_tiles = (a.nwords + kImmWords - 1) / kImmWords;
-    const long long n_items = (long long)n_tiles * a.groups;
-    BB200_REQUIRE(n_items < (1LL << 31) - 4096, BBCU_ERR_TOO_LARGE);
-    long long grid = device_info().sm_count;
-    if (grid > n_items) grid = n_items;
-    launch(k_binary_lut6_imm, (unsigned)grid, kBlWarps * 32, kImmSmem, as_stream(stream), a, n_tiles);
-    return launch_status();
+    a.groups = 0;
+    a.Tw = 0;
+    BB200_REQUIRE(imm_fits(a), BBCU_ERR_TOO_LARGE);
+    return launch_immediate(a, as_stream(stream));
 }
 
 extern "C" int bbcu_bit_BinatyLut6_Forward(const int *x, int *y, const int *idx, const int *table, int node_size, int frame_size,

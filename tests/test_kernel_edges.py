@@ -55,6 +55,26 @@ def test_binary_lut6_words_and_pipeline(ops, n_in, n_out, frames, stride):
     assert ((y.cpu().numpy().view(np.uint32)[:, :words] ^ want[:, :words]) & live == 0).all()
 
 
+# table bytes as immediates: one quad of words, a segment and a quad, whole tiles and a part of one; two tiles a node, the last run of one tile (2000 nodes)
+@pytest.mark.parametrize("n_in,n_out,words,spare", [(6, 1, 1, 5), (9, 13, 260, 0), (64, 777, 1024, 3), (50, 37, 2051, 31), (300, 1501, 1300, 1), (300, 2000, 3 * 1024 - 2, 9)])
+def test_binary_lut6_by_immediates(ops, n_in, n_out, words, spare):
+    import torch
+    from gpu_util import dev, wiring
+    rng = np.random.default_rng(words)
+    F, stride = words * 32 - spare, (words + 3) // 4 * 4 + 4
+    x = rng.integers(-2**31, 2**31, (n_in, stride), dtype=np.int64).astype(np.int32)
+    idx, table = wiring(rng, n_in, n_out), rng.integers(-2**31, 2**31, (n_out, 2), dtype=np.int64).astype(np.int32)
+    table[0] = [0x03020100, 0x7f80feff]
+    want = port.binary_lut6_forward(x.view(np.uint32), idx, table, F)
+    live = np.full(words, 0xffffffff, np.uint32)
+    live[-1] >>= spare
+    for forced in (True, False):
+        y = torch.full((n_out, stride), 0x5a5a5a5a, dtype=torch.int32, device="cuda")
+        y = ops.binary_lut6_forward(dev(x), dev(idx), dev(table), F, y=y, lop3_immediate=forced).cpu().numpy().view(np.uint32)
+        assert ((y[:, :words] ^ want[:, :words]) & live == 0).all()
+        assert (y[:, (words + 3) // 4 * 4:] == 0x5a5a5a5a).all()
+
+
 # one chunk, a first and a last chunk only, full-width chunks with a one-word remainder
 @pytest.mark.parametrize("n_in,n_out,words,spare", [(9, 7, 1, 0), (700, 400, 130, 30), (4096, 64, 257, 31), (1024, 1100, 1793, 5)])
 def test_binary_lut6_host_chunks(ops, n_in, n_out, words, spare):
