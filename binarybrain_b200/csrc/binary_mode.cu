@@ -277,7 +277,7 @@ struct BitBwdArgs {
     const int *heavy_count;
     int heavy_from, heavy_chunk, heavy_ctas;
     int I, O, F, groups, tile_frames, tiles, nc, split;
-    int vec;                            // dy and dx (and fp32 x) rows start on 16-byte boundaries
+    int vec, xvec;                      // dy and dx (and fp32 x) rows start on 16-byte boundaries; bit-packed x rows do
     long long xs, fs, ps;               // word stride of x, float stride of dy / dx, stride of pat
 };
 
@@ -329,7 +329,9 @@ k_pack_bits(const float *__restrict__ x, uint32_t *__restrict__ bits, int I, int
 // -- column `lane` of [64 patterns][32 lanes], free of bank conflicts and of atomics -- and the columns are added up once per tile.
 // (Float atomics on one shared histogram per warp, compare-and-swap loops in hardware, took 0.68 ms for 8192 nodes x 16384 frames.)
 // Shared memory takes four clocks per warp and 32 frames (a 64-bit load and store per frame), about as long as reading dy takes; with
-// only 12 warps per SM (16 KiB of columns each) the loads have to be far ahead, so 512 frames of dy are in flight per warp.
+// only 12 warps per SM (16 KiB of columns each) the loads have to be far ahead: 512 frames of dy are in flight per warp, and the lines of the 512 after
+// them on their way to L2 (186 -> 166 us under ncu for 8192 x 8192 nodes x 16384 frames; four loads of a word instead of one of four 195; reading dy
+// and writing the patterns takes 105 at HBM speed.  One or two warps a CTA: 172 to 179).
 constexpr int kPsWarps = 4;
 template <bool BN> struct PatternSlot { float s; uint32_t n; };      // n: count, bit 31: the pattern's mask bit
 template <> struct PatternSlot<false> { float s; };
@@ -402,25 +404,30 @@ k_pattern_sums(const BitBwdArgs a)
     int f = f_begin + 4 * lane;
     if constexpr (!XF32) {
         // 512 frames per step while whole steps are left; the loads of the next step are issued before this one is used, into the
-        // other of two sets of registers
+        // other of two sets of registers.  Here a lane's frames are those of four neighbouring words of x, four of each, so that a row's words
+        // come with one 128-bit load instead of four loads (and dy and the patterns still in whole 128 and 32 bytes).
         constexpr int NC = 4, kStep = 128 * NC;
-        struct Set { uint32_t w[NC][6]; float4 dy[NC]; };
-        const int steps = a.vec ? (f_end - f_begin) / kStep : 0;
+        struct Set { uint4 w[6]; float4 dy[NC]; };
+        const int steps = a.vec && a.xvec ? (f_end - f_begin) / kStep : 0;
+        const int fl = f_begin + 128 * (lane >> 3) + 4 * (lane & 7);
         auto fetch = [&](Set &b, int k) {
             if (k < steps) {
+                if (lane < 16 && k + 2 < steps) asm volatile("prefetch.global.L2 [%0];" ::"l"(dyrow + f_begin + (k + 2) * kStep + 32 * lane));
 #pragma unroll
-                for (int c = 0; c < NC; ++c) {
+                for (int j = 0; j < 6; ++j) b.w[j] = __ldg(reinterpret_cast<const uint4 *>(rows[j] + ((fl + k * kStep) >> 5)));
 #pragma unroll
-                    for (int j = 0; j < 6; ++j) b.w[c][j] = __ldg(rows[j] + ((f + k * kStep) >> 5) + 4 * c);
-                    b.dy[c] = __ldg(reinterpret_cast<const float4 *>(dyrow + f + k * kStep + 128 * c));
-                }
+                for (int c = 0; c < NC; ++c) b.dy[c] = __ldg(reinterpret_cast<const float4 *>(dyrow + fl + k * kStep + 32 * c));
             }
         };
         auto use = [&](const Set &b, int k) {
             if (k < steps) {
 #pragma unroll
-                for (int c = 0; c < NC; ++c)
-                    *reinterpret_cast<uint32_t *>(prow + f + k * kStep + 128 * c) = pattern_columns_add<BN>(mine, pattern_bytes(b.w[c], lane), b.dy[c], 4);
+                for (int c = 0; c < NC; ++c) {
+                    uint32_t w[6];
+#pragma unroll
+                    for (int j = 0; j < 6; ++j) w[j] = c == 0 ? b.w[j].x : c == 1 ? b.w[j].y : c == 2 ? b.w[j].z : b.w[j].w;
+                    *reinterpret_cast<uint32_t *>(prow + fl + k * kStep + 32 * c) = pattern_columns_add<BN>(mine, pattern_bytes(w, lane), b.dy[c], 4);
+                }
             }
         };
         Set s0, s1;
@@ -1468,7 +1475,7 @@ bool input_side(BitBwdArgs &a, int I, bool x_is_fp32, bool packed, cudaStream_t 
     a.I = I;
     gather_shape(a);
     const int edges = 6 * a.O;
-    const long long ws = (a.F + 31) / 32;
+    const long long ws = ((long long)a.F + 127) / 128 * 4;                  // whole 16-byte pieces
     // a heavy row has more than heavy_from >= 2 heavy_chunk consumers, so its chunks number at most 3 / 2 of its consumers over heavy_chunk
     const size_t heavy_most = (size_t)edges / (size_t)a.heavy_chunk * 3 / 2 + 2;
     const size_t list_bytes = (heavy_most * sizeof(int2) + (2 * (size_t)I + 2 + (size_t)edges) * sizeof(int) + 255) & ~(size_t)255;
@@ -1500,6 +1507,7 @@ template <bool XF32>
 int launch_pattern_sums(BitBwdArgs a, bool bn, cudaStream_t st)
 {
     a.groups = (a.O + kPsWarps - 1) / kPsWarps;
+    a.xvec = (reinterpret_cast<uintptr_t>(a.x) & 15) == 0 && a.xs % 4 == 0;
     if (XF32) a.vec = a.vec && (reinterpret_cast<uintptr_t>(a.x) & 15) == 0 && a.xs % 4 == 0;
     long long tile = ((long long)a.F + 127) / 128 * 128;
     while (tile > 1024 && (long long)a.O * ((a.F + tile - 1) / tile) < 24LL * device_info().sm_count) tile = (tile / 2 + 127) / 128 * 128;
