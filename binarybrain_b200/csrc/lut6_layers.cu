@@ -200,7 +200,7 @@ k_lut6_forward(const FwdArgs a)
 // flight.  (Bulk copies with an mbarrier did the same with seven copy instructions per item, but each of them cost five moves
 // into uniform registers plus the election of the issuing lane: a fifth of the kernel's issue slots.)
 // The table normally arrives ready to use: a small kernel in front (k_table_coeffs) has turned every node's 64 entries
-// into the 32 x (c0, c0, c1, c1) packed-operand form once per launch, so no warp repeats that butterfly (ten shuffles
+// into coefficients in the half-packed form once per launch, so no warp repeats that butterfly (ten shuffles
 // in a dependent chain) for every item.  Tables have a ring of three slots per warp because the table of item j is
 // still being read while the copies of item j+2 are started.  Without the scratch table (a.coef == nullptr) the raw
 // entries are copied instead and converted in place.
@@ -211,7 +211,7 @@ constexpr int kFpStages        = 2;
 constexpr int kFpStageBytes    = 6 * kFpMaxItemFrames * 4;                             // six row segments
 constexpr int kFpRowsBytes     = kWarpsPerCta * kFpStages * kFpStageBytes;
 constexpr int kFpTabSlots      = 3;
-constexpr int kFpTabSlotBytes  = 32 * 16;
+constexpr int kFpTabSlotBytes  = 16 * 16;
 constexpr int kFpTabBytes      = kWarpsPerCta * kFpTabSlots * kFpTabSlotBytes;
 constexpr int kFpSmem          = kFpRowsBytes + kFpTabBytes;
 static_assert(kFpCtas * (kFpSmem + 1024) <= 227 * 1024, "the CTAs of one SM must fit");
@@ -281,14 +281,13 @@ __device__ __forceinline__ void fp_issue(const FwdArgs &a, FpPos pos, bool exist
                 }
             }
         }
-        if (a.coef)         cp_async16(tab_slot + 16 * lane, a.coef + (size_t)node * 32 + lane, true);
-        else if (lane < 16) cp_async16(tab_slot + 16 * lane, a.W + (size_t)node * 64 + 4 * lane, true);
+        if (lane < 16) cp_async16(tab_slot + 16 * lane, a.coef ? a.coef + (size_t)node * 16 + lane : reinterpret_cast<const float4 *>(a.W + (size_t)node * 64) + lane, true);
     }
     cp_async_commit();
 }
 
-// Every node's table as 32 x (c0, c0, c1, c1): the polynomial coefficients, each duplicated for the two halves of a packed operand.  On the
-// way it clears the node's batch sums, when there are any.
+// Every node's table in the half-packed form of lut6_forward_halves: 16 x (c[2k], c[2k+32], c[2k+1], c[2k+33]).  On the way it clears the node's
+// batch sums, when there are any.
 __global__ void __launch_bounds__(kWarpsPerCta * 32)
 k_table_coeffs(const float *__restrict__ W, float4 *__restrict__ coef, double *__restrict__ sums, int O, int lut_binarize)
 {
@@ -299,7 +298,8 @@ k_table_coeffs(const float *__restrict__ W, float4 *__restrict__ coef, double *_
     float2 v = reinterpret_cast<const float2 *>(W + (size_t)node * 64)[lane];
     if (lut_binarize) { v.x = v.x > 0.5f ? 1.0f : 0.0f; v.y = v.y > 0.5f ? 1.0f : 0.0f; }
     v = table_to_coeffs(v, lane);
-    coef[(size_t)node * 32 + lane] = make_float4(v.x, v.x, v.y, v.y);
+    const float hx = __shfl_down_sync(kFull, v.x, 16), hy = __shfl_down_sync(kFull, v.y, 16);
+    if (lane < 16) coef[(size_t)node * 16 + lane] = make_float4(v.x, hx, v.y, hy);
     if (sums != nullptr && lane < 2) sums[2 * (size_t)node + lane] = 0.0;
 }
 
@@ -357,12 +357,13 @@ k_lut6_forward_pipe(const FwdArgs a, int n_tiles)
         float4 *tab = reinterpret_cast<float4 *>(my_tabs + ts * kFpTabSlotBytes);
         unsigned char *tab_refill = my_tabs + (ts == 0 ? 2 : ts - 1) * kFpTabSlotBytes;      // slot (k + 2) mod 3, last read by item k - 1
         ts = ts == 2 ? 0 : ts + 1;
-        if (a.coef == nullptr) {   // raw W[64] arrived: convert in place to 32 x (c0, c0, c1, c1)
+        if (a.coef == nullptr) {   // raw W[64] arrived: convert in place
             float2 v = reinterpret_cast<const float2 *>(tab)[lane];
             if (a.lut_binarize) { v.x = v.x > 0.5f ? 1.0f : 0.0f; v.y = v.y > 0.5f ? 1.0f : 0.0f; }
             v = table_to_coeffs(v, lane);
+            const float hx = __shfl_down_sync(kFull, v.x, 16), hy = __shfl_down_sync(kFull, v.y, 16);
             __syncwarp();
-            tab[lane] = make_float4(v.x, v.x, v.y, v.y);
+            if (lane < 16) tab[lane] = make_float4(v.x, hx, v.y, hy);
             __syncwarp();
         }
         double s1 = 0.0, s2 = 0.0;
@@ -370,53 +371,48 @@ k_lut6_forward_pipe(const FwdArgs a, int n_tiles)
         float *yrow = PHASE == PH_BWD ? nullptr : a.y + (size_t)node * a.ys + f0 + 4 * lane;
         const float *dyrow = PHASE == PH_BWD ? a.dy + (size_t)node * a.dys + f0 + 4 * lane : nullptr;
         const float rstd2 = scale * scale;                 // PH_BWD
-        // One walk of the tree carries NP frame pairs per lane.  A lane owns four consecutive frames of every 128 (frames 128h + 4 lane
-        // + 0..3, h < NP/2; pairs (0, 1) and (2, 3)), so its inputs come out of shared memory with one 128-bit load per row and half and
-        // its outputs leave with one 128-bit store per half: 4 pairs when the item is 256 frames wide, 2 pairs for a 128-frame item.
+        // A lane owns four consecutive frames of every 128 (frames 128 h + 4 lane + 0..3), so its inputs come out of shared memory with one
+        // 128-bit load per row and half and its outputs leave with one 128-bit store per half.  Both halves of the table travel in the two
+        // halves of packed operands: the coefficients are read once for four frames, and every node of a level shares the operand of its
+        // input, which counts: a packed FMA with three operands that are not the one before's takes three clocks, with two 2.4
+        // (registers have two read ports).  The tree alone takes 80 clocks per frame and scheduler this way, 95 with frame pairs in the packed
+        // operands and the coefficients duplicated.
         const FpPos p3 = fp_advance(p2, dt, dg, a.groups);
-        auto walk = [&](auto np_tag) {
-            constexpr int NP = decltype(np_tag)::value;
-            f32x2 up[6][NP], yp[NP];
-            float g4[NP / 2][4];                                   // PH_BWD: dy of the lane's frames, fetched ahead of the tree
-            if (PHASE == PH_BWD) {
+        auto walk = [&](auto nh_tag) {
+            constexpr int NH = decltype(nh_tag)::value;
 #pragma unroll
-                for (int h = 0; h < NP / 2; ++h) {
-                    const int fl = 128 * h + 4 * lane;
+            for (int h = 0; h < NH; ++h) {
+                const int fl = 128 * h + 4 * lane;                 // first of the lane's four frames, relative to the item
+                float g4[4];                                       // PH_BWD: dy of the lane's frames, fetched ahead of the tree
+                if (PHASE == PH_BWD) {
                     if (fl + 3 < nf) {
                         const float4 q = __ldg(reinterpret_cast<const float4 *>(dyrow + 128 * h));
-                        g4[h][0] = q.x; g4[h][1] = q.y; g4[h][2] = q.z; g4[h][3] = q.w;
+                        g4[0] = q.x; g4[1] = q.y; g4[2] = q.z; g4[3] = q.w;
                     } else {
 #pragma unroll
-                        for (int i = 0; i < 4; ++i) g4[h][i] = fl + i < nf ? __ldg(dyrow + 128 * h + i) : 0.0f;
+                        for (int i = 0; i < 4; ++i) g4[i] = fl + i < nf ? __ldg(dyrow + 128 * h + i) : 0.0f;
                     }
                 }
-            }
+                float4 r[6];
 #pragma unroll
-            for (int j = 0; j < 6; ++j) {
-#pragma unroll
-                for (int h = 0; h < NP / 2; ++h) {
-                    const float4 r = *reinterpret_cast<const float4 *>(xs0 + j * kFpMaxItemFrames + 128 * h + 4 * lane);
-                    // the same values as condition_u()
-                    if (BINARY) {
-                        up[j][2 * h]     = pack2(r.x > 0.5f ? a.bias : -a.bias, r.y > 0.5f ? a.bias : -a.bias);
-                        up[j][2 * h + 1] = pack2(r.z > 0.5f ? a.bias : -a.bias, r.w > 0.5f ? a.bias : -a.bias);
-                    } else {
-                        up[j][2 * h]     = pack2(__saturatef(r.x) - 0.5f, __saturatef(r.y) - 0.5f);
-                        up[j][2 * h + 1] = pack2(__saturatef(r.z) - 0.5f, __saturatef(r.w) - 0.5f);
-                    }
+                for (int j = 0; j < 6; ++j) r[j] = *reinterpret_cast<const float4 *>(xs0 + j * kFpMaxItemFrames + 128 * h + 4 * lane);
+                if (h == NH - 1) {
+                    // the stage has been read out: hand it back to the copies of item k+2 before the last of the math
+                    __syncwarp();
+                    fp_issue(a, p2, p2.tile < n_tiles, row2, warp, lane, stage, tab_refill);
+                    if (p3.tile < n_tiles) row2 = fp_row(a, p3, warp, lane);
                 }
-            }
-            // the stage has been read out: hand it back to the copy engine for item k+2 before doing the math
-            __syncwarp();
-            fp_issue(a, p2, p2.tile < n_tiles, row2, warp, lane, stage, tab_refill);
-            if (p3.tile < n_tiles) row2 = fp_row(a, p3, warp, lane);
-            lut6_forward_x2<NP>(tab, up, yp);
-#pragma unroll
-            for (int h = 0; h < NP / 2; ++h) {
                 float v[4];
-                unpack2(yp[2 * h], v[0], v[1]);
-                unpack2(yp[2 * h + 1], v[2], v[3]);
-                const int fl = 128 * h + 4 * lane;                 // first of the lane's four frames, relative to the item
+#pragma unroll
+                for (int i = 0; i < 4; ++i) {
+                    float u[6];
+#pragma unroll
+                    for (int j = 0; j < 6; ++j) {
+                        const float xv = i == 0 ? r[j].x : i == 1 ? r[j].y : i == 2 ? r[j].z : r[j].w;
+                        u[j] = BINARY ? (xv > 0.5f ? a.bias : -a.bias) : __saturatef(xv) - 0.5f;           // the same values as condition_u()
+                    }
+                    v[i] = lut6_forward_halves(tab, u);
+                }
 #pragma unroll
                 for (int i = 0; i < 4; ++i) {
                     if (PHASE == PH_STATS) {
@@ -424,7 +420,7 @@ k_lut6_forward_pipe(const FwdArgs a, int n_tiles)
                     } else if (PHASE == PH_BWD) {
                         if (store && fl + i < nf) {                // DifferentiableLutN.h:1190-1215, as k_lut6_backward_stats
                             const float tanh_x = ((v[i] - mean) * scale) * a.gamma + a.beta;
-                            float g = g4[h][i];
+                            float g = g4[i];
                             if (tanh_x <= 0.0f || tanh_x >= 1.0f) g = 0.0f;
                             const float dxn = a.gamma * g;
                             s1 -= (double)(dxn * (v[i] - mean) * rstd2);
@@ -449,8 +445,8 @@ k_lut6_forward_pipe(const FwdArgs a, int n_tiles)
                 }
             }
         };
-        if (kFpMaxItemFrames > kFramesPerIter && nf > kFramesPerIter) walk(std::integral_constant<int, kFpMaxItemFrames / 64>());
-        else                                                          walk(std::integral_constant<int, 2>());
+        if (nf > kFramesPerIter) walk(std::integral_constant<int, kFpMaxItemFrames / kFramesPerIter>());
+        else                     walk(std::integral_constant<int, 1>());
         if (PHASE == PH_STATS || PHASE == PH_BWD) {
             // both sums in one butterfly: the lower half of the lanes goes on with s1, the upper half with s2 (two full ones, twice the
             // shuffles, took 4.5 % of the kernel: 1.24 -> 1.19 ms for 65536 nodes x 4096 frames)
