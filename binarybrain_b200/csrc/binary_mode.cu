@@ -1204,7 +1204,11 @@ k_small_binary_backward(const SmallBinArgs a, const GridClear clear)
 // 129 / 115; and however few the nodes, a CTA works through its frames alone: 64 x 16384 125 / 64.
 bool small_layer(int O, int F) { return (long long)O * F <= kSmallLayer && F <= 4096; }
 
+// The forward's registers leave an SM 64 warps: as many as there are rounds of frames.  Of the backward it holds 24, and a wave costs about as much as a
+// round, 2.7 us (sweep of 58 layers with 1, 2, 3, 4 and 8 warps; as many warps as rounds -> this rule, in us: 1024 nodes x 512 frames 14.6 -> 12.3,
+// 982 x 1670 35.6 -> 28.9, 550 x 927 16.3 -> 13.8, 3428 x 415 28.4 -> 25.9, 2816 x 596 34.1 -> 28.6).
 unsigned small_threads(int F) { return 32u * (unsigned)(F > 128 * kWarpsPerCta ? kWarpsPerCta : (F + 127) / 128); }
+unsigned small_backward_threads(int O, int F) { return small_layer_threads(O, F, 24, 27, 27); }
 
 struct Scratch {
     float    *Y;        // [O][64]
@@ -1594,7 +1598,7 @@ int bit_backward_by_table(bool bn, bool x_is_fp32, const void *x, const float *d
         if (rcc) return rcc;
         auto kern = x_is_fp32 ? (bn ? k_small_binary_backward<false, true> : k_small_binary_backward<false, false>)
                               : (bn ? k_small_binary_backward<true, true> : k_small_binary_backward<true, false>);
-        launch(kern, O, small_threads(F), 0, st, a, clear);
+        launch(kern, O, small_backward_threads(O, F), 0, st, a, clear);
         return launch_status();
     }
     BitBwdArgs a;

@@ -100,6 +100,11 @@ struct SmallLayerArgs {
 };
 constexpr long long kSmallProbability = BBCU_B200_SMALL_NODE_FRAMES;       // see small_probability_layer()
 bool small_probability_layer(int O, int F);
+
+// Threads of the one-launch kernels, whose CTA is a node with all of its frames (four a lane and round): a warp for every 128 frames, up to
+// eight, or fewer that take several rounds, so that more nodes share an SM and the layer takes fewer waves of CTAs.  A wave costs `fixed` and each of its
+// rounds `per_round`; `sm_warps`: warps of the kernel that an SM holds (at least eight).
+unsigned small_layer_threads(int O, int F, int sm_warps, int fixed, int per_round);
 int small_forward(int mode, const SmallLayerArgs &a, int O, cudaStream_t st);
 int small_backward(bool bn, const SmallLayerArgs &a, int I, int O, cudaStream_t st);
 

@@ -264,9 +264,27 @@ k_lut6_small_backward(const SmallLayerArgs a, const GridClear clear)
     }
 }
 
-unsigned threads_for(int F) { return 32u * (unsigned)(F > 128 * kWarpsPerCta ? kWarpsPerCta : (F + 127) / 128); }
+// Registers leave an SM 20 warps of the forward kernels and 8 of the backward ones.  In units of 0.1 us a wave of the forward costs about 20 and 6 a
+// round, of the backward 23 and 18 (a sweep of 58 layers with 1, 2, 4 and 8 warps; forward / backward in us, as many warps as rounds -> this rule:
+// 1024 nodes x 512 frames 7.8 / 17.8 -> 6.2 / 14.1, 4096 x 512 21.6 / 57 -> 16.8 / 43.7, 3015 x 260 14.7 / 43 -> 12.3 / 29, 982 x 1670 19.6 / 54 ->
+// 14.1 / 37.8, 420 x 512 4.0 / 10.4 -> 3.9 / 9.3; on the worst layer 10 % from the best count).
+unsigned forward_threads(int O, int F)  { return small_layer_threads(O, F, 20, 20, 6); }
+unsigned backward_threads(int O, int F) { return small_layer_threads(O, F, 8, 23, 18); }
 
 }   // namespace
+
+unsigned small_layer_threads(int O, int F, int sm_warps, int fixed, int per_round)
+{
+    const int all = F > 128 * kWarpsPerCta ? kWarpsPerCta : (F + 127) / 128;                 // warps that one round of frames keeps busy
+    int best = all;
+    long long best_cost = -1;
+    for (int w = all; w >= 1; --w) {
+        const long long slots = (long long)device_info().sm_count * (sm_warps / w), rounds = (F + 128 * w - 1) / (128 * w);
+        const long long cost = (O + slots - 1) / slots * (fixed + per_round * rounds);
+        if (best_cost < 0 || cost < best_cost) { best = w; best_cost = cost; }
+    }
+    return 32u * (unsigned)best;
+}
 
 // Measured on B200 against the persistent kernels, training forward / batch-normalised backward of a layer: 360 nodes x 100 frames 6 / 9 us
 // (18 / 33), 1024 x 512 10 / 21 (20 / 46), 4096 x 512 24 / 60 (34 / 80), 2048 x 1000 27 / 72 (33 / 81; 64 from the saved output): even at
@@ -275,7 +293,7 @@ bool small_probability_layer(int O, int F) { return O > 0 && F > 0 && (long long
 
 int small_forward(int mode, const SmallLayerArgs &a, int O, cudaStream_t st)
 {
-    const unsigned threads = threads_for(a.F);
+    const unsigned threads = forward_threads(O, a.F);
     if (mode == kSmallTrain) {
         const int round = 4 * (int)threads;
         launch(k_lut6_small_forward<kSmallTrain>, O, threads, (a.F + round - 1) / round * round * (int)sizeof(float), st, a);
@@ -292,8 +310,8 @@ int small_backward(bool bn, const SmallLayerArgs &a, int I, int O, cudaStream_t 
     GridClear clear;
     const int rc = grid_clear_setup(clear, a.dx, (size_t)I * (size_t)a.fs, st);
     if (rc) return rc;
-    if (bn) launch(k_lut6_small_backward<true>, O, threads_for(a.F), 0, st, a, clear);
-    else    launch(k_lut6_small_backward<false>, O, threads_for(a.F), 0, st, a, clear);
+    if (bn) launch(k_lut6_small_backward<true>, O, backward_threads(O, a.F), 0, st, a, clear);
+    else    launch(k_lut6_small_backward<false>, O, backward_threads(O, a.F), 0, st, a, clear);
     return launch_status();
 }
 

@@ -148,6 +148,13 @@ def test_small_probability_layers_edges(ops, I, O, F, stride):
     parity._dl6_fp32_check(ops, x, idx, W, dy, rng.random(O, dtype=np.float32), rng.random(O, dtype=np.float32) + 0.5, dict(binary=0, lut_binarize=0), stride)
 
 
+# many nodes: CTAs of fewer warps than rounds of 128 frames, of whole and of ragged rounds, aligned rows and others
+@pytest.mark.parametrize("I,O,F,stride", [(60, 1300, 701, None), (33, 3100, 259, 263)])
+def test_small_layers_of_several_rounds(ops, I, O, F, stride):
+    test_small_probability_layers_edges(ops, I, O, F, stride)
+    test_two_valued_layers_edges(ops, I, O, F, stride)
+
+
 # above the one-launch range: persistent kernels (tile remainders, a short last group of nodes, one and several chunks of the statistics), rows that are not aligned
 @pytest.mark.parametrize("I,O,F,stride", [(6, 1, 4097, None), (33, 17, 4225, 4228), (33, 17, 4225, 4227), (700, 1025, 2049, None), (9, 5, 20011, None)])
 def test_large_probability_layers_edges(ops, I, O, F, stride):
