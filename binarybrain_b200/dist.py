@@ -66,12 +66,12 @@ class ShardedDifferentiableLut6:
         """x: this rank's [n_in, stride] shard with `frames` valid frames; total_frames: frames of the whole step."""
         # One rank needs no exchange point: the unsplit operators, which take the per-pattern table route in binary mode and run a small
         # layer in one launch.  (A large layer in probability mode keeps the split operators, whose backward reads the saved output.)
-        self._fused = (hasattr(self.ops, "differentiable_lut6_forward_training") and self.world == 1 and
-                       (self.binary or (frames == total_frames and frames <= self.ops.SMALL_FRAMES and
-                                        frames * self.n_out <= self.ops.SMALL_NODE_FRAMES)))
+        ops = self.ops
+        self._fused = (hasattr(ops, "differentiable_lut6_forward_training") and (not self.sharded or self.world == 1) and
+                       (self.binary or (frames == total_frames and frames <= ops.SMALL_FRAMES and frames * self.n_out <= ops.SMALL_NODE_FRAMES)))
         if self._fused:
             # the statistics stay in the same two tensors, as with the split operators
-            y, _, _ = self.ops.differentiable_lut6_forward_training(
+            y, _, _ = ops.differentiable_lut6_forward_training(
                 x, self.idx, self.W, self.running_mean, self.running_var, frames, y=y, gamma=self.gamma, beta=self.beta, momentum=self.momentum,
                 lut_binarize=self.lut_binarize, binary=self.binary, mean=self.mean, rstd=self.rstd)
             self._x, self._frames, self._total, self._y = x, frames, total_frames, None
@@ -91,10 +91,11 @@ class ShardedDifferentiableLut6:
     def backward(self, dy, dx=None):
         """Returns dx for this rank's frames; dW (local partial) is all-reduced asynchronously -- call wait_grad() before using it."""
         x, frames, total = self._x, self._frames, self._total
-        kw = dict(gamma=self.gamma, beta=self.beta, lut_binarize=self.lut_binarize, binary=self.binary)
         if getattr(self, "_fused", False):
             self._x = None
-            return self.ops.differentiable_lut6_backward(x, dy, self.idx, self.W, self.dW, self.mean, self.rstd, self.n_in, frames, dx=dx, **kw)
+            return self.ops.differentiable_lut6_backward(x, dy, self.idx, self.W, self.dW, self.mean, self.rstd, self.n_in, frames, dx=dx, gamma=self.gamma,
+                                                         beta=self.beta, lut_binarize=self.lut_binarize, binary=self.binary)
+        kw = dict(gamma=self.gamma, beta=self.beta, lut_binarize=self.lut_binarize, binary=self.binary)
         if dx is None:
             dx = torch.empty((self.n_in, dy.shape[1]), dtype=torch.float32, device=dy.device)
         if self._y is not None and self._y.shape[1] == dy.shape[1]:

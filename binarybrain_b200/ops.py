@@ -107,20 +107,16 @@ def stochastic_lut6_backward(x, dy, idx, W, dW, n_in, frames, dx=None, binary=Fa
 def differentiable_lut6_forward_training(x, idx, W, running_mean, running_var, frames, y=None, gamma=0.3, beta=0.5, momentum=0.9,
                                          bias=BIAS, lut_binarize=False, binary=True, mean=None, rstd=None):
     """Returns (y, mean, rstd), in `mean` and `rstd` where they are given; running_mean / running_var are updated in place.  Bit x gives bit y."""
+    if x.dtype == torch.float32:
+        return _n.train_forward(x, y, idx, W, mean, rstd, running_mean, running_var, gamma, beta, momentum, bias, frames, lut_binarize, binary)
+    _chk(x, torch.int32, "x")
     O = idx.shape[0]
     mean = _n.vector_f32(x, O) if mean is None else mean
     rstd = _n.vector_f32(x, O) if rstd is None else rstd
-    if x.dtype == torch.float32:
-        if y is None:
-            y = _n.empty_f32(x, O, x.shape[1])
-        _n.bbcu_fp32_DifferentiableLut6_ForwardTrainingRows(x, y, idx, W, mean, rstd, running_mean, running_var, gamma, beta, momentum, bias,
-                                                            x.shape[0], O, frames, x.shape[1], int(lut_binarize), int(binary))
-    else:
-        _chk(x, torch.int32, "x")
-        if y is None:
-            y = _bits(x, O, frames, x.shape[1])
-        _n.bbcu_bit_fp32_DifferentiableLut6_ForwardTraining(x, y, idx, W, mean, rstd, running_mean, running_var, gamma, beta, momentum, bias, O,
-                                                            frames, x.shape[1], int(lut_binarize))
+    if y is None:
+        y = _bits(x, O, frames, x.shape[1])
+    _n.bbcu_bit_fp32_DifferentiableLut6_ForwardTraining(x, y, idx, W, mean, rstd, running_mean, running_var, gamma, beta, momentum, bias, O, frames,
+                                                        x.shape[1], int(lut_binarize))
     return y, mean, rstd
 
 
@@ -142,6 +138,8 @@ def differentiable_lut6_forward_inference(x, idx, W, running_mean, running_var, 
 
 def differentiable_lut6_backward(x, dy, idx, W, dW, mean, rstd, n_in, frames, dx=None, gamma=0.3, beta=0.5, bias=BIAS, lut_binarize=False,
                                  binary=True, dx_tmp=None):
+    if dx_tmp is None and x.dtype == torch.float32:
+        return _n.train_backward(x, dy, dx, idx, W, dW, mean, rstd, gamma, beta, bias, n_in, frames, lut_binarize, binary)
     O = idx.shape[0]
     if dx is None:
         dx = _n.empty_f32(dy, n_in, dy.shape[1])
@@ -151,8 +149,7 @@ def differentiable_lut6_backward(x, dy, idx, W, dW, mean, rstd, n_in, frames, dx
     if x.dtype == torch.float32:
         assert x.shape[1] == dy.shape[1]
         _n.bbcu_fp32_DifferentiableLut6_Backward(x, dy, dx, dx_tmp, idx, 0, W, dW, mean, rstd, dmean, dvar, gamma, beta, bias, 0, n_in, O, frames,
-                                                 dy.shape[1], 0 if dx_tmp is None else dx_tmp.shape[1], 0 if dx_tmp is None else dx_tmp.shape[1],
-                                                 int(lut_binarize), int(binary))
+                                                 dy.shape[1], dx_tmp.shape[1], dx_tmp.shape[1], int(lut_binarize), int(binary))
     else:
         _n.bbcu_bit_fp32_DifferentiableLut6_Backward(x, dy, dx, 0, idx, 0, W, dW, mean, rstd, dmean, dvar, gamma, beta, bias, 0, n_in, O, frames,
                                                      dy.shape[1], x.shape[1], 0, 0, int(lut_binarize))
@@ -219,8 +216,9 @@ def clamp_(t, lo=0.0, hi=1.0):
 
 def softmax_cross_entropy(y, t, frames, pix_size=1):
     """bb::LossSoftmaxCrossEntropy::CalculateLoss: returns (dy, loss) with loss = -sum(loss_buf) / t_sum (the mean over frames)."""
-    dy, loss = _n.empty_f32(y, y.shape[0], y.shape[1]), _n.scalar_f64(y)
-    _n.bbcu_fp32_LossSoftmaxCrossEntropyMean(y, t, dy, loss, pix_size, y.shape[0] // pix_size, frames, y.shape[1])
+    rows, stride = y.shape
+    dy, loss = _n.empty_f32(y, rows, stride), _n.scalar_f64(y)
+    _n.bbcu_fp32_LossSoftmaxCrossEntropyMean(y, t, dy, loss, pix_size, rows // pix_size, frames, stride)
     return dy, loss
 
 
@@ -238,16 +236,18 @@ def mean_squared_error(y, t, frames, batch_size=None, loss_buf=None, dy=None):
 
 def reduce_forward(x, out_nodes, frames, y=None):
     """bb::Reduce forward: y[o] = mean_i x[out_nodes * i + o]."""
+    rows, stride = x.shape
     if y is None:
-        y = _n.empty_f32(x, out_nodes, x.shape[1])
-    _n.bbcu_fp32_Reduce_Forward(x, y, x.shape[0], out_nodes, frames, x.shape[1], y.shape[1])
+        y = _n.empty_f32(x, out_nodes, stride)
+    _n.bbcu_fp32_Reduce_Forward(x, y, rows, out_nodes, frames, stride, y.shape[1])
     return y
 
 
 def reduce_backward(dy, in_nodes, frames, dx=None):
+    rows, stride = dy.shape
     if dx is None:
-        dx = _n.empty_f32(dy, in_nodes, dy.shape[1])
-    _n.bbcu_fp32_Reduce_Backward(dy, dx, in_nodes, dy.shape[0], frames, dy.shape[1], dx.shape[1])
+        dx = _n.empty_f32(dy, in_nodes, stride)
+    _n.bbcu_fp32_Reduce_Backward(dy, dx, in_nodes, rows, frames, stride, dx.shape[1])
     return dx
 
 
