@@ -181,6 +181,21 @@ def test_mean_loss_and_adam_update(ops, classes, frames):
         assert np.abs(Wd.cpu().numpy() - W).max() <= 1e-6 and not dWd.any()
 
 
+# a frame per thread (up to 16 classes and 1024 frames): one class, all sixteen and one more, whole and ragged warps, one block's frames and one more;
+# frames with one target above 0, several and none
+@pytest.mark.parametrize("classes,frames", [(1, 33), (2, 1), (16, 1024), (16, 1025), (17, 64), (10, 100)])
+def test_mean_loss_of_weighted_targets(ops, classes, frames):
+    from gpu_util import dev_fp32, host_fp32
+    rng = np.random.default_rng(classes * frames)
+    y = (rng.standard_normal((classes, frames)) * 4).astype(np.float32)
+    t = (rng.random((classes, frames)) * (rng.random((classes, frames)) < 1.5 / classes)).astype(np.float32)
+    t[0, 0] = 0.75
+    dy, loss = ops.softmax_cross_entropy(dev_fp32(y), dev_fp32(t), frames)
+    dy_w, loss_w = port.softmax_cross_entropy(y, t)
+    # both sides form a frame's loss in fp32, each to 8 ulp of it (exponentials, their sum, the quotient, its logarithm, the weight): 16 * 2^-24 of the sum
+    assert np.abs(host_fp32(dy, frames) - dy_w).max() <= 1e-6 and abs(float(loss.item()) - loss_w) <= 16 * 2**-24 * max(1.0, abs(loss_w))
+
+
 # Im2Col by quads of pixels (filters 3 and 5 wide, one band and several, a short last band, every border) and bit Im2Col with several word columns
 # a block, several periods a warp, split blocks, windows beyond four and words without any
 @pytest.mark.parametrize("c,h,w,fh,fw,ys,xs,pad,F", [
