@@ -992,6 +992,8 @@ k_small_binary_forward(const SmallBinArgs a)
     size_t rows[6];
 #pragma unroll
     for (int j = 0; j < 6; ++j) rows[j] = (size_t)__ldg(a.idx + (size_t)node * 6 + j) * a.xs;
+    const int f_first = 4 * (int)threadIdx.x;
+    const uint32_t p_first = small_patterns<XBIT>(a, rows, f_first, lane);       // under way while the table is evaluated, and kept for the output
     float y0 = 0.0f, y1 = 0.0f;
     if (warp == 0) {
         s_cnt[lane] = 0u;
@@ -1009,8 +1011,8 @@ k_small_binary_forward(const SmallBinArgs a)
     }
     __syncthreads();
     const int step = 4 * (int)blockDim.x;
-    for (int f = 4 * (int)threadIdx.x; f < a.F; f += step) {
-        const uint32_t p4 = small_patterns<XBIT>(a, rows, f, lane);
+    for (int f = f_first; f < a.F; f += step) {
+        const uint32_t p4 = f == f_first ? p_first : small_patterns<XBIT>(a, rows, f, lane);
 #pragma unroll
         for (int i = 0; i < 4; ++i)
             if (f + i < a.F) atomicAdd(&s_cnt[(p4 >> (8 * i)) & 63u], 1u);
@@ -1041,7 +1043,7 @@ k_small_binary_forward(const SmallBinArgs a)
     const uint32_t lo = s_table[0], hi = s_table[1];
     for (int base = 4 * 32 * warp; base < a.F; base += step) {               // warp-uniform: bit outputs shuffle
         const int f = base + 4 * lane;
-        const uint32_t p4 = small_patterns<XBIT>(a, rows, f, lane);
+        const uint32_t p4 = f == f_first ? p_first : small_patterns<XBIT>(a, rows, f, lane);
         uint32_t bits = 0u;
 #pragma unroll
         for (int i = 0; i < 4; ++i) {
@@ -1086,8 +1088,13 @@ k_small_binary_backward(const SmallBinArgs a, const GridClear clear)
     for (int j = 0; j < 6; ++j) {
         const size_t r = (size_t)__ldg(a.idx + (size_t)node * 6 + j);
         rows[j] = r * a.xs;
-        out[j] = r * a.fs;
+        out[j] = XBIT ? r * a.fs : rows[j];                                     // fp32 x shares the stride of dx
     }
+    const float *dyrow = a.dy + (size_t)node * a.fs;
+    // under way while the patterns are evaluated, and kept for the second pass
+    const int f_first = 4 * (int)threadIdx.x;
+    const uint32_t p_first = small_patterns<XBIT>(a, rows, f_first, lane);
+    const float4 g_first = load_frames(dyrow, f_first, a.F, a.vec);
     float y[2], d[2][6], mean = 0.0f, rstd = 0.0f;
     bool m[2] = {false, false};
     if (warp == 0) {
@@ -1113,11 +1120,10 @@ k_small_binary_backward(const SmallBinArgs a, const GridClear clear)
     }
     grid_clear_slices(clear);
     __syncthreads();
-    const float *dyrow = a.dy + (size_t)node * a.fs;
     const int step = 4 * (int)blockDim.x;
-    for (int f = 4 * (int)threadIdx.x; f < a.F; f += step) {
-        const uint32_t p4 = small_patterns<XBIT>(a, rows, f, lane);
-        const float4 g = load_frames(dyrow, f, a.F, a.vec);
+    for (int f = f_first; f < a.F; f += step) {
+        const uint32_t p4 = f == f_first ? p_first : small_patterns<XBIT>(a, rows, f, lane);
+        const float4 g = f == f_first ? g_first : load_frames(dyrow, f, a.F, a.vec);
         const float gv[4] = {g.x, g.y, g.z, g.w};
 #pragma unroll
         for (int i = 0; i < 4; ++i)
@@ -1168,8 +1174,8 @@ k_small_binary_backward(const SmallBinArgs a, const GridClear clear)
     const uint32_t mask_lo = BN ? s_mask[0] : 0u, mask_hi = BN ? s_mask[1] : 0u;
     for (int f_warp = 4 * 32 * warp; f_warp < a.F; f_warp += step) {
         const int f = f_warp + 4 * lane;
-        const uint32_t p4 = small_patterns<XBIT>(a, rows, f, lane);
-        const float4 gq = load_frames(dyrow, f, a.F, a.vec);
+        const uint32_t p4 = f == f_first ? p_first : small_patterns<XBIT>(a, rows, f, lane);
+        const float4 gq = f == f_first ? g_first : load_frames(dyrow, f, a.F, a.vec);
         float g[4] = {gq.x, gq.y, gq.z, gq.w};
         const uint32_t q2[2] = {__byte_perm(p4, 0u, 0x4140) * 65u, __byte_perm(p4, 0u, 0x4342) * 65u};
         if (BN) {
