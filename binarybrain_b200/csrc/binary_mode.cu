@@ -569,6 +569,7 @@ __device__ __forceinline__ void pattern_gather(const BitBwdArgs &a, const int *l
         }
 #pragma unroll
         for (int c = 0; c < NC; ++c) {
+            if (!WHOLE && f0 - 4 * lane + 128 * c >= a.F) break;           // no frame of the chunk exists
             const float dyv[4] = {dyq[c].x, dyq[c].y, dyq[c].z, dyq[c].w};
             const uint32_t rot = ((q4[c] >> (j + 1)) & low) | ((q4[c] << (5 - j)) & ~low);        // (bits 6 and 7 of the bytes: anything)
 #pragma unroll
