@@ -47,13 +47,20 @@ k_conv_bit_to_real(const uint32_t *__restrict__ x, float *__restrict__ y, float 
     float *yr = y + (size_t)node * y_stride;
     const int f0 = chunk * kFbChunk, f1 = min(frame_size, f0 + kFbChunk);
     if (vec) {
-        for (int f = f0 + 4 * threadIdx.x; f < f1; f += 1024) {
-            const uint32_t w = __ldg(xr + (f >> 5)) >> (f & 31);          // f is a multiple of 4: the four bits sit in one word
+        uint32_t w[kFbChunk / 1024];                                     // a thread's words first, then its stores
+#pragma unroll
+        for (int k = 0; k < kFbChunk / 1024; ++k) {
+            const int f = f0 + 4 * (int)threadIdx.x + 1024 * k;
+            w[k] = f < f1 ? __ldg(xr + (f >> 5)) >> (f & 31) : 0u;       // f is a multiple of 4: the four bits sit in one word
+        }
+#pragma unroll
+        for (int k = 0; k < kFbChunk / 1024; ++k) {
+            const int f = f0 + 4 * (int)threadIdx.x + 1024 * k;
             if (f + 3 < f1) {
-                *reinterpret_cast<float4 *>(yr + f) = make_float4((w & 1u) ? value1 : value0, (w & 2u) ? value1 : value0, (w & 4u) ? value1 : value0,
-                                                                  (w & 8u) ? value1 : value0);
+                *reinterpret_cast<float4 *>(yr + f) = make_float4((w[k] & 1u) ? value1 : value0, (w[k] & 2u) ? value1 : value0, (w[k] & 4u) ? value1 : value0,
+                                                                  (w[k] & 8u) ? value1 : value0);
             } else {
-                for (int i = 0; f + i < f1; ++i) yr[f + i] = ((w >> i) & 1u) ? value1 : value0;
+                for (int i = 0; f + i < f1; ++i) yr[f + i] = ((w[k] >> i) & 1u) ? value1 : value0;
             }
         }
     } else {
