@@ -286,8 +286,7 @@ __device__ __forceinline__ void fp_issue(const FwdArgs &a, FpPos pos, bool exist
     cp_async_commit();
 }
 
-// Every node's table in the half-packed form of lut6_forward_halves: 16 x (c[2k], c[2k+32], c[2k+1], c[2k+33]).  On the way it clears the node's
-// batch sums, when there are any.
+// Every node's table in the half-packed form of lut6_forward_halves.  On the way it clears the node's batch sums, when there are any.
 __global__ void __launch_bounds__(kWarpsPerCta * 32)
 k_table_coeffs(const float *__restrict__ W, float4 *__restrict__ coef, double *__restrict__ sums, int O, int lut_binarize)
 {
@@ -299,7 +298,7 @@ k_table_coeffs(const float *__restrict__ W, float4 *__restrict__ coef, double *_
     if (lut_binarize) { v.x = v.x > 0.5f ? 1.0f : 0.0f; v.y = v.y > 0.5f ? 1.0f : 0.0f; }
     v = table_to_coeffs(v, lane);
     const float hx = __shfl_down_sync(kFull, v.x, 16), hy = __shfl_down_sync(kFull, v.y, 16);
-    if (lane < 16) coef[(size_t)node * 16 + lane] = make_float4(v.x, hx, v.y, hy);
+    if (lane < 16) store_coeff_pairs(coef + (size_t)node * 16, lane, make_float2(v.x, hx), make_float2(v.y, hy));
     if (sums != nullptr && lane < 2) sums[2 * (size_t)node + lane] = 0.0;
 }
 
@@ -363,7 +362,7 @@ k_lut6_forward_pipe(const FwdArgs a, int n_tiles)
             v = table_to_coeffs(v, lane);
             const float hx = __shfl_down_sync(kFull, v.x, 16), hy = __shfl_down_sync(kFull, v.y, 16);
             __syncwarp();
-            if (lane < 16) tab[lane] = make_float4(v.x, hx, v.y, hy);
+            if (lane < 16) store_coeff_pairs(tab, lane, make_float2(v.x, hx), make_float2(v.y, hy));
             __syncwarp();
         }
         double s1 = 0.0, s2 = 0.0;
@@ -821,7 +820,7 @@ static_assert(kBvSmem <= 227 * 1024, "one CTA per SM must fit");
 static_assert(6 * kBvRowBytes <= kBvTrBytes, "dx staging fits the transpose buffer");
 
 // Everything the persistent backward wants done before it, in one launch: every node's table in the half-packed form of
-// lut6_forward_keep_halves (16 x (c[2k], c[2k+32], c[2k+1], c[2k+33])), cleared coefficient gradients, the node's dmean and dvar from the
+// lut6_forward_keep_halves, cleared coefficient gradients, the node's dmean and dvar from the
 // batch sums (`sums` not null), and dx cleared by all threads of the grid with 128-bit stores (`zero` not null; a large cudaMemsetAsync
 // ran at about half of the copy bandwidth).
 struct BwdPrepare {
@@ -848,7 +847,7 @@ k_backward_prepare(const BwdPrepare a)
         if (a.lut_binarize) { v.x = v.x > 0.5f ? 1.0f : 0.0f; v.y = v.y > 0.5f ? 1.0f : 0.0f; }
         v = table_to_coeffs(v, lane);
         const float hx = __shfl_down_sync(kFull, v.x, 16), hy = __shfl_down_sync(kFull, v.y, 16);
-        if (lane < 16) a.coef[(size_t)node * 16 + lane] = make_float4(v.x, hx, v.y, hy);
+        if (lane < 16) store_coeff_pairs(a.coef + (size_t)node * 16, lane, make_float2(v.x, hx), make_float2(v.y, hy));
         a.dC[(size_t)node * 32 + lane] = make_float2(0.0f, 0.0f);
         if (a.sums != nullptr && lane == 0) bn_backward_finalize(a.sums, node, a.mean, a.rstd, a.dmean, a.dvar, a.total_frames);
     }
@@ -856,7 +855,7 @@ k_backward_prepare(const BwdPrepare a)
     for (size_t i = (size_t)blockIdx.x * blockDim.x + threadIdx.x; i < a.zero_quads; i += (size_t)gridDim.x * blockDim.x) a.zero[i] = z;
 }
 
-// dW += adjoint butterfly of the coefficient gradients (dC in the half-packed layout of k_backward_prepare); one warp per node.
+// dW += adjoint butterfly of the coefficient gradients (dC: 16 x (dc[2k], dc[2k+32], dc[2k+1], dc[2k+33])); one warp per node.
 __global__ void __launch_bounds__(kWarpsPerCta * 32)
 k_coeff_grads_to_dw(const float4 *__restrict__ dC, float *__restrict__ dW, int O)
 {
@@ -1003,37 +1002,67 @@ k_lut6_backward_pipe(const BwdArgs a, const float4 *__restrict__ coef, float *__
             const int f0 = f_tile + cc.c * kFramesPerIter;
             // lane l takes the frame pairs 64 h + 2 l + {0, 1}, h = 0, 1: one 64-bit shared load per row and pair, one 64-bit store per
             // input gradient and pair (both conflict-free)
+            auto inputs = [&](const float2 (&xp)[6], int e, float (&u)[6]) {
 #pragma unroll
-            for (int h = 0; h < 2; ++h) {
-                float2 xp[6];
+                for (int j = 0; j < 6; ++j) {
+                    const float v = e ? xp[j].y : xp[j].x;
+                    u[j] = BINARY ? (v > 0.5f ? a.bias : -a.bias) : __saturatef(v) - 0.5f;               // the same values as condition_u()
+                }
+            };
+            auto load_pair = [&](int h, float2 (&xp)[6], float2 &gp) {
 #pragma unroll
                 for (int j = 0; j < 6; ++j) xp[j] = *reinterpret_cast<const float2 *>(st2 + j * kFramesPerIter + 64 * h);
-                const float2 gp = *reinterpret_cast<const float2 *>(st2 + 6 * kFramesPerIter + 64 * h);
-                float dxp[6][2];
+                gp = *reinterpret_cast<const float2 *>(st2 + 6 * kFramesPerIter + 64 * h);
+            };
+            auto store_pair = [&](int h, const float (&dxp)[2][6]) {
 #pragma unroll
-                for (int e = 0; e < 2; ++e) {
-                    float u[6];
-#pragma unroll
-                    for (int j = 0; j < 6; ++j) {
-                        const float v = e ? xp[j].y : xp[j].x;
-                        u[j] = BINARY ? (v > 0.5f ? a.bias : -a.bias) : __saturatef(v) - 0.5f;           // the same values as condition_u()
-                    }
-                    KeptHalves D;
-                    const float v = lut6_forward_keep_halves(tab, u, D);
-                    float g = e ? gp.y : gp.x;
-                    if (BN) {
-                        const float tanh_x = ((v - mean) * rstd) * a.gamma + a.beta;
-                        if (tanh_x <= 0.0f || tanh_x >= 1.0f) g = 0.0f;
-                        g = fmaf(v, dvar_rF, fmaf(g, grstd, dmean));
-                    }
+                for (int j = 0; j < 6; ++j) *reinterpret_cast<float2 *>(tr + j * kFramesPerIter + 64 * h + 2 * lane) = make_float2(dxp[0][j], dxp[1][j]);
+            };
+            if constexpr (BN) {
+                // A frame's forward pass and batch norm stand between the two parts of the reverse pass of the frame before, which does not wait
+                // for them: the chain from the inputs to g shows otherwise, with two warps a scheduler.
+                float u[2][6], dxp[2][6], g;
+                float2 xp[6], gp;
+                KeptHalves D;
+                auto front = [&](int q) {
+                    const int h = q >> 1, e = q & 1;
+                    if (e == 0) load_pair(h, xp, gp);
+                    inputs(xp, e, u[e]);
+                    const float v = lut6_forward_keep_halves(tab, u[e], D);
+                    const float tanh_x = ((v - mean) * rstd) * a.gamma + a.beta;
+                    g = e ? gp.y : gp.x;
+                    if (tanh_x <= 0.0f || tanh_x >= 1.0f) g = 0.0f;
+                    g = fmaf(v, dvar_rF, fmaf(g, grstd, dmean));
                     if (f0 + 64 * h + 2 * lane + e >= a.F || !live_node) g = 0.0f;
-                    float dxv[6];
-                    lut6_reverse_halves(tab, u, D, g, acc2, dxv);
+                };
+                front(0);
 #pragma unroll
-                    for (int j = 0; j < 6; ++j) dxp[j][e] = dxv[j];
+                for (int q = 0; q < 4; ++q) {
+                    ReverseState R;
+                    lut6_reverse_halves_top(u[q & 1], D, g, R, dxp[q & 1][5]);
+                    if (q < 3) front(q + 1);
+                    lut6_reverse_halves_bottom(tab, u[q & 1], R, acc2, dxp[q & 1]);
+                    if (q & 1) store_pair(q >> 1, dxp);
                 }
+            } else {
+                // g needs no forward pass here: two frames share the coefficients' loads
 #pragma unroll
-                for (int j = 0; j < 6; ++j) *reinterpret_cast<float2 *>(tr + j * kFramesPerIter + 64 * h + 2 * lane) = make_float2(dxp[j][0], dxp[j][1]);
+                for (int h = 0; h < 2; ++h) {
+                    float2 xp[6], gp;
+                    float u[2][6], dxp[2][6], unused[2];
+                    KeptHalves D[2];
+                    load_pair(h, xp, gp);
+                    inputs(xp, 0, u[0]);
+                    inputs(xp, 1, u[1]);
+                    lut6_forward_keep_halves_pair(tab, u, D, unused);
+#pragma unroll
+                    for (int e = 0; e < 2; ++e) {
+                        float g = e ? gp.y : gp.x;
+                        if (f0 + 64 * h + 2 * lane + e >= a.F || !live_node) g = 0.0f;
+                        lut6_reverse_halves(tab, u[e], D[e], g, acc2, dxp[e]);
+                    }
+                    store_pair(h, dxp);
+                }
             }
             __syncwarp();
             const bool write = f0 + 4 * lane < a.F && live_node;
