@@ -355,6 +355,7 @@ __device__ __forceinline__ void lut6_reverse_halves_bottom(const float4 *tab2, c
     }
 }
 
+// Both parts in one, written out: put together from the two above it takes 664 instead of 616 us for 216 nodes x 262144 frames without batch norm.
 __device__ __forceinline__ void lut6_reverse_halves(const float4 *tab2, const float (&u)[6], const KeptHalves &D, float g,
                                                     f32x2 (&acc2)[32], float (&dx)[6])
 {
