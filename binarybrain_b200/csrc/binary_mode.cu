@@ -330,8 +330,9 @@ k_pack_bits(const float *__restrict__ x, uint32_t *__restrict__ bits, int I, int
 // (Float atomics on one shared histogram per warp, compare-and-swap loops in hardware, took 0.68 ms for 8192 nodes x 16384 frames.)
 // Shared memory takes four clocks per warp and 32 frames (a 64-bit load and store per frame), about as long as reading dy takes; with
 // only 12 warps per SM (16 KiB of columns each) the loads have to be far ahead: 512 frames of dy are in flight per warp, and the lines of the 512 after
-// them on their way to L2 (186 -> 166 us under ncu for 8192 x 8192 nodes x 16384 frames; four loads of a word instead of one of four 195; reading dy
-// and writing the patterns takes 105 at HBM speed.  One or two warps a CTA: 172 to 179).
+// them on their way to L2 (186 -> 166 us under ncu for 8192 x 8192 nodes x 16384 frames; reading dy and writing the patterns takes 105 at HBM
+// speed.  One or two warps a CTA: 172 to 179).  Rows of x that do not start on 16-byte boundaries take the same loop with four loads of a word: a backward
+// of 316 rows, 617 nodes and 49185 frames without batch norm 137 us, 134 with aligned rows (191 through the loop of 128 frames).
 constexpr int kPsWarps = 4;
 template <bool BN> struct PatternSlot { float s; uint32_t n; };      // n: count, bit 31: the pattern's mask bit
 template <> struct PatternSlot<false> { float s; };
@@ -405,16 +406,19 @@ k_pattern_sums(const BitBwdArgs a)
     if constexpr (!XF32) {
         // 512 frames per step while whole steps are left; the loads of the next step are issued before this one is used, into the
         // other of two sets of registers.  Here a lane's frames are those of four neighbouring words of x, four of each, so that a row's words
-        // come with one 128-bit load instead of four loads (and dy and the patterns still in whole 128 and 32 bytes).
+        // come with one 128-bit load (and dy and the patterns still in whole 128 and 32 bytes), or four loads where rows of x start elsewhere.
         constexpr int NC = 4, kStep = 128 * NC;
         struct Set { uint4 w[6]; float4 dy[NC]; };
-        const int steps = a.vec && a.xvec ? (f_end - f_begin) / kStep : 0;
+        const int steps = a.vec ? (f_end - f_begin) / kStep : 0;
         const int fl = f_begin + 128 * (lane >> 3) + 4 * (lane & 7);
         auto fetch = [&](Set &b, int k) {
             if (k < steps) {
                 if (lane < 16 && k + 2 < steps) asm volatile("prefetch.global.L2 [%0];" ::"l"(dyrow + f_begin + (k + 2) * kStep + 32 * lane));
 #pragma unroll
-                for (int j = 0; j < 6; ++j) b.w[j] = __ldg(reinterpret_cast<const uint4 *>(rows[j] + ((fl + k * kStep) >> 5)));
+                for (int j = 0; j < 6; ++j) {
+                    const uint32_t *x = rows[j] + ((fl + k * kStep) >> 5);
+                    b.w[j] = a.xvec ? __ldg(reinterpret_cast<const uint4 *>(x)) : make_uint4(__ldg(x), __ldg(x + 1), __ldg(x + 2), __ldg(x + 3));
+                }
 #pragma unroll
                 for (int c = 0; c < NC; ++c) b.dy[c] = __ldg(reinterpret_cast<const float4 *>(dyrow + fl + k * kStep + 32 * c));
             }
