@@ -14,7 +14,7 @@
 
 #include <climits>
 #include <cstdint>
-#include <stdexcept>
+#include <exception>
 #include <tuple>
 #include <type_traits>
 #include <utility>
@@ -188,56 +188,73 @@ template <class F> F *bound(F *&fn, const char *name)
     return fn;
 }
 
-// the tensor in `o`, which has to be of two dimensions where `matrix`; null with a Python error set
-const at::Tensor *tensor_of(PyObject *o, bool matrix, const char *name)
+// the tensor in `o`, which has to have `dims` dimensions at least; null with a Python error set
+const at::Tensor *tensor_of(PyObject *o, int64_t dims, const char *name)
 {
     if (!THPVariable_Check(o)) { PyErr_Format(PyExc_TypeError, "%s: expected a tensor", name); return nullptr; }
     const at::Tensor &t = THPVariable_Unpack(o);
-    if (matrix && t.dim() != 2) { PyErr_Format(PyExc_ValueError, "%s: expected two dimensions", name); return nullptr; }
+    if (t.dim() < dims) { PyErr_Format(PyExc_IndexError, "%s: expected %d dimensions", name, (int)dims); return nullptr; }
     return &t;
 }
 
-// the given tensor, or a new uninitialised fp32 one beside `like`
-at::Tensor given_or_new(PyObject *o, const at::Tensor &like, at::IntArrayRef size)
+// a flag, or any number that int() takes
+bool parse_flag(PyObject *o, int &v)
 {
-    if (o != Py_None) {
-        if (!THPVariable_Check(o)) throw std::invalid_argument("expected a tensor or None");
-        return THPVariable_Unpack(o);
-    }
-    return at::empty(size, at::TensorOptions().dtype(at::kFloat).device(like.device()));
+    if (PyLong_Check(o)) return parse(o, v);
+    PyObject *n = PyNumber_Long(o);
+    if (!n) return false;
+    const bool ok = parse(n, v);
+    Py_DECREF(n);
+    return ok;
 }
+
+// an fp32 output: memory of the given tensor, the given address, or, for None, a new tensor beside `like`; false with a Python error set
+struct Output {
+    PyObject *given;
+    at::Tensor made;
+    float *data = nullptr;
+
+    bool take(PyObject *o, const at::Tensor &like, at::IntArrayRef size)
+    {
+        given = o;
+        if (o != Py_None) return parse(o, data);
+        made = at::empty(size, at::TensorOptions().dtype(at::kFloat).device(like.device()));
+        data = static_cast<float *>(made.mutable_data_ptr());
+        return true;
+    }
+    PyObject *result() const { return given != Py_None ? Py_NewRef(given) : THPVariable_Wrap(made); }
+};
 
 // train_forward(x, y, idx, W, mean, rstd, running_mean, running_var, gamma, beta, momentum, bias, frames, lut_binarize, binary) -> (y, mean, rstd)
 PyObject *train_forward(PyObject *, PyObject *const *o, Py_ssize_t n)
 {
     static decltype(&bbcu_fp32_DifferentiableLut6_ForwardTrainingRows) fn = nullptr;
     if (n != 15) { PyErr_SetString(PyExc_TypeError, "train_forward takes 15 arguments"); return nullptr; }
-    float gamma, beta, momentum, bias;
+    float gamma, beta, momentum, bias, *running_mean, *running_var;
+    const float *x, *W;
+    const int *index;
     int frames, lut_binarize, binary;
-    const at::Tensor *x = tensor_of(o[0], true, "x"), *idx = x ? tensor_of(o[2], true, "idx") : nullptr;
-    if (!idx || !parse(o[8], gamma) || !parse(o[9], beta) || !parse(o[10], momentum) || !parse(o[11], bias) || !parse(o[12], frames) ||
-        !parse(o[13], lut_binarize) || !parse(o[14], binary) || !bound(fn, "bbcu_fp32_DifferentiableLut6_ForwardTrainingRows")) return nullptr;
-    const float *W;
-    float *running_mean, *running_var;
-    if (!parse(o[3], W) || !parse(o[6], running_mean) || !parse(o[7], running_var)) return nullptr;
     try {
-        const int64_t rows = x->size(0), stride = x->size(1), nodes = idx->size(0);
+        const at::Tensor *xt = tensor_of(o[0], 2, "x"), *idx = xt ? tensor_of(o[2], 1, "idx") : nullptr;
+        if (!idx || !parse(o[0], x) || !parse(o[2], index) || !parse(o[3], W) || !parse(o[6], running_mean) || !parse(o[7], running_var) ||
+            !parse(o[8], gamma) || !parse(o[9], beta) || !parse(o[10], momentum) || !parse(o[11], bias) || !parse(o[12], frames) ||
+            !parse_flag(o[13], lut_binarize) || !parse_flag(o[14], binary) || !bound(fn, "bbcu_fp32_DifferentiableLut6_ForwardTrainingRows")) return nullptr;
+        const int64_t rows = xt->size(0), stride = xt->size(1), nodes = idx->size(0);
         if (rows > INT_MAX || stride > INT_MAX || nodes > INT_MAX) { PyErr_SetString(PyExc_OverflowError, "a size does not fit the operator"); return nullptr; }
-        const at::Tensor y = given_or_new(o[1], *x, {nodes, stride}), mean = given_or_new(o[4], *x, {nodes}), rstd = given_or_new(o[5], *x, {nodes});
-        const auto *xp = static_cast<const float *>(x->const_data_ptr());
-        const auto *ip = static_cast<const int *>(idx->const_data_ptr());
-        auto *yp = static_cast<float *>(y.mutable_data_ptr()), *mp = static_cast<float *>(mean.mutable_data_ptr()), *rp = static_cast<float *>(rstd.mutable_data_ptr());
+        Output y, mean, rstd;
+        if (!y.take(o[1], *xt, {nodes, stride}) || !mean.take(o[4], *xt, {nodes}) || !rstd.take(o[5], *xt, {nodes})) return nullptr;
         const auto stream = reinterpret_cast<bbcu_stream_t>(c10::cuda::getCurrentCUDAStream().stream());
         int status = 0;
         Py_BEGIN_ALLOW_THREADS
-        status = fn(xp, yp, ip, W, mp, rp, running_mean, running_var, gamma, beta, momentum, bias, (int)rows, (int)nodes, frames, (int)stride, lut_binarize, binary, stream);
+        status = fn(x, y.data, index, W, mean.data, rstd.data, running_mean, running_var, gamma, beta, momentum, bias, (int)rows, (int)nodes, frames, (int)stride,
+                    lut_binarize, binary, stream);
         Py_END_ALLOW_THREADS
         if (status != 0) return raise_status("bbcu_fp32_DifferentiableLut6_ForwardTrainingRows", status);
         PyObject *r = PyTuple_New(3);
         if (!r) return nullptr;
-        const at::Tensor *made[3] = {&y, &mean, &rstd};
-        const int from[3] = {1, 4, 5};
-        for (int i = 0; i < 3; ++i) PyTuple_SET_ITEM(r, i, o[from[i]] != Py_None ? Py_NewRef(o[from[i]]) : THPVariable_Wrap(*made[i]));
+        PyTuple_SET_ITEM(r, 0, y.result());
+        PyTuple_SET_ITEM(r, 1, mean.result());
+        PyTuple_SET_ITEM(r, 2, rstd.result());
         return r;
     } catch (const std::exception &e) {
         PyErr_SetString(PyExc_RuntimeError, e.what());
@@ -250,30 +267,28 @@ PyObject *train_backward(PyObject *, PyObject *const *o, Py_ssize_t n)
 {
     static decltype(&bbcu_fp32_DifferentiableLut6_Backward) fn = nullptr;
     if (n != 15) { PyErr_SetString(PyExc_TypeError, "train_backward takes 15 arguments"); return nullptr; }
-    float gamma, beta, bias;
+    float gamma, beta, bias, *dW;
+    const float *x, *dy, *W, *mean, *rstd;
+    const int *index;
     int n_in, frames, lut_binarize, binary;
-    const at::Tensor *xt = tensor_of(o[0], true, "x"), *dy = xt ? tensor_of(o[1], true, "dy") : nullptr, *idx = dy ? tensor_of(o[3], true, "idx") : nullptr;
-    if (!idx || !parse(o[8], gamma) || !parse(o[9], beta) || !parse(o[10], bias) || !parse(o[11], n_in) || !parse(o[12], frames) ||
-        !parse(o[13], lut_binarize) || !parse(o[14], binary) || !bound(fn, "bbcu_fp32_DifferentiableLut6_Backward")) return nullptr;
-    const float *x, *W, *mean, *rstd;
-    float *dW;
-    if (!parse(o[0], x) || !parse(o[4], W) || !parse(o[5], dW) || !parse(o[6], mean) || !parse(o[7], rstd)) return nullptr;
     try {
-        const int64_t stride = dy->size(1), nodes = idx->size(0);
+        const at::Tensor *xt = tensor_of(o[0], 2, "x"), *dyt = xt ? tensor_of(o[1], 2, "dy") : nullptr, *idx = dyt ? tensor_of(o[3], 1, "idx") : nullptr;
+        if (!idx || !parse(o[0], x) || !parse(o[1], dy) || !parse(o[3], index) || !parse(o[4], W) || !parse(o[5], dW) || !parse(o[6], mean) ||
+            !parse(o[7], rstd) || !parse(o[8], gamma) || !parse(o[9], beta) || !parse(o[10], bias) || !parse(o[11], n_in) || !parse(o[12], frames) ||
+            !parse_flag(o[13], lut_binarize) || !parse_flag(o[14], binary) || !bound(fn, "bbcu_fp32_DifferentiableLut6_Backward")) return nullptr;
+        const int64_t stride = dyt->size(1), nodes = idx->size(0);
         if (xt->size(1) != stride) { PyErr_SetString(PyExc_AssertionError, "x and dy differ in their stride"); return nullptr; }
         if (stride > INT_MAX || nodes > INT_MAX) { PyErr_SetString(PyExc_OverflowError, "a size does not fit the operator"); return nullptr; }
-        const at::Tensor dx = given_or_new(o[2], *dy, {n_in, stride}), scratch = given_or_new(Py_None, *dy, {2 * nodes});
-        const auto *dyp = static_cast<const float *>(dy->const_data_ptr());
-        const auto *ip = static_cast<const int *>(idx->const_data_ptr());
-        auto *dxp = static_cast<float *>(dx.mutable_data_ptr()), *sp = static_cast<float *>(scratch.mutable_data_ptr());
+        Output dx, scratch;
+        if (!dx.take(o[2], *dyt, {n_in, stride}) || !scratch.take(Py_None, *dyt, {2 * nodes})) return nullptr;
         const auto stream = reinterpret_cast<bbcu_stream_t>(c10::cuda::getCurrentCUDAStream().stream());
         int status = 0;
         Py_BEGIN_ALLOW_THREADS
-        status = fn(x, dyp, dxp, nullptr, ip, nullptr, W, dW, mean, rstd, sp, sp + nodes, gamma, beta, bias, 0, n_in, (int)nodes, frames, (int)stride, 0, 0,
-                    lut_binarize, binary, stream);
+        status = fn(x, dy, dx.data, nullptr, index, nullptr, W, dW, mean, rstd, scratch.data, scratch.data + nodes, gamma, beta, bias, 0, n_in, (int)nodes, frames,
+                    (int)stride, 0, 0, lut_binarize, binary, stream);
         Py_END_ALLOW_THREADS
         if (status != 0) return raise_status("bbcu_fp32_DifferentiableLut6_Backward", status);
-        return o[2] != Py_None ? Py_NewRef(o[2]) : THPVariable_Wrap(dx);
+        return dx.result();
     } catch (const std::exception &e) {
         PyErr_SetString(PyExc_RuntimeError, e.what());
         return nullptr;
