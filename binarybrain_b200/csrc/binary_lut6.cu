@@ -653,8 +653,8 @@ extern "C" int bbcu_bit_BinaryLut6_Forward(const int *x, int *y, const int *idx,
     return launch_status();
 }
 
-// The same operator through the truth-table-immediate kernel whatever the size.  Rows must be 16-byte aligned (stride a multiple of 4 words,
-// aligned base pointers).
+// The same operator through the truth-table-immediate kernel wherever its 32-bit arithmetic reaches, through the kernels above beyond.  Rows must be
+// 16-byte aligned (stride a multiple of 4 words, aligned base pointers).
 extern "C" int bbcu_bit_BinaryLut6_Forward_Lop3Immediate(const int *x, int *y, const int *idx, const int *table, int node_size, int frame_size,
                                                          int frame_stride, bbcu_stream_t stream)
 {
@@ -670,7 +670,7 @@ extern "C" int bbcu_bit_BinaryLut6_Forward_Lop3Immediate(const int *x, int *y, c
     a.nwords = ((frame_size + 31) / 32 + 3) & ~3;
     a.groups = 0;
     a.Tw = 0;
-    BB200_REQUIRE(imm_fits(a), BBCU_ERR_TOO_LARGE);
+    if (!imm_fits(a)) return bbcu_bit_BinaryLut6_Forward(x, y, idx, table, node_size, frame_size, frame_stride, stream);
     return launch_immediate(a, as_stream(stream));
 }
 

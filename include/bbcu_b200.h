@@ -187,8 +187,10 @@ int bbcu_bit_BinatyLut6_Forward(const int *dev_x_buf, int *dev_y_buf, const int 
                                 int node_size, int frame_size, int frame_stride, bbcu_stream_t stream);
 
 /* Additive: the same operator evaluated with the table bytes as lop3 immediates (15 logic operations per 32 frames instead of 63, one
- * indexed branch per table byte) whatever the size; the operator above takes that kernel by itself where it is the faster one.  Bit-identical
- * results.  Rows must be 16-byte aligned: frame_stride a multiple of 4 words and aligned base pointers, BBCU_ERR_BAD_STRIDE otherwise. */
+ * indexed branch per table byte) also where the operator above, which takes that kernel by itself where it is the faster one, would not.
+ * Bit-identical results.  Rows must be 16-byte aligned: frame_stride a multiple of 4 words and aligned base pointers,
+ * BBCU_ERR_BAD_STRIDE otherwise.  Beyond the kernel's 32-bit arithmetic (frame_stride from 2^30 words, or about 2^30 nodes) the
+ * operator above does the call. */
 int bbcu_bit_BinaryLut6_Forward_Lop3Immediate(const int *dev_x_buf, int *dev_y_buf, const int *dev_input_index, const int *dev_table,
                                               int node_size, int frame_size, int frame_stride, bbcu_stream_t stream);
 

@@ -75,6 +75,28 @@ def test_binary_lut6_by_immediates(ops, n_in, n_out, words, spare):
         assert (y[:, (words + 3) // 4 * 4:] == 0x5a5a5a5a).all()
 
 
+# rows 2^30 words apart, beyond the 32-bit arithmetic of that kernel
+def test_binary_lut6_by_immediates_of_far_rows(ops):
+    import torch
+    from gpu_util import dev
+    rng = np.random.default_rng(5)
+    F, stride, words = 250, 1 << 30, 8
+    x, table = rng.integers(-2**31, 2**31, (2, words)).astype(np.int32), rng.integers(-2**31, 2**31, (2, 2)).astype(np.int32)
+    idx = np.array([[0, 1, 0, 0, 1, 1], [1, 1, 0, 1, 0, 0]], np.int32)
+    xd, yd = torch.empty(stride + words, dtype=torch.int32, device="cuda"), torch.empty(stride + words, dtype=torch.int32, device="cuda")
+    for k in range(2):
+        xd[k * stride: k * stride + words] = dev(x[k])
+    from binarybrain_b200 import abi
+    idx_d, table_d = dev(idx), dev(table)
+    abi.call("bbcu_bit_BinaryLut6_Forward_Lop3Immediate", xd.data_ptr(), yd.data_ptr(), idx_d.data_ptr(), table_d.data_ptr(), 2, F, stride, None)
+    torch.cuda.synchronize()
+    y = np.stack([yd[k * stride: k * stride + words].cpu().numpy() for k in range(2)]).view(np.uint32)
+    want = port.binary_lut6_forward(x.view(np.uint32), idx, table, F)
+    live = np.full(words, 0xffffffff, np.uint32)
+    live[-1] >>= words * 32 - F
+    assert ((y ^ want[:, :words]) & live == 0).all()
+
+
 # one chunk, a first and a last chunk only, full-width chunks with a one-word remainder
 @pytest.mark.parametrize("n_in,n_out,words,spare", [(9, 7, 1, 0), (700, 400, 130, 30), (4096, 64, 257, 31), (1024, 1100, 1793, 5)])
 def test_binary_lut6_host_chunks(ops, n_in, n_out, words, spare):
