@@ -1482,6 +1482,17 @@ void gather_shape(BitBwdArgs &a)
     a.heavy_ctas = 8 * di.sm_count;
 }
 
+// Words of a packed row: whole 16-byte pieces, which k_pattern_sums reads with one load, or no padding where only then the rows take no more than the
+// limit.  (Beyond it a backward goes through the per-node kernels.)
+constexpr long long kPackedBytes = 1LL << 30;
+constexpr long long packed_row_words(long long rows, long long frames)
+{
+    const long long padded = (frames + 127) / 128 * 4;
+    return rows * padded * 4 <= kPackedBytes ? padded : (frames + 31) / 32;
+}
+static_assert(packed_row_words(1LL << 26, 33) == 4 && packed_row_words((1LL << 26) + 1, 33) == 2 && packed_row_words(1LL << 27, 33) * (1LL << 27) * 4 == kPackedBytes,
+              "whatever fits without padding is packed");
+
 // Slot 3 of the stream's scratch: consumer lists, the chunks of heavy rows, and the bits of the I rows where x is fp32.  The block is the same
 // size when they need not be packed, so that a call after which that is known does not have to grow it.
 bool input_side(BitBwdArgs &a, int I, bool x_is_fp32, bool packed, cudaStream_t st)
@@ -1490,12 +1501,12 @@ bool input_side(BitBwdArgs &a, int I, bool x_is_fp32, bool packed, cudaStream_t 
     a.I = I;
     gather_shape(a);
     const int edges = 6 * a.O;
-    const long long ws = ((long long)a.F + 127) / 128 * 4;                  // whole 16-byte pieces
+    const long long ws = packed_row_words(I, a.F);
     // a heavy row has more than heavy_from >= 2 heavy_chunk consumers, so its chunks number at most 3 / 2 of its consumers over heavy_chunk
     const size_t heavy_most = (size_t)edges / (size_t)a.heavy_chunk * 3 / 2 + 2;
     const size_t list_bytes = (heavy_most * sizeof(int2) + (2 * (size_t)I + 2 + (size_t)edges) * sizeof(int) + 255) & ~(size_t)255;
     size_t bit_bytes = x_is_fp32 ? (size_t)I * (size_t)ws * 4 : 0;
-    if (bit_bytes > ((size_t)1 << 30)) {
+    if (bit_bytes > (size_t)kPackedBytes) {
         if (!packed) return false;
         bit_bytes = 0;
     }
