@@ -84,8 +84,9 @@ k_softmax_cross_entropy_one(const float *__restrict__ y, const float *__restrict
 }
 
 // The same for one pixel, up to ROWS classes and a frame per thread: everything is read once, all loads of a frame in flight together, and a frame
-// with one target above 0 takes one logarithm.  Latency is all there is to it (10 classes: 100 frames 6.9 -> 5.0 us, 512 7.9 -> 5.8, 1024 10.2 -> 7.9;
-// 16 classes, 1000 frames 14.9 -> 10.0).
+// with one target above 0 takes one logarithm.  Latency is all there is to it (k_softmax_cross_entropy_one -> this, in us: 10 classes, 100 frames
+// 6.7 -> 5.8, 512 7.8 -> 6.8, 1000 11.4 -> 9.3; 16 classes, 1000 frames 15.1 -> 12.2).  Every thread walks through all ROWS, so there are kernels
+// for 4, 8 and 16: 3 classes, 1024 frames 5.5, with 16 rows 6.0, with 4 rows 5.1; 5 classes 6.6, 7.0, with 8 rows 5.5.
 template <int ROWS>
 __global__ void __launch_bounds__(1024)
 k_softmax_cross_entropy_frames(const float *__restrict__ y, const float *__restrict__ t, float *dy, double *loss, int ch_size, int F, long long stride)
@@ -241,7 +242,8 @@ extern "C" int bbcu_fp32_LossSoftmaxCrossEntropyMean(const float *y, const float
     double *work = rows * frame_size <= kOneCta ? nullptr : static_cast<double *>(stream_scratch(st, 2 * sizeof(double)));
     if (pix_size == 1 && ch_size <= 16 && frame_size <= 1024) {
         const int threads = frame_size > 32 ? (frame_size + 31) / 32 * 32 : 32;
-        launch(k_softmax_cross_entropy_frames<16>, 1, threads, 0, st, y, t, dy, loss, ch_size, frame_size, frame_stride);
+        auto kern = ch_size <= 4 ? k_softmax_cross_entropy_frames<4> : ch_size <= 8 ? k_softmax_cross_entropy_frames<8> : k_softmax_cross_entropy_frames<16>;
+        launch(kern, 1, threads, 0, st, y, t, dy, loss, ch_size, frame_size, frame_stride);
         return launch_status();
     }
     if (work == nullptr) {                                    // (a heap that declines it: slower, not an error)

@@ -259,6 +259,12 @@ def test_mean_loss_of_weighted_targets(ops, classes, frames):
     assert np.abs(host_fp32(dy, frames) - dy_w).max() <= 1e-6 and abs(float(loss.item()) - loss_w) <= 16 * 2**-24 * max(1.0, abs(loss_w))
 
 
+# the kernels for up to 4, 8 and 16 classes: the most and the fewest of each
+@pytest.mark.parametrize("classes,frames", [(4, 1024), (5, 1000), (8, 65), (9, 1024)])
+def test_mean_loss_of_few_classes(ops, classes, frames):
+    test_mean_loss_of_weighted_targets(ops, classes, frames)
+
+
 # Im2Col by quads of pixels (filters 3 and 5 wide, one band and several, a short last band, every border) and bit Im2Col with several word columns
 # a block, several periods a warp, split blocks, windows beyond four and words without any
 @pytest.mark.parametrize("c,h,w,fh,fw,ys,xs,pad,F", [
