@@ -273,17 +273,20 @@ unsigned backward_threads(int O, int F) { return small_layer_threads(O, F, 8, 23
 
 }   // namespace
 
+// On the way of calls of 3 us: the device is asked for once, and not at all where one warp does (eight look-ups and 64-bit divisions took 0.35 us).
 unsigned small_layer_threads(int O, int F, int sm_warps, int fixed, int per_round)
 {
-    const int all = F > 128 * kWarpsPerCta ? kWarpsPerCta : (F + 127) / 128;                 // warps that one round of frames keeps busy
-    int best = all;
-    long long best_cost = -1;
-    for (int w = all; w >= 1; --w) {
-        const long long slots = (long long)device_info().sm_count * (sm_warps / w), rounds = (F + 128 * w - 1) / (128 * w);
-        const long long cost = (O + slots - 1) / slots * (fixed + per_round * rounds);
-        if (best_cost < 0 || cost < best_cost) { best = w; best_cost = cost; }
+    const unsigned all = F > 128 * kWarpsPerCta ? kWarpsPerCta : (unsigned)(F + 127) / 128;      // warps that one round of frames keeps busy
+    if (all == 1) return 32u;
+    const unsigned sms = (unsigned)device_info().sm_count;
+    if ((unsigned)O <= sms * ((unsigned)sm_warps / all)) return 32u * all;                       // one wave as it is
+    unsigned best = all, best_cost = ~0u;
+    for (unsigned w = all; w >= 1; --w) {
+        const unsigned slots = sms * ((unsigned)sm_warps / w), rounds = ((unsigned)F + 128 * w - 1) / (128 * w);
+        const unsigned cost = ((unsigned)O + slots - 1) / slots * ((unsigned)fixed + (unsigned)per_round * rounds);
+        if (cost < best_cost) { best = w; best_cost = cost; }
     }
-    return 32u * (unsigned)best;
+    return 32u * best;
 }
 
 // Measured on B200 against the persistent kernels, training forward / batch-normalised backward of a layer: 360 nodes x 100 frames 6 / 9 us

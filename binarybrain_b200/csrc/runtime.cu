@@ -62,8 +62,12 @@ const DeviceInfo &device_info()
 {
     static std::mutex mu;
     static std::map<int, DeviceInfo> infos;
+    static std::atomic<const DeviceInfo *> known[16];                    // entries of `infos`, which stay where they are
     int dev = 0;
     cudaGetDevice(&dev);
+    if (dev >= 0 && dev < 16) {
+        if (const DeviceInfo *di = known[dev].load(std::memory_order_acquire)) return *di;
+    }
     std::lock_guard<std::mutex> g(mu);
     auto it = infos.find(dev);
     if (it == infos.end()) {
@@ -74,6 +78,7 @@ const DeviceInfo &device_info()
         if (cudaDeviceGetAttribute(&v, cudaDevAttrMultiProcessorCount, dev) == cudaSuccess && v > 0) di.sm_count = v;
         if (cudaDeviceGetAttribute(&v, cudaDevAttrL2CacheSize, dev) == cudaSuccess && v > 0) di.l2_bytes = (size_t)v;
         it = infos.emplace(dev, di).first;
+        if (dev >= 0 && dev < 16) known[dev].store(&it->second, std::memory_order_release);
     }
     return it->second;
 }
