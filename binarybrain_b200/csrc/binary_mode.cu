@@ -985,8 +985,9 @@ __device__ __forceinline__ uint32_t small_patterns(const SmallBinArgs &a, const 
 }
 
 // Training forward of a batch-normalised layer on two-valued inputs: the arithmetic of k_pattern_values and k_dl6_bit_train_finalize.
-template <bool XBIT>
-__global__ void __launch_bounds__(kWarpsPerCta * 32)
+// WARPS: how many an SM has to hold.  64 leave 32 registers, with which the rows are waited for sooner than need be.
+template <bool XBIT, int WARPS>
+__global__ void __launch_bounds__(kWarpsPerCta * 32, WARPS / kWarpsPerCta)
 k_small_binary_forward(const SmallBinArgs a)
 {
     grid_dependency();
@@ -994,6 +995,9 @@ k_small_binary_forward(const SmallBinArgs a)
     __shared__ unsigned s_cnt[64];
     __shared__ unsigned s_table[2];
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, node = blockIdx.x;
+    const float2 *table = reinterpret_cast<const float2 *>(a.W + (size_t)node * 64) + lane;
+    float2 w = make_float2(0.0f, 0.0f);
+    if (!XBIT && warp == 0) w = *table;                                                     // (bit rows are here sooner: 2 % slower that way)
     size_t rows[6];
 #pragma unroll
     for (int j = 0; j < 6; ++j) rows[j] = (size_t)__ldg(a.idx + (size_t)node * 6 + j) * a.xs;
@@ -1003,7 +1007,7 @@ k_small_binary_forward(const SmallBinArgs a)
     if (warp == 0) {
         s_cnt[lane] = 0u;
         s_cnt[lane + 32] = 0u;
-        stage_table_x2(s_tab, a.W, node, lane, a.lut_binarize);
+        stage_table_x2(s_tab, XBIT ? *table : w, lane, a.lut_binarize);
         f32x2 up[6][1], yp[1];
 #pragma unroll
         for (int j = 0; j < 5; ++j) {
@@ -1075,9 +1079,9 @@ k_small_binary_forward(const SmallBinArgs a)
     }
 }
 
-// Backward (BN: batch-normalised layer): the arithmetic of k_bit_backward_finalize and k_pattern_gather.
-template <bool XBIT, bool BN>
-__global__ void __launch_bounds__(kWarpsPerCta * 32)
+// Backward (BN: batch-normalised layer): the arithmetic of k_bit_backward_finalize and k_pattern_gather.  WARPS as above: 24 leave 80 registers.
+template <bool XBIT, bool BN, int WARPS>
+__global__ void __launch_bounds__(kWarpsPerCta * 32, WARPS / kWarpsPerCta)
 k_small_binary_backward(const SmallBinArgs a, const GridClear clear)
 {
     grid_dependency();
@@ -1088,6 +1092,8 @@ k_small_binary_backward(const SmallBinArgs a, const GridClear clear)
     __shared__ float s_node[2];
     __shared__ unsigned s_mask[2];
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, node = blockIdx.x;
+    float2 w = make_float2(0.0f, 0.0f);
+    if (warp == 0) w = reinterpret_cast<const float2 *>(a.W + (size_t)node * 64)[lane];          // on its way before the rows are waited for
     size_t rows[6], out[6];
 #pragma unroll
     for (int j = 0; j < 6; ++j) {
@@ -1107,7 +1113,7 @@ k_small_binary_backward(const SmallBinArgs a, const GridClear clear)
         s_hdy[lane + 32] = 0.0f;
         s_cnt[lane] = 0u;
         s_cnt[lane + 32] = 0u;
-        stage_table_halves(s_tab, a.W, node, lane, a.lut_binarize);
+        stage_table_halves(s_tab, w, lane, a.lut_binarize);
         eval_pattern_pair(s_tab, lane, a.bias, y, d);
         if (BN) {
             mean = a.mean_in[node];
@@ -1215,11 +1221,21 @@ k_small_binary_backward(const SmallBinArgs a, const GridClear clear)
 // 129 / 115; and however few the nodes, a CTA works through its frames alone: 64 x 16384 125 / 64.
 bool small_layer(int O, int F) { return (long long)O * F <= kSmallLayer && F <= 4096; }
 
-// The forward's registers leave an SM 64 warps: as many as there are rounds of frames.  Of the backward it holds 24, and a wave costs about as much as a
+// Warps of a CTA: in the forward as many as there are rounds of frames.  In the backward, of which an SM holds 24, a wave costs about as much as a
 // round, 2.7 us (sweep of 58 layers with 1, 2, 3, 4 and 8 warps; as many warps as rounds -> this rule, in us: 1024 nodes x 512 frames 14.6 -> 12.3,
 // 982 x 1670 35.6 -> 28.9, 550 x 927 16.3 -> 13.8, 3428 x 415 28.4 -> 25.9, 2816 x 596 34.1 -> 28.6).
 unsigned small_threads(int F) { return 32u * (unsigned)(F > 128 * kWarpsPerCta ? kWarpsPerCta : (F + 127) / 128); }
 unsigned small_backward_threads(int O, int F) { return small_layer_threads(O, F, 24, 27, 27); }
+
+// Whether O CTAs take no more waves on SMs that hold `few` warps (and 32 CTAs) than on SMs that hold `many`: then the kernel with more registers is the
+// faster one.  In us with many / few: forward on fp32 rows 948 nodes x 1174 frames 10.8 / 14.5, 393 x 1032 8.8 / 8.4, 8635 x 78 14.5 / 14.0; backward on
+// bit rows 948 x 1174 16.3 / 24.0, 393 x 1032 10.7 / 16.4, 1159 x 115 9.0 / 8.1, 1930 x 158 12.0 / 11.3.
+bool waves_as_few(int O, unsigned threads, int few, int many)
+{
+    const int warps = (int)threads / 32, sms = device_info().sm_count;
+    auto waves = [&](int hold) { const int slots = sms * (hold / warps < 32 ? hold / warps : 32); return (O + slots - 1) / slots; };
+    return waves(few) <= waves(many);
+}
 
 struct Scratch {
     float    *Y;        // [O][64]
@@ -1315,7 +1331,7 @@ int dl6_bit_forward_training_by_table(const int *x, int *y, const int *idx, cons
         SmallBinArgs a = {};
         a.x = x; a.y = y; a.idx = idx; a.W = W; a.mean = mean; a.rstd = rstd; a.running_mean = rmean; a.running_var = rvar;
         a.gamma = gamma; a.beta = beta; a.momentum = momentum; a.bias = bias; a.F = F; a.lut_binarize = lut_binarize; a.xs = stride; a.ys = stride;
-        launch(k_small_binary_forward<true>, O, small_threads(F), 0, st, a);
+        launch(k_small_binary_forward<true, 64>, O, small_threads(F), 0, st, a);
         return launch_status();
     }
     Scratch s;
@@ -1373,7 +1389,8 @@ int f32_binary_forward_by_table(int mode, const float *x, float *y, const int *i
         SmallBinArgs a = {};
         a.x = x; a.y = y; a.idx = idx; a.W = W; a.mean = mean; a.rstd = rstd; a.running_mean = rmean; a.running_var = rvar;
         a.gamma = gamma; a.beta = beta; a.momentum = momentum; a.bias = bias; a.F = F; a.lut_binarize = lut_binarize; a.xs = fs; a.ys = fs; a.vec = aligned;
-        launch(k_small_binary_forward<false>, O, small_threads(F), 0, st, a);
+        const unsigned threads = small_threads(F);
+        launch(waves_as_few(O, threads, 48, 64) ? k_small_binary_forward<false, 48> : k_small_binary_forward<false, 64>, O, threads, 0, st, a);
         return launch_status();
     }
     if (!aligned) return BBCU_ERR_NO_MEMORY;
@@ -1618,9 +1635,11 @@ int bit_backward_by_table(bool bn, bool x_is_fp32, const void *x, const float *d
         GridClear clear;
         const int rcc = grid_clear_setup(clear, dx, (size_t)I * (size_t)fs, st);
         if (rcc) return rcc;
-        auto kern = x_is_fp32 ? (bn ? k_small_binary_backward<false, true> : k_small_binary_backward<false, false>)
-                              : (bn ? k_small_binary_backward<true, true> : k_small_binary_backward<true, false>);
-        launch(kern, O, small_backward_threads(O, F), 0, st, a, clear);
+        const unsigned threads = small_backward_threads(O, F);
+        auto kern = x_is_fp32 ? (bn ? k_small_binary_backward<false, true, 24> : k_small_binary_backward<false, false, 24>)
+                  : waves_as_few(O, threads, 16, 24) ? (bn ? k_small_binary_backward<true, true, 16> : k_small_binary_backward<true, false, 16>)
+                                                     : (bn ? k_small_binary_backward<true, true, 24> : k_small_binary_backward<true, false, 24>);
+        launch(kern, O, threads, 0, st, a, clear);
         return launch_status();
     }
     BitBwdArgs a;

@@ -123,10 +123,10 @@ __device__ __forceinline__ f32x2 add2(f32x2 a, f32x2 b) { f32x2 d; asm("add.rn.f
 
 // Per-node table for the packed path: 32 entries of (c0, c0, c1, c1), the coefficient pair of a level-1 node duplicated for
 // both halves of a packed operand, so that level 1 reads both operands with one 128-bit load.
-__device__ __forceinline__ void stage_table_x2(float4 *tab, const float *__restrict__ W, int node, int lane, int lut_binarize)
+// `v`: the lane's two entries of the node's table.
+__device__ __forceinline__ void stage_table_x2(float4 *tab, float2 v, int lane, int lut_binarize)
 {
     __syncwarp();
-    float2 v = reinterpret_cast<const float2 *>(W + (size_t)node * 64)[lane];
     if (lut_binarize) {
         v.x = v.x > 0.5f ? 1.0f : 0.0f;
         v.y = v.y > 0.5f ? 1.0f : 0.0f;
@@ -134,6 +134,10 @@ __device__ __forceinline__ void stage_table_x2(float4 *tab, const float *__restr
     v = table_to_coeffs(v, lane);
     tab[lane] = make_float4(v.x, v.x, v.y, v.y);
     __syncwarp();
+}
+__device__ __forceinline__ void stage_table_x2(float4 *tab, const float *__restrict__ W, int node, int lane, int lut_binarize)
+{
+    stage_table_x2(tab, reinterpret_cast<const float2 *>(W + (size_t)node * 64)[lane], lane, lut_binarize);
 }
 
 template <int L, int K, int NP>
@@ -185,10 +189,10 @@ __device__ __forceinline__ void store_coeff_pairs(float4 *tab2, int k, float2 ev
     dst[2] = odd;
 }
 
-__device__ __forceinline__ void stage_table_halves(float4 *tab2, const float *__restrict__ W, int node, int lane, int lut_binarize)
+// `v`: the lane's two entries of the node's table.
+__device__ __forceinline__ void stage_table_halves(float4 *tab2, float2 v, int lane, int lut_binarize)
 {
     __syncwarp();
-    float2 v = reinterpret_cast<const float2 *>(W + (size_t)node * 64)[lane];
     if (lut_binarize) {
         v.x = v.x > 0.5f ? 1.0f : 0.0f;
         v.y = v.y > 0.5f ? 1.0f : 0.0f;
@@ -197,6 +201,10 @@ __device__ __forceinline__ void stage_table_halves(float4 *tab2, const float *__
     const float hx = __shfl_down_sync(kFull, v.x, 16), hy = __shfl_down_sync(kFull, v.y, 16);
     if (lane < 16) store_coeff_pairs(tab2, lane, make_float2(v.x, hx), make_float2(v.y, hy));
     __syncwarp();
+}
+__device__ __forceinline__ void stage_table_halves(float4 *tab2, const float *__restrict__ W, int node, int lane, int lut_binarize)
+{
+    stage_table_halves(tab2, reinterpret_cast<const float2 *>(W + (size_t)node * 64)[lane], lane, lut_binarize);
 }
 
 // The odd operands of levels 2..5 (both halves) and of level 6, kept between the forward and the reverse pass.
