@@ -25,6 +25,7 @@ struct BlArgs {
     const int *idx;
     const int *table;
     int O, nwords, Tw, groups;
+    int run_rows;                       // k_binary_lut6_imm: input rows of which Tw tiles stay in L2
     long long stride;
 };
 
@@ -468,6 +469,27 @@ __device__ __forceinline__ void lut6_words_by_immediates(uint32_t (&x)[3][8], ui
 #undef BB200_LOAD4
 #undef BB200_LOAD5
 
+// Whether a node's run is two tiles by the input rows, whose number is not among the operator's arguments: it is the range of the wiring's entries, of
+// which every warp reads the same 256 (not a microsecond of calls of 70 and more).  Rows of two tiles that do not stay in L2 come from HBM once more for every
+// reader.  Two to three rows a node are for two tiles where they do stay; up to two are either way within 5 %, sustained for two, cool for one; and
+// beyond three few rows have a second reader.  In us by k_binary_lut6_pipe / with one tile / with two, cool: 8192 nodes x 2^20 frames reading 8192 rows
+// 982 / 733 / 671, 16384 rows 984 / 759 / 791, 24576 983 / 775 / 944, 49152 1008 / 883 / 1126; 4000 x 2^20 reading 8000 rows 530 / 365 / 335, 12000
+// 501 / 371 / 359, 24000 497 / 412 / 486; 2000 x 2^21 reading 12000 497 / 401 / 430; 13000 x 2^18 reading 3900 423 / 322 / 282, 39000 412 / 327 / 401.
+__device__ __forceinline__ bool imm_two_tiles(const BlArgs &a, int lane)
+{
+    constexpr int kLook = 8;
+    const long long entries = 6LL * a.O;
+    unsigned lo = ~0u, hi = 0u;
+#pragma unroll
+    for (int k = 0; k < kLook; ++k) {
+        const unsigned row = (unsigned)__ldg(a.idx + (entries * (32 * k + lane)) / (32 * kLook));
+        lo = min(lo, row);
+        hi = max(hi, row);
+    }
+    const long long rows = (long long)__reduce_max_sync(0xffffffffu, hi) - __reduce_min_sync(0xffffffffu, lo);
+    return rows <= 2LL * a.O || (rows <= a.run_rows && rows <= 3LL * a.O);
+}
+
 // Persistent: a group of four warps takes (tile of 1024 words, node) items in tile-major order, each warp a segment of 256 words.  x0..x2 go to
 // registers at the start of an item, and the copies of the next item's follow at once; x3..x5 are used from shared memory, in two buffers.
 // Every lane copies, with cp.async, the 16-byte pieces that it will itself read: no barrier and no cross-lane dependence.
@@ -483,22 +505,23 @@ k_binary_lut6_imm(const BlArgs a)
     const int tiles = a.nwords > segment ? (a.nwords - segment - 1) / kImmTile + 1 : 0;      // tiles that have words for this warp, and
     const int whole = (a.nwords + kImmTile - kPipeWords - segment) / kImmTile;               // those in which it has all 256
     const int step = (int)gridDim.x * kGroups, first = (int)blockIdx.x * kGroups + warp / kImmGroup;
-    // A node's run is a.Tw tiles (a power of two); the runs of a group are `first`, first + step, ...
-    const int dt = step / a.O, dn = step - dt * a.O, last = a.Tw - 1;
+    // A node's run is one or two tiles; the runs of a group are `first`, first + step, ...
+    const int run = a.Tw == 2 && imm_two_tiles(a, lane) ? 2 : 1;
+    const int dt = step / a.O, dn = step - dt * a.O, last = run - 1;
     auto advance = [&](PipePos p) {
         if ((p.tile & last) != last && p.tile + 1 < tiles) {
             ++p.tile;
             return p;
         }
-        p.tile = (p.tile & ~last) + dt * a.Tw;
+        p.tile = (p.tile & ~last) + dt * run;
         p.node += dn;
-        if (p.node >= a.O) { p.node -= a.O; p.tile += a.Tw; }
+        if (p.node >= a.O) { p.node -= a.O; p.tile += run; }
         return p;
     };
     PipePos p0;
     p0.tile = first / a.O;
     p0.node = first - p0.tile * a.O;
-    p0.tile *= a.Tw;
+    p0.tile *= run;
     // three rows, from input `J` on, of item p to `dst`; lane j of `row` holds the item's input row j
     const uint32_t row_bytes = (uint32_t)a.stride * 4u;
     const uint64_t mine = (uint64_t)__cvta_generic_to_global(a.x) + (uint64_t)(segment + 4 * lane) * 4;
@@ -572,10 +595,11 @@ long long imm_rounds(const BlArgs &a)
     return ((a.nwords + kImmTile - 1) / kImmTile * (long long)a.O + groups - 1) / groups;
 }
 
-// Tiles that a group takes of a node before the next node.  Two halve the case bodies to fetch, but the rows of both, 8 KiB a node, have to stay
-// in L2, and they make the rounds coarser: 8192 nodes x 2^20 frames 982 us by k_binary_lut6_pipe, 727 with one tile, 668 with two, 796 with
-// four; 20000 x 2^18 606, 467, 479, 618; 318 x 56770 (one round) 4.5, 4.6, 5.9, 5.9.
-int imm_run(const BlArgs &a) { return imm_rounds(a) >= 8 && 2LL * kImmTile * 4 * a.O <= (long long)(device_info().l2_bytes / 10 * 9) ? 2 : 1; }
+// Most tiles that a group takes of a node before the next node.  Two halve the case bodies to fetch, but the rows of both, 8 KiB an input, have to stay
+// in L2 (of the inputs only the wiring tells: imm_two_tiles()), and they make the rounds coarser: 8192 nodes x 2^20 frames 982 us by
+// k_binary_lut6_pipe, 727 with one tile, 668 with two, 796 with four; 20000 x 2^18 606, 467, 479, 618; 318 x 56770 (one round) 4.5, 4.6, 5.9, 5.9.
+int imm_run_rows() { return (int)((long long)(device_info().l2_bytes / 10 * 9) / (2LL * kImmTile * 4)); }
+int imm_run(const BlArgs &a) { return imm_rounds(a) >= 8 && a.O <= imm_run_rows() ? 2 : 1; }
 
 // What the kernel's 32-bit arithmetic can take.
 bool imm_fits(const BlArgs &a)
@@ -586,6 +610,7 @@ bool imm_fits(const BlArgs &a)
 int launch_immediate(BlArgs a, cudaStream_t st)
 {
     a.Tw = imm_run(a);
+    a.run_rows = imm_run_rows();
     const long long tiles = (a.nwords + kImmTile - 1) / kImmTile, runs = (tiles + a.Tw - 1) / a.Tw * a.O, groups = kImmWarps / kImmGroup;
     const long long grid = (runs + groups - 1) / groups;
     launch(k_binary_lut6_imm, (unsigned)(grid < device_info().sm_count ? grid : device_info().sm_count), kImmWarps * 32, kImmSmem, st, a);

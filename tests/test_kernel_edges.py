@@ -75,6 +75,12 @@ def test_binary_lut6_by_immediates(ops, n_in, n_out, words, spare):
         assert (y[:, (words + 3) // 4 * 4:] == 0x5a5a5a5a).all()
 
 
+# more input rows than two tiles of a node at a time are for, and the most for which they are
+@pytest.mark.parametrize("n_in,n_out,words,spare", [(7000, 2000, 3 * 1024 - 2, 9), (6001, 2000, 3 * 1024 - 2, 9)])
+def test_binary_lut6_by_immediates_of_many_rows(ops, n_in, n_out, words, spare):
+    test_binary_lut6_by_immediates(ops, n_in, n_out, words, spare)
+
+
 # rows 2^30 words apart, beyond the 32-bit arithmetic of that kernel
 def test_binary_lut6_by_immediates_of_far_rows(ops):
     import torch
