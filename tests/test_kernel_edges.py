@@ -230,6 +230,28 @@ def test_large_probability_layers_edges(ops, I, O, F, stride):
     test_small_probability_layers_edges(ops, I, O, F, stride)
 
 
+# The reverse pass stands in one piece and in two, the forward pass that keeps its operands for one frame and for two: the same operations, whose results
+# agree in every bit.  Two at once and one piece in the plain backward, one and two pieces behind batch norm (here the identity, which has no part in the
+# gradients), one and one piece in the one-launch layers.  Every input feeds one node, so that a gradient is no sum.
+@pytest.mark.parametrize("O,F", [(3, 4097), (40, 5000)])
+def test_forms_of_the_forward_and_reverse_pass_agree(ops, O, F):
+    import torch
+    g = torch.Generator(device="cuda").manual_seed(O)
+    I, stride, small = 6 * O, ops.fp32_stride(F), 4096
+    x, dy = torch.rand((I, stride), device="cuda", generator=g) * 1.2 - 0.1, torch.randn((O, stride), device="cuda", generator=g)
+    idx = torch.randperm(I, device="cuda", generator=g).to(torch.int32).reshape(O, 6)
+    W = torch.rand((O, 64), device="cuda", generator=g) * 0.8 + 0.1                      # inside the band that the batch norm's clipping passes
+    dW = [torch.zeros((O, 64), device="cuda") for _ in range(3)]
+    plain = ops.stochastic_lut6_backward(x, dy, idx, W, dW[0], I, F)
+    bn = ops.dl6_backward_apply(x, dy, torch.empty_like(x), idx, W, dW[1], torch.zeros(O, device="cuda"), torch.ones(O, device="cuda"),
+                                torch.zeros((O, 2), dtype=torch.float64, device="cuda"), I, F, F, gamma=1.0, beta=0.0, binary=False)
+    one = ops.stochastic_lut6_backward(x[:, :small].contiguous(), dy[:, :small].contiguous(), idx, W, dW[2], I, small)
+    assert plain[:, :F].any() and torch.equal(plain[:, :F], bn[:, :F]) and torch.equal(plain[:, :small], one)
+    # sums of the same products in another order: F roundings of the sum of their magnitudes, which is no more than that of |dy|, each to 2^-24
+    bound = F * 2.0**-24 * dy[:, :F].abs().sum(1, keepdim=True)
+    assert ((dW[0] - dW[1]).abs() <= bound).all()
+
+
 # one CTA (up to 2^14 target values) and the general form; Adam with the gradients cleared on the way, whole quads and a remainder
 @pytest.mark.parametrize("classes,frames", [(1, 1), (10, 129), (10, 3276), (10, 3277), (3, 20000)])
 def test_mean_loss_and_adam_update(ops, classes, frames):
