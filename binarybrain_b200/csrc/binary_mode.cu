@@ -277,7 +277,7 @@ struct BitBwdArgs {
     const int *heavy_count;
     int heavy_from, heavy_chunk, heavy_ctas;
     int I, O, F, groups, tile_frames, tiles, nc, split;
-    int vec, xvec;                      // dy and dx (and fp32 x) rows start on 16-byte boundaries; bit-packed x rows do
+    int vec;                            // dy and dx (and fp32 x) rows start on 16-byte boundaries
     long long xs, fs, ps;               // word stride of x, float stride of dy / dx, stride of pat
 };
 
@@ -375,8 +375,9 @@ __device__ __forceinline__ void pattern_columns_reduce(const PatternSlot<BN> *sl
     }
 }
 
-// XF32 (the statistics half of a sharded backward, always batch-normalised): the patterns come from fp32 rows.
-template <bool XF32, bool BN>
+// XF32 (the statistics half of a sharded backward, always batch-normalised): the patterns come from fp32 rows.  XVEC: bit rows start on 16-byte
+// boundaries (as a question to the arguments it cost those rows 2 %).
+template <bool XF32, bool BN, bool XVEC>
 __global__ void __launch_bounds__(kPsWarps * 32)
 k_pattern_sums(const BitBwdArgs a)
 {
@@ -417,7 +418,7 @@ k_pattern_sums(const BitBwdArgs a)
 #pragma unroll
                 for (int j = 0; j < 6; ++j) {
                     const uint32_t *x = rows[j] + ((fl + k * kStep) >> 5);
-                    b.w[j] = a.xvec ? __ldg(reinterpret_cast<const uint4 *>(x)) : make_uint4(__ldg(x), __ldg(x + 1), __ldg(x + 2), __ldg(x + 3));
+                    b.w[j] = XVEC ? __ldg(reinterpret_cast<const uint4 *>(x)) : make_uint4(__ldg(x), __ldg(x + 1), __ldg(x + 2), __ldg(x + 3));
                 }
 #pragma unroll
                 for (int c = 0; c < NC; ++c) b.dy[c] = __ldg(reinterpret_cast<const float4 *>(dyrow + fl + k * kStep + 32 * c));
@@ -1550,8 +1551,8 @@ template <bool XF32>
 int launch_pattern_sums(BitBwdArgs a, bool bn, cudaStream_t st)
 {
     a.groups = (a.O + kPsWarps - 1) / kPsWarps;
-    a.xvec = (reinterpret_cast<uintptr_t>(a.x) & 15) == 0 && a.xs % 4 == 0;
-    if (XF32) a.vec = a.vec && (reinterpret_cast<uintptr_t>(a.x) & 15) == 0 && a.xs % 4 == 0;
+    const bool xvec = (reinterpret_cast<uintptr_t>(a.x) & 15) == 0 && a.xs % 4 == 0;
+    if (XF32) a.vec = a.vec && xvec;
     long long tile = ((long long)a.F + 127) / 128 * 128;
     while (tile > 1024 && (long long)a.O * ((a.F + tile - 1) / tile) < 24LL * device_info().sm_count) tile = (tile / 2 + 127) / 128 * 128;
     a.tile_frames = (int)tile;
@@ -1563,8 +1564,11 @@ int launch_pattern_sums(BitBwdArgs a, bool bn, cudaStream_t st)
         if (bn) BB200_CUDA(cudaMemsetAsync(a.hist, 0, (size_t)a.O * 256, st));
     }
     const int smem = kPsWarps * 64 * 32 * (int)(bn ? sizeof(PatternSlot<true>) : sizeof(PatternSlot<false>));
-    void (*kern)(BitBwdArgs) = k_pattern_sums<XF32, true>;
-    if constexpr (!XF32) { if (!bn) kern = k_pattern_sums<false, false>; }
+    void (*kern)(BitBwdArgs) = k_pattern_sums<XF32, true, true>;
+    if constexpr (!XF32) {
+        if (!bn) kern = xvec ? k_pattern_sums<false, false, true> : k_pattern_sums<false, false, false>;
+        else if (!xvec) kern = k_pattern_sums<false, true, false>;
+    }
     BB200_REQUIRE(allow_big_smem(kern, smem), BBCU_ERR_NO_MEMORY);
     launch(kern, (unsigned)blocks, kPsWarps * 32, smem, st, a);
     return launch_status();
