@@ -49,8 +49,9 @@ FLOPS_FWD, FLOPS_BWD = 126.0, 505.0
 # what the centred-polynomial kernels issue instead (a packed FMA is four): 63 FMA forward; backward 31 packed FMA and one scalar in the
 # forward halves, 47 packed FMA, 27 packed products and sums and 7 scalar operations in the reverse pass; 12 for conditioning the inputs
 FLOPS_FWD_EXECUTED, FLOPS_BWD_EXECUTED = 126.0 + 12.0, 4.0 * (31 + 47) + 2.0 * (1 + 27) + 7.0 + 12.0
-# dram__bytes_read.sum + dram__bytes_write.sum of one k_binary_lut6_pipe launch: ncu on a 131072-frame launch; traffic grows with frames
-NCU_BL6_TRAFFIC_BYTES_PER_FRAME = (457.5e6 + 244.4e6) / 131072
+# dram__bytes_read.sum + dram__bytes_write.sum of one k_binary_lut6_imm launch: ncu on a 131072-frame launch of the same layer, which walks the same
+# tiles of 32768 frames, a tile of a node at a time; traffic grows with frames
+NCU_BL6_TRAFFIC_BYTES_PER_FRAME = (469.27e6 + 245.19e6) / 131072
 # the same for one k_lut6_backward_pipe<BN> launch on a 65536 -> 65536 x 4096-frame layer: 12.325 GB read + 5.616 GB written for 2.68e8
 # node-frames.  backward_pipe_tile() gives this layer 1408-frame tiles at 4096, 8192, 16384 and 32768 frames alike, so the traffic grows in
 # proportion to the frames of a launch
@@ -389,13 +390,8 @@ def binary_lut6_section(torch, ops, dist, world, rank, steps, warmup, frames, ex
                        "inputs exceed L2, no flush)", "metric": "BinaryLut6 forward node-frames/s", "value": world * BL6_NODES * frames / sec,
            "unit": "node-frames/s", "ms_per_step": sec * 1e3, "steps": steps, "scaling": "weak", "dtype": "u32 bit-packed", "gpu_launches": steps,
            "roofline": {"bound": "hbm", "achieved": achieved, "peak": hbm, "unit": "GB/s", "frac": achieved / hbm,
-                        "traffic": NCU_BL6_TRAFFIC_BYTES_PER_FRAME * frames, "peak_source": f"of {which}", "kernel": "k_binary_lut6_pipe",
+                        "traffic": NCU_BL6_TRAFFIC_BYTES_PER_FRAME * frames, "peak_source": f"of {which}", "kernel": "k_binary_lut6_imm",
                         "algorithmic_bytes_per_launch": algo_bytes}}
-    if extras and rank == 0:
-        # the same launch through the truth-table-immediate kernel (15 logic operations per word instead of 63, one indexed branch per
-        # table byte): kept measurable because it is the formulation with the fewest operations and still the slower one
-        sec_imm = time_op(torch, lambda: ops.binary_lut6_forward(x, idx, table, frames, y=y, lop3_immediate=True), max(2, min(steps, 5)))
-        out["lop3_immediate_variant"] = {"ms_per_step": sec_imm * 1e3, "frac": algo_bytes / sec_imm / 1e9 / hbm, "kernel": "k_binary_lut6_imm"}
     if extras and world == 1:
         # end to end through the operator with host buffers: H2D of x, kernel, D2H of y, every step (chunk-pipelined inside the call)
         hx = torch.empty(x.shape, dtype=torch.int32).pin_memory()
