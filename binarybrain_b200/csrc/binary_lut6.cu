@@ -1,14 +1,15 @@
 // BinaryLut6: bit-packed 6-input LUT inference forward.
 //
 // Semantics of BinaryBrain include/bb/BinaryLutN.h:436-463: for every frame the six input bits form an
-// index (input k -> bit k) into the node's 64-entry truth table.  Frames are processed 32 per word
-// as a multiplexer tree over whole words: 32 two-way selects on x0 between table constants, then
-// 16/8/4/2/1 selects on x1..x5 -- 63 three-input logic ops (LOP3) per 32 frames, against the 448 of
-// the reference kernel's 64 masked AND chains (cuda/BinaryLut6.cu:82-160).
+// index (input k -> bit k) into the node's 64-entry truth table.  Frames are processed 32 per word, by logic on whole words, against the
+// 448 operations a word of the reference kernel's 64 masked AND chains (cuda/BinaryLut6.cu:82-160).
 //
-// Mapping: one warp per output node, one 128-bit load per lane and input row, so a warp reads 512
-// contiguous bytes of each of its six rows per iteration; CTAs of consecutive node groups share a
-// word tile so the tile's input rows stay in L2 for the ~6 nodes that read each of them.
+// Four ways, chosen in bbcu_bit_BinaryLut6_Forward, where the rules and both sides of each stand:
+//   k_binary_lut6_imm    15 operations a word with the table bytes as lop3 immediates: layers of several rounds of its grid
+//   k_binary_lut6_pipe   a multiplexer tree, 63 operations a word, fed by bulk copies: the other layers with rows on 16-byte boundaries
+//   k_binary_lut6_words  the tree, a word of a node per thread: the smallest calls
+//   k_binary_lut6        the tree, rows that start anywhere (k_binary_lut6_2pipe: 16-byte boundaries where the others cannot be set up)
+// All but the words keep the nodes of one tile of words in flight together, so that the tile's input rows stay in L2 for their readers.
 
 #include <type_traits>
 
@@ -83,7 +84,7 @@ k_binary_lut6(const BlArgs a)
 }
 
 // ---------------------------------------------------------------------------------------------
-// Two-pipe variant (the one the launcher uses for aligned rows).
+// Two-pipe variant (aligned rows where the persistent kernels below cannot be set up; its tree is theirs).
 //   * Level 1 of the tree only ever produces one of {0, x0, ~x0, ~0}.  In two's complement that is
 //     x0 * a + b with (a, b) in {(0,0), (1,0), (-1,-1), (0,-1)}: an integer multiply-add, which issues to the
 //     FMA pipe and leaves the 31 selects of levels 2..6 to the INT/logic pipe, so the two pipes split the
@@ -186,7 +187,7 @@ struct MuxTree<1, K, NW> {
 };
 
 // ---------------------------------------------------------------------------------------------
-// Persistent, bulk-copy-pipelined variant (aligned rows; the launcher's default).
+// Persistent, bulk-copy-pipelined variant (aligned rows; layers of few rounds, or whose rows fill the tiles of k_binary_lut6_imm badly).
 // Work item = (word tile of 256 words, node) of one warp; the warps of the grid take the items in order, so that those in
 // flight sweep the nodes of one tile together and the tile's rows stay in L2.  (Items of a CTA and eight nodes left warps
 // idle where the nodes are no multiple of 8: 36 nodes x 2^20 frames 8.9 -> 8.1 us.)  Each warp runs its own two-stage
@@ -370,9 +371,10 @@ k_binary_lut6_words(const BlArgs a)
 // its own node 169, two sharing one 112, four 65, seven (all of a scheduler) 56, all 28 46, and four with two segments each 57; the
 // multiplexer tree of k_binary_lut6_pipe takes 106 whatever is shared.
 // The bodies write one set of registers, which costs four moves a word: with a second set of bodies for the odd bytes, 80 KiB of code in all,
-// fetching them bounds the kernel again (1000 nodes x 2^20 frames 130 us instead of 92).  16384 x 2^20: 1951 -> 1483 us, 5000 x 2^20 609 -> 414,
-// 216 x 2^20 30.3 -> 22.7; 46 instructions and 93 clocks per word and scheduler (of 127), issue 0.5, the rest latency of branches, fetches and
-// shared memory at 20 warps per SM (24 do not leave it the registers: 110 us instead of 92).
+// fetching them bounds the kernel again (1000 nodes x 2^20 frames 130 us instead of 92).  16384 x 2^20: 1951 -> 1483 us at the full clock, 5000 x 2^20
+// 609 -> 414, 216 x 2^20 30.3 -> 22.7.  Under ncu (16384 nodes x 131072 frames, caches cold) 205 us against 272 of the tree: 47 instructions and 105
+// clocks per word and scheduler, 45 % of the issue slots, no unit above 52 %: latency at 20 warps per SM, of shared memory and copies, of the branches
+// and of the fetches (24 warps do not leave it the registers: 110 us instead of 92).
 // %0-%7 x0 and the result, %8-%15 x1, %16-%23 x2, %24 / %25 the table words, %26 the lane's first piece of x3 in shared memory; x3, x4 and x5 are
 // read there when they are needed (24 registers fewer).
 // ---------------------------------------------------------------------------------------------

@@ -788,7 +788,7 @@ k_lut6_backward(const BwdArgs a)
 // of the group.  What the kernel is bound by: an SM sub-partition issues one instruction per clock and a packed f32x2
 // instruction takes two issue slots (measured: 32 packed FMAs take 65 clocks per warp, and scalar FMAs, logic ops or anything
 // else issued beside them add their own clocks in full), so the time is the weighted instruction count -- 105 packed (210
-// slots) + 109 others per frame with batch norm -- over the issue rate.  Everything here is about the "others":
+// slots) + 111 others per frame with batch norm, in 404 clocks of a scheduler -- over the issue rate.  Everything here is about the "others":
 //   * the per-node table arrives ready to use (k_backward_prepare has converted every table once per launch);
 //   * global -> shared: a warp streams its item in 128-frame chunks through a three-stage ring; every lane copies 16 bytes (four
 //     consecutive frames) of each of the six input rows and of dy with cp.async, two chunks ahead of the arithmetic, so the
@@ -1130,8 +1130,8 @@ static int launch_forward(FwdArgs a, int max_tile, cudaStream_t st)
                              (a.xs % 4) == 0 && (a.ys % 4) == 0;
         auto kern = a.binary ? k_lut6_forward_pipe<PHASE, true> : k_lut6_forward_pipe<PHASE, false>;
         if (aligned && allow_big_smem(kern, kFpSmem)) {
-            // 256-frame items whenever there are that many frames: four frame pairs per lane share every table read and the
-            // per-item costs halve.  Measured on B200: 65536 -> 65536 nodes x 4096 frames 1.89 ms (128) vs 1.49 ms (256), although
+            // 256-frame items whenever there are that many frames: the per-item costs halve.  Measured on B200 with the version before, in
+            // which all frames of an item shared every table read: 65536 -> 65536 nodes x 4096 frames 1.89 ms (128) vs 1.49 ms (256), although
             // the 256-frame tile of such a layer (64 MiB of gathered rows) no longer fits a fifth of L2.
             a.T = a.F > kFramesPerIter ? kFpMaxItemFrames : kFramesPerIter;
             const long long n_items = (long long)((a.F + a.T - 1) / a.T) * a.groups;
