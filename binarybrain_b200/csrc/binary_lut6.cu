@@ -26,7 +26,6 @@ struct BlArgs {
     const int *idx;
     const int *table;
     int O, nwords, Tw, groups;
-    int run_rows;                       // k_binary_lut6_imm: input rows of which Tw tiles stay in L2
     long long stride;
 };
 
@@ -477,9 +476,9 @@ __device__ __forceinline__ void lut6_words_by_immediates(uint32_t (&x)[3][8], ui
 // beyond three few rows have a second reader.  In us by k_binary_lut6_pipe / with one tile / with two, cool: 8192 nodes x 2^20 frames reading 8192 rows
 // 982 / 733 / 671, 16384 rows 984 / 759 / 791, 24576 983 / 775 / 944, 49152 1008 / 883 / 1126; 4000 x 2^20 reading 8000 rows 530 / 365 / 335, 12000
 // 501 / 371 / 359, 24000 497 / 412 / 486; 2000 x 2^21 reading 12000 497 / 401 / 430; 13000 x 2^18 reading 3900 423 / 322 / 282, 39000 412 / 327 / 401.
-__device__ __forceinline__ bool imm_two_tiles(const BlArgs &a, int lane)
+__device__ __forceinline__ bool imm_two_tiles(const BlArgs &a, int run_rows, int lane)
 {
-    constexpr int kLook = 8;
+    constexpr int kLook = 2;
     const long long entries = 6LL * a.O;
     unsigned lo = ~0u, hi = 0u;
 #pragma unroll
@@ -489,14 +488,16 @@ __device__ __forceinline__ bool imm_two_tiles(const BlArgs &a, int lane)
         hi = max(hi, row);
     }
     const long long rows = (long long)__reduce_max_sync(0xffffffffu, hi) - __reduce_min_sync(0xffffffffu, lo);
-    return rows <= 2LL * a.O || (rows <= a.run_rows && rows <= 3LL * a.O);
+    return rows <= 2LL * a.O || (rows <= run_rows && rows <= 3LL * a.O);
 }
 
 // Persistent: a group of four warps takes (tile of 1024 words, node) items in tile-major order, each warp a segment of 256 words.  x0..x2 go to
 // registers at the start of an item, and the copies of the next item's follow at once; x3..x5 are used from shared memory, in two buffers.
 // Every lane copies, with cp.async, the 16-byte pieces that it will itself read: no barrier and no cross-lane dependence.
+// TWO: a node's run may be two tiles, up to run_rows input rows (of which two tiles stay in L2).
+template <bool TWO>
 __global__ void __launch_bounds__(kImmWarps * 32, 1)
-k_binary_lut6_imm(const BlArgs a)
+k_binary_lut6_imm(const BlArgs a, int run_rows)
 {
     grid_dependency();
     extern __shared__ __align__(128) unsigned char smem_raw[];
@@ -508,7 +509,11 @@ k_binary_lut6_imm(const BlArgs a)
     const int whole = (a.nwords + kImmTile - kPipeWords - segment) / kImmTile;               // those in which it has all 256
     const int step = (int)gridDim.x * kGroups, first = (int)blockIdx.x * kGroups + warp / kImmGroup;
     // A node's run is one or two tiles; the runs of a group are `first`, first + step, ...
-    const int run = a.Tw == 2 && imm_two_tiles(a, lane) ? 2 : 1;
+    PipePos p0;
+    p0.tile = first / a.O;
+    p0.node = first - p0.tile * a.O;
+    const int row0 = pipe_row(a, p0.node, lane);          // on its way while the wiring is looked at; a node's run does not move it
+    const int run = TWO && imm_two_tiles(a, run_rows, lane) ? 2 : 1;
     const int dt = step / a.O, dn = step - dt * a.O, last = run - 1;
     auto advance = [&](PipePos p) {
         if ((p.tile & last) != last && p.tile + 1 < tiles) {
@@ -520,9 +525,6 @@ k_binary_lut6_imm(const BlArgs a)
         if (p.node >= a.O) { p.node -= a.O; p.tile += run; }
         return p;
     };
-    PipePos p0;
-    p0.tile = first / a.O;
-    p0.node = first - p0.tile * a.O;
     p0.tile *= run;
     // three rows, from input `J` on, of item p to `dst`; lane j of `row` holds the item's input row j
     const uint32_t row_bytes = (uint32_t)a.stride * 4u;
@@ -552,7 +554,6 @@ k_binary_lut6_imm(const BlArgs a)
     int row1 = 0, row2 = 0;                              // input rows of items k + 1 and k + 2 (lanes 0..5)
     uint2 table = make_uint2(0u, 0u);
     {
-        const int row0 = p0.tile < tiles ? pipe_row(a, p0.node, lane) : 0;
         if (p1.tile < tiles) row1 = pipe_row(a, p1.node, lane);
         issue(p0, row0, Hi{}, upper);
         issue(p0, row0, Lo{}, lower);
@@ -606,16 +607,17 @@ int imm_run(const BlArgs &a) { return imm_rounds(a) >= 8 && a.O <= imm_run_rows(
 // What the kernel's 32-bit arithmetic can take.
 bool imm_fits(const BlArgs &a)
 {
-    return a.stride < (1 << 30) && ((long long)a.nwords / kImmTile + 2) * a.O < (1LL << 31) - 65536 && allow_big_smem(k_binary_lut6_imm, kImmSmem);
+    return a.stride < (1 << 30) && ((long long)a.nwords / kImmTile + 2) * a.O < (1LL << 31) - 65536 && allow_big_smem(k_binary_lut6_imm<true>, kImmSmem) &&
+           allow_big_smem(k_binary_lut6_imm<false>, kImmSmem);
 }
 
 int launch_immediate(BlArgs a, cudaStream_t st)
 {
     a.Tw = imm_run(a);
-    a.run_rows = imm_run_rows();
     const long long tiles = (a.nwords + kImmTile - 1) / kImmTile, runs = (tiles + a.Tw - 1) / a.Tw * a.O, groups = kImmWarps / kImmGroup;
     const long long grid = (runs + groups - 1) / groups;
-    launch(k_binary_lut6_imm, (unsigned)(grid < device_info().sm_count ? grid : device_info().sm_count), kImmWarps * 32, kImmSmem, st, a);
+    launch(a.Tw == 2 ? k_binary_lut6_imm<true> : k_binary_lut6_imm<false>, (unsigned)(grid < device_info().sm_count ? grid : device_info().sm_count),
+           kImmWarps * 32, kImmSmem, st, a, imm_run_rows());
     return launch_status();
 }
 
