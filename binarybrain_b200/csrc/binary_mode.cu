@@ -544,7 +544,8 @@ __device__ __forceinline__ uint32_t prmt(uint32_t v)
 // loads, 27 warps per SM): two shuffles, 5 bytes and 16 instructions per consumer and frame.  With batch norm g is put together here;
 // writing g out once and reading it back would spare a shuffle and six instructions, but costs 10 bytes per node-frame of HBM traffic.
 // Several rows one after the other in a CTA keep more tiles in flight than L2 holds (8 rows: 509 -> 617 us for 16384 frames).
-template <bool BN, int NC, bool WHOLE>
+// SHORT: a row's last tile, of which the last chunks have no frames and are left out.
+template <bool BN, int NC, bool WHOLE, bool SHORT>
 __device__ __forceinline__ void pattern_gather(const BitBwdArgs &a, const int *list, int n, int part, int f0, int lane, float (&acc)[NC][4])
 {
     int e_n = part < n ? __ldg(list + part) : 0;
@@ -574,7 +575,7 @@ __device__ __forceinline__ void pattern_gather(const BitBwdArgs &a, const int *l
         }
 #pragma unroll
         for (int c = 0; c < NC; ++c) {
-            if (!WHOLE && f0 - 4 * lane + 128 * c >= a.F) break;           // no frame of the chunk exists
+            if (SHORT && f0 - 4 * lane + 128 * c >= a.F) break;
             const float dyv[4] = {dyq[c].x, dyq[c].y, dyq[c].z, dyq[c].w};
             const uint32_t rot = ((q4[c] >> (j + 1)) & low) | ((q4[c] << (5 - j)) & ~low);        // (bits 6 and 7 of the bytes: anything)
 #pragma unroll
@@ -606,8 +607,12 @@ __device__ __forceinline__ void gather_tile(const BitBwdArgs &a, int row, const 
     for (int c = 0; c < NC; ++c)
 #pragma unroll
         for (int i = 0; i < 4; ++i) acc[c][i] = 0.0f;
-    if (a.vec && f_begin + 128 * NC <= a.F) pattern_gather<BN, NC, true>(a, list, n, part, f0, lane, acc);
-    else if (f_begin < a.F)                 pattern_gather<BN, NC, false>(a, list, n, part, f0, lane, acc);
+    // A last tile most of whose chunks have frames has a form of its own without batch norm, where asking for each costs more than it saves (500 rows, 20000
+    // nodes, 1000 frames 212.5 -> 210.3 us for the operator; 92 frames in the last tile, 3000 rows and nodes: 91.9 without asking, 90.4 with).  With batch norm
+    // that form costs the others 1 % (8192 rows and nodes, 16384 frames 793 -> 801): SHORT = BN, so that none is built there.
+    if (a.vec && f_begin + 128 * NC <= a.F)       pattern_gather<BN, NC, true, false>(a, list, n, part, f0, lane, acc);
+    else if (!BN && f_begin + 64 * NC < a.F)      pattern_gather<BN, NC, false, BN>(a, list, n, part, f0, lane, acc);
+    else if (f_begin < a.F)                       pattern_gather<BN, NC, false, true>(a, list, n, part, f0, lane, acc);
     if (a.split > 1) {
         if (ADD) __syncthreads();                                       // (the tile before has been read)
 #pragma unroll

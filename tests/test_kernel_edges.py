@@ -160,6 +160,12 @@ def test_large_two_valued_layers_edges(ops, I, O, F, stride):
     test_two_valued_layers_edges(ops, I, O, F, stride)
 
 
+# the gather's last tile of 512 and of 256 frames: half of its chunks have frames, one frame more, and all but one frame
+@pytest.mark.parametrize("I,O,F,stride", [(300, 60, 4352, None), (300, 60, 4353, None), (300, 60, 4607, None), (200, 60, 4224, None), (200, 60, 4225, None)])
+def test_last_tile_of_the_gather(ops, I, O, F, stride):
+    test_two_valued_layers_edges(ops, I, O, F, stride)
+
+
 # bit rows that start anywhere beside gradients on 16-byte boundaries, above the one-launch range: whole steps of 512 frames, a remainder and one frame more
 @pytest.mark.parametrize("I,O,F", [(30, 600, 4608), (50, 700, 5121), (9, 40, 60001)])
 def test_bit_rows_that_start_anywhere(ops, I, O, F):
