@@ -51,7 +51,7 @@ FLOPS_FWD, FLOPS_BWD = 126.0, 505.0
 FLOPS_FWD_EXECUTED, FLOPS_BWD_EXECUTED = 126.0 + 12.0, 4.0 * (31 + 47) + 2.0 * (1 + 27) + 7.0 + 12.0
 # dram__bytes_read.sum + dram__bytes_write.sum of one k_binary_lut6_imm launch: ncu on a 131072-frame launch of the same layer, which walks the same
 # tiles of 32768 frames, a tile of a node at a time; traffic grows with frames
-NCU_BL6_TRAFFIC_BYTES_PER_FRAME = (469.27e6 + 245.19e6) / 131072
+NCU_BL6_TRAFFIC_BYTES_PER_FRAME = (467.27e6 + 243.48e6) / 131072
 # the same for one k_lut6_backward_pipe<BN> launch on a 65536 -> 65536 x 4096-frame layer: 12.325 GB read + 5.616 GB written for 2.68e8
 # node-frames.  backward_pipe_tile() gives this layer 1408-frame tiles at 4096, 8192, 16384 and 32768 frames alike, so the traffic grows in
 # proportion to the frames of a launch

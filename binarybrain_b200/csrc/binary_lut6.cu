@@ -371,8 +371,8 @@ k_binary_lut6_words(const BlArgs a)
 // multiplexer tree of k_binary_lut6_pipe takes 106 whatever is shared.
 // The bodies write one set of registers, which costs four moves a word: with a second set of bodies for the odd bytes, 80 KiB of code in all,
 // fetching them bounds the kernel again (1000 nodes x 2^20 frames 130 us instead of 92).  16384 x 2^20: 1951 -> 1483 us at the full clock, 5000 x 2^20
-// 609 -> 414, 216 x 2^20 30.3 -> 22.7.  Under ncu (16384 nodes x 131072 frames, caches cold) 205 us against 272 of the tree: 47 instructions and 105
-// clocks per word and scheduler, 45 % of the issue slots, no unit above 52 %: latency at 20 warps per SM, of shared memory and copies, of the branches
+// 609 -> 414, 216 x 2^20 30.3 -> 22.7.  Under ncu (16384 nodes x 131072 frames, caches cold) 204 us against 272 of the tree: 46 instructions and 104
+// clocks per word and scheduler, 45 % of the issue slots, no unit above 54 %: latency at 20 warps per SM, of shared memory and copies, of the branches
 // and of the fetches (24 warps do not leave it the registers: 110 us instead of 92).
 // %0-%7 x0 and the result, %8-%15 x1, %16-%23 x2, %24 / %25 the table words, %26 the lane's first piece of x3 in shared memory; x3, x4 and x5 are
 // read there when they are needed (24 registers fewer).
@@ -471,7 +471,9 @@ __device__ __forceinline__ void lut6_words_by_immediates(uint32_t (&x)[3][8], ui
 #undef BB200_LOAD5
 
 // Whether a node's run is two tiles by the input rows, whose number is not among the operator's arguments: it is the range of the wiring's entries, of
-// which every warp reads the same 256 (not a microsecond of calls of 70 and more).  Rows of two tiles that do not stay in L2 come from HBM once more for every
+// which every warp reads the same 64 while the rows of its first item are on their way (256 of them, before anything else, made 1000 nodes x 300000 frames
+// 30.2 -> 30.6 us, and asking every call 216 x 262144, which is too short for two tiles, 9.0 -> 9.2; now 30.5 in a run where not asking takes 30.5,
+// and 8.8).  Rows of two tiles that do not stay in L2 come from HBM once more for every
 // reader.  Two to three rows a node are for two tiles where they do stay; up to two are either way within 5 %, sustained for two, cool for one; and
 // beyond three few rows have a second reader.  In us by k_binary_lut6_pipe / with one tile / with two, cool: 8192 nodes x 2^20 frames reading 8192 rows
 // 982 / 733 / 671, 16384 rows 984 / 759 / 791, 24576 983 / 775 / 944, 49152 1008 / 883 / 1126; 4000 x 2^20 reading 8000 rows 530 / 365 / 335, 12000
